@@ -100,6 +100,9 @@ def draw(rng):
         learned = form == "fp32" and rng.random() < 0.5
         case.update(flow=rng.choice(["shear", "turbulent"]), drops=between(1, most), steps=rng.choice([1, 3, 20]),
                     learned=learned)
+        h = spacing(case)
+        while learned and case["nz"] * h / case["nz"] != h:  # the network wants the same spacing to the last bit
+            case["nz"] += 1
     elif kind == "projection":
         case.update(walls_y=rng.random() < 0.4)
         if case["walls_y"]:
