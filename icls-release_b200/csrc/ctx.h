@@ -36,7 +36,8 @@ struct LsTask {
   double bg, bgg;        // far-field values of the apron: rows 0..k1 / ghost rows
   const double* phi0;    // RK base (read at the thread's own cell only)
   const double* phis;    // stage input (stencil reads)
-  const double* orig;    // reinitialisation: sgn source
+  const double* orig;    // reinitialisation: sgn source; mass correction: the drop's curvature (shape C)
+  double* aux;           // mass correction: |grad phi| (shape I) of the curvature sweep, then H (shape C); else null
   double* out;
   uint8_t* mask;         // the drop's band mask (tube writes, advection reads)
   Region vin;            // tube: phi0 holds valid data on vin's written cells,
@@ -55,6 +56,12 @@ struct ReinitState {
   double last;      // residual of the last completed iteration
   int done;         // residual < dz**5 reached
   int iters;
+};
+
+// per-drop state of a mass correction (levelset.f90:407-582)
+struct InflateState {
+  double temp;      // the correction's normal speed (levelset.f90:514)
+  double gain;      // blend factor of the gain-one correction
 };
 
 // Sweep state of one drop's level set.  Outside valid's written cells every
@@ -101,13 +108,11 @@ struct Ctx {
   double *px = nullptr, *py = nullptr, *pz = nullptr, *pxold = nullptr, *pyold = nullptr, *pzold = nullptr;
   double *pjump = nullptr, *miu = nullptr, *rho = nullptr, *jiemian = nullptr;
   double *curv = nullptr;      // curv_cmn: re_curvature of the last drop (get_curvature in TwoD)
-  double *dheav = nullptr, *kappa = nullptr;
   // shape I
   double *duold[2] = {nullptr, nullptr}, *dvold[2] = {nullptr, nullptr}, *dwold[2] = {nullptr, nullptr};
   int hist = 0;  // which duold buffer holds the current history
   double *rho_u = nullptr, *rho_v = nullptr, *rho_w = nullptr;
   double *ucc = nullptr, *vcc = nullptr, *wcc = nullptr, *nrm_m = nullptr;
-  double *ulc = nullptr, *vlc = nullptr, *wlc = nullptr;
   // level sets (shape L): one buffer per drop
   std::vector<double*> lv;
   // working buffers of the drops of one group (drop l uses member l % G):
@@ -149,7 +154,8 @@ struct Ctx {
   double* dmaxchk = nullptr;            // per drop maxchk of the last inflation
   ReinitState* drs = nullptr;           // per drop
   double* stage = nullptr;              // precision form: FP64 staging of one field (upload/download)
-  double* hpart = nullptr;              // per-tile exact sums of H (XSum), red_cap per drop
+  double* hpart = nullptr;              // per (tile, chunk): exact sums of H (XSum), hcap per drop, then area sums
+  InflateState* dinf = nullptr;         // per drop
   int red_cap = 0;                      // column tiles of a whole x-y plane
   int hcap = 0;                         // Heaviside partials per drop: red_cap x the z chunks of shape C
   // pinned host mirrors
@@ -208,16 +214,15 @@ void launch_reinit_check(Ctx& c, const LsBatch& b, int it, int maxiter, double t
 void launch_heaviside(Ctx& c, const LsBatch& b);
 void launch_fill(Ctx& c, double* a, long long n, double v, bool tfield);
 void launch_materials_final(Ctx& c, const double* outside, const int* ntiles);
-void launch_inflate_sums(Ctx& c, const LsBatch& b, double outside);
-void launch_inflate_vel(Ctx& c, const LsBatch& b);
-void launch_region_copy(Ctx& c, const LsBatch& b);
-void launch_gain(Ctx& c, const LsBatch& b, double outside);
+// mass correction of the tasks' drops; LsTask::far holds the interior cells outside a drop's region
+void launch_inflate_sums(Ctx& c, const LsBatch& b);
+void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt);
+void launch_gain(Ctx& c, const LsBatch& b);
 void launch_region_blend(Ctx& c, const LsBatch& b);
 void launch_band_list(Ctx& c, const LsBatch& b);
 void launch_adv_split(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                       const double* vu, const double* vv, const double* vw, long long need);
-void launch_volume_now(Ctx& c, const LsBatch& b, double outside);
-void launch_copy(Ctx& c, double* dst, const double* src, long long n);
+void launch_volume_now(Ctx& c, const LsBatch& b);
 void launch_boundmls(Ctx& c, double* phi);
 void launch_materialize(Ctx& c, const Region& r, double bg, double bgg, double* phi);
 void launch_to_float(Ctx& c, double* dst_f32, const double* src, long long n);

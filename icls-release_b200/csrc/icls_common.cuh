@@ -331,10 +331,6 @@ struct DevScalars {
   double norm;            // main.f90:173-175
   double norm_old;        // main.f90:183
   double residual;        // levelset.f90:831
-  double area;            // levelset.f90:499-501
-  double heav_sum;        // levelset.f90:505
-  double inflate_temp;    // levelset.f90:514
-  double inflate_gain;    // blend factor of the last gain-one inflation
   double maxchk;          // levelset.f90:521
   double divtot, divmax;  // chkdiv.f90
   double umax, vmax, wmax;// chkdt.f90:42-44

@@ -100,7 +100,7 @@ __device__ __forceinline__ T curvature_at(const Params& p, const T* __restrict__
 }
 
 // get_curvature + boundc over the tasks' shape-C regions (phi0 = the
-// drop's level set, out = its curvature): wall rows stay 0, halos are the
+// drop's level set, out = its curvature, aux = its |grad phi| where set): wall rows stay 0, halos are the
 // periodic copies (bound.f90:292-305), the apron (far field, |phi| > 5dz)
 // is 0.
 template <typename T>
@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(NT, 4) k_curvature(Params p, const __grid_cons
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
   const T* phi = cT<T>(t.phi0);
   T* out = mT<T>(t.out);
+  T* aux = mT<T>(t.aux);
   const T lim = TC(4. * p.dz);
   const unsigned lane = threadIdx.x & 31u;
   // every lane of the warp walks the same rows, so the ballots line up
@@ -121,6 +122,7 @@ __global__ void __launch_bounds__(NT, 4) k_curvature(Params p, const __grid_cons
         T m;
         v = curvature_at(p, phi, c.i, c.j, k, m);
         if (nrm_m) nrm_m[idxI(p, c.i, c.j, k)] = m;
+        if (aux) aux[idxI(p, c.i, c.j, k)] = m;
       }
       putC(p, out, c.i, c.j, k, v);
     }

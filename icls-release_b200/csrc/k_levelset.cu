@@ -325,10 +325,83 @@ __device__ __forceinline__ T adv_rhs(const Params& p, const Axial19<T>& S, T vu,
 #undef PZ
   return (udfdx + vdfdy) + wdfdz;
 }
-template <int SCHEME, typename T, int PW>
+// u_lc, v_lc, w_lc of levelset.f90:527-548, with u_l,v_l,w_l of 530-532
+// after bounduvw evaluated on the fly
+template <typename T>
+__device__ __forceinline__ T infl_face(const Params& p, const T* __restrict__ dheav, T temp, int axis, int i, int j,
+                                       int k) {
+  const long long n = idxC(p, i, j, k);
+  if (axis == 0) return -divx(p, temp * (dheav[n + 1] - dheav[n]));
+  if (axis == 1) return -divy(p, temp * (dheav[n + p.nCx] - dheav[n]));
+  return -divz(p, temp * (dheav[n + (long long)p.nCx * p.nCy] - dheav[n]));
+}
+// v_l(i,0,k) and v_l(i,jmax,k) with the y walls of boundp(dheav) and
+// bounduvw(u_l,v_l,w_l) (levelset.f90:466-478, bound.f90:81-282) for
+// BC_in_y = Walls, InOut, OutOut: v_l = 0 on a wall, v_inflow at the inlet,
+// the OutOut extrapolation at y = 0, and dheav(i,j1,k) = -dheav(i,jmax,k) at
+// an outflow end
+template <typename T>
+__device__ __forceinline__ T infl_v_front(const Params& p, const T* __restrict__ dheav, T temp, int i, int k,
+                                          const double* __restrict__ vin) {
+  if (p.bcy == ICLS_BCY_WALLS) return TC(0.);
+  if (p.bcy == ICLS_BCY_INOUT) return TC(vin[i + (long long)(p.i1 + 1) * k]);
+  const T wl_1 = (k == p.kmax) ? TC(0.) : infl_face(p, dheav, temp, 2, i, 1, k);
+  const T wl_0 = (k == 1) ? TC(0.) : infl_face(p, dheav, temp, 2, i, 1, k - 1);
+  return infl_face(p, dheav, temp, 1, i, 1, k) + TC(p.dy / p.dz) * (wl_1 - wl_0);
+}
+template <typename T>
+__device__ __forceinline__ T infl_v_back(const Params& p, const T* __restrict__ dheav, T temp, int i, int k) {
+  if (p.bcy == ICLS_BCY_WALLS) return TC(0.);
+  const T h = dheav[idxC(p, i, p.jmax, k)];
+  return -divy(p, temp * (-h - h));
+}
+// (a, b, c) = u_lc, v_lc, w_lc at an interior cell; false where H is uniform
+// around it (the velocity is then +-0 and moves nothing)
+template <typename T>
+__device__ __forceinline__ bool infl_velocity(const Params& p, const T* __restrict__ dheav,
+                                              const T* __restrict__ kappa, T temp, int i, int j, int k,
+                                              const double* __restrict__ vin, T& a, T& b, T& cc) {
+  const long long n = idxC(p, i, j, k), sy = p.nCx, sz = (long long)p.nCx * p.nCy;
+  const bool inner_y = p.bcy == ICLS_BCY_PERIODIC || (j != 1 && j != p.jmax);
+  const T h0 = dheav[n];
+  if (inner_y && isfinite(temp) && dheav[n + 1] == h0 && dheav[n - 1] == h0 && dheav[n + sy] == h0 &&
+      dheav[n - sy] == h0 && dheav[n + sz] == h0 && dheav[n - sz] == h0)
+    return false;
+  const T ul_m = infl_face(p, dheav, temp, 0, wrapx(p, i - 1), j, k);
+  const T ul_0 = infl_face(p, dheav, temp, 0, i, j, k);
+  T vl_m, vl_0;
+  if (inner_y) {
+    vl_m = infl_face(p, dheav, temp, 1, i, wrapy(p, j - 1), k);
+    vl_0 = infl_face(p, dheav, temp, 1, i, j, k);
+  } else {
+    vl_m = j == 1 ? infl_v_front(p, dheav, temp, i, k, vin) : infl_face(p, dheav, temp, 1, i, j - 1, k);
+    vl_0 = j == p.jmax ? infl_v_back(p, dheav, temp, i, k) : infl_face(p, dheav, temp, 1, i, j, k);
+  }
+  const T wl_m = (k == 1) ? TC(0.) : infl_face(p, dheav, temp, 2, i, j, k - 1);
+  const T wl_0 = (k == p.kmax) ? TC(0.) : infl_face(p, dheav, temp, 2, i, j, k);
+  a = (ul_m + ul_0) / TC(2.);
+  b = (vl_m + vl_0) / TC(2.);
+  cc = (wl_m + wl_0) / TC(2.);
+  if (p.ispeed_curv) {
+    const T kp = kappa[n];
+    a = a * kp;
+    b = b * kp;
+    cc = cc * kp;
+  }
+  return true;
+}
+
+// INFL: a stage of the mass correction.  The velocity is u_lc, v_lc, w_lc of
+// the inflation, formed at the cell (infl_velocity); where H is uniform
+// around the cell it is an exact zero and the value keeps its base without
+// the stencil (the correction moves only cells within 1.5dz of the
+// interface and their neighbours, a fifth of the band).
+template <int SCHEME, typename T, int PW, bool INFL>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Params p, const __grid_constant__ LsBatch B, int stage1,
                                                      double a_, double bb_, double fdt_, const T* __restrict__ vu,
-                                                     const T* __restrict__ vv, const T* __restrict__ vw) {
+                                                     const T* __restrict__ vv, const T* __restrict__ vw,
+                                                     const InflateState* __restrict__ inf,
+                                                     const double* __restrict__ vin) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -348,6 +421,8 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Para
   T* const o2 = jj != INT_MIN ? out + idxL(p, i, jj, 0) : nullptr;
   T* const o3 = (ii != INT_MIN && jj != INT_MIN) ? out + idxL(p, ii, jj, 0) : nullptr;
   const long long qc = idxI(p, i, j, 1);  // row k at qc + (k - 1) * szI
+  T temp = TC(0.);
+  if constexpr (INFL) temp = TC(inf[t.l].temp);
   auto put = [&](int k, T v) {
     const int o = k * sz;
     o0[o] = v;
@@ -379,9 +454,27 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Para
         val = stage1 ? f0 : a * f0 + bb * fsc[o];
       } else {
         const long long q = qc + (long long)(k - 1) * szI;
-        const uint8_t m = t.mask[q];
-        const T u = vu[q], v = vv[q], w = vw[q];
+        uint8_t m = t.mask[q];
         const T* f = fsc + o;
+        T u, v, w;
+        if constexpr (INFL) {
+          u = v = w = TC(0.);
+          if (m) m = infl_velocity(p, cT<T>(t.aux), cT<T>(t.orig), temp, i, j, k, vin, u, v, w) ? 1 : 0;
+          if (!m) {
+            val = stage1 ? f0 : a * f0 + bb * f[0];
+            if (k == 1) v1 = val;
+            if (k == 2) v2 = val;
+            if (k == p.kmax - 1) vkm = val;
+            if (k == p.kmax) vk = val;
+            put(k, val);
+            if (k == 2 && wall0) put(0, TC(2.) * v1 - v2);
+            continue;
+          }
+        } else {
+          u = vu[q];
+          v = vv[q];
+          w = vw[q];
+        }
         Axial19<T> S;
         S.c = f[0];
 #pragma unroll
@@ -967,22 +1060,35 @@ __global__ void __launch_bounds__(NT) k_materials_rows2(Params p, const T* __res
 }
 
 // ------------------------------------------------------------ inflation
-// dheav with boundp semantics over the task's shape-C region (one task),
-// the far-field value 1 on its apron, and per-tile area/volume sums (FP64)
-// over its interior computed cells (levelset.f90:493-507, 525)
+// a Heaviside value into an exact sum: the zeros add nothing and the ones
+// (most cells of a box) are counted, so only interface cells pay the limb
+// arithmetic
+template <typename T>
+__device__ __forceinline__ void heav_add(XSum& s, int& ones, T H) {
+  if (H == TC(1.)) ++ones;
+  else if (H != TC(0.)) xs_add(s, (double)H);
+}
+
+// dheav with boundp semantics over the tasks' shape-C regions (aux: the
+// drop's |grad phi|, orig: its curvature; out: dheav), the far-field value 1
+// on their aprons, and per-(tile, chunk) area and volume sums (FP64) over the
+// interior computed cells (levelset.f90:493-507, 525)
 template <typename T>
 __global__ void __launch_bounds__(NT) k_inflate_sums(Params p, const __grid_constant__ LsBatch B,
-                                                     const T* __restrict__ kappa, const T* __restrict__ nrm_m,
-                                                     T* __restrict__ dheav, double* __restrict__ part_area,
-                                                     XSum* __restrict__ part_heav) {
+                                                     double* __restrict__ part_area,
+                                                     XSum* __restrict__ part_heav, int cap) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
   const T s1 = TC(1.5 * p.dz);
   const T* phi = cT<T>(t.phi0);
+  const T* __restrict__ kappa = cT<T>(t.orig);
+  const T* __restrict__ nrm_m = cT<T>(t.aux);
+  T* dheav = mT<T>(t.out);
   double sa = 0.;
   XSum sh;
   xs_zero(sh);
+  int ones = 0;
   if (c.ok) {
     const int i = c.i, j = c.j;
     for (int k = c.ka; k <= c.kb; ++k) {
@@ -991,49 +1097,60 @@ __global__ void __launch_bounds__(NT) k_inflate_sums(Params p, const __grid_cons
         continue;
       }
       const int K = k == 0 ? 1 : (k == p.k1 ? p.kmax : k);
-      putC(p, dheav, i, j, k, heav_trig(p, phi[idxL(p, i, j, K)], s1));
+      const T ph = phi[idxL(p, i, j, K)];
+      const T H = heav_trig(p, ph, s1);
+      putC(p, dheav, i, j, k, H);
       if (k >= 1 && k <= p.kmax) {
-        const T ph = phi[idxL(p, i, j, k)];
-        const T H = heav_trig(p, ph, s1);
+        heav_add(sh, ones, H);
         const T del = dirac_trig(p, ph, s1);
-        const T m = nrm_m[idxI(p, i, j, k)];
-        sa += (double)(p.ispeed_curv ? (del * kappa[idxC(p, i, j, k)]) * m : del * m);
-        xs_add(sh, (double)H);
+        if (del != TC(0.)) {
+          const T m = nrm_m[idxI(p, i, j, k)];
+          sa += (double)(p.ispeed_curv ? (del * kappa[idxC(p, i, j, k)]) * m : del * m);
+        }
       }
     }
   }
+  xs_add_count(sh, ones);
   const double ba = block_sum<double, NT>(sa);
   const XSum bh = block_xsum<NT>(sh);
   if (flat_tid() == 0) {
-    part_area[c.tile] = ba;
-    part_heav[c.tile] = bh;
+    const long long at = (long long)t.l * cap + c.tile + (long long)t.tx * t.ty * c.ch;
+    part_area[at] = ba;
+    part_heav[at] = bh;
   }
 }
 
-__global__ void k_inflate_final(Params p, const double* __restrict__ part_area,
-                                const XSum* __restrict__ part_heav, int nblk, int l, double istep_dt,
-                                double outside, double* __restrict__ vol, const double* __restrict__ vol0,
-                                double* __restrict__ maxchk, DevScalars* __restrict__ dsc) {
-  if (threadIdx.x != 0) return;
-  double sa = 0.;
+// the partials of one task (block blockIdx.x), added in a fixed order: every
+// thread's strided share, then a fixed tree
+constexpr int kFinalThreads = 256;
+__device__ __forceinline__ XSum task_heav(const LsTask& t, const XSum* __restrict__ part, int cap) {
   XSum hs;
   xs_zero(hs);
-  for (int b = 0; b < nblk; ++b) {
-    sa += part_area[b];
-    xs_merge(hs, part_heav[b]);
-  }
-  xs_add_count(hs, (long long)outside);
-  const double sh = xs_value(hs);
+  const int n = t.tx * t.ty * t.nch;
+  for (int b = threadIdx.x; b < n; b += kFinalThreads) xs_merge(hs, part[(long long)t.l * cap + b]);
+  hs = block_xsum<kFinalThreads>(hs);
+  xs_add_count(hs, (long long)t.far);
+  return hs;
+}
+__global__ void __launch_bounds__(kFinalThreads)
+    k_inflate_final(Params p, const __grid_constant__ LsBatch B, const double* __restrict__ part_area,
+                    const XSum* __restrict__ part_heav, int cap, double istep_dt, double* __restrict__ vol,
+                    const double* __restrict__ vol0, double* __restrict__ maxchk, InflateState* __restrict__ inf) {
+  const LsTask& t = B.t[blockIdx.x];
+  const int l = t.l, n = t.tx * t.ty * t.nch;
+  double sa = 0.;
+  for (int b = threadIdx.x; b < n; b += kFinalThreads) sa += part_area[(long long)l * cap + b];
+  sa = block_sum<double, kFinalThreads>(sa);
+  const XSum hs = task_heav(t, part_heav, cap);
+  if (threadIdx.x != 0) return;
   double area = sa * p.dx * p.dy * p.dz;
   if (p.TwoD) area = area / p.lx;
-  const double volume = 1. - sh / ((1. * p.imax * p.jmax) * p.kmax);
+  const double volume = 1. - xs_value(hs) / ((1. * p.imax * p.jmax) * p.kmax);
   vol[l] = volume;
   double loss_rate = p.lx * p.ly * p.lz * (volume - vol0[l]) / istep_dt;
   if (p.TwoD) loss_rate = loss_rate / p.lx;
   const double temp = loss_rate / area;
-  dsc->inflate_temp = temp;
-  dsc->area = area;
-  dsc->heav_sum = sh;
+  inf[l].temp = temp;
   maxchk[l] = temp / (1.5 * p.dz);
 }
 
@@ -1046,22 +1163,10 @@ __global__ void k_inflate_final(Params p, const double* __restrict__ part_area,
 // volumes before (V) and after (V1) the inflation: the blend removes the
 // measured error to first order in the (small) displacement.
 
-// t.out = t.phi0 on the task's written cells (rows of the chunk, images)
-template <typename T>
-__global__ void __launch_bounds__(NT) k_region_copy(Params p, const __grid_constant__ LsBatch B) {
-  const int ti = task_of(B);
-  const LsTask& t = B.t[ti];
-  const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
-  if (!c.ok) return;
-  const T* __restrict__ src = cT<T>(t.phi0);
-  T* __restrict__ dst = mT<T>(t.out);
-  for (int k = c.ka; k <= c.kb; ++k) putL(p, dst, c.i, c.j, k, src[idxL(p, c.i, c.j, k)]);
-}
-
-// per-tile exact sums of H(phi1) over the task's computed interior cells
+// per-(tile, chunk) exact sums of H(phi0) over the tasks' computed interior cells
 template <typename T>
 __global__ void __launch_bounds__(NT) k_region_heav(Params p, const __grid_constant__ LsBatch B,
-                                                    XSum* __restrict__ part) {
+                                                    XSum* __restrict__ part, int cap) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -1069,118 +1174,53 @@ __global__ void __launch_bounds__(NT) k_region_heav(Params p, const __grid_const
   const T* __restrict__ phi = cT<T>(t.phi0);
   XSum sh;
   xs_zero(sh);
+  int ones = 0;
   if (c.ok)
     for (int k = max(c.ka, 1); k <= min(c.kb, p.kmax); ++k)
-      if (computed(c, t.r, k)) xs_add(sh, (double)heav_trig(p, phi[idxL(p, c.i, c.j, k)], s1));
+      if (computed(c, t.r, k)) heav_add(sh, ones, heav_trig(p, phi[idxL(p, c.i, c.j, k)], s1));
+  xs_add_count(sh, ones);
   const XSum bh = block_xsum<NT>(sh);
-  if (flat_tid() == 0) part[c.tile] = bh;
+  if (flat_tid() == 0) part[(long long)t.l * cap + c.tile + (long long)t.tx * t.ty * c.ch] = bh;
 }
 
-// g = (V0 - V)/(V1 - V), V1 from the tiles and the far-field count
-__global__ void k_gain_final(Params p, const XSum* __restrict__ part, int nblk, int l, double outside,
-                             const double* __restrict__ vol, const double* __restrict__ vol0,
-                             DevScalars* __restrict__ dsc) {
+// g = (V0 - V)/(V1 - V) of each task's drop, V1 from the partials and the far-field count
+__global__ void __launch_bounds__(kFinalThreads)
+    k_gain_final(Params p, const __grid_constant__ LsBatch B, const XSum* __restrict__ part, int cap,
+                 const double* __restrict__ vol, const double* __restrict__ vol0, InflateState* __restrict__ inf) {
+  const LsTask& t = B.t[blockIdx.x];
+  const XSum hs = task_heav(t, part, cap);
   if (threadIdx.x != 0) return;
-  XSum hs;
-  xs_zero(hs);
-  for (int b = 0; b < nblk; ++b) xs_merge(hs, part[b]);
-  xs_add_count(hs, (long long)outside);
+  const int l = t.l;
   const double v1 = 1. - xs_value(hs) / ((1. * p.imax * p.jmax) * p.kmax);
   const double d = v1 - vol[l];
-  dsc->inflate_gain = d != 0. ? (vol0[l] - vol[l]) / d : 0.;
+  inf[l].gain = d != 0. ? (vol0[l] - vol[l]) / d : 0.;
 }
 
-// the volume of drop l now, from the tiles and the far-field count
-__global__ void k_volume_now(Params p, const XSum* __restrict__ part, int nblk, int l, double outside,
-                             double* __restrict__ vnow) {
-  if (threadIdx.x != 0) return;
-  XSum hs;
-  xs_zero(hs);
-  for (int b = 0; b < nblk; ++b) xs_merge(hs, part[b]);
-  xs_add_count(hs, (long long)outside);
-  vnow[l] = 1. - xs_value(hs) / ((1. * p.imax * p.jmax) * p.kmax);
+// the volume of each task's drop now
+__global__ void __launch_bounds__(kFinalThreads)
+    k_volume_now(Params p, const __grid_constant__ LsBatch B, const XSum* __restrict__ part, int cap,
+                 double* __restrict__ vnow) {
+  const LsTask& t = B.t[blockIdx.x];
+  const XSum hs = task_heav(t, part, cap);
+  if (threadIdx.x == 0) vnow[t.l] = 1. - xs_value(hs) / ((1. * p.imax * p.jmax) * p.kmax);
 }
 
-// t.out (phi1, in place) = phi0 + g (phi1 - phi0) on the written cells
+// out (the level set before the correction) += g (phi0 - out), phi0 the
+// inflated one, on the written cells
 template <typename T>
 __global__ void __launch_bounds__(NT) k_region_blend(Params p, const __grid_constant__ LsBatch B,
-                                                     const DevScalars* __restrict__ dsc) {
+                                                     const InflateState* __restrict__ inf) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
   if (!c.ok) return;
-  const double g = dsc->inflate_gain;
-  const T* __restrict__ p0 = cT<T>(t.phi0);
-  T* __restrict__ p1 = mT<T>(t.out);
+  const double g = inf[t.l].gain;
+  const T* __restrict__ p1 = cT<T>(t.phi0);
+  T* __restrict__ p0 = mT<T>(t.out);
   for (int k = c.ka; k <= c.kb; ++k) {
     const long long n = idxL(p, c.i, c.j, k);
     const double a0 = (double)p0[n];
-    putL(p, p1, c.i, c.j, k, TC(a0 + g * ((double)p1[n] - a0)));
-  }
-}
-
-// u_lc, v_lc, w_lc of levelset.f90:527-548, with u_l,v_l,w_l of 530-532
-// after bounduvw evaluated on the fly; computed interior cells of r
-template <typename T>
-__device__ __forceinline__ T infl_face(const Params& p, const T* __restrict__ dheav, T temp, int axis, int i, int j,
-                                       int k) {
-  const long long n = idxC(p, i, j, k);
-  if (axis == 0) return -divx(p, temp * (dheav[n + 1] - dheav[n]));
-  if (axis == 1) return -divy(p, temp * (dheav[n + p.nCx] - dheav[n]));
-  return -divz(p, temp * (dheav[n + (long long)p.nCx * p.nCy] - dheav[n]));
-}
-// v_l(i,0,k) and v_l(i,jmax,k) with the y walls of boundp(dheav) and
-// bounduvw(u_l,v_l,w_l) (levelset.f90:466-478, bound.f90:81-282) for
-// BC_in_y = Walls, InOut, OutOut: v_l = 0 on a wall, v_inflow at the inlet,
-// the OutOut extrapolation at y = 0, and dheav(i,j1,k) = -dheav(i,jmax,k) at
-// an outflow end
-template <typename T>
-__device__ __forceinline__ T infl_v_front(const Params& p, const T* __restrict__ dheav, T temp, int i, int k,
-                                          const double* __restrict__ vin) {
-  if (p.bcy == ICLS_BCY_WALLS) return TC(0.);
-  if (p.bcy == ICLS_BCY_INOUT) return TC(vin[i + (long long)(p.i1 + 1) * k]);
-  const T wl_1 = (k == p.kmax) ? TC(0.) : infl_face(p, dheav, temp, 2, i, 1, k);
-  const T wl_0 = (k == 1) ? TC(0.) : infl_face(p, dheav, temp, 2, i, 1, k - 1);
-  return infl_face(p, dheav, temp, 1, i, 1, k) + TC(p.dy / p.dz) * (wl_1 - wl_0);
-}
-template <typename T>
-__device__ __forceinline__ T infl_v_back(const Params& p, const T* __restrict__ dheav, T temp, int i, int k) {
-  if (p.bcy == ICLS_BCY_WALLS) return TC(0.);
-  const T h = dheav[idxC(p, i, p.jmax, k)];
-  return -divy(p, temp * (-h - h));
-}
-template <typename T>
-__global__ void __launch_bounds__(NT) k_inflate_vel(Params p, const __grid_constant__ LsBatch B,
-                                                    const T* __restrict__ dheav, const T* __restrict__ kappa,
-                                                    const DevScalars* __restrict__ dsc, T* __restrict__ ulc,
-                                                    T* __restrict__ vlc, T* __restrict__ wlc,
-                                                    const double* __restrict__ vin) {
-  const int ti = task_of(B);
-  const LsTask& t = B.t[ti];
-  const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
-  if (!c.ok || !c.cxy) return;
-  const int i = c.i, j = c.j;
-  const T temp = TC(dsc->inflate_temp);
-  for (int k = max(c.ka, max(t.r.cz0, 1)); k <= min(c.kb, min(t.r.cz1, p.kmax)); ++k) {
-    const long long q = idxI(p, i, j, k);
-    const T ul_m = infl_face(p, dheav, temp, 0, wrapx(p, i - 1), j, k);
-    const T ul_0 = infl_face(p, dheav, temp, 0, i, j, k);
-    T vl_m, vl_0;
-    if (p.bcy == ICLS_BCY_PERIODIC || (j != 1 && j != p.jmax)) {
-      vl_m = infl_face(p, dheav, temp, 1, i, wrapy(p, j - 1), k);
-      vl_0 = infl_face(p, dheav, temp, 1, i, j, k);
-    } else {
-      vl_m = j == 1 ? infl_v_front(p, dheav, temp, i, k, vin) : infl_face(p, dheav, temp, 1, i, j - 1, k);
-      vl_0 = j == p.jmax ? infl_v_back(p, dheav, temp, i, k) : infl_face(p, dheav, temp, 1, i, j, k);
-    }
-    const T wl_m = (k == 1) ? TC(0.) : infl_face(p, dheav, temp, 2, i, j, k - 1);
-    const T wl_0 = (k == p.kmax) ? TC(0.) : infl_face(p, dheav, temp, 2, i, j, k);
-    T a = (ul_m + ul_0) / TC(2.), b = (vl_m + vl_0) / TC(2.), cc = (wl_m + wl_0) / TC(2.);
-    if (p.ispeed_curv) {
-      const T kp = kappa[idxC(p, i, j, k)];
-      a = a * kp; b = b * kp; cc = cc * kp;
-    }
-    ulc[q] = a; vlc[q] = b; wlc[q] = cc;
+    putL(p, p0, c.i, c.j, k, TC(a0 + g * ((double)p1[n] - a0)));
   }
 }
 
@@ -1221,12 +1261,6 @@ __global__ void __launch_bounds__(NT) k_materialize(Params p, Region r, double b
   int i, j, k;
   if (!cell3(r0, r1, i, j, k)) return;
   if (!in_written(p, r, i, j, k)) y[idxL(p, i, j, k)] = (k < 0 || k > p.k1) ? TC(bgg) : TC(bg);
-}
-
-template <typename T>
-__global__ void k_copy(T* __restrict__ dst, const T* __restrict__ src, long long n) {
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-    dst[q] = src[q];
 }
 
 // field conversions of the precision form (upload / download)
@@ -1381,7 +1415,7 @@ void launch_band_extents(Ctx& c, int l) {
           (k_band_extents<double><<<g, NT, 0, c.s>>>(c.P, c.lv[l], l, lo, hi)));
 }
 
-template <typename T>
+template <typename T, bool INFL>
 void adv_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt, const double* vu,
                 const double* vv, const double* vw) {
   const T* u = reinterpret_cast<const T*>(vu);
@@ -1391,12 +1425,13 @@ void adv_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, doub
   // the FP32 form always takes the product by the reciprocal)
   const unsigned g = b.start[b.n];
   const bool pw = c.P.pow2 || sizeof(T) == 4;
+  auto go = [&](auto kernel) { kernel<<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w, c.dinf, c.vin); };
   if (scheme == ICLS_HOUC5) {
-    if (pw) k_adv_stage<ICLS_HOUC5, T, 1><<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w);
-    else k_adv_stage<ICLS_HOUC5, T, 0><<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w);
+    if (pw) go(k_adv_stage<ICLS_HOUC5, T, 1, INFL>);
+    else go(k_adv_stage<ICLS_HOUC5, T, 0, INFL>);
   } else {
-    if (pw) k_adv_stage<ICLS_WENO5, T, 1><<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w);
-    else k_adv_stage<ICLS_WENO5, T, 0><<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w);
+    if (pw) go(k_adv_stage<ICLS_WENO5, T, 1, INFL>);
+    else go(k_adv_stage<ICLS_WENO5, T, 0, INFL>);
   }
 }
 // the band list of a batch (its tasks' masks set): entries in c.band_list,
@@ -1444,8 +1479,14 @@ void launch_adv_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a
                       const double* vu, const double* vv, const double* vw) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "adv_stage", 1);
-  BY_FORM(c, adv_launch<float>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw),
-          adv_launch<double>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw));
+  BY_FORM(c, (adv_launch<float, false>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw)),
+          (adv_launch<double, false>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw)));
+}
+void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt) {
+  if (b.n == 0) return;
+  Scope sc_(c.prof, c.s, "inflate_stage", 1);
+  BY_FORM(c, (adv_launch<float, true>(c, b, scheme, stage1, a, bb, fdt, nullptr, nullptr, nullptr)),
+          (adv_launch<double, true>(c, b, scheme, stage1, a, bb, fdt, nullptr, nullptr, nullptr)));
 }
 
 void launch_reinit_stage(Ctx& c, const LsBatch& b, int stage, double dtau) {
@@ -1532,57 +1573,42 @@ void launch_materials_final(Ctx& c, const double* outside, const int* ntiles) {
   }
 }
 
-// b: one task (shape-C region of the drop, apron 1), phi0 = its level set
-void launch_inflate_sums(Ctx& c, const LsBatch& b, double outside) {
+// the area sums behind the exact sums
+double* aparts(Ctx& c) { return c.hpart + (size_t)4 * c.P.L * c.hcap; }
+// tasks: the drops' shape-C regions, apron 1, in z chunks of kStageRows (at
+// most hcap partials per drop), phi0 = their level sets, far = the interior
+// cells outside them
+void launch_inflate_sums(Ctx& c, const LsBatch& b) {
+  if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "inflate_sums", 2);
-  double* pa = c.hpart;
-  XSum* ph = reinterpret_cast<XSum*>(c.hpart + c.red_cap);
-  if (c.P.f32) {
-    auto f = [](double* q) { return reinterpret_cast<float*>(q); };
-    k_inflate_sums<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, f(c.kappa), f(c.nrm_m), f(c.dheav), pa, ph);
-  } else {
-    k_inflate_sums<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.kappa, c.nrm_m, c.dheav, pa, ph);
-  }
-  k_inflate_final<<<1, 32, 0, c.s>>>(c.P, pa, ph, b.start[b.n], b.t[0].l, (double)c.cfg.inflate_step * c.dt, outside,
-                                     c.dvol, c.dvol0, c.dmaxchk, c.dsc);
+  BY_FORM(c, (k_inflate_sums<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, aparts(c), hparts(c), c.hcap)),
+          (k_inflate_sums<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, aparts(c), hparts(c), c.hcap)));
+  k_inflate_final<<<b.n, kFinalThreads, 0, c.s>>>(c.P, b, aparts(c), hparts(c), c.hcap,
+                                                  (double)c.cfg.inflate_step * c.dt, c.dvol, c.dvol0, c.dmaxchk,
+                                                  c.dinf);
 }
-
-// gain-one inflation: phi0 copy, the volume after, and the blend
-void launch_region_copy(Ctx& c, const LsBatch& b) {
-  Scope sc_(c.prof, c.s, "gain_one", 1);
-  BY_FORM(c, (k_region_copy<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b)),
-          (k_region_copy<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b)));
+// gain-one inflation: the volume after it, and the blend
+void launch_region_heav(Ctx& c, const LsBatch& b) {
+  BY_FORM(c, (k_region_heav<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, hparts(c), c.hcap)),
+          (k_region_heav<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, hparts(c), c.hcap)));
 }
-void launch_gain(Ctx& c, const LsBatch& b, double outside) {
+void launch_gain(Ctx& c, const LsBatch& b) {
+  if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "gain_one", 2);
-  XSum* ph = reinterpret_cast<XSum*>(c.hpart + c.red_cap);
-  BY_FORM(c, (k_region_heav<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, ph)),
-          (k_region_heav<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, ph)));
-  k_gain_final<<<1, 32, 0, c.s>>>(c.P, ph, b.start[b.n], b.t[0].l, outside, c.dvol, c.dvol0, c.dsc);
+  launch_region_heav(c, b);
+  k_gain_final<<<b.n, kFinalThreads, 0, c.s>>>(c.P, b, hparts(c), c.hcap, c.dvol, c.dvol0, c.dinf);
 }
-void launch_volume_now(Ctx& c, const LsBatch& b, double outside) {
+void launch_volume_now(Ctx& c, const LsBatch& b) {
+  if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "gain_one", 2);
-  XSum* ph = reinterpret_cast<XSum*>(c.hpart + c.red_cap);
-  BY_FORM(c, (k_region_heav<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, ph)),
-          (k_region_heav<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, ph)));
-  k_volume_now<<<1, 32, 0, c.s>>>(c.P, ph, b.start[b.n], b.t[0].l, outside, c.dvolnow);
+  launch_region_heav(c, b);
+  k_volume_now<<<b.n, kFinalThreads, 0, c.s>>>(c.P, b, hparts(c), c.hcap, c.dvolnow);
 }
 void launch_region_blend(Ctx& c, const LsBatch& b) {
+  if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "gain_one", 1);
-  BY_FORM(c, (k_region_blend<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dsc)),
-          (k_region_blend<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dsc)));
-}
-
-// b: one task (shape-C region of the drop, apron 0)
-void launch_inflate_vel(Ctx& c, const LsBatch& b) {
-  Scope sc_(c.prof, c.s, "inflate_vel", 1);
-  if (c.P.f32) {
-    auto f = [](double* q) { return reinterpret_cast<float*>(q); };
-    k_inflate_vel<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, f(c.dheav), f(c.kappa), c.dsc, f(c.ulc), f(c.vlc),
-                                                           f(c.wlc), c.vin);
-  } else {
-    k_inflate_vel<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dheav, c.kappa, c.dsc, c.ulc, c.vlc, c.wlc, c.vin);
-  }
+  BY_FORM(c, (k_region_blend<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf)),
+          (k_region_blend<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf)));
 }
 
 void launch_boundmls(Ctx& c, double* phi) {
@@ -1598,11 +1624,6 @@ void launch_materialize(Ctx& c, const Region& r, double bg, double bgg, double* 
   BY_FORM(c,
           (k_materialize<float><<<grid_of(r0, r1), kBlock, 0, c.s>>>(c.P, r, bg, bgg, reinterpret_cast<float*>(phi))),
           (k_materialize<double><<<grid_of(r0, r1), kBlock, 0, c.s>>>(c.P, r, bg, bgg, phi)));
-}
-
-void launch_copy(Ctx& c, double* dst, const double* src, long long n) {
-  Scope sc_(c.prof, c.s, "copy", 1);
-  k_copy<double><<<1184, 256, 0, c.s>>>(dst, src, n);
 }
 
 void launch_to_float(Ctx& c, double* dst_f32, const double* src, long long n) {
