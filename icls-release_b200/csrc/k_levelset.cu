@@ -893,6 +893,15 @@ __device__ __forceinline__ void min_into(float* a, float v) {
     old = prev;
   }
 }
+// a Heaviside value into an exact sum: the zeros add nothing and the ones
+// (most cells of a box) are counted, so only interface cells pay the limb
+// arithmetic
+template <typename T>
+__device__ __forceinline__ void heav_add(XSum& s, int& ones, T H) {
+  if (H == TC(1.)) ++ones;
+  else if (H != TC(0.)) xs_add(s, (double)H);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(NT, 4) k_heaviside(Params p, const __grid_constant__ LsBatch B,
                                                   T* __restrict__ jiemian, XSum* __restrict__ part, int cap) {
@@ -903,6 +912,7 @@ __global__ void __launch_bounds__(NT, 4) k_heaviside(Params p, const __grid_cons
   const T* __restrict__ phi = cT<T>(t.phi0);
   XSum s;
   xs_zero(s);
+  int ones = 0;
   if (c.ok && c.cxy) {
     const int i = c.i, j = c.j;
     const int ii = image_of<1>(i, p.imax), jj = image_of<1>(j, p.jmax);
@@ -927,11 +937,12 @@ __global__ void __launch_bounds__(NT, 4) k_heaviside(Params p, const __grid_cons
               if (ii != INT_MIN) min_into(jiemian + idxC(p, ii, jj, k), H);
             }
           }
-          if (k >= 1 && k <= p.kmax) xs_add(s, (double)H);
+          if (k >= 1 && k <= p.kmax) heav_add(s, ones, H);
         }
       }
     }
   }
+  xs_add_count(s, ones);
   const XSum bs = block_xsum<NT>(s);
   // one partial per (column tile, z chunk) of the task
   if (flat_tid() == 0) part[(long long)t.l * cap + c.tile + (long long)t.tx * t.ty * c.ch] = bs;
@@ -1060,15 +1071,6 @@ __global__ void __launch_bounds__(NT) k_materials_rows2(Params p, const T* __res
 }
 
 // ------------------------------------------------------------ inflation
-// a Heaviside value into an exact sum: the zeros add nothing and the ones
-// (most cells of a box) are counted, so only interface cells pay the limb
-// arithmetic
-template <typename T>
-__device__ __forceinline__ void heav_add(XSum& s, int& ones, T H) {
-  if (H == TC(1.)) ++ones;
-  else if (H != TC(0.)) xs_add(s, (double)H);
-}
-
 // dheav with boundp semantics over the tasks' shape-C regions (aux: the
 // drop's |grad phi|, orig: its curvature; out: dheav), the far-field value 1
 // on their aprons, and per-(tile, chunk) area and volume sums (FP64) over the
