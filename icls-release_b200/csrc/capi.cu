@@ -200,6 +200,7 @@ int allocate(Ctx& c) {
   for (int l = 0; l < P.L; ++l) AL(c.lv[l], tn(P, P.nL));
   if (P.f32) AL(c.stage, (size_t)P.nL);
   AL(c.d_nbcnt, (size_t)P.L);
+  for (uint8_t** m : {&c.seg_mat[0], &c.seg_mat[1], &c.seg_jmp[0], &c.seg_jmp[1]}) AL(*m, (size_t)seg_count(P));
   AL(c.spec, (size_t)P.nI);
   AL(c.twx, (size_t)P.imax);
   AL(c.twy, (size_t)std::max(P.jmax, P.kmax));  // y twiddles, or z twiddles of solver2d_cos
@@ -258,7 +259,8 @@ int allocate(Ctx& c) {
   // list build included);
   // ICLS_CORREC=shapec: the fused correction one thread per shape-C cell
   // in place of one per interior cell writing the images;
-  // ICLS_MATERIALS=rows1: the materials one row per thread, not two.
+  // ICLS_MATERIALS=rows1: the materials one thread per cell of the whole
+  // arrays in place of the segments near the drops.
   const char* ab = std::getenv("ICLS_AB2");
   c.ab2_ring = !(ab && std::strcmp(ab, "tma") == 0);
   const char* cv = std::getenv("ICLS_CORREC");
@@ -312,6 +314,8 @@ void release(Ctx& c) {
     if (m.mask) cudaFree(m.mask);
   }
   if (c.d_nbcnt) cudaFree(c.d_nbcnt);
+  for (uint8_t* m : {c.seg_mat[0], c.seg_mat[1], c.seg_jmp[0], c.seg_jmp[1]})
+    if (m) cudaFree(m);
   if (c.twx) cudaFree(c.twx);
   if (c.twy) cudaFree(c.twy);
   if (c.czw) cudaFree(c.czw);
@@ -526,9 +530,41 @@ void make_full(Ctx& c, int l) {
   w.have_D = false;
 }
 
+// a caller writes field `id`: what its segment map says of it no longer holds
+void field_written(Ctx& c, int id) {
+  const size_t n = (size_t)seg_count(c.P);
+  switch (id) {
+    case ICLS_F_MIU: case ICLS_F_RHO: case ICLS_F_JIEMIAN: case ICLS_F_RHO_U: case ICLS_F_RHO_V: case ICLS_F_RHO_W:
+      c.mat_dirty = true;
+      cudaMemsetAsync(c.seg_mat[c.mat_cur], 1, n, c.s);
+      break;
+    case ICLS_F_PX: case ICLS_F_PY: case ICLS_F_PZ: case ICLS_F_PXOLD: case ICLS_F_PYOLD: case ICLS_F_PZOLD: {
+      const int h = id >= ICLS_F_PXOLD ? 1 : 0;
+      c.jmp_dirty[h] = true;
+      cudaMemsetAsync(c.seg_jmp[h], 1, n, c.s);
+      break;
+    }
+    case ICLS_F_PJUMP:
+      c.pjump_dirty = true;
+      cudaMemsetAsync(c.seg_jmp[0], 1, n, c.s);
+      break;
+    default:
+      break;
+  }
+}
+
 void update_materials(Ctx& c) {
   const int L = c.P.L;
-  launch_fill(c, c.jiemian, c.P.nC, 1.0, true);
+  const size_t ns = (size_t)seg_count(c.P);
+  const int prev = c.mat_cur;
+  if (c.mat_dirty || c.materials_rows1) {
+    cudaMemsetAsync(c.seg_mat[prev], 1, ns, c.s);
+    launch_fill(c, c.jiemian, c.P.nC, 1.0, true);
+  } else {
+    launch_seg_reset(c, c.seg_mat[prev]);
+  }
+  c.mat_cur ^= 1;
+  cudaMemsetAsync(c.seg_mat[c.mat_cur], 0, ns, c.s);
   std::vector<int> all(L);
   for (int l = 0; l < L; ++l) all[l] = l;
   std::vector<int> ntiles(L, 0);  // partial sums per drop: column tiles x z chunks
@@ -540,7 +576,10 @@ void update_materials(Ctx& c) {
     launch_heaviside(c, b);
   }
   for (int l = 0; l < L; ++l) c.outside[l] = outside_count(c, c.win[l].box);
-  launch_materials_final(c, c.outside.data(), ntiles.data());
+  launch_volumes(c, c.outside.data(), ntiles.data());
+  if (c.materials_rows1) launch_materials(c, nullptr, nullptr);
+  else launch_materials(c, c.seg_mat[c.mat_cur], c.seg_mat[prev]);
+  c.mat_dirty = false;
   cudaMemcpyAsync(c.h_vol, c.dvol, sizeof(double) * L, cudaMemcpyDeviceToHost, c.s);
   cudaEventRecord(c.ev_vol, c.s);
   c.vol_pending = true;
@@ -1045,11 +1084,18 @@ int gfm4p(Ctx& c) {
   std::swap(c.px, c.pxold);
   std::swap(c.py, c.pyold);
   std::swap(c.pz, c.pzold);
+  std::swap(c.seg_jmp[0], c.seg_jmp[1]);
+  std::swap(c.jmp_dirty[0], c.jmp_dirty[1]);
+  // the jump fields start at zero: p_x, p_y, p_z where the step before last
+  // left jumps, p_jump where the last one did
   const size_t bytes = sizeof(double) * (size_t)c.P.nC, tbytes = sizeof(double) * tn(c.P, c.P.nC);
-  cudaMemsetAsync(c.px, 0, tbytes, c.s);
-  cudaMemsetAsync(c.py, 0, tbytes, c.s);
-  cudaMemsetAsync(c.pz, 0, tbytes, c.s);
-  cudaMemsetAsync(c.pjump, 0, bytes, c.s);
+  const size_t ns = (size_t)seg_count(c.P);
+  if (c.jmp_dirty[0])
+    for (double* f : {c.px, c.py, c.pz}) cudaMemsetAsync(f, 0, tbytes, c.s);
+  if (c.pjump_dirty) cudaMemsetAsync(c.pjump, 0, bytes, c.s);
+  launch_seg_clear_jumps(c, c.seg_jmp[0], c.seg_jmp[1]);
+  cudaMemsetAsync(c.seg_jmp[0], 0, ns, c.s);
+  c.jmp_dirty[0] = c.pjump_dirty = false;
   for (int g = 0; g < n_groups(c); ++g) {
     const std::vector<int> drops = group_drops(c, g);
     std::vector<LsBatch> b1 = make_batches(drops, kStageRows, [&](int l) { return c_region(c.P, c.win[l].box, 1); });
@@ -1222,6 +1268,7 @@ int icls_upload_field(icls_ctx* h, int id, int l, const double* host) {
   } else {
     CK(cudaMemcpyAsync(d, host, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c.s));
   }
+  field_written(c, id);
   CK(cudaStreamSynchronize(c.s));
   if (id == ICLS_F_LVSET) {  // a new level set: sweep it whole until its band is measured
     collect_bbox(c);
@@ -1371,6 +1418,8 @@ int icls_init_program(icls_ctx* h) {
   CK(cudaMemcpyAsync(c.pxold, c.px, bytes, cudaMemcpyDeviceToDevice, c.s));
   CK(cudaMemcpyAsync(c.pyold, c.py, bytes, cudaMemcpyDeviceToDevice, c.s));
   CK(cudaMemcpyAsync(c.pzold, c.pz, bytes, cudaMemcpyDeviceToDevice, c.s));
+  CK(cudaMemcpyAsync(c.seg_jmp[1], c.seg_jmp[0], (size_t)seg_count(c.P), cudaMemcpyDeviceToDevice, c.s));
+  c.jmp_dirty[1] = c.jmp_dirty[0];
   CK(cudaStreamSynchronize(c.s));
   c.initialised = true;
   return check_launch();
@@ -1446,6 +1495,7 @@ int icls_boundp(icls_ctx* h, int id) {
   double* d = field_ptr(h->c, id, 1, &n);
   if (!d || n != h->c.P.nC) return ICLS_E_ARG;
   launch_boundp(h->c, d, tfield(id));
+  field_written(h->c, id);
   return check_launch();
 }
 

@@ -82,6 +82,24 @@ struct DropWin {
   int grow = 0;
 };
 
+// Segment maps.  Away from the drops the materials hold the carrier's values
+// and the face jumps are zero: at 256^3 with 48 drops nine tenths of the
+// domain.  A map has one byte per 32 consecutive interior cells of a row,
+// rows k = 0..k1 (a warp's share), nonzero where the field may differ from
+// that constant in the segment's own cells.  The sweeps that produce the
+// fields set the bytes, and clear or complete only the segments that are, or
+// were, set; a field that a caller writes (upload, boundp) has its whole map
+// set, so what follows treats it as unknown everywhere.
+constexpr int kSeg = 32;
+__host__ __device__ __forceinline__ int seg_row(const Params& p) { return (p.imax + kSeg - 1) / kSeg; }
+__host__ __device__ __forceinline__ long long seg_count(const Params& p) {
+  return (long long)seg_row(p) * p.jmax * p.nCz;
+}
+// the segment of interior column (i, j), row k in 0..k1
+__host__ __device__ __forceinline__ long long seg_of(const Params& p, int i, int j, int k) {
+  return (i - 1) / kSeg + (long long)seg_row(p) * ((j - 1) + (long long)p.jmax * k);
+}
+
 // z rows per chunk of update_materials' Heaviside sweep (one exact partial
 // sum per column tile and chunk)
 constexpr int kHeavRows = 8;
@@ -137,6 +155,13 @@ struct Ctx {
   double* cosb = nullptr, *cosf = nullptr;
   double2* czw = nullptr;               // (cos, sin)(pi k/(2 kmax)), k < kmax
   double* vin = nullptr;
+  // segment maps: seg_mat[mat_cur] where jiemian may differ from 1 (the other
+  // buffer: before the last update_materials); seg_jmp[0] belongs to p_x, p_y,
+  // p_z and swaps with them, seg_jmp[1] to their old values.  dirty: written
+  // by a caller since (halo cells included), so cleared or rebuilt whole.
+  uint8_t *seg_mat[2] = {nullptr, nullptr}, *seg_jmp[2] = {nullptr, nullptr};
+  int mat_cur = 0;
+  bool mat_dirty = true, jmp_dirty[2] = {false, false}, pjump_dirty = false;
   // reductions and device scalars
   double* partials = nullptr;           // kRedBlocks * max(L,4)
   double* diag = nullptr;               // disp partials: 7 * kRedBlocks, then the 7 sums
@@ -213,7 +238,10 @@ void launch_reinit_reset(Ctx& c, const LsBatch& b, int maxiter);
 void launch_reinit_check(Ctx& c, const LsBatch& b, int it, int maxiter, double thr);
 void launch_heaviside(Ctx& c, const LsBatch& b);
 void launch_fill(Ctx& c, double* a, long long n, double v, bool tfield);
-void launch_materials_final(Ctx& c, const double* outside, const int* ntiles);
+void launch_seg_reset(Ctx& c, const uint8_t* seg);
+void launch_volumes(Ctx& c, const double* outside, const int* ntiles);
+void launch_materials(Ctx& c, const uint8_t* cur, const uint8_t* prev);
+void launch_seg_clear_jumps(Ctx& c, const uint8_t* faces, const uint8_t* lap);
 // mass correction of the tasks' drops; LsTask::far holds the interior cells outside a drop's region
 void launch_inflate_sums(Ctx& c, const LsBatch& b);
 void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt);

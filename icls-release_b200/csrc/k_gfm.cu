@@ -223,7 +223,7 @@ __device__ __forceinline__ double axis_jump(const Params& p, const T* __restrict
 template <typename T>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_jumps(Params p, const __grid_constant__ LsBatch B,
                                               double* __restrict__ pjump, T* __restrict__ px,
-                                              T* __restrict__ py, T* __restrict__ pz) {
+                                              T* __restrict__ py, T* __restrict__ pz, uint8_t* __restrict__ seg) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const T* __restrict__ cv = cT<T>(t.phis);
@@ -249,10 +249,14 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_jumps(Params p
     } else {
       pj = 0.; fx = 0.; fy = 0.; fz = 0.;
     }
+    // most cells of the shell have no crossing next to them: adding their
+    // zeros to fields that start at +0 changes nothing
+    if (pj == 0. && fx == 0. && fy == 0. && fz == 0.) continue;
+    seg[seg_of(p, i, j, k)] = 1;
     atomicAdd(pjump + cc, pj);
-    atomicAdd(px + cc, (T)fx);  // assembled in FP64, stored in the field type
-    atomicAdd(py + cc, (T)fy);
-    atomicAdd(pz + cc, (T)fz);
+    if (fx != 0.) atomicAdd(px + cc, (T)fx);  // assembled in FP64, stored in the field type
+    if (fy != 0.) atomicAdd(py + cc, (T)fy);
+    if (fz != 0.) atomicAdd(pz + cc, (T)fz);
   }
 }
 
@@ -332,9 +336,10 @@ void launch_jumps(Ctx& c, const LsBatch& b) {
   Scope sc_(c.prof, c.s, "jumps", 1);
   if (c.P.f32)
     k_jumps<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.pjump, reinterpret_cast<float*>(c.px),
-                                                     reinterpret_cast<float*>(c.py), reinterpret_cast<float*>(c.pz));
+                                                     reinterpret_cast<float*>(c.py), reinterpret_cast<float*>(c.pz),
+                                                     c.seg_jmp[0]);
   else
-    k_jumps<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.pjump, c.px, c.py, c.pz);
+    k_jumps<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.pjump, c.px, c.py, c.pz, c.seg_jmp[0]);
 }
 // the periodic column spans a..a+la-1 and b..b+lb-1 of n columns share a
 // column (two arcs meet iff one starts inside the other)
