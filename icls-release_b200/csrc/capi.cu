@@ -201,6 +201,7 @@ int allocate(Ctx& c) {
   if (P.f32) AL(c.stage, (size_t)P.nL);
   AL(c.d_nbcnt, (size_t)P.L);
   for (uint8_t** m : {&c.seg_mat[0], &c.seg_mat[1], &c.seg_jmp[0], &c.seg_jmp[1]}) AL(*m, (size_t)seg_count(P));
+  AL(c.row_jmp, (size_t)P.jmax * P.nCz);
   AL(c.spec, (size_t)P.nI);
   AL(c.twx, (size_t)P.imax);
   AL(c.twy, (size_t)std::max(P.jmax, P.kmax));  // y twiddles, or z twiddles of solver2d_cos
@@ -314,7 +315,7 @@ void release(Ctx& c) {
     if (m.mask) cudaFree(m.mask);
   }
   if (c.d_nbcnt) cudaFree(c.d_nbcnt);
-  for (uint8_t* m : {c.seg_mat[0], c.seg_mat[1], c.seg_jmp[0], c.seg_jmp[1]})
+  for (uint8_t* m : {c.seg_mat[0], c.seg_mat[1], c.seg_jmp[0], c.seg_jmp[1], c.row_jmp})
     if (m) cudaFree(m);
   if (c.twx) cudaFree(c.twx);
   if (c.twy) cudaFree(c.twy);
@@ -547,6 +548,7 @@ void field_written(Ctx& c, int id) {
     case ICLS_F_PJUMP:
       c.pjump_dirty = true;
       cudaMemsetAsync(c.seg_jmp[0], 1, n, c.s);
+      cudaMemsetAsync(c.row_jmp, 1, (size_t)c.P.jmax * c.P.nCz, c.s);
       break;
     default:
       break;
@@ -1095,6 +1097,7 @@ int gfm4p(Ctx& c) {
   if (c.pjump_dirty) cudaMemsetAsync(c.pjump, 0, bytes, c.s);
   launch_seg_clear_jumps(c, c.seg_jmp[0], c.seg_jmp[1]);
   cudaMemsetAsync(c.seg_jmp[0], 0, ns, c.s);
+  cudaMemsetAsync(c.row_jmp, 0, (size_t)c.P.jmax * c.P.nCz, c.s);
   c.jmp_dirty[0] = c.pjump_dirty = false;
   for (int g = 0; g < n_groups(c); ++g) {
     const std::vector<int> drops = group_drops(c, g);

@@ -160,6 +160,7 @@ struct Ctx {
   // p_z and swaps with them, seg_jmp[1] to their old values.  dirty: written
   // by a caller since (halo cells included), so cleared or rebuilt whole.
   uint8_t *seg_mat[2] = {nullptr, nullptr}, *seg_jmp[2] = {nullptr, nullptr};
+  uint8_t* row_jmp = nullptr;  // per row (j, k): seg_jmp[0] holds a set byte there (p_jump may be nonzero)
   int mat_cur = 0;
   bool mat_dirty = true, jmp_dirty[2] = {false, false}, pjump_dirty = false;
   // reductions and device scalars

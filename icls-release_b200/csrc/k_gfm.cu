@@ -223,7 +223,8 @@ __device__ __forceinline__ double axis_jump(const Params& p, const T* __restrict
 template <typename T>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_jumps(Params p, const __grid_constant__ LsBatch B,
                                               double* __restrict__ pjump, T* __restrict__ px,
-                                              T* __restrict__ py, T* __restrict__ pz, uint8_t* __restrict__ seg) {
+                                              T* __restrict__ py, T* __restrict__ pz, uint8_t* __restrict__ seg,
+                                              uint8_t* __restrict__ row) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const T* __restrict__ cv = cT<T>(t.phis);
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_jumps(Params p
     // zeros to fields that start at +0 changes nothing
     if (pj == 0. && fx == 0. && fy == 0. && fz == 0.) continue;
     seg[seg_of(p, i, j, k)] = 1;
+    row[(j - 1) + (long long)p.jmax * k] = 1;
     atomicAdd(pjump + cc, pj);
     if (fx != 0.) atomicAdd(px + cc, (T)fx);  // assembled in FP64, stored in the field type
     if (fy != 0.) atomicAdd(py + cc, (T)fy);
@@ -337,9 +339,9 @@ void launch_jumps(Ctx& c, const LsBatch& b) {
   if (c.P.f32)
     k_jumps<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.pjump, reinterpret_cast<float*>(c.px),
                                                      reinterpret_cast<float*>(c.py), reinterpret_cast<float*>(c.pz),
-                                                     c.seg_jmp[0]);
+                                                     c.seg_jmp[0], c.row_jmp);
   else
-    k_jumps<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.pjump, c.px, c.py, c.pz, c.seg_jmp[0]);
+    k_jumps<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.pjump, c.px, c.py, c.pz, c.seg_jmp[0], c.row_jmp);
 }
 // the periodic column spans a..a+la-1 and b..b+lb-1 of n columns share a
 // column (two arcs meet iff one starts inside the other)

@@ -338,15 +338,16 @@ __device__ __forceinline__ void reg_dft(double2 (&x)[R], const double2* __restri
 }
 
 // The Poisson right-hand side of fillps (fillps.f90:36-53), plus p_jump when
-// add is set, at shape-C index c from the predicted velocities of type T
+// add is set (the row's map byte: adding the zeros of the other rows changes
+// nothing but the sign of a zero), at shape-C index c from the predicted velocities of type T
 // (float in the FP32 form): the expression of k_fillps, so the same bits.
 struct RhsArgs {
   const void *du, *dv, *dw;
   const double* pj;
-  int add;
+  const uint8_t* row;  // rows (j, k) whose p_jump may be nonzero; null: p_jump is not added
 };
 template <typename T>
-__device__ __forceinline__ double rhs_at(const Params& p, const RhsArgs& r, long long c) {
+__device__ __forceinline__ double rhs_at(const Params& p, const RhsArgs& r, long long c, bool add) {
   const T* __restrict__ du = static_cast<const T*>(r.du);
   const T* __restrict__ dv = static_cast<const T*>(r.dv);
   const T* __restrict__ dw = static_cast<const T*>(r.dw);
@@ -357,7 +358,7 @@ __device__ __forceinline__ double rhs_at(const Params& p, const RhsArgs& r, long
   const double vel_y = __dmul_rn(__dsub_rn((double)dv[c], (double)dv[c - p.nCx]), p.dyi);
   const double vel_z = __dmul_rn(__dsub_rn((double)dw[c], (double)dw[c - (long long)p.nCx * p.nCy]), p.dzi);
   double v = __dmul_rn(coef, __dadd_rn(__dadd_rn(vel_x, vel_y), vel_z));
-  if (r.add) v = __dadd_rn(v, r.pj[c]);
+  if (add) v = __dadd_rn(v, r.pj[c]);
   return v;
 }
 
@@ -422,12 +423,20 @@ __global__ void __launch_bounds__(256, (R1 > 16 || R2 > 16) ? 1 : 2)
   // step 1: lane n2 < R2 transforms z[R2 n1 + n2] over n1
   if (lane < R2 && live) {
     double2 x[R1];
+    bool adda = false, addb = false;
+    if constexpr (RHS != 0) {
+      if (ra.row) {
+        adda = ra.row[(ja - 1) + (long long)p.jmax * ka] != 0;
+        addb = ra.row[(jb - 1) + (long long)p.jmax * kb] != 0;
+      }
+    }
 #pragma unroll
     for (int n1 = 0; n1 < R1; ++n1) {
       const int n = R2 * n1 + lane;
       if constexpr (RHS != 0) {  // dir 0: lines a and b start at columns 1 of (ja,ka), (jb,kb)
         using T = typename std::conditional<RHS == 4, float, double>::type;
-        x[n1] = make_double2(rhs_at<T>(p, ra, idxC(p, 1, ja, ka) + n), rhs_at<T>(p, ra, idxC(p, 1, jb, kb) + n));
+        x[n1] = make_double2(rhs_at<T>(p, ra, idxC(p, 1, ja, ka) + n, adda),
+                             rhs_at<T>(p, ra, idxC(p, 1, jb, kb) + n, addb));
       } else {
         x[n1] = dir == 0 ? make_double2(A[n * st], B[n * st]) : pack_hc(A, B, N, n, st);
       }
@@ -960,7 +969,7 @@ void launch_fillps_solver2d(Ctx& c, int write_halos, int add) {
     launch_solver2d(c, write_halos);
     return;
   }
-  RhsArgs ra{c.dudt, c.dvdt, c.dwdt, c.pjump, add};
+  RhsArgs ra{c.dudt, c.dvdt, c.dwdt, c.pjump, add ? c.row_jmp : nullptr};
   solver2d_periodic(c, write_halos, &ra);
 }
 void solver2d_periodic(Ctx& c, int write_halos, const RhsArgs* ra) {
