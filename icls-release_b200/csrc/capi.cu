@@ -223,8 +223,10 @@ int allocate(Ctx& c) {
   AL(c.dsc, 1);
   AL(c.dvol, (size_t)P.L); AL(c.dvol0, (size_t)P.L); AL(c.dmaxchk, (size_t)P.L);
   AL(c.dvolnow, (size_t)P.L);
-  // band list of the advection stages: up to one entry per interior cell
-  c.band_cap = P.nI;
+  // band list of the advection stages: an entry per interior cell, and on
+  // small grids, where the drops' boxes add up to more than the domain, up to
+  // 16M (128 MB)
+  c.band_cap = std::max<long long>(P.nI, std::min<long long>((long long)P.L * P.nI, 1LL << 24));
   if (cudaMalloc(&c.band_list, (size_t)c.band_cap * 8) != cudaSuccess) return ICLS_E_NOMEM;
   if (cudaMalloc((void**)&c.band_count, sizeof(int)) != cudaSuccess) return ICLS_E_NOMEM;
   AL(c.drs, (size_t)P.L);
@@ -255,9 +257,8 @@ int allocate(Ctx& c) {
   // ICLS_AB2=tma: the FP64 predictor on the TMA-fed kernel in place of the
   // cp.async-ring one (the ring kernel measured faster at 256^3, 1.37 vs
   // 1.68 ms);
-  // ICLS_ADV=band: the advection stages after tube_construction as the
-  // band-list split (measured no faster in FP64, slower in FP32, with the
-  // list build included);
+  // ICLS_ADV=column: the advection stages after tube_construction as
+  // sweeps of each drop's columns in place of the list of its band cells;
   // ICLS_CORREC=shapec: the fused correction one thread per shape-C cell
   // in place of one per interior cell writing the images;
   // ICLS_MATERIALS=rows1: the materials one thread per cell of the whole
@@ -269,7 +270,7 @@ int allocate(Ctx& c) {
   const char* mv = std::getenv("ICLS_MATERIALS");
   c.materials_rows1 = mv && std::strcmp(mv, "rows1") == 0;
   const char* av = std::getenv("ICLS_ADV");
-  c.adv_column = !(av && std::strcmp(av, "band") == 0);
+  c.adv_column = av && std::strcmp(av, "column") == 0;
   // working buffers of a group of drops: as many drops as half the free
   // HBM holds (ICLS_GROUP=n caps the group, e.g. to test the grouped path)
   {
@@ -588,35 +589,34 @@ void update_materials(Ctx& c) {
   std::fill(c.vol_dirty.begin(), c.vol_dirty.end(), 0);
 }
 
-// tube_construction (levelset.f90:87-197) of the batches' drops into
+// tube_construction (levelset.f90:87-197) of the batch's drops into
 // their members' s1 and band masks; every cell outside the measured band
-// box is +6dz afterwards
-void tube_batches(Ctx& c, std::vector<LsBatch>& bs) {
-  for (LsBatch& b : bs) {
-    for (int q = 0; q < b.n; ++q) {
-      LsTask& t = b.t[q];
-      const DropWin& w = c.win[t.l];
-      t.phi0 = c.lv[t.l];
-      t.vin = w.valid;
-      t.bgin = w.bg;
-      t.bggin = w.bg_ghost;
-      t.out = member(c, t.l).s1;
-      t.mask = member(c, t.l).mask;
-    }
-    launch_tube(c, b);
-    for (int q = 0; q < b.n; ++q) {
-      DropWin& w = c.win[b.t[q].l];
-      w.valid = w.box;
-      w.bg = c.P.NB;
-      w.bg_ghost = c.P.NB;
-      w.bg_valid = true;
-    }
+// box is +6dz afterwards.  list: the band cells into c.band_list, and the
+// clipped values into s2 and s3 too.
+void tube_batch(Ctx& c, LsBatch& b, bool list) {
+  for (int q = 0; q < b.n; ++q) {
+    LsTask& t = b.t[q];
+    const DropWin& w = c.win[t.l];
+    const Ctx::Member& m = member(c, t.l);
+    t.phi0 = c.lv[t.l];
+    t.vin = w.valid;
+    t.bgin = w.bg;
+    t.bggin = w.bg_ghost;
+    t.out = m.s1;
+    t.out2 = m.s2;
+    t.out3 = m.s3;
+    t.mask = m.mask;
+  }
+  launch_tube(c, b, list);
+  for (int q = 0; q < b.n; ++q) {
+    DropWin& w = c.win[b.t[q].l];
+    w.valid = w.box;
+    w.bg = c.P.NB;
+    w.bg_ghost = c.P.NB;
+    w.bg_valid = true;
   }
 }
 
-// SSP-RK3 of ls_advection / inflation (levelset.f90:235-243, 558-565) on
-// the batches' drops, with their members' buffers: from_tube, s1 -> s2 ->
-// s3 -> the drop's own array; else the drop's array -> s1 -> s2 -> itself
 // the band cells a batch's list can hold at most: its tasks' computed
 // interior cells
 long long band_bound(const Ctx& c, const LsBatch& b) {
@@ -629,57 +629,69 @@ long long band_bound(const Ctx& c, const LsBatch& b) {
   return n;
 }
 
-void rk3_batches(Ctx& c, std::vector<LsBatch>& bs, int scheme, bool from_tube, const double* vu, const double* vv,
-                 const double* vw) {
+// the RK3 combinations, in a stage's arithmetic, of a value that no stage moves
+template <typename T>
+T rk3_still(T x) {
+  const T y = (T)(3. / 4.) * x + (T)(1. / 4.) * x;
+  return (T)(1. / 3.) * x + (T)(2. / 3.) * y;
+}
+// the stages return NB and the far-field values g, h for NB
+template <typename T>
+bool rk3_keeps(double NB, double g, double h) {
+  const T nb = (T)NB;
+  return rk3_still(nb) == nb && (T)g == nb && (T)h == nb;
+}
+
+// SSP-RK3 of ls_advection (levelset.f90:235-243, 558-565) on the batch's
+// drops, with their members' buffers, tiles of kStageRows.  After a tube
+// (from_tube) s1 holds the base: with its list (need >= 0: the list's bound)
+// s1 -> s2 -> s3 -> s1, which then becomes the drop's array; by columns s1 ->
+// s2 -> s3 -> the drop's array.  Else the drop's array -> s1 -> s2 -> itself.
+void rk3_batch(Ctx& c, LsBatch& b, int scheme, bool from_tube, long long need) {
   const double dt = c.dt;
-  for (LsBatch& b : bs) {
-    // after tube_construction the band flags are fresh: one band list serves
-    // the three stages
-    // (a list entry holds i and j in 12 bits each)
-    const bool packs = c.P.imax <= 4096 && c.P.jmax <= 4096;
-    const long long need = from_tube && !c.adv_column && packs ? band_bound(c, b) : -1;
-    const bool split = need >= 0 && need <= c.band_cap;
-    if (split) {
-      for (int q = 0; q < b.n; ++q) b.t[q].mask = member(c, b.t[q].l).mask;
-      launch_band_list(c, b);
-    }
-    double g[kTasks][4], h[kTasks][4];
+  const bool list = need >= 0;
+  set_tiles(b, kStageRows);
+  double g[kTasks][4], h[kTasks][4];
+  for (int q = 0; q < b.n; ++q) {
+    const DropWin& w = c.win[b.t[q].l];
+    g[q][0] = w.bg;
+    h[q][0] = w.bg_ghost;
+    g[q][1] = g[q][0];
+    h[q][1] = h[q][0];
+    g[q][2] = 3. / 4. * g[q][0] + 1. / 4. * g[q][1];
+    h[q][2] = 3. / 4. * h[q][0] + 1. / 4. * h[q][1];
+    g[q][3] = 1. / 3. * g[q][0] + 2. / 3. * g[q][2];
+    h[q][3] = 1. / 3. * h[q][0] + 2. / 3. * h[q][2];
+  }
+  bool keeps = true;
+  for (int q = 0; q < b.n; ++q)
+    keeps = keeps && (c.P.f32 ? rk3_keeps<float>(c.P.NB, g[q][3], h[q][3]) : rk3_keeps<double>(c.P.NB, g[q][3], h[q][3]));
+  auto stage = [&](int st, double a, double bb, double fdt) {
     for (int q = 0; q < b.n; ++q) {
-      const DropWin& w = c.win[b.t[q].l];
-      g[q][0] = w.bg;
-      h[q][0] = w.bg_ghost;
-      g[q][1] = g[q][0];
-      h[q][1] = h[q][0];
-      g[q][2] = 3. / 4. * g[q][0] + 1. / 4. * g[q][1];
-      h[q][2] = 3. / 4. * h[q][0] + 1. / 4. * h[q][1];
-      g[q][3] = 1. / 3. * g[q][0] + 2. / 3. * g[q][2];
-      h[q][3] = 1. / 3. * h[q][0] + 2. / 3. * h[q][2];
+      LsTask& t = b.t[q];
+      Ctx::Member& m = member(c, t.l);
+      double* src = from_tube ? m.s1 : c.lv[t.l];
+      double* A = from_tube ? m.s2 : m.s1;
+      double* S = from_tube ? m.s3 : m.s2;
+      t.mask = m.mask;
+      t.phi0 = src;
+      t.phis = st == 1 ? src : (st == 2 ? A : S);
+      t.out = st == 1 ? A : (st == 2 ? S : (list ? src : c.lv[t.l]));
+      t.bg = g[q][st];
+      t.bgg = h[q][st];
     }
-    auto stage = [&](int st, double a, double bb, double fdt) {
-      for (int q = 0; q < b.n; ++q) {
-        LsTask& t = b.t[q];
-        Ctx::Member& m = member(c, t.l);
-        const double* src = from_tube ? m.s1 : c.lv[t.l];
-        double* A = from_tube ? m.s2 : m.s1;
-        double* B = from_tube ? m.s3 : m.s2;
-        t.mask = m.mask;
-        t.phi0 = src;
-        t.phis = st == 1 ? src : (st == 2 ? A : B);
-        t.out = st == 1 ? A : (st == 2 ? B : c.lv[t.l]);
-        t.bg = g[q][st];
-        t.bgg = h[q][st];
-      }
-      if (split) launch_adv_split(c, b, scheme, st == 1 ? 1 : 0, a, bb, fdt, vu, vv, vw, need);
-      else launch_adv_stage(c, b, scheme, st == 1 ? 1 : 0, a, bb, fdt, vu, vv, vw);
-    };
-    stage(1, 1., 0., 1. * dt);
-    stage(2, 3. / 4., 1. / 4., 1. / 4. * dt);
-    stage(3, 1. / 3., 2. / 3., 2. / 3. * dt);
-    for (int q = 0; q < b.n; ++q) {
-      DropWin& w = c.win[b.t[q].l];
-      w.bg = g[q][3];
-      w.bg_ghost = h[q][3];
-    }
+    if (list) launch_adv_band(c, b, scheme, st == 1 ? 1 : 0, a, bb, fdt, c.ucc, c.vcc, c.wcc, need, st == 3 && !keeps);
+    else launch_adv_stage(c, b, scheme, st == 1 ? 1 : 0, a, bb, fdt, c.ucc, c.vcc, c.wcc);
+  };
+  stage(1, 1., 0., 1. * dt);
+  stage(2, 3. / 4., 1. / 4., 1. / 4. * dt);
+  stage(3, 1. / 3., 2. / 3., 2. / 3. * dt);
+  if (list)
+    for (int q = 0; q < b.n; ++q) std::swap(c.lv[b.t[q].l], member(c, b.t[q].l).s1);
+  for (int q = 0; q < b.n; ++q) {
+    DropWin& w = c.win[b.t[q].l];
+    w.bg = g[q][3];
+    w.bg_ghost = h[q][3];
   }
 }
 
@@ -690,7 +702,7 @@ std::vector<LsBatch> single(const Ctx& c, int l, int kc, const Region& r) {
 
 void ls_advection(Ctx& c, int l) {
   std::vector<LsBatch> bs = single(c, l, kStageRows, c.win[l].box);
-  rk3_batches(c, bs, c.cfg.ls_adv_space, false, c.ucc, c.vcc, c.wcc);
+  rk3_batch(c, bs[0], c.cfg.ls_adv_space, false, -1);
 }
 
 // inflation (levelset.f90:407-582) of the given drops, all in the same
@@ -929,7 +941,7 @@ void ls_reinit(Ctx& c, int l) {
 void tube_construction(Ctx& c, int l) {
   std::vector<LsBatch> bs = single(c, l, kStageRows, c.win[l].box);
   cudaMemsetAsync(c.d_nbcnt + l, 0, sizeof(long long), c.s);
-  tube_batches(c, bs);
+  tube_batch(c, bs[0], false);
   std::swap(c.lv[l], member(c, l).s1);
 }
 
@@ -1018,15 +1030,22 @@ int ls_main(Ctx& c, int istep) {
   for (int g = 0; g < n_groups(c); ++g) {
     const std::vector<int> drops = group_drops(c, g);
     std::vector<LsBatch> bs = make_batches(drops, kStageRows, [&](int l) { return c.win[l].box; });
-    bool unmeasured = false;
-    for (int l : drops) unmeasured = unmeasured || (c.use_boxes && !c.win[l].have_D);
-    tube_batches(c, bs);
-    if (unmeasured) {
-      rc = narrow_after_tube(c, drops, g_now);
-      if (rc) return rc;
-      bs = make_batches(drops, kStageRows, [&](int l) { return c.win[l].box; });
+    for (LsBatch& b : bs) {
+      // the tube's list serves the stages (its entries hold i and j in 12 bits each)
+      const long long bound = band_bound(c, b);
+      const bool list = !c.adv_column && c.P.imax <= 4096 && c.P.jmax <= 4096 && bound <= c.band_cap;
+      bool unmeasured = false;
+      for (int q = 0; q < b.n; ++q) unmeasured = unmeasured || (c.use_boxes && !c.win[b.t[q].l].have_D);
+      tube_batch(c, b, list);
+      if (unmeasured) {
+        std::vector<int> in_b;
+        for (int q = 0; q < b.n; ++q) in_b.push_back(b.t[q].l);
+        rc = narrow_after_tube(c, in_b, g_now);
+        if (rc) return rc;
+        for (int q = 0; q < b.n; ++q) b.t[q].r = c.win[b.t[q].l].box;
+      }
+      rk3_batch(c, b, c.cfg.ls_adv_space, true, list ? bound : -1);
     }
-    rk3_batches(c, bs, c.cfg.ls_adv_space, true, c.ucc, c.vcc, c.wcc);
     // the reference corrects the volume before reinitialising; with the
     // gain-one correction the order is swapped, so that one correction also
     // removes the volume change of the reinitialisation in the same step

@@ -39,6 +39,7 @@ struct LsTask {
   const double* orig;    // reinitialisation: sgn source; mass correction: the drop's curvature (shape C)
   double* aux;           // mass correction: |grad phi| (shape I) of the curvature sweep, then H (shape C); else null
   double* out;
+  double *out2, *out3;   // tube with a band list: the clipped values go here as well
   uint8_t* mask;         // the drop's band mask (tube writes, advection reads)
   Region vin;            // tube: phi0 holds valid data on vin's written cells,
   double bgin, bggin;    //       these far-field values elsewhere
@@ -175,7 +176,7 @@ struct Ctx {
   void* band_list = nullptr;
   int* band_count = nullptr;
   long long band_cap = 0;
-  bool adv_column = true;               // the one-kernel column stage (else the band-list split: ICLS_ADV=band)
+  bool adv_column = false;              // the column stage in place of the band list (ICLS_ADV=column)
   double* h_volnow = nullptr;           // pinned host copy
   double* dmaxchk = nullptr;            // per drop maxchk of the last inflation
   ReinitState* drs = nullptr;           // per drop
@@ -231,7 +232,8 @@ Region full_region(const Params& P);
 bool region_full(const Params& P, const Region& r);
 Region c_region(const Params& P, const Region& r, int apron);
 void set_tiles(LsBatch& b, int kc, bool flat = true);
-void launch_tube(Ctx& c, const LsBatch& b);
+// tube_construction; list: the band cells also into c.band_list (sets the batch's own tiles)
+void launch_tube(Ctx& c, LsBatch& b, bool list);
 void launch_adv_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                       const double* vu, const double* vv, const double* vw);
 void launch_reinit_stage(Ctx& c, const LsBatch& b, int stage, double dtau);
@@ -248,9 +250,10 @@ void launch_inflate_sums(Ctx& c, const LsBatch& b);
 void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt);
 void launch_gain(Ctx& c, const LsBatch& b);
 void launch_region_blend(Ctx& c, const LsBatch& b);
-void launch_band_list(Ctx& c, const LsBatch& b);
-void launch_adv_split(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
-                      const double* vu, const double* vv, const double* vw, long long need);
+// one RK3 stage over the band cells that the batch's tube listed; rest: and
+// the last stage's combination on the other cells
+void launch_adv_band(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
+                     const double* vu, const double* vv, const double* vw, long long need, bool rest);
 void launch_volume_now(Ctx& c, const LsBatch& b);
 void launch_boundmls(Ctx& c, double* phi);
 void launch_materialize(Ctx& c, const Region& r, double bg, double bgg, double* phi);

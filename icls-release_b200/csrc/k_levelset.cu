@@ -104,6 +104,12 @@ __global__ void __launch_bounds__(NT) k_band_extents(Params p, const T* __restri
 }
 
 // ---------------------------------------------------------------- tube
+// A band cell of a batch: (i-1) | (j-1) << 12 | task << 24, and k.
+struct BandCell {
+  unsigned ijt;
+  int k;
+};
+
 // Clip to +-NB (levelset.f90:120-128) and the band mask (130-160) over the
 // tasks' regions.  phi0 holds valid data on vin's written cells, bgin
 // (rows 0..k1) or bggin (ghost rows) elsewhere.  Counts the band per drop
@@ -112,131 +118,162 @@ __global__ void __launch_bounds__(NT) k_band_extents(Params p, const T* __restri
 // shifted by jmax/2, z.  A far-field cell is outside the band only if all
 // 15 axial neighbours clip to +-NB, so the test stops at the first that
 // does not (the reference's sums of |clip|-NB <= 0 are zero exactly then).
+//
+// With a list, the band cells of the batch are also appended to it for the
+// advection stages (k_adv_band), and the clipped values go to out2 and out3
+// as well, where those stages read neighbours that they do not write.
+//
+// A thread marches one column of a flat tile up a chunk of at most 31 rows.
+// It reads its own column once (a register window of five rows) and the
+// eight x and y neighbours within two cells; each neighbouring column is
+// either held by the input region or far field throughout.  Bound by
+// instruction issue: the version before staged 2-D tiles of flags in shared
+// memory with a barrier per row and 64-bit index products per store, 580
+// instructions a warp row.  With the list and the two more copies a sweep
+// takes 0.25 ms instead of 0.20 (256^3 x 48, FP64; FP32 0.16 instead of 0.14),
+// and the three stages 0.34 instead of 0.67 ms (FP32 0.19 instead of 0.31).
+constexpr int kTubeRows = 16;
 template <typename T>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_tube(Params p, const __grid_constant__ LsBatch B,
                                              long long* __restrict__ cnt, int* __restrict__ bbox_lo,
-                                             int* __restrict__ bbox_hi) {
+                                             int* __restrict__ bbox_hi, BandCell* __restrict__ list,
+                                             int* __restrict__ count) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
   const T NB = TC(p.NB);
-  const T* __restrict__ in = cT<T>(t.phi0);
-  T* __restrict__ out = mT<T>(t.out);
   const T bgin = TC(t.bgin), bggin = TC(t.bggin);
-  int band = 0;
-  int lo[5] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX, INT_MAX};
-  int hi[5] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN};
-  // The band test reads, per row, in-band flags |clip(phi)| != NB of the
-  // tile's columns and a 2-column halo from a shared-memory plane (double
-  // buffered, one barrier per row) and of its own column's rows k-2..k+2
-  // from a register window.  Every flag comes from the input as the
-  // original reads did: the input region's value where it holds the
-  // column (tested on the wrapped column index) and row, else its far-field
-  // value.
-  __shared__ uint8_t F[2][TBY + 4][TBX + 4];
-  const int tx = (int)threadIdx.x, ty = (int)threadIdx.y, tid = tx + TBX * ty;
-  const int X0 = c.X - tx, Y0 = c.Y - ty;  // the tile's first column in region coordinates
-  auto wrapn = [](int v, int n) { v %= n; return v < 0 ? v + n : v; };
-  auto column = [&](int X, int Y, int& iw, int& jw, bool& held) {
-    iw = wrapn(t.r.xa - 1 + X, p.imax) + 1;
-    jw = wrapn(t.r.ya - 1 + Y, p.jmax) + 1;
-    held = span_has(t.vin.xa, t.vin.xn, p.imax, iw) && span_has(t.vin.ya, t.vin.yn, p.jmax, jw);
-  };
-  auto rdo = [&](long long at, bool held, int k) -> T {
-    return (held && k >= t.vin.z0 && k <= t.vin.z1) ? in[at] : ((k < 0 || k > p.k1) ? bggin : bgin);
-  };
-  auto flag = [&](T v) -> uint8_t { return fabs(clipNB(v, NB)) != NB ? 1 : 0; };
-  const long long sz = (long long)p.nLx * p.nLy;
-  // this thread's column (in or out of the region) and its halo cell, if any
-  int iw, jw, hi_w = 0, hj_w = 0, hxs = 0, hys = 0;
-  bool held, hheld = false;
-  column(c.X, c.Y, iw, jw, held);
-  const bool has_halo = tid < 4 * TBY + 4 * TBX;  // 4 halo columns x TBY rows, 4 halo rows x TBX columns
-  if (has_halo) {
-    int xo, yo;
-    if (tid < 4 * TBY) {
-      const int side = tid / TBY;  // columns -2, -1, TBX, TBX+1
-      xo = side < 2 ? side - 2 : TBX + side - 2;
-      yo = tid % TBY;
-    } else {
-      const int u = tid - 4 * TBY, side = u / TBX;  // rows -2, -1, TBY, TBY+1
-      xo = u % TBX;
-      yo = side < 2 ? side - 2 : TBY + side - 2;
-    }
-    column(X0 + xo, Y0 + yo, hi_w, hj_w, hheld);
-    hxs = xo + 2;
-    hys = yo + 2;
-  }
-  const long long cw = idxL(p, iw, jw, 0), hw = idxL(p, hi_w, hj_w, 0);
-  // z window: flags of this column at rows k-2 .. k+2 (slots 1..4 hold rows
-  // ka-2..ka+1; each row shifts down one slot and reads row k+2 into slot 4)
-  uint8_t fz[5];
-  fz[0] = 0;
-#pragma unroll
-  for (int d = -2; d <= 1; ++d) fz[d + 3] = flag(rdo(cw + (c.ka + d) * sz, held, c.ka + d));
-  // the values a row turns into flags (row k+2 of this column, row k of the
-  // halo cell) were read one row earlier, so a barrier waits on no fresh load
-  T nz = rdo(cw + (c.ka + 2) * sz, held, c.ka + 2);
-  T nh = has_halo ? rdo(hw + c.ka * sz, hheld, c.ka) : bgin;
+  const int sy = p.nLx, sz = p.nLx * p.nLy, szI = p.imax * p.jmax;
   const int i = c.i, j = c.j;
-  const int hx = p.imax / 2, hy = p.jmax / 2;
-  const int ib = i + hx > p.imax ? i + hx - p.imax : i + hx;
-  const int jb = j + hy > p.jmax ? j + hy - p.jmax : j + hy;
-  const bool colin = held;
-  for (int k = c.ka; k <= c.kb; ++k) {
+  unsigned rows = 0;  // bit r: row ka + r is a band cell
+  int kmin = INT_MAX, kmax = INT_MIN;
+  if (c.ok) {
+    const int col = (int)idxL(p, i, j, 0);
+    const T* __restrict__ in = cT<T>(t.phi0) + col;
+    T* const out = mT<T>(t.out);
+    T* const out2 = list ? mT<T>(t.out2) : nullptr;
+    T* const out3 = list ? mT<T>(t.out3) : nullptr;
+    // the column's storage and that of its periodic images
+    const int ii = image_of<3>(i, p.imax), jj = image_of<3>(j, p.jmax);
+    const int o1 = ii != INT_MIN ? (int)idxL(p, ii, j, 0) : -1;
+    const int o2 = jj != INT_MIN ? (int)idxL(p, i, jj, 0) : -1;
+    const int o3 = (ii != INT_MIN && jj != INT_MIN) ? (int)idxL(p, ii, jj, 0) : -1;
+    auto store = [&](T* a, int o, T v) {
+      a[col + o] = v;
+      if (o1 >= 0) a[o1 + o] = v;
+      if (o2 >= 0) {
+        a[o2 + o] = v;
+        if (o3 >= 0) a[o3 + o] = v;
+      }
+    };
+    // columns that the input region holds: x offsets -2..2 (bits 0..4, bit 2
+    // this column), y offsets -2..2 (bits 5..9)
+    unsigned held = 0;
+    {
+      const bool yh = span_has(t.vin.ya, t.vin.yn, p.jmax, j), xh = span_has(t.vin.xa, t.vin.xn, p.imax, i);
 #pragma unroll
-    for (int d = 0; d < 4; ++d) fz[d] = fz[d + 1];
-    fz[4] = flag(nz);
-    nz = rdo(cw + (k + 3) * sz, held, k + 3);
-    const int buf = k & 1;
-    F[buf][ty + 2][tx + 2] = fz[2];
-    if (has_halo) {
-      F[buf][hys][hxs] = flag(nh);
-      nh = rdo(hw + (k + 1) * sz, hheld, k + 1);
+      for (int d = -2; d <= 2; ++d) {
+        if (yh && span_has(t.vin.xa, t.vin.xn, p.imax, wrapx(p, i + d))) held |= 1u << (d + 2);
+        if (xh && span_has(t.vin.ya, t.vin.yn, p.jmax, wrapy(p, j + d))) held |= 1u << (d + 7);
+      }
     }
-    __syncthreads();
-    if (c.ok) {
+    auto far = [&](int k) { return (k < 0 || k > p.k1) ? bggin : bgin; };
+    auto own = [&](int k) -> T {
+      return ((held & 4u) && k >= t.vin.z0 && k <= t.vin.z1) ? in[k * sz] : far(k);
+    };
+    // |clip(v)| != NB (true for NaN)
+    auto in_band = [&](T v) { return !(fabs(v) >= NB); };
+    // own column, rows k-2 .. k+2
+    T a0 = own(c.ka - 2), a1 = own(c.ka - 1), a2 = own(c.ka), a3 = own(c.ka + 1), a4 = own(c.ka + 2);
+    for (int k = c.ka; k <= c.kb; ++k) {
+      const T nxt = own(k + 3);
+      const int o = k * sz;
       T val;
-      const long long c0 = idxL(p, i, j, k);
       if (!computed(c, t.r, k)) {
-        val = clipNB((k < 0 || k > p.k1) ? bggin : bgin, NB);
+        val = clipNB(far(k), NB);
       } else {
-        if (k == 0)
-          val = TC(2.) * clipNB(rdo(c0 + sz, colin, 1), NB) - clipNB(rdo(c0 + 2 * sz, colin, 2), NB);
-        else if (k == p.k1)
-          val = TC(2.) * clipNB(rdo(c0 - sz, colin, p.kmax), NB) - clipNB(rdo(c0 - 2 * sz, colin, p.kmax - 1), NB);
-        else
-          val = clipNB(rdo(c0, colin, k), NB);
+        if (k == 0) val = TC(2.) * clipNB(a3, NB) - clipNB(a4, NB);
+        else if (k == p.k1) val = TC(2.) * clipNB(a1, NB) - clipNB(a0, NB);
+        else val = clipNB(a2, NB);
         if (k >= 1 && k <= p.kmax) {
-          const uint8_t(&Fp)[TBY + 4][TBX + 4] = F[buf];
-          const int m = (fz[2] | Fp[ty + 2][tx] | Fp[ty + 2][tx + 1] | Fp[ty + 2][tx + 3] | Fp[ty + 2][tx + 4] |
-                         Fp[ty][tx + 2] | Fp[ty + 1][tx + 2] | Fp[ty + 3][tx + 2] | Fp[ty + 4][tx + 2] | fz[0] |
-                         fz[1] | fz[3] | fz[4]) != 0;
-          t.mask[idxI(p, i, j, k)] = (uint8_t)m;
-          band += m;
+          bool m = in_band(a0) | in_band(a1) | in_band(a2) | in_band(a3) | in_band(a4);
+          if (!m) {
+            const T fk = far(k);
+            const bool kin = k >= t.vin.z0 && k <= t.vin.z1;
+#pragma unroll
+            for (int d = -2; d <= 2; ++d) {
+              if (d == 0) continue;
+              const T vx = (kin && (held >> (d + 2) & 1u)) ? in[o + d] : fk;
+              const T vy = (kin && (held >> (d + 7) & 1u)) ? in[o + d * sy] : fk;
+              m = m | in_band(vx) | in_band(vy);
+            }
+          }
+          t.mask[(i - 1) + p.imax * (j - 1) + szI * (k - 1)] = m ? 1 : 0;
+          if (m) rows |= 1u << (k - c.ka);
         }
         if (val != NB) {
-          lo[0] = min(lo[0], i); hi[0] = max(hi[0], i);
-          lo[1] = min(lo[1], ib); hi[1] = max(hi[1], ib);
-          lo[2] = min(lo[2], j); hi[2] = max(hi[2], j);
-          lo[3] = min(lo[3], jb); hi[3] = max(hi[3], jb);
-          lo[4] = min(lo[4], k); hi[4] = max(hi[4], k);
+          kmin = min(kmin, k);
+          kmax = k;
         }
       }
-      putL(p, out, i, j, k, val);
+      store(out, o, val);
+      if (list) {
+        store(out2, o, val);
+        store(out3, o, val);
+      }
+      a0 = a1; a1 = a2; a2 = a3; a3 = a4; a4 = nxt;
     }
   }
-  const int bs = block_sum<int, NT>(band);
-  if (flat_tid() == 0 && bs) atomicAdd((unsigned long long*)(cnt + t.l), (unsigned long long)bs);
-  for (int a = 0; a < 5; ++a) {
-    int l = lo[a], h = hi[a];
-    for (int o = 16; o > 0; o >>= 1) {
-      l = min(l, __shfl_down_sync(0xffffffffu, l, o));
-      h = max(h, __shfl_down_sync(0xffffffffu, h, o));
+  const int lane = flat_tid() & 31, warp = flat_tid() >> 5;
+  // the warp's band cells, then the block's: one addition to the drop's count
+  // and one to the list per block; within a warp the rows in order, lanes (x
+  // fastest) within a row
+  __shared__ int wsum[NT / 32], base_sh;
+  int n = 0;
+  for (unsigned any = __reduce_or_sync(0xffffffffu, rows), r = any; r; r &= r - 1)
+    n += __popc(__ballot_sync(0xffffffffu, rows >> (__ffs(r) - 1) & 1u));
+  if (lane == 0) wsum[warp] = n;
+  __syncthreads();
+  if (flat_tid() == 0) {
+    int tot = 0;
+    for (int w = 0; w < NT / 32; ++w) {
+      const int v = wsum[w];
+      wsum[w] = tot;
+      tot += v;
     }
-    if ((flat_tid() & 31) == 0 && l != INT_MAX) {
-      atomicMin(&bbox_lo[5 * t.l + a], l);
-      atomicMax(&bbox_hi[5 * t.l + a], h);
+    if (tot) atomicAdd((unsigned long long*)(cnt + t.l), (unsigned long long)tot);
+    base_sh = (tot && list) ? atomicAdd(count, tot) : 0;
+  }
+  __syncthreads();
+  if (list && n) {
+    int at = base_sh + wsum[warp];
+    const unsigned ijt = (unsigned)(i - 1) | ((unsigned)(j - 1) << 12) | ((unsigned)ti << 24);
+    for (unsigned r = __reduce_or_sync(0xffffffffu, rows); r; r &= r - 1) {
+      const int row = __ffs(r) - 1;
+      const unsigned m = __ballot_sync(0xffffffffu, rows >> row & 1u);
+      if (rows >> row & 1u) list[at + __popc(m & ((1u << lane) - 1u))] = BandCell{ijt, c.ka + row};
+      at += __popc(m);
+    }
+  }
+  int lo[5] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX, INT_MAX};
+  int hi[5] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN};
+  if (kmin != INT_MAX) {
+    const int hx = p.imax / 2, hy = p.jmax / 2;
+    lo[0] = hi[0] = i;
+    lo[1] = hi[1] = i + hx > p.imax ? i + hx - p.imax : i + hx;
+    lo[2] = hi[2] = j;
+    lo[3] = hi[3] = j + hy > p.jmax ? j + hy - p.jmax : j + hy;
+    lo[4] = kmin;
+    hi[4] = kmax;
+  }
+  if (__any_sync(0xffffffffu, kmin != INT_MAX)) {
+#pragma unroll
+    for (int a = 0; a < 5; ++a) {
+      const int l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
+      if (lane == 0) {
+        atomicMin(&bbox_lo[5 * t.l + a], l);
+        atomicMax(&bbox_hi[5 * t.l + a], h);
+      }
     }
   }
 }
@@ -499,119 +536,92 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Para
 }
 
 // ------------------------------------------------- band-list advection
-// One RK stage of k_adv_stage split in three launches over the same tasks,
-// with the same arithmetic per cell (bit-identical):
-//   k_adv_base   every written cell its value without the transport term:
-//                the far field outside the computed part, else f0 (stage
-//                1) or a f0 + bb fs; the wall rows 0 and k1 are left
-//   k_adv_band   adds fdt * dfdt on the band cells of a compacted list
-//                (k_band_list, built once after tube_construction for all
-//                three stages): full warps, and no lane walks a clipped
-//                column only to copy it
-//   k_adv_walls  rows 0 and k1 from the finished rows next to them, under
-//                the conditions k_adv_stage writes them
-// The list holds the computed interior cells whose band flag is set, as
-// (i-1) | (j-1) << 12 | task << 24 and k.
-struct BandCell {
-  unsigned ijt;
-  int k;
-};
-
-template <typename T>
-__global__ void __launch_bounds__(NT) k_band_list(Params p, const __grid_constant__ LsBatch B,
-                                                  BandCell* __restrict__ list, int* __restrict__ count, int cap) {
-  const int ti = task_of(B);
-  const LsTask& t = B.t[ti];
-  const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
-  const unsigned lane = threadIdx.x & 31u;
-  const long long q0 = c.ok ? idxI(p, c.i, c.j, 1) : 0;
-  const long long szI = (long long)p.imax * p.jmax;
-  // every lane of a block walks the same rows, so the ballots line up
-  for (int k = max(c.ka, 1); k <= min(c.kb, p.kmax); ++k) {
-    const bool take = c.ok && computed(c, t.r, k) && t.mask[q0 + (k - 1) * szI];
-    const unsigned msk = __ballot_sync(0xffffffffu, take);
-    if (!msk) continue;
-    int base = 0;
-    if (lane == (unsigned)(__ffs(msk) - 1)) base = atomicAdd(count, __popc(msk));
-    base = __shfl_sync(0xffffffffu, base, __ffs(msk) - 1);
-    const int slot = base + __popc(msk & ((1u << lane) - 1u));
-    if (take && slot < cap)
-      list[slot] = BandCell{(unsigned)(c.i - 1) | ((unsigned)(c.j - 1) << 12) | ((unsigned)ti << 24), k};
+// One RK stage over the batch's list of band cells (k_tube), one thread per
+// cell, the arithmetic of k_adv_stage.  Cells outside the band are exactly
+// +-NB: the first two stages leave them, and the tube wrote them to every
+// buffer the stages read; the last one rounds a/3 + 2a/3, which returns NB
+// where the spacing is a power of two and is applied by k_adv_rest where it
+// does not.  Rows outside 1..kmax of drops next to a wall follow in
+// k_adv_ghosts.
+// Bound by the latency of the 19 stencil loads (a quarter of the box's cells
+// are band cells; the column stage loads all of them and walks every row):
+// 256^3 x 48, FP64 0.223 -> 0.112 ms, FP32 0.104 -> 0.063 ms per stage.
+template <int SCHEME, typename T, int PW>
+__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4))
+    k_adv_band(Params p, const __grid_constant__ LsBatch B, const BandCell* __restrict__ list,
+               const int* __restrict__ count, int stage1, double a_, double bb_, double fdt_,
+               const T* __restrict__ vu, const T* __restrict__ vv, const T* __restrict__ vw) {
+  const int total = *count;
+  const T a = TC(a_), bb = TC(bb_), fdt = TC(fdt_);
+  const int sy = p.nLx, sz = p.nLx * p.nLy;
+  for (int n = (int)(blockIdx.x * NT + threadIdx.x); n < total; n += (int)gridDim.x * NT) {
+    const BandCell bc = list[n];
+    const int i = (int)(bc.ijt & 0xFFFu) + 1, j = (int)((bc.ijt >> 12) & 0xFFFu) + 1, k = bc.k;
+    const LsTask& t = B.t[bc.ijt >> 24];
+    const int o = (int)idxL(p, i, j, k);
+    const int q = (i - 1) + p.imax * ((j - 1) + p.jmax * (k - 1));
+    const T* f = cT<T>(t.phis) + o;
+    const T f0 = cT<T>(t.phi0)[o];
+    const T u = vu[q], v = vv[q], w = vw[q];
+    Axial19<T> S;
+    S.c = f[0];
+#pragma unroll
+    for (int d = -3; d <= 3; ++d) {
+      if (d == 0) continue;
+      S.x[d + 3] = f[d];
+      S.y[d + 3] = f[d * sy];
+      S.z[d + 3] = f[d * sz];
+    }
+    S.x[3] = S.y[3] = S.z[3] = S.c;
+    const T val = (stage1 ? f0 : a * f0 + bb * S.c) + fdt * adv_rhs<SCHEME, PW>(p, S, u, v, w, k);
+    T* const out = mT<T>(t.out);
+    out[o] = val;
+    if (i <= 3 || i > p.imax - 3 || j <= 3 || j > p.jmax - 3) putL(p, out, i, j, k, val);
   }
 }
 
+// After a band stage, the rows outside 1..kmax of the tasks whose computed
+// part holds them: the ghost rows by the stage's combination, the wall rows
+// from the two rows next to them
 template <typename T>
-__global__ void __launch_bounds__(NT) k_adv_base(Params p, const __grid_constant__ LsBatch B, int stage1, double a_,
-                                                 double bb_) {
+__global__ void __launch_bounds__(NT) k_adv_ghosts(Params p, const __grid_constant__ LsBatch B, int stage1, double a_,
+                                                   double bb_) {
+  const int ti = task_of(B);
+  const LsTask& t = B.t[ti];
+  const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
+  if (!c.ok || !c.cxy || t.r.cz0 > -2) return;
+  const T a = TC(a_), bb = TC(bb_);
+  const T* f0 = cT<T>(t.phi0);
+  const T* fs = cT<T>(t.phis);
+  T* out = mT<T>(t.out);
+  auto at = [&](int k) { return idxL(p, c.i, c.j, k); };
+  for (int k : {-2, -1, p.k1 + 1, p.k1 + 2}) {
+    const T v = f0[at(k)];
+    putL(p, out, c.i, c.j, k, stage1 ? v : a * v + bb * fs[at(k)]);
+  }
+  putL(p, out, c.i, c.j, 0, TC(2.) * out[at(1)] - out[at(2)]);
+  putL(p, out, c.i, c.j, p.k1, TC(2.) * out[at(p.kmax)] - out[at(p.kmax - 1)]);
+}
+
+// After the last band stage, where its combination rounds NB: the interior
+// rows' cells outside the band in place (the RK3 combinations of a value that
+// no stage moves), and the far-field value on the aprons
+template <typename T>
+__global__ void __launch_bounds__(NT) k_adv_rest(Params p, const __grid_constant__ LsBatch B) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
   if (!c.ok) return;
-  const T a = TC(a_), bb = TC(bb_);
-  const T* __restrict__ f0c = cT<T>(t.phi0);
-  const T* __restrict__ fsc = cT<T>(t.phis);
   T* out = mT<T>(t.out);
   for (int k = c.ka; k <= c.kb; ++k) {
     if (!computed(c, t.r, k)) {
       putL(p, out, c.i, c.j, k, (k < 0 || k > p.k1) ? TC(t.bgg) : TC(t.bg));
       continue;
     }
-    if (k == 0 || k == p.k1) continue;  // k_adv_walls
-    const long long o = idxL(p, c.i, c.j, k);
-    const T f0 = f0c[o];
-    putL(p, out, c.i, c.j, k, stage1 ? f0 : a * f0 + bb * fsc[o]);
-  }
-}
-
-template <int SCHEME, typename T, int PW>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 4 : 3))
-    k_adv_band(Params p, const __grid_constant__ LsBatch B, const BandCell* __restrict__ list,
-               const int* __restrict__ count, double fdt_, const T* __restrict__ vu, const T* __restrict__ vv,
-               const T* __restrict__ vw) {
-  const int n = (int)(blockIdx.x * NT + threadIdx.x);
-  if (n >= *count) return;
-  const BandCell bc = list[n];
-  const int i = (int)(bc.ijt & 0xFFFu) + 1, j = (int)((bc.ijt >> 12) & 0xFFFu) + 1, ti = (int)(bc.ijt >> 24);
-  const int k = bc.k;
-  const LsTask& t = B.t[ti];
-  const T fdt = TC(fdt_);
-  const long long sy = p.nLx, sz = (long long)p.nLx * p.nLy;
-  const long long o = idxL(p, i, j, k);
-  const long long q = idxI(p, i, j, k);
-  const T* __restrict__ f = cT<T>(t.phis) + o;
-  T* out = mT<T>(t.out);
-  const T base = out[o];  // k_adv_base's value of this cell
-  Axial19<T> S;
-  S.c = f[0];
-#pragma unroll
-  for (int d = -3; d <= 3; ++d) {
-    if (d == 0) continue;
-    S.x[d + 3] = f[d];
-    S.y[d + 3] = f[d * sy];
-    S.z[d + 3] = f[d * sz];
-  }
-  S.x[3] = S.y[3] = S.z[3] = S.c;
-  putL(p, out, i, j, k, base + fdt * adv_rhs<SCHEME, PW>(p, S, vu[q], vv[q], vw[q], k));
-}
-
-template <typename T>
-__global__ void __launch_bounds__(NT) k_adv_walls(Params p, const __grid_constant__ LsBatch B) {
-  const int ti = task_of(B);
-  const LsTask& t = B.t[ti];
-  const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
-  if (!c.ok) return;
-  T* out = mT<T>(t.out);
-  auto at = [&](int k) { return out[idxL(p, c.i, c.j, k)]; };
-  // the rows of this block's chunk that were computed, as k_adv_stage sees them
-  auto row = [&](int k) { return k >= c.ka && k <= c.kb && computed(c, t.r, k); };
-  // k = 0: written when row 2 of the same chunk was computed, from rows 1
-  // (0 if not computed) and 2
-  if (row(0) && row(2)) putL(p, out, c.i, c.j, 0, TC(2.) * (row(1) ? at(1) : TC(0.)) - at(2));
-  // k = k1: from rows kmax and kmax-1 of the same chunk (0 where not computed)
-  if (row(p.k1)) {
-    const T vk = row(p.kmax) ? at(p.kmax) : TC(0.);
-    const T vkm = row(p.kmax - 1) ? at(p.kmax - 1) : TC(0.);
-    putL(p, out, c.i, c.j, p.k1, TC(2.) * vk - vkm);
+    if (k < 1 || k > p.kmax || t.mask[idxI(p, c.i, c.j, k)]) continue;
+    const T x = out[idxL(p, c.i, c.j, k)];
+    const T y = TC(3. / 4.) * x + TC(1. / 4.) * x;
+    putL(p, out, c.i, c.j, k, TC(1. / 3.) * x + TC(2. / 3.) * y);
   }
 }
 
@@ -1436,37 +1446,17 @@ void set_tiles(LsBatch& b, int kc, bool flat) {
     }                                   \
   } while (0)
 
-void launch_tube(Ctx& c, const LsBatch& flat) {
-  if (flat.n == 0) return;
+void launch_tube(Ctx& c, LsBatch& b, bool list) {
+  if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "tube", 1);
-  // k_tube stages a TBX x TBY tile with its halo in shared memory: the same
-  // tasks on 2-D tiles, in z chunks of kTubeRows rows (its register window
-  // along z favours longer chunks than the stage kernels': 16 rows measured
-  // 0.135 -> 0.128 ms FP32, 0.206 -> 0.188 ms FP64 against 8)
-  constexpr int kTubeRows = 16;
-  LsBatch b = flat;
-  int s = 0;
-  for (int q = 0; q < b.n; ++q) {
-    LsTask& t = b.t[q];
-    t.flat = 0;
-    t.tx = (t.r.xn + TBX - 1) / TBX;
-    t.ty = (t.r.yn + TBY - 1) / TBY;
-    const int nz = t.r.z1 - t.r.z0 + 1;
-    if (kTubeRows >= nz) {
-      t.nch = 1;
-      t.kc = nz;
-    } else {
-      t.nch = nz / kTubeRows;
-      t.kc = kTubeRows;
-    }
-    b.start[q] = s;
-    s += t.tx * t.ty * t.nch;
-  }
-  b.start[b.n] = s;
+  // chunks of 16 rows: the register window along z is filled once per chunk
+  set_tiles(b, kTubeRows);
   int* lo = c.d_bbox;
   int* hi = c.d_bbox + 5 * c.P.L;
-  BY_FORM(c, (k_tube<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.d_nbcnt, lo, hi)),
-          (k_tube<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.d_nbcnt, lo, hi)));
+  if (list) cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
+  BandCell* l = list ? reinterpret_cast<BandCell*>(c.band_list) : nullptr;
+  BY_FORM(c, (k_tube<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)),
+          (k_tube<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)));
 }
 
 void launch_band_extents(Ctx& c, int l) {
@@ -1497,47 +1487,43 @@ void adv_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, doub
     else go(k_adv_stage<ICLS_WENO5, T, 0, INFL>);
   }
 }
-// the band list of a batch (its tasks' masks set): entries in c.band_list,
-// their number in c.band_count on the device; need = the upper bound the
-// caller checked against c.band_cap
-void launch_band_list(Ctx& c, const LsBatch& b) {
-  if (b.n == 0) return;
-  Scope sc_(c.prof, c.s, "band_list", 1);
-  cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
-  BandCell* list = reinterpret_cast<BandCell*>(c.band_list);
-  BY_FORM(c, (k_band_list<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, list, c.band_count, (int)c.band_cap)),
-          (k_band_list<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, list, c.band_count, (int)c.band_cap)));
-}
+// one RK stage over the batch from the list of its tube sweep; need = the
+// upper bound of its length that the caller checked against c.band_cap
 template <typename T>
-void adv_split_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
-                      const double* vu, const double* vv, const double* vw, long long need) {
+void adv_band_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
+                     const double* vu, const double* vv, const double* vw, long long need, bool rest, bool walls) {
   const T* u = reinterpret_cast<const T*>(vu);
   const T* v = reinterpret_cast<const T*>(vv);
   const T* w = reinterpret_cast<const T*>(vw);
   const BandCell* list = reinterpret_cast<const BandCell*>(c.band_list);
-  const unsigned nb = (unsigned)((need + NT - 1) / NT);
-  k_adv_base<T><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, stage1, a, bb);
+  const unsigned nb = (unsigned)std::min<long long>((need + NT - 1) / NT, 8 * 148);
+  const bool pw = c.P.pow2 || sizeof(T) == 4;
+  auto go = [&](auto kernel) { kernel<<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, stage1, a, bb, fdt, u, v, w); };
   if (nb > 0) {
-    const bool pw = c.P.pow2 || sizeof(T) == 4;
     if (scheme == ICLS_HOUC5) {
-      if (pw) k_adv_band<ICLS_HOUC5, T, 1><<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, fdt, u, v, w);
-      else k_adv_band<ICLS_HOUC5, T, 0><<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, fdt, u, v, w);
+      if (pw) go(k_adv_band<ICLS_HOUC5, T, 1>);
+      else go(k_adv_band<ICLS_HOUC5, T, 0>);
     } else {
-      if (pw) k_adv_band<ICLS_WENO5, T, 1><<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, fdt, u, v, w);
-      else k_adv_band<ICLS_WENO5, T, 0><<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, fdt, u, v, w);
+      if (pw) go(k_adv_band<ICLS_WENO5, T, 1>);
+      else go(k_adv_band<ICLS_WENO5, T, 0>);
     }
   }
-  k_adv_walls<T><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b);
+  if (rest) k_adv_rest<T><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b);
+  if (walls) {
+    LsBatch w1 = b;
+    set_tiles(w1, 0);
+    k_adv_ghosts<T><<<w1.start[w1.n], kTile, 0, c.s>>>(c.P, w1, stage1, a, bb);
+  }
 }
-// one RK stage over the batch from its band list (launch_band_list first)
-void launch_adv_split(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
-                      const double* vu, const double* vv, const double* vw, long long need) {
+void launch_adv_band(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
+                     const double* vu, const double* vv, const double* vw, long long need, bool rest) {
   if (b.n == 0) return;
-  Scope sc_(c.prof, c.s, "adv_stage", 3);
-  BY_FORM(c, adv_split_launch<float>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need),
-          adv_split_launch<double>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need));
+  bool walls = false;
+  for (int q = 0; q < b.n; ++q) walls = walls || b.t[q].r.cz0 <= -2;
+  Scope sc_(c.prof, c.s, "adv_stage", 1 + (walls ? 1 : 0) + (rest ? 1 : 0));
+  BY_FORM(c, adv_band_launch<float>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need, rest, walls),
+          adv_band_launch<double>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need, rest, walls));
 }
-
 void launch_adv_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                       const double* vu, const double* vv, const double* vw) {
   if (b.n == 0) return;

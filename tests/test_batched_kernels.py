@@ -6,7 +6,7 @@ expressions per cell, so the fields have to be the same bits.
 import numpy as np
 import pytest
 
-from icls_gpu import FP32, FP64, HOUC5, Solver, init_drops, initial_velocity, make_config
+from icls_gpu import FP32, FP64, HOUC5, WENO5, Solver, init_drops, initial_velocity, make_config
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +80,32 @@ def test_segment_maps_equal_whole_sweeps(n, precision):
     rows.gfm4p()
     for name in ("miu", "p_x", "p_jump"):
         assert np.array_equal(plain.download(name), rows.download(name)), name
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32])
+@pytest.mark.parametrize("grid,scheme,drops", [((64, 48, 50), HOUC5, 3), ((96, 48, 40), WENO5, 3),
+                                               ((96, 48, 40), HOUC5, 3), ((32, 32, 32), HOUC5, 66)])
+def test_band_list_equals_columns(grid, scheme, drops, precision):
+    """The advection stages over the tube's list of band cells against the
+    column sweeps (ICLS_ADV=column): a drop across the seam, one whose region
+    holds the wall and ghost rows, spacings where a/3 + 2a/3 is and is not a,
+    reinitialisation and corrections in between, and more drops than one
+    batch holds."""
+    nx, ny, nz = grid
+    h = 1.0 / max(nx, ny)
+    cfg = make_config(itot=nx, jtot=ny, ktot=nz, lmax=drops, lx=nx * h, ly=ny * h, lz=nz * h, timestep=1e-3,
+                      rho2=10.0, miu2=10.0, Re=100.0, We=0.5, v_wall_lower=-1.0, v_wall_upper=1.0,
+                      ls_adv_space=scheme, reinit_step=2, inflate_step=3, mass_threshold=1e-9, mass_gain_one=1,
+                      precision=precision)
+    at = [((0.02, 0.4, 0.55), 11.0), ((0.5, 0.3, 0.2), 7.0), ((0.6, 0.75, 0.6), 8.0)]
+    at = [at[l % 3] for l in range(drops)]
+    ls = init_drops(cfg, [(x * cfg.lx, y * cfg.ly, z * cfg.lz) for (x, y, z), _ in at],
+                    [r * h * (nx / 64 if drops > 3 else 1.0) for _, r in at], all_images=True)
+    lists = run_steps(cfg, ls, 5)
+    cols = run_steps(cfg, ls, 5, ICLS_ADV="column")
+    for l in list(range(1, min(drops, 3) + 1)) + [drops]:
+        assert np.array_equal(lists.download("lvset", l), cols.download("lvset", l)), l
+        assert lists.band_count(l) == cols.band_count(l)
+    for name in ("u", "v", "w", "pnew", "jiemian", "curv"):
+        assert np.array_equal(lists.download(name), cols.download(name)), name
+    assert np.array_equal(lists.volumes()[0], cols.volumes()[0])
