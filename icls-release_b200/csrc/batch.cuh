@@ -72,6 +72,40 @@ __device__ __forceinline__ bool computed(const Col& c, const Region& r, int k) {
   return c.cxy && k >= r.cz0 && k <= r.cz1;
 }
 
+// A block's queue of cells of its chunk (at most kQueueRows rows of 256
+// columns): a sweep pushes the few cells that need real work, and the block
+// works them off with full warps after a barrier.
+constexpr int kQueueRows = 16;
+struct CellQueue {
+  uint16_t cell[kQueueRows * TBX * TBY];
+  uint16_t ci[TBX * TBY], cj[TBX * TBY];
+  int n;
+};
+__device__ __forceinline__ void queue_init(CellQueue& q, const Col& c) {
+  const int tid = flat_tid();
+  if (tid == 0) q.n = 0;
+  q.ci[tid] = (uint16_t)c.i;
+  q.cj[tid] = (uint16_t)c.j;
+  __syncthreads();
+}
+// every lane of a warp calls this, with its row of the chunk
+__device__ __forceinline__ void queue_push(CellQueue& q, bool take, int row) {
+  const unsigned m = __ballot_sync(0xffffffffu, take);
+  if (!m) return;
+  const int tid = flat_tid(), lane = tid & 31;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(&q.n, __popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+  if (take) q.cell[at] = (uint16_t)((row << 8) | tid);
+}
+// cell e of the queue, of a chunk that starts at row ka
+__device__ __forceinline__ void queue_cell(const CellQueue& q, int e, int ka, int& i, int& j, int& k) {
+  const int v = q.cell[e];
+  i = q.ci[v & 255];
+  j = q.cj[v & 255];
+  k = ka + (v >> 8);
+}
+
 // the halo copy of column i in an array with H halo layers, INT_MIN if none
 template <int H>
 __device__ __forceinline__ int image_of(int i, int n) {

@@ -519,6 +519,8 @@ constexpr int kStageRows = 8;  // z rows per block of the level-set stage kernel
 // written by the thread that holds rows 1 and 2 (measured: 8 rows beat 4
 // and 16)
 static_assert(kStageRows >= 5, "level-set chunks must span rows -2..2");
+// and a chunk of up to 2 kStageRows - 1 rows fits a block's queue (batch.cuh)
+static_assert(2 * kStageRows - 1 <= 16, "a chunk's cells must fit the queue");
 
 Ctx::Member& member(Ctx& c, int l) { return c.mem[l % (int)c.mem.size()]; }
 
@@ -1126,26 +1128,17 @@ int gfm4p(Ctx& c) {
       for (int q = 0; q < b.n; ++q) {
         LsTask& t = b.t[q];
         t.phi0 = c.lv[t.l];
-        t.out = c.cfg.TwoD ? member(c, t.l).cv : member(c, t.l).fit;
+        t.out = member(c, t.l).fit;
       }
       const bool mlp = c.cfg.curvature_model == ICLS_CURV_MLP;
       launch_curvature(c, b, nullptr, mlp);
       if (mlp) launch_mlp_curvature(c, b);
     }
-    if (!c.cfg.TwoD)
-      for (LsBatch& b : b1) {
-        for (int q = 0; q < b.n; ++q) {
-          LsTask& t = b.t[q];
-          t.phis = member(c, t.l).fit;
-          t.out = member(c, t.l).cv;
-        }
-        launch_recurvature(c, b);
-      }
     for (LsBatch& b : b0) {
       for (int q = 0; q < b.n; ++q) {
         LsTask& t = b.t[q];
         t.phi0 = c.lv[t.l];
-        t.phis = member(c, t.l).cv;
+        t.phis = member(c, t.l).fit;
       }
       launch_jumps(c, b);
     }

@@ -715,7 +715,6 @@ __device__ __forceinline__ T reinit_val(int stage, T f0, T fs, T dtau, T rhs) {
 // evaluated where they occurred 21 of 32 lanes took part (256^3 x 48 FP64
 // 1.11 -> 0.78 ms, FP32 0.44 -> 0.38 ms per stage; 96 x 192 x 100 with ten
 // drops, FP64 and a spacing that divides, 0.37 -> 0.21 ms).
-constexpr int kReinitRows = 16;  // most rows of a chunk
 template <typename T, int PW>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 4 : 3)) k_reinit_stage(Params p, const __grid_constant__ LsBatch B, int stage,
                                                         double dtau_, ReinitState* __restrict__ rs) {
@@ -730,21 +729,14 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 4 : 3)) k_reinit_stage(P
       for (int k = c.ka; k <= c.kb; ++k) putL(p, out, c.i, c.j, k, phi0[idxL(p, c.i, c.j, k)]);
     return;
   }
-  __shared__ uint16_t queue[kReinitRows * NT];
-  __shared__ uint16_t ci[NT], cj[NT];
-  __shared__ int nqueue;
-  const int tid = flat_tid();
-  if (tid == 0) nqueue = 0;
-  ci[tid] = (uint16_t)c.i;
-  cj[tid] = (uint16_t)c.j;
-  __syncthreads();
+  __shared__ CellQueue queue;
+  queue_init(queue, c);
   const T dtau = TC(dtau_);
   const T* phis = cT<T>(t.phis);
   const T* orig = cT<T>(t.orig);
   const int sy = p.nLx, sz = p.nLx * p.nLy;
   const int col = (int)idxL(p, c.ok ? c.i : 1, c.ok ? c.j : 1, 0);
   const T lim = TC(p.NB + p.dz);
-  const int lane = tid & 31;
   double r = 0.;
   for (int k = c.ka; k <= c.kb; ++k) {
     bool heavy = false;
@@ -775,17 +767,12 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 4 : 3)) k_reinit_stage(P
         }
       }
     }
-    const unsigned m = __ballot_sync(0xffffffffu, heavy);
-    if (m) {
-      int at = 0;
-      if (lane == 0) at = atomicAdd(&nqueue, __popc(m));
-      at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-      if (heavy) queue[at] = (uint16_t)(((k - c.ka) << 8) | tid);
-    }
+    queue_push(queue, heavy, k - c.ka);
   }
   __syncthreads();
-  for (int e = tid; e < nqueue; e += NT) {
-    const int q = queue[e], i = ci[q & 255], j = cj[q & 255], k = c.ka + (q >> 8);
+  for (int e = flat_tid(); e < queue.n; e += NT) {
+    int i, j, k;
+    queue_cell(queue, e, c.ka, i, j, k);
     const int n = (int)idxL(p, i, j, k);
     const T f0 = phi0[n];
     const T rhs = reinit_rhs<PW>(p, phis, reinit_sgn(p, orig[n]), n, k);
