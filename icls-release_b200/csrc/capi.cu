@@ -142,6 +142,7 @@ void fill_params(Ctx& c) {
   P.NB = 6. * P.dz;
   P.pi = std::acos(-1.);
   P.dt = f.timestep;
+  P.cdx = P.dt * P.dxi; P.cdy = P.dt * P.dyi; P.cdz = P.dt * P.dzi;
   P.rho1 = f.rho1; P.rho2 = f.rho2; P.miu1 = f.miu1; P.miu2 = f.miu2;
   P.rho0 = std::min(f.rho1, f.rho2);  // param.f90:63
   P.rrho0 = 1. / P.rho0;

@@ -31,6 +31,7 @@ struct Params {
   double pi;
   double dt;
   double rho1, rho2, miu1, miu2, rho0, visc, iFr, nondi;
+  double cdx, cdy, cdz;      // dt dxi, dt dyi, dt dzi (correc's first products)
   double rrho0;              // 1./rho0, the IEEE quotient the reference evaluates per cell
   int rho0_pow2;             // rho0 is a power of two: x / rho0 == x * rrho0 exactly
   double g1, g2, g3;

@@ -175,87 +175,103 @@ __global__ void __launch_bounds__(NT) k_correc_fused(Params p, CorrArgs a) {
   }
 }
 
-// One correc value (correc.f90:27-39) at shape-C index c: d - dt dhi
-// ((p(c+off) - p(c)) - jump) / rho0, the expression of corr_u/v/w, with
-// the division by rho0 chosen at compile time (RP 1: rho0 a power of two,
-// the product by its exact reciprocal)
+// One correc value (correc.f90:27-39), d - dt dhi ((p+ - p) - jump) / rho0:
+// the expression of corr_u/v/w with cd = dt dhi (the reference's first
+// product) and the division by rho0 chosen at compile time (RP 1: rho0 a power
+// of two, the product by its exact reciprocal)
 template <typename T, int RP>
-__device__ __forceinline__ T corr_at(const Params& p, const T* __restrict__ d, const double* __restrict__ pp,
-                                     T jump, long long c, long long off, double dhi) {
-  const double a = p.dt * dhi * ((pp[c + off] - pp[c]) - (double)jump);
+__device__ __forceinline__ T corr_val(const Params& p, T d, double pp, double p0, T jump, double cd) {
+  const double a = cd * ((pp - p0) - (double)jump);
   const double g = RP == 1 ? a * p.rrho0 : a / p.rho0;
-  if (sizeof(T) == sizeof(double)) return (T)((double)d[c] - g);
-  return d[c] - (T)g;
+  if (sizeof(T) == sizeof(double)) return (T)((double)d - g);
+  return d - (T)g;
 }
 
 // k_correc_fused's fields with one thread per interior cell: the thread
-// writes its cell's u, v, w with their periodic images (putC), at k = 1 and
+// writes its cell's u, v, w with their periodic images, at k = 1 and
 // k = kmax the wall rows k = 0 and k1 with theirs, and the cell-centre
 // velocities.  The halo and wall cells are the images k_correc_fused
 // computes from the same source cells, so the fields are the same bits;
 // every warp is a full row segment and no thread recomputes a source
 // column's corrections for a halo cell.  The face jumps are read where the
 // segment map says that they can be nonzero (a warp is one segment of a row);
-// at 256^3 with 48 drops that leaves 10 of the 13 fields: FP64 0.378 -> 0.300 ms, FP32
-// 0.260 -> 0.241 ms.
+// at 256^3 with 48 drops that leaves 10 of the 13 fields.  The pressure of the
+// cell serves its west, south and lower neighbours' corrections (its images
+// are the same value).  Instruction issue bounds the FP32 form (77 % busy), so
+// indices are 32-bit (an array has less than 2^30 elements) and the images'
+// tests are made once per thread: with the map, FP64 0.373 -> 0.293 ms and
+// FP32 0.257 -> 0.232 ms; 128 x 128 x 256 FP64 with a rho0 that divides 0.126 ->
+// 0.093 ms.
 template <typename T, int RP>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 8 : 5)) k_correc_own(Params p, CorrArgs a) {
-  int i, j, k;
-  if (!cell3(kI0, cI1(p).v, i, j, k)) return;
-  const long long sy = p.nCx, sz = (long long)p.nCx * p.nCy;
-  const long long c = idxC(p, i, j, k);
+  const int i = 1 + BX * (int)blockIdx.x + (int)threadIdx.x, j = 1 + BY * (int)blockIdx.y + (int)threadIdx.y;
+  const int k = 1 + (int)blockIdx.z;
+  if (i > p.imax || j > p.jmax) return;
+  const int sy = p.nCx, sz = p.nCx * p.nCy;
+  const int c = i + sy * j + sz * k;
+  const int cx = i > 1 ? c - 1 : c + p.imax - 1, cy = j > 1 ? c - sy : c + sy * (p.jmax - 1), cz = c - sz;
   const T* __restrict__ du = cT<T>(a.dudt);
   const T* __restrict__ dv = cT<T>(a.dvdt);
   const T* __restrict__ dw = cT<T>(a.dwdt);
-  const T* __restrict__ px = cT<T>(a.px);
-  const T* __restrict__ py = cT<T>(a.py);
-  const T* __restrict__ pz = cT<T>(a.pz);
   const double* __restrict__ pp = a.p;
-  // the cell-centre average's (i-1), (j-1) and (k-1) corrections
-  const long long cx = idxC(p, wrapx(p, i - 1), j, k), cy = idxC(p, i, wrapy(p, j - 1), k);
+  const int nsx = seg_row(p), sp = nsx * p.jmax;
+  const uint8_t* __restrict__ seg = a.seg + ((int)blockIdx.x + nsx * (j - 1) + sp * k);
+  const uint8_t own = seg[0], west = seg[blockIdx.x ? -1 : nsx - 1];
+  const uint8_t south = seg[j > 1 ? -nsx : sp - nsx], below = seg[-sp];
+  const double p0 = pp[c];
+  const double pe = pp[c + 1], pn = pp[c + sy], pu = pp[c + sz], pw = pp[cx], ps = pp[cy], pd = pp[cz];
+  const T d0 = du[c], d1 = dv[c], d2 = dw[c], e0 = du[cx], e1 = dv[cy], e2 = dw[cz];
   T qx = TC(0.), qy = TC(0.), qz = TC(0.), qxm = TC(0.), qym = TC(0.), qzm = TC(0.);
-  {
-    const int nsx = seg_row(p);
-    const long long q = seg_of(p, i, j, k);
-    const uint8_t own = a.seg[q], west = a.seg[blockIdx.x ? q - 1 : q + nsx - 1];
-    const uint8_t south = a.seg[j > 1 ? q - nsx : q + (long long)nsx * (p.jmax - 1)];
-    const uint8_t below = a.seg[q - (long long)nsx * p.jmax];
-    if (own) {
-      qx = px[c];
-      qy = py[c];
-      qz = pz[c];
-    }
-    if (own | west) qxm = px[cx];
-    if (south) qym = py[cy];
-    if (below) qzm = pz[c - sz];
+  if (own) {
+    qx = cT<T>(a.px)[c];
+    qy = cT<T>(a.py)[c];
+    qz = cT<T>(a.pz)[c];
   }
-  const T uu = corr_at<T, RP>(p, du, pp, qx, c, 1, p.dxi);
-  const T vv = corr_at<T, RP>(p, dv, pp, qy, c, sy, p.dyi);
-  const T ww = (k == p.kmax) ? TC(0.) : corr_at<T, RP>(p, dw, pp, qz, c, sz, p.dzi);
-  const T um = corr_at<T, RP>(p, du, pp, qxm, cx, 1, p.dxi);
-  const T vm = corr_at<T, RP>(p, dv, pp, qym, cy, sy, p.dyi);
-  const T wl = corr_at<T, RP>(p, dw, pp, qzm, c - sz, sz, p.dzi);
-  const T wm = (k == 1) ? TC(0.) : wl;
-  T* u = mT<T>(a.u);
-  T* v = mT<T>(a.v);
-  T* w = mT<T>(a.w);
-  putC(p, u, i, j, k, uu);
-  putC(p, v, i, j, k, vv);
-  putC(p, w, i, j, k, ww);
-  if (k == 1) {
-    putC(p, u, i, j, 0, -uu);
-    putC(p, v, i, j, 0, TC(2. * p.v_lower) - vv);
-    putC(p, w, i, j, 0, TC(0.));
-  }
-  if (k == p.kmax) {
-    putC(p, u, i, j, p.k1, -uu);
-    putC(p, v, i, j, p.k1, TC(2. * p.v_upper) - vv);
-    putC(p, w, i, j, p.k1, wl);
-  }
-  const long long q = idxI(p, i, j, k);
+  if (own | west) qxm = cT<T>(a.px)[cx];
+  if (south) qym = cT<T>(a.py)[cy];
+  if (below) qzm = cT<T>(a.pz)[cz];
+  const T uu = corr_val<T, RP>(p, d0, pe, p0, qx, p.cdx);
+  const T vv = corr_val<T, RP>(p, d1, pn, p0, qy, p.cdy);
+  const T ww = (k == p.kmax) ? TC(0.) : corr_val<T, RP>(p, d2, pu, p0, qz, p.cdz);
+  // the cell-centre average's (i-1), (j-1) and (k-1) corrections
+  const T um = corr_val<T, RP>(p, e0, p0, pw, qxm, p.cdx);
+  const T vm = corr_val<T, RP>(p, e1, p0, ps, qym, p.cdy);
+  const T wl = corr_val<T, RP>(p, e2, p0, pd, qzm, p.cdz);
+  T* __restrict__ u = mT<T>(a.u);
+  T* __restrict__ v = mT<T>(a.v);
+  T* __restrict__ w = mT<T>(a.w);
+  const int q = (i - 1) + p.imax * ((j - 1) + p.jmax * (k - 1));
+  u[c] = uu;
+  v[c] = vv;
+  w[c] = ww;
   mT<T>(a.ucc)[q] = (um + uu) / TC(2.);
   mT<T>(a.vcc)[q] = (vm + vv) / TC(2.);
-  mT<T>(a.wcc)[q] = (wm + ww) / TC(2.);
+  mT<T>(a.wcc)[q] = (((k == 1) ? TC(0.) : wl) + ww) / TC(2.);
+  const bool ex = i == 1 || i == p.imax, ey = j == 1 || j == p.jmax;
+  if (!(ex | ey | (k == 1) | (k == p.kmax))) return;
+  // images and wall rows
+  const int di = ex ? (i == 1 ? p.imax : -p.imax) : 0, dj = ey ? sy * (j == 1 ? p.jmax : -p.jmax) : 0;
+  auto put = [&](T* __restrict__ f, int n, T x) {
+    f[n] = x;
+    if (di) f[n + di] = x;
+    if (dj) {
+      f[n + dj] = x;
+      if (di) f[n + di + dj] = x;
+    }
+  };
+  put(u, c, uu);
+  put(v, c, vv);
+  put(w, c, ww);
+  if (k == 1) {
+    put(u, c - sz, -uu);
+    put(v, c - sz, TC(2. * p.v_lower) - vv);
+    put(w, c - sz, TC(0.));
+  }
+  if (k == p.kmax) {
+    put(u, c + sz, -uu);
+    put(v, c + sz, TC(2. * p.v_upper) - vv);
+    put(w, c + sz, wl);
+  }
   if (i == 1 && j == 1 && k == 1 && isnan(vv)) a.dsc->nan_flag = 1;
 }
 
