@@ -20,6 +20,9 @@ struct MomArgs {
   const double *duold, *dvold, *dwold;
   const double *pnew, *pold, *px, *py, *pz, *pxold, *pyold, *pzold;
   const double* rho_avr;
+  // far rows (k_ab2): one byte per tile and row, and nonzero where a pressure is not finite
+  const uint8_t* near;
+  const int* p_bad;
 };
 
 namespace {
@@ -32,10 +35,10 @@ namespace {
 // U(di,dj,dk) returns u at (i+di, j+dj, k+dk), likewise V, W and M (miu):
 // the same expressions serve the shared-memory march of k_ab2 and the
 // global-memory k_mom_main.  T is the form's field type; TC(x) the
-// constant x in T.
-template <typename T, int PW = -1, class FU, class FV, class FW, class FM>
+// constant x in T.  by_rho(x) is x over the component's face density.
+template <typename T, int PW = -1, class FU, class FV, class FW, class FM, class FD>
 __device__ __forceinline__ T rhs_u(const Params& p, const FU& U, const FV& V, const FW& W, const FM& M,
-                                        T rho_u, T rho_avr) {
+                                   const FD& by_rho, T rho_avr) {
   T RCu = TC(0.);
   if (!p.TwoD) {
     T uuip = TC(0.25) * (U(1, 0, 0) + U(0, 0, 0)) * (U(1, 0, 0) + U(0, 0, 0));
@@ -67,19 +70,19 @@ __device__ __forceinline__ T rhs_u(const Params& p, const FU& U, const FV& V, co
     T RD3 = divy<PW>(p, (dvdxp * ma2 - dvdxm * ma1));
     T RD4 = divz<PW>(p, (dudzp * ma4 - dudzm * ma3));
     T RD5 = divz<PW>(p, (dwdxp * ma4 - dwdxm * ma3));
-    RDu = ((((RD1 + RD2) + RD3) + RD4) + RD5) / rho_u;
+    RDu = by_rho((((RD1 + RD2) + RD3) + RD4) + RD5);
   }
   // buoyancy iFr (1 - rho_avr/rho) g: skipped (with its divide) where iFr or
   // this component of g is zero; the term is then an exact +-0, which
   // changes the sum at most in the sign of an exactly zero result
   if (p.TwoD || p.iFr == 0. || p.g1 == 0.) return RCu + RDu * TC(p.visc);
-  T RGu = TC(p.iFr) * (TC(1.) - rho_avr / rho_u) * TC(p.g1);
+  T RGu = TC(p.iFr) * (TC(1.) - by_rho(rho_avr)) * TC(p.g1);
   return (RCu + RDu * TC(p.visc)) + RGu;
 }
 
-template <typename T, int PW = -1, class FU, class FV, class FW, class FM>
+template <typename T, int PW = -1, class FU, class FV, class FW, class FM, class FD>
 __device__ __forceinline__ T rhs_v(const Params& p, const FU& U, const FV& V, const FW& W, const FM& M,
-                                        T rv, T rho_avr) {
+                                   const FD& by_rho, T rho_avr) {
   T uvip = TC(0.25) * (U(0, 0, 0) + U(0, 1, 0)) * (V(0, 0, 0) + V(1, 0, 0));
   T uvim = TC(0.25) * (U(-1, 0, 0) + U(-1, 1, 0)) * (V(0, 0, 0) + V(-1, 0, 0));
   T vvjp = TC(0.25) * (V(0, 0, 0) + V(0, 1, 0)) * (V(0, 0, 0) + V(0, 1, 0));
@@ -106,15 +109,15 @@ __device__ __forceinline__ T rhs_v(const Params& p, const FU& U, const FV& V, co
   T RD3 = divy<PW>(p, TC(2.) * (dvdyp * M(0, 1, 0) - dvdym * M(0, 0, 0)));
   T RD4 = divz<PW>(p, (dvdzp * ma7 - dvdzm * ma6));
   T RD5 = divz<PW>(p, (dwdyp * ma7 - dwdym * ma6));
-  T RDv = ((((RD1 + RD2) + RD3) + RD4) + RD5) / rv;
+  T RDv = by_rho((((RD1 + RD2) + RD3) + RD4) + RD5);
   if (p.iFr == 0. || p.g2 == 0.) return RCv + RDv * TC(p.visc);  // buoyancy as in rhs_u
-  T RGv = TC(p.iFr) * (TC(1.) - rho_avr / rv) * TC(p.g2);
+  T RGv = TC(p.iFr) * (TC(1.) - by_rho(rho_avr)) * TC(p.g2);
   return (RCv + RDv * TC(p.visc)) + RGv;
 }
 
-template <typename T, int PW = -1, class FU, class FV, class FW, class FM>
+template <typename T, int PW = -1, class FU, class FV, class FW, class FM, class FD>
 __device__ __forceinline__ T rhs_w(const Params& p, const FU& U, const FV& V, const FW& W, const FM& M,
-                                        T rw, T rho_avr) {
+                                   const FD& by_rho, T rho_avr) {
   T uwip = TC(0.25) * (W(0, 0, 0) + W(1, 0, 0)) * (U(0, 0, 0) + U(0, 0, 1));
   T uwim = TC(0.25) * (W(0, 0, 0) + W(-1, 0, 0)) * (U(-1, 0, 0) + U(-1, 0, 1));
   T vwjp = TC(0.25) * (W(0, 0, 0) + W(0, 1, 0)) * (V(0, 0, 0) + V(0, 0, 1));
@@ -141,15 +144,15 @@ __device__ __forceinline__ T rhs_w(const Params& p, const FU& U, const FV& V, co
   T RD3 = divy<PW>(p, (dwdyp * ma7 - dwdym * ma9));
   T RD4 = divy<PW>(p, (dvdzp * ma7 - dvdzm * ma9));
   T RD5 = divz<PW>(p, TC(2.) * (dwdzp * M(0, 0, 1) - dwdzm * M(0, 0, 0)));
-  T RDw = ((((RD1 + RD2) + RD3) + RD4) + RD5) / rw;
+  T RDw = by_rho((((RD1 + RD2) + RD3) + RD4) + RD5);
   if (p.iFr == 0. || p.g3 == 0.) return RCw + RDw * TC(p.visc);  // buoyancy as in rhs_u
-  T RGw = TC(p.iFr) * (TC(1.) - rho_avr / rw) * TC(p.g3);
+  T RGw = TC(p.iFr) * (TC(1.) - by_rho(rho_avr)) * TC(p.g3);
   return (RCw + RDw * TC(p.visc)) + RGw;
 }
 
 // ---- the ab2 update of one component (ab2.f90:51-61, 79-129) -------------
-// u0 = u at the cell, R = its mom_main RHS, rold the previous RHS, rf its
-// face density, dhi the 1/dx of the component's axis; the pressure-split
+// u0 = u at the cell, R = its mom_main RHS, rold the previous RHS, irf one
+// over its face density, dhi the 1/dx of the component's axis; the pressure-split
 // term is formed in FP64 (the pressures are FP64 fields) from: ph_p / ph_0 the
 // extrapolated pressures 2 pnew - pold at the + neighbour and the cell,
 // pjh the extrapolated pressure gradient 2 p_x - p_x,old
@@ -157,10 +160,10 @@ __device__ __forceinline__ T rhs_w(const Params& p, const FU& U, const FV& V, co
 // form, whose pressures are stored in FP32, the term is formed in FP32 too
 // (it is part of the momentum predictor, which that form computes in FP32)
 template <typename T, typename PT>
-__device__ __forceinline__ T ab2_update_v(const Params& p, T u0, T R, T rold, T rf, PT ph_p, PT ph_0, PT pjh,
+__device__ __forceinline__ T ab2_update_v(const Params& p, T u0, T R, T rold, PT irf, PT ph_p, PT ph_0, PT pjh,
                                           double dhi) {
   T d = u0 + TC(p.dt) * (TC(1.5) * R - TC(0.5) * rold);
-  const PT dn = -((PT(1.) / (PT)rf - (PT)p.rrho0) * (PT)dhi * ((ph_p - pjh) - ph_0));
+  const PT dn = -((irf - (PT)p.rrho0) * (PT)dhi * ((ph_p - pjh) - ph_0));
   return d + TC((PT)p.dt * dn);
 }
 
@@ -196,147 +199,218 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // (the slot a row's copies fill is not one any thread can still be reading).
 // A thread writes its column's periodic halo images and, at k = 1 and
 // k = kmax, the wall rows k = 0 and k = k1.  Every plane row starts at
-// column i0 - 1 (even).
-constexpr int MX = 32, MY = 8, MSX = MX + 2, MSY = MY + 2, MPY = MY + 1, MRING = 4;
+// column i0 - 1 (even).  Indices are 32-bit: an array has less than 2^30
+// elements.
+//
+// FAR: rows that a byte per tile and row (k_ab2_near) says have no drop next
+// to them.  There the viscosity and the face densities are the carrier's and
+// the face jumps zero, so these ten of the 24 fields are not read, and the row
+// runs the same expressions with one viscosity and one density: the same
+// bits.  Where the carrier is the lighter phase the pressure-split factor
+// 1/rho1 - 1/rho0 is exactly zero too, and while every pressure is finite
+// (p_bad) its product is: the two pressures are not read either.  Nine tenths
+// of the rows are far at 256^3 with 48 drops.  FAR false: the fields were
+// written by a caller, every row is general.
+// The planes arrive one row ahead of their use, and so do the AB2 history
+// values; a near row's other operands are read at the row.  (Waiting for a
+// row's planes right after issuing them, the long-scoreboard and barrier
+// stalls were a third of the FP64 form's issue slots.)
+//
+// 256^3 with 48 drops: FP64 0.843 -> 0.626 ms, FP32 0.489 -> 0.357 ms; every row
+// general: FP64 0.842 -> 0.762 ms, 384 x 192 x 150 FP32 0.360 -> 0.283 ms.  FP64
+// takes two blocks per SM at 128 registers (three at 80: 0.660 and 0.808 ms),
+// FP32 four.  Two cells per thread (adjacent in y, sharing their stencil) were
+// slower in both forms (FP64 0.743, FP32 0.396): the registers they take cost
+// more warps than the shared loads save.
+constexpr int MX = kAb2X, MY = kAb2Y, MSX = MX + 2, MSY = MY + 2, MPY = MY + 1, MRING = 4;
+static_assert(MX == kSeg, "a tile is one segment wide");
 template <typename T>
 constexpr int ab2_smem() {
   return (int)(4 * MRING * MSY * MSX * sizeof(T) + 2 * MRING * MPY * MSX * sizeof(T));
 }
-template <typename T, int PW, int MB>
+template <typename T, int PW, int MB, bool FAR>
 __global__ void __launch_bounds__(MX * MY, MB)
     k_ab2(Params p, MomArgs a, T* __restrict__ dudt, T* __restrict__ dvdt, T* __restrict__ dwdt,
-          T* __restrict__ duold_out, T* __restrict__ dvold_out, T* __restrict__ dwold_out, int kc, int nch) {
+          T* __restrict__ duold_out, T* __restrict__ dvold_out, T* __restrict__ dwold_out, int kc) {
   extern __shared__ __align__(16) unsigned char ab2_dyn[];
+  typedef T PT;  // the pressure term's arithmetic
   typedef T Plane[MSY][MSX];
   typedef T PPlane[MPY][MSX];  // pnew, pold (columns i0-1.., rows j0..) in the form's field type
+  constexpr int NTH = MX * MY;
   Plane* ring = reinterpret_cast<Plane*>(ab2_dyn);  // [field * MRING + slot]
   PPlane* pring = reinterpret_cast<PPlane*>(ab2_dyn + 4 * MRING * sizeof(Plane));
   const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + MX * ty;
   const int i0 = 1 + MX * (int)blockIdx.x, j0 = 1 + MY * (int)blockIdx.y;
-  const int ch = blockIdx.z;
-  const int ka = 1 + ch * kc, kb = (ch == nch - 1) ? p.kmax : ka + kc - 1;
+  const int ka = 1 + (int)blockIdx.z * kc, kb = blockIdx.z == gridDim.z - 1 ? p.kmax : ka + kc - 1;
   const int i = i0 + tx, j = j0 + ty;
   const bool ok = i <= p.imax && j <= p.jmax;
-  const T* __restrict__ F[4] = {cT<T>(a.u), cT<T>(a.v), cT<T>(a.w), cT<T>(a.miu)};
-  const T* __restrict__ rhu = cT<T>(a.rho_u);
-  const T* __restrict__ rhv = cT<T>(a.rho_v);
-  const T* __restrict__ rhw = cT<T>(a.rho_w);
-  const T* __restrict__ hu = cT<T>(a.duold);
-  const T* __restrict__ hv = cT<T>(a.dvold);
-  const T* __restrict__ hw = cT<T>(a.dwold);
-  // FP64: imax is even (every FFT length validate() admits is), so the rows
-  // of shape C have an even length and each plane row's first element
-  // (column i0-1, even) sits at an even index: 16-byte pair copies are
-  // aligned, and halve the copy instructions (1.37 -> 1.30 ms at 256^3).
-  // FP32 keeps one 4-byte copy per element: at its 64-register budget the
-  // pair loop spilled and measured slower (0.77 -> 0.84 ms).
-  // This thread's copy slots, the same for every row: slot r is element
-  // tid + r MX MY of a plane (a pair of elements in FP64), at plane offset
-  // gi + nCx gj of storage row 0 (row kk is kk nCx nCy further), -1 where
-  // the element lies outside the grid.  NS slots cover a plane.
-  constexpr int EPC = sizeof(T) == 8 ? 2 : 1;  // elements per copy
-  constexpr int RW = MSX / EPC;                // copies per plane row
-  constexpr int NS = (RW * MSY + MX * MY - 1) / (MX * MY);
+  // imax is even (every FFT length validate() admits is), so the rows of
+  // shape C have an even length and each plane row's first element (column
+  // i0-1, even) sits at an even index: pair copies (8 bytes in FP32, 16 in
+  // FP64) are aligned.
+  // This thread's copy slots, the same for every row: slot r is the pair
+  // tid + r 256 of a plane, at plane offset gi + nCx gj of storage row 0 (row
+  // kk is kk nCx nCy further), -1 where it lies outside the grid.
+  constexpr int RW = MSX / 2;  // copies per plane row
+  constexpr int NS = (RW * MSY + NTH - 1) / NTH;
   int ro[NS], po[NS];
 #pragma unroll
   for (int r = 0; r < NS; ++r) {
-    const int e = tid + r * MX * MY;
-    const int sy = e / RW, sx = EPC * (e - sy * RW);
-    const int gi = i0 - 1 + sx;
-    // gi even in FP64: gi + 1 <= imax + 1
-    const bool xin = sizeof(T) == 8 ? gi <= p.imax : gi <= p.imax + 1;
-    ro[r] = (e < RW * MSY && xin && j0 - 1 + sy <= p.jmax + 1) ? gi + p.nCx * (j0 - 1 + sy) : -1;
-    // pnew, pold rows start at j0; their column i0-1 is not read (FP32
-    // skips it, FP64 copies it with its pair)
-    po[r] = (e < RW * MPY && xin && j0 + sy <= p.jmax + 1 && (sizeof(T) == 8 || sx > 0)) ? gi + p.nCx * (j0 + sy)
-                                                                                        : -1;
+    const int e = tid + r * NTH;
+    const int sy = e / RW, gi = i0 - 1 + 2 * (e - sy * RW);
+    // gi even: gi + 1 <= imax + 1
+    ro[r] = (e < RW * MSY && gi <= p.imax && j0 - 1 + sy <= p.jmax + 1) ? gi + p.nCx * (j0 - 1 + sy) : -1;
+    // pnew, pold rows start at j0
+    po[r] = (e < RW * MPY && gi <= p.imax && j0 + sy <= p.jmax + 1) ? gi + p.nCx * (j0 + sy) : -1;
   }
-  const long long psz = (long long)p.nCx * p.nCy;
-  auto issue_plane = [&](int kk) {
-    const int s = kk & (MRING - 1);
-    const long long kb = (long long)kk * psz;
+  const int psz = p.nCx * p.nCy;
+  const T* __restrict__ fu = cT<T>(a.u);
+  const T* __restrict__ fv = cT<T>(a.v);
+  const T* __restrict__ fw = cT<T>(a.w);
+  auto issue_uvw = [&](int kk) {
+    const int s = kk & (MRING - 1), o = kk * psz;
 #pragma unroll
-    for (int r = 0; r < NS; ++r) {
-      const int e = EPC * (tid + r * MX * MY);  // element offset in the plane
+    for (int r = 0; r < NS; ++r)
       if (ro[r] >= 0) {
-        const long long g = kb + ro[r];
+        const int g = o + ro[r], e = 2 * (tid + r * NTH);
+        cp_async_pair(&ring[0 * MRING + s][0][0] + e, fu + g);
+        cp_async_pair(&ring[1 * MRING + s][0][0] + e, fv + g);
+        cp_async_pair(&ring[2 * MRING + s][0][0] + e, fw + g);
+      }
+  };
+  auto issue_miu = [&](int kk) {
+    const int s = kk & (MRING - 1), o = kk * psz;
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          T* dst = &ring[f * MRING + s][0][0] + e;
-          if constexpr (sizeof(T) == 8) cp_async_pair(dst, F[f] + g);
-          else cp_async_el(dst, F[f] + g);
-        }
-      }
+    for (int r = 0; r < NS; ++r)
+      if (ro[r] >= 0) cp_async_pair(&ring[3 * MRING + s][0][0] + 2 * (tid + r * NTH), cT<T>(a.miu) + (o + ro[r]));
+  };
+  auto issue_p = [&](int kk) {
+    const int s = kk & (MRING - 1), o = kk * psz;
+#pragma unroll
+    for (int r = 0; r < NS; ++r)
       if (po[r] >= 0) {
-        const long long g = kb + po[r];
-        T* d0 = &pring[s][0][0] + e;
-        T* d1 = &pring[MRING + s][0][0] + e;
-        if constexpr (sizeof(T) == 8) {
-          cp_async_pair(d0, cT<T>(a.pnew) + g);
-          cp_async_pair(d1, cT<T>(a.pold) + g);
-        } else {
-          cp_async_el(d0, cT<T>(a.pnew) + g);
-          cp_async_el(d1, cT<T>(a.pold) + g);
-        }
+        const int g = o + po[r], e = 2 * (tid + r * NTH);
+        cp_async_pair(&pring[s][0][0] + e, cT<T>(a.pnew) + g);
+        cp_async_pair(&pring[MRING + s][0][0] + e, cT<T>(a.pold) + g);
       }
+  };
+  const T rho1 = TC(p.rho1), miu1 = TC(p.miu1), rrho1 = TC(p.rrho1);
+  const PT irho1 = PT(1.) / (PT)rho1;
+  __shared__ uint8_t near_row[kAb2Rows + 2];  // [1 + r] row ka + r; 0 before the first and after the last
+  bool noP = false;
+  if constexpr (FAR) {
+    noP = *a.p_bad == 0 && irho1 - (PT)p.rrho0 == PT(0.);
+    const uint8_t* near = a.near + ((long long)blockIdx.x + (long long)gridDim.x * blockIdx.y) * p.nCz + ka;
+    if (tid < kAb2Rows + 2) near_row[tid] = (tid >= 1 && tid <= kb - ka + 1) ? near[tid - 1] : 0;
+  }
+  // row kk of the viscosity is read by the near rows among kk-1..kk+1, of
+  // the pressures by rows kk-1 and kk
+  auto near_at = [&](int k) -> bool { return !FAR || near_row[1 + k - ka]; };
+  auto issue_rest = [&](int kk) {
+    const bool lo = kk > ka && near_at(kk - 1), at = kk >= ka && kk <= kb && near_at(kk);
+    if (lo || at || (kk < kb && near_at(kk + 1))) issue_miu(kk);
+    if (!noP || lo || at) issue_p(kk);
+  };
+  issue_uvw(ka - 1);
+  issue_uvw(ka);
+  issue_uvw(ka + 1);
+  if constexpr (FAR) __syncthreads();
+  issue_rest(ka - 1);
+  issue_rest(ka);
+  issue_rest(ka + 1);
+  const T rho_avr = TC(*a.rho_avr);
+  // the thread's column in the arrays, and its periodic images
+  const int cc0 = i + p.nCx * j, q0 = (i - 1) + p.imax * (j - 1), szI = p.imax * p.jmax;
+  const int di = i == 1 ? p.imax : (i == p.imax ? -p.imax : 0);
+  const int dj = j == 1 ? p.nCx * p.jmax : (j == p.jmax ? -p.nCx * p.jmax : 0);
+  auto put = [&](T* __restrict__ f, int c, T v) {
+    f[c] = v;
+    if (di) f[c + di] = v;
+    if (dj) {
+      f[c + dj] = v;
+      if (di) f[c + di + dj] = v;
     }
   };
-  issue_plane(ka - 1);
-  issue_plane(ka);
-  const T rho_avr = TC(*a.rho_avr);
-  T dw_km1 = TC(0.);
+  T dw_km1 = TC(0.), ou = TC(0.), ov = TC(0.), ow = TC(0.);
+  auto history = [&](int k) {
+    if (!ok) return;
+    const int q = q0 + (k - 1) * szI;
+    ou = cT<T>(a.duold)[q];
+    ov = cT<T>(a.dvold)[q];
+    ow = cT<T>(a.dwold)[q];
+  };
+  history(ka);
   for (int k = ka; k <= kb; ++k) {
-    // this cell's own operands, in flight together with row k+1's planes
-    T ru = TC(1.), rv = TC(1.), rw = TC(1.), ou = TC(0.), ov = TC(0.), ow = TC(0.);
-    typedef typename std::conditional<sizeof(T) == 8, double, float>::type PT;
-    PT qx = 0., qxo = 0., qy = 0., qyo = 0., qz = 0., qzo = 0.;
-    const long long c = idxC(p, i, j, k), q = idxI(p, i, j, k);
-    if (ok) {
-      ru = rhu[q]; rv = rhv[q]; rw = rhw[q];
-      ou = hu[q]; ov = hv[q]; ow = hw[q];
-      qx = (PT)cT<T>(a.px)[c]; qxo = (PT)cT<T>(a.pxold)[c];
-      qy = (PT)cT<T>(a.py)[c]; qyo = (PT)cT<T>(a.pyold)[c];
-      qz = (PT)cT<T>(a.pz)[c]; qzo = (PT)cT<T>(a.pzold)[c];
+    const bool near = near_at(k);
+    const int c = cc0 + k * psz, q = q0 + (k - 1) * szI;
+    T ru = rho1, rv = rho1, rw = rho1;
+    PT jx = PT(0.), jy = PT(0.), jz = PT(0.);
+    if (near && ok) {  // the near row's own operands
+      ru = cT<T>(a.rho_u)[q]; rv = cT<T>(a.rho_v)[q]; rw = cT<T>(a.rho_w)[q];
+      jx = PT(2.) * cT<T>(a.px)[c] - cT<T>(a.pxold)[c];
+      jy = PT(2.) * cT<T>(a.py)[c] - cT<T>(a.pyold)[c];
+      jz = PT(2.) * cT<T>(a.pz)[c] - cT<T>(a.pzold)[c];
     }
-    issue_plane(k + 1);
-    cp_async_wait_all();
-    __syncthreads();
-    if (ok) {
-      const int s_m = (k - 1) & (MRING - 1), s_0 = k & (MRING - 1), s_p = (k + 1) & (MRING - 1);
-      auto sl = [&](int dk) { return dk < 0 ? s_m : (dk > 0 ? s_p : s_0); };
-      auto U = [&](int di, int dj, int dk) { return ring[0 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
-      auto V = [&](int di, int dj, int dk) { return ring[1 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
-      auto W = [&](int di, int dj, int dk) { return ring[2 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
-      auto M = [&](int di, int dj, int dk) { return ring[3 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
-      auto PH = [&](int di, int dj, int dk) {
-        return PT(2.) * (PT)pring[sl(dk)][ty + dj][tx + 1 + di] - (PT)pring[MRING + sl(dk)][ty + dj][tx + 1 + di];
-      };
+    cp_async_wait_all();  // row k+1's planes, issued a row ago
+    __syncthreads();      // everyone's; and everyone is done with the slot of row k-2
+    if (k < kb) {
+      issue_uvw(k + 2);
+      issue_rest(k + 2);
+    }
+    const int s_m = (k - 1) & (MRING - 1), s_0 = k & (MRING - 1), s_p = (k + 1) & (MRING - 1);
+    auto sl = [&](int dk) { return dk < 0 ? s_m : (dk > 0 ? s_p : s_0); };
+    auto U = [&](int di, int dj, int dk) { return ring[0 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
+    auto V = [&](int di, int dj, int dk) { return ring[1 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
+    auto W = [&](int di, int dj, int dk) { return ring[2 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
+    auto M = [&](int di, int dj, int dk) { return ring[3 * MRING + sl(dk)][ty + 1 + dj][tx + 1 + di]; };
+    auto PH = [&](int di, int dj, int dk) {
+      return PT(2.) * (PT)pring[sl(dk)][ty + dj][tx + 1 + di] - (PT)pring[MRING + sl(dk)][ty + dj][tx + 1 + di];
+    };
+    T Ru, Rv, Rw, du, dv, dw;
+    if (near) {
+      Ru = rhs_u<T, PW>(p, U, V, W, M, [&](T x) { return x / ru; }, rho_avr);
+      Rv = rhs_v<T, PW>(p, U, V, W, M, [&](T x) { return x / rv; }, rho_avr);
+      Rw = rhs_w<T, PW>(p, U, V, W, M, [&](T x) { return x / rw; }, rho_avr);
+    } else {
+      auto M1 = [&](int, int, int) { return miu1; };
+      // a power-of-two density: the product by its reciprocal is the quotient
+      auto by_rho = [&](T x) { return p.rho1_pow2 ? x * rrho1 : x / rho1; };
+      Ru = rhs_u<T, PW>(p, U, V, W, M1, by_rho, rho_avr);
+      Rv = rhs_v<T, PW>(p, U, V, W, M1, by_rho, rho_avr);
+      Rw = rhs_w<T, PW>(p, U, V, W, M1, by_rho, rho_avr);
+    }
+    if (near || !noP) {
       const PT ph0 = PH(0, 0, 0);
-      const T Ru = rhs_u<T, PW>(p, U, V, W, M, ru, rho_avr);
-      const T Rv = rhs_v<T, PW>(p, U, V, W, M, rv, rho_avr);
-      const T Rw = rhs_w<T, PW>(p, U, V, W, M, rw, rho_avr);
-      const T du = ab2_update_v<T, PT>(p, U(0, 0, 0), Ru, ou, ru, PH(1, 0, 0), ph0, PT(2.) * qx - qxo, p.dxi);
-      T dv = ab2_update_v<T, PT>(p, V(0, 0, 0), Rv, ov, rv, PH(0, 1, 0), ph0, PT(2.) * qy - qyo, p.dyi);
-      if (p.forceytot != 0.) dv = dv - TC(p.forceytot * p.dt) / rv;  // constPoi driving (exact zero otherwise)
-      T dw = ab2_update_v<T, PT>(p, W(0, 0, 0), Rw, ow, rw, PH(0, 0, 1), ph0, PT(2.) * qz - qzo, p.dzi);
-      duold_out[q] = Ru;
-      dvold_out[q] = Rv;
-      dwold_out[q] = Rw;
-      if (k == p.kmax - 1) dw_km1 = dw;
-      if (k == p.kmax) dw = TC(0.);
-      putC(p, dudt, i, j, k, du);
-      putC(p, dvdt, i, j, k, dv);
-      putC(p, dwdt, i, j, k, dw);
-      if (k == 1) {
-        putC(p, dudt, i, j, 0, -du);
-        putC(p, dvdt, i, j, 0, TC(2. * p.v_lower) - dv);
-        putC(p, dwdt, i, j, 0, TC(0.));
-      }
-      if (k == p.kmax) {
-        putC(p, dudt, i, j, p.k1, -du);
-        putC(p, dvdt, i, j, p.k1, TC(2. * p.v_upper) - dv);
-        putC(p, dwdt, i, j, p.k1, dw_km1);
-      }
+      const PT iu = near ? PT(1.) / (PT)ru : irho1, iv = near ? PT(1.) / (PT)rv : irho1,
+               iw = near ? PT(1.) / (PT)rw : irho1;
+      du = ab2_update_v<T, PT>(p, U(0, 0, 0), Ru, ou, iu, PH(1, 0, 0), ph0, jx, p.dxi);
+      dv = ab2_update_v<T, PT>(p, V(0, 0, 0), Rv, ov, iv, PH(0, 1, 0), ph0, jy, p.dyi);
+      dw = ab2_update_v<T, PT>(p, W(0, 0, 0), Rw, ow, iw, PH(0, 0, 1), ph0, jz, p.dzi);
+    } else {
+      du = U(0, 0, 0) + TC(p.dt) * (TC(1.5) * Ru - TC(0.5) * ou);
+      dv = V(0, 0, 0) + TC(p.dt) * (TC(1.5) * Rv - TC(0.5) * ov);
+      dw = W(0, 0, 0) + TC(p.dt) * (TC(1.5) * Rw - TC(0.5) * ow);
+    }
+    if (p.forceytot != 0.) dv = dv - TC(p.forceytot * p.dt) / rv;  // constPoi driving (exact zero otherwise)
+    if (k < kb) history(k + 1);
+    if (!ok) continue;
+    duold_out[q] = Ru;
+    dvold_out[q] = Rv;
+    dwold_out[q] = Rw;
+    if (k == p.kmax - 1) dw_km1 = dw;
+    if (k == p.kmax) dw = TC(0.);
+    put(dudt, c, du);
+    put(dvdt, c, dv);
+    put(dwdt, c, dw);
+    if (k == 1) {
+      put(dudt, c - psz, -du);
+      put(dvdt, c - psz, TC(2. * p.v_lower) - dv);
+      put(dwdt, c - psz, TC(0.));
+    }
+    if (k == p.kmax) {
+      put(dudt, c + psz, -du);
+      put(dvdt, c + psz, TC(2. * p.v_upper) - dv);
+      put(dwdt, c + psz, dw_km1);
     }
   }
 }
@@ -344,35 +418,36 @@ __global__ void __launch_bounds__(MX * MY, MB)
 template <typename T>
 T* ab2_ptr(double* q) { return reinterpret_cast<T*>(q); }
 
-template <typename T, int PW, int MB>
-void ab2_launch_pw(Ctx& c, const MomArgs& a, int o) {
-  // rows per block: 32 for the FP32 form (four blocks per SM, shorter
-  // ring prologues), 16 for FP64 (three blocks per SM, more blocks per wave)
-  const int kc = sizeof(T) == 8 ? 16 : 32, nch = std::max(1, c.P.kmax / kc);
-  const dim3 grid((unsigned)((c.P.imax + MX - 1) / MX), (unsigned)((c.P.jmax + MY - 1) / MY), (unsigned)nch);
+template <typename T, int PW, int MB, bool FAR>
+void ab2_launch_far(Ctx& c, const MomArgs& a, int o) {
+  int kc;
+  const dim3 grid = ab2_grid(c.P, sizeof(T) == 8, kc);
   static unsigned attr = 0;  // devices this instance's shared-memory limit is raised on
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr & (1u << (dev & 31)))) {
-    cudaFuncSetAttribute(k_ab2<T, PW, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, ab2_smem<T>());
+    cudaFuncSetAttribute(k_ab2<T, PW, MB, FAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, ab2_smem<T>());
     attr |= 1u << (dev & 31);
   }
-  k_ab2<T, PW, MB><<<grid, dim3(MX, MY, 1), ab2_smem<T>(), c.s>>>(
+  k_ab2<T, PW, MB, FAR><<<grid, dim3(MX, MY, 1), ab2_smem<T>(), c.s>>>(
       c.P, a, ab2_ptr<T>(c.dudt), ab2_ptr<T>(c.dvdt), ab2_ptr<T>(c.dwdt), ab2_ptr<T>(c.duold[o]),
-      ab2_ptr<T>(c.dvold[o]), ab2_ptr<T>(c.dwold[o]), nch == 1 ? c.P.kmax : kc, nch);
+      ab2_ptr<T>(c.dvold[o]), ab2_ptr<T>(c.dwold[o]), kc);
+}
+template <typename T, int PW, int MB>
+void ab2_launch_pw(Ctx& c, const MomArgs& a, int o) {
+  if (a.near) ab2_launch_far<T, PW, MB, true>(c, a, o);
+  else ab2_launch_far<T, PW, MB, false>(c, a, o);
 }
 // one instance per spacing case: with power-of-two spacings every a/dx is
 // the product, so neither the test nor the division is in the kernel.  The
 // FP32 form, held to tolerances rather than to the reference's rounding,
 // always takes the product by the reciprocal (within an ulp of the quotient).
-// MB: blocks per SM the registers are budgeted for.  FP64 three (80
-// registers, a few spilled: 0.895 -> 0.840 ms at 256^3 against two blocks
-// at 120 registers); FP32 four (64 registers).
+// The instance's blocks per SM as measured (k_ab2).
 template <typename T>
 void ab2_launch(Ctx& c, const MomArgs& a, int o) {
   if constexpr (sizeof(T) == 8) {
-    if (c.P.pow2) ab2_launch_pw<T, 1, 3>(c, a, o);
-    else ab2_launch_pw<T, 0, 3>(c, a, o);
+    if (c.P.pow2) ab2_launch_pw<T, 1, 2>(c, a, o);
+    else ab2_launch_pw<T, 0, 2>(c, a, o);
   } else {
     ab2_launch_pw<T, 1, 4>(c, a, o);
   }

@@ -149,6 +149,8 @@ void fill_params(Ctx& c) {
   {
     int e2;
     P.rho0_pow2 = std::frexp(P.rho0, &e2) == 0.5 ? 1 : 0;
+    P.rrho1 = 1. / P.rho1;
+    P.rho1_pow2 = std::frexp(P.rho1, &e2) == 0.5 ? 1 : 0;
   }
   P.f32 = f.precision == ICLS_FP32 ? 1 : 0;
   P.visc = 1. / f.Re;                 // param.f90:73
@@ -221,6 +223,7 @@ int allocate(Ctx& c) {
   AL(c.partials, (size_t)kRedBlocks * std::max(P.L, 4) + (size_t)P.imax + 8);
   AL(c.diag, (size_t)7 * kRedBlocks + 8);
   AL(c.lpartials, (size_t)kRedBlocks);
+  AL(c.ab2_near, (size_t)seg_row(P) * ((P.jmax + kAb2Y - 1) / kAb2Y) * P.nCz);
   AL(c.dsc, 1);
   AL(c.dvol, (size_t)P.L); AL(c.dvol0, (size_t)P.L); AL(c.dmaxchk, (size_t)P.L);
   AL(c.dvolnow, (size_t)P.L);
@@ -317,7 +320,7 @@ void release(Ctx& c) {
     if (m.mask) cudaFree(m.mask);
   }
   if (c.d_nbcnt) cudaFree(c.d_nbcnt);
-  for (uint8_t* m : {c.seg_mat[0], c.seg_mat[1], c.seg_jmp[0], c.seg_jmp[1], c.row_jmp})
+  for (uint8_t* m : {c.seg_mat[0], c.seg_mat[1], c.seg_jmp[0], c.seg_jmp[1], c.row_jmp, c.ab2_near})
     if (m) cudaFree(m);
   if (c.twx) cudaFree(c.twx);
   if (c.twy) cudaFree(c.twy);
@@ -553,6 +556,9 @@ void field_written(Ctx& c, int id) {
       c.pjump_dirty = true;
       cudaMemsetAsync(c.seg_jmp[0], 1, n, c.s);
       cudaMemsetAsync(c.row_jmp, 1, (size_t)c.P.jmax * c.P.nCz, c.s);
+      break;
+    case ICLS_F_PNEW: case ICLS_F_POLD:
+      c.p_dirty = true;
       break;
     default:
       break;
@@ -1436,6 +1442,7 @@ int icls_init_program(icls_ctx* h) {
   CK(cudaMemcpyAsync(c.pzold, c.pz, bytes, cudaMemcpyDeviceToDevice, c.s));
   CK(cudaMemcpyAsync(c.seg_jmp[1], c.seg_jmp[0], (size_t)seg_count(c.P), cudaMemcpyDeviceToDevice, c.s));
   c.jmp_dirty[1] = c.jmp_dirty[0];
+  c.p_dirty = true;
   CK(cudaStreamSynchronize(c.s));
   c.initialised = true;
   return check_launch();

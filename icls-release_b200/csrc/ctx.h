@@ -101,6 +101,21 @@ __host__ __device__ __forceinline__ long long seg_of(const Params& p, int i, int
   return (i - 1) / kSeg + (long long)seg_row(p) * ((j - 1) + (long long)p.jmax * k);
 }
 
+// Tiles of the AB2 predictor (ab2.cuh): 32 x 8 columns, kc rows: 16 for FP64
+// (32 rows: 0.643 instead of 0.626 ms at 256^3), 8 for FP32 (32 rows: 0.375
+// instead of 0.357), and fewer while the grid does not fill the SMs once (64^3
+// FP64: 64 blocks of 16 rows 62 us, 256 of 4 rows 28 us).  The last chunk takes
+// the remainder, so every chunk has at least kc rows (the wall row k1 needs
+// rows kmax-1 and kmax in one block).
+constexpr int kAb2X = 32, kAb2Y = 8, kAb2Rows = 2 * 16;
+inline dim3 ab2_grid(const Params& p, bool fp64, int& kc) {
+  const unsigned gx = (unsigned)((p.imax + kAb2X - 1) / kAb2X), gy = (unsigned)((p.jmax + kAb2Y - 1) / kAb2Y);
+  const long long full = (long long)(fp64 ? 2 : 4) * 148;
+  kc = fp64 ? 16 : 8;
+  while (kc > 4 && (long long)gx * gy * (p.kmax / kc) < full) kc /= 2;
+  return dim3(gx, gy, (unsigned)(p.kmax / kc > 0 ? p.kmax / kc : 1));
+}
+
 // z rows per chunk of update_materials' Heaviside sweep (one exact partial
 // sum per column tile and chunk)
 constexpr int kHeavRows = 8;
@@ -168,6 +183,8 @@ struct Ctx {
   double* partials = nullptr;           // kRedBlocks * max(L,4)
   double* diag = nullptr;               // disp partials: 7 * kRedBlocks, then the 7 sums
   long long* lpartials = nullptr;
+  uint8_t* ab2_near = nullptr;          // per predictor tile and row: a drop next to it (k_ab2_near)
+  bool p_dirty = true;                  // pnew or pold written by a caller since the last pressure update
   DevScalars* dsc = nullptr;
   double* dvol = nullptr;               // volume(1:L)
   double* dvol0 = nullptr;              // init_volume(1:L)

@@ -34,6 +34,8 @@ struct Params {
   double cdx, cdy, cdz;      // dt dxi, dt dyi, dt dzi (correc's first products)
   double rrho0;              // 1./rho0, the IEEE quotient the reference evaluates per cell
   int rho0_pow2;             // rho0 is a power of two: x / rho0 == x * rrho0 exactly
+  double rrho1;              // 1/rho1, and the same for rho1
+  int rho1_pow2;
   double g1, g2, g3;
   double v_lower, v_upper;
   double forceytot;
@@ -341,6 +343,7 @@ struct DevScalars {
   int reinit_iters;
   int nan_flag;           // main.f90:207
   int wait_err;           // a kernel's bounded mbarrier wait gave up
+  int p_bad;              // the last pressure update wrote a value that is not finite
 };
 
 }  // namespace icls

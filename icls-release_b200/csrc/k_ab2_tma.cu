@@ -272,13 +272,13 @@ __global__ void __launch_bounds__(kThreadsTma, 1)
         const double ru = pi[oi], rv = pi[IB + oi], rw = pi[2 * IB + oi];
         const double ou = pi[3 * IB + oi], ov = pi[4 * IB + oi], ow = pi[5 * IB + oi];
         const double ph0 = PH(0, 0, 0);
-        const double Ru = rhs_u<double>(p, U, V, W, M, ru, rho_avr);
-        const double Rv = rhs_v<double>(p, U, V, W, M, rv, rho_avr);
-        const double Rw = rhs_w<double>(p, U, V, W, M, rw, rho_avr);
-        const double du = ab2_update_v(p, U(0, 0, 0), Ru, ou, ru, PH(1, 0, 0), ph0, 2. * qx - qxo, p.dxi);
-        double dv = ab2_update_v(p, V(0, 0, 0), Rv, ov, rv, PH(0, 1, 0), ph0, 2. * qy - qyo, p.dyi);
+        const double Ru = rhs_u<double>(p, U, V, W, M, [&](double x) { return x / ru; }, rho_avr);
+        const double Rv = rhs_v<double>(p, U, V, W, M, [&](double x) { return x / rv; }, rho_avr);
+        const double Rw = rhs_w<double>(p, U, V, W, M, [&](double x) { return x / rw; }, rho_avr);
+        const double du = ab2_update_v(p, U(0, 0, 0), Ru, ou, 1. / ru, PH(1, 0, 0), ph0, 2. * qx - qxo, p.dxi);
+        double dv = ab2_update_v(p, V(0, 0, 0), Rv, ov, 1. / rv, PH(0, 1, 0), ph0, 2. * qy - qyo, p.dyi);
         if (p.forceytot != 0.) dv = dv - (p.forceytot * p.dt) / rv;
-        double dw = ab2_update_v(p, W(0, 0, 0), Rw, ow, rw, PH(0, 0, 1), ph0, 2. * qz - qzo, p.dzi);
+        double dw = ab2_update_v(p, W(0, 0, 0), Rw, ow, 1. / rw, PH(0, 0, 1), ph0, 2. * qz - qzo, p.dzi);
         const long long q = idxI(p, i, j, k);
         duold_out[q] = Ru;
         dvold_out[q] = Rv;

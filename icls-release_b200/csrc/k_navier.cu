@@ -66,9 +66,45 @@ __global__ void __launch_bounds__(NT) k_mom_main(Params p, MomArgs a, T* __restr
   auto V = [&](int di, int dj, int dk) { return v[c + di + dj * sy + dk * sz]; };
   auto W = [&](int di, int dj, int dk) { return w[c + di + dj * sy + dk * sz]; };
   auto M = [&](int di, int dj, int dk) { return miu[c + di + dj * sy + dk * sz]; };
-  ru[q] = rhs_u<T>(p, U, V, W, M, cT<T>(a.rho_u)[q], rho_avr);
-  rv[q] = rhs_v<T>(p, U, V, W, M, cT<T>(a.rho_v)[q], rho_avr);
-  rw[q] = rhs_w<T>(p, U, V, W, M, cT<T>(a.rho_w)[q], rho_avr);
+  ru[q] = rhs_u<T>(p, U, V, W, M, [&](T x) { return x / cT<T>(a.rho_u)[q]; }, rho_avr);
+  rv[q] = rhs_v<T>(p, U, V, W, M, [&](T x) { return x / cT<T>(a.rho_v)[q]; }, rho_avr);
+  rw[q] = rhs_w<T>(p, U, V, W, M, [&](T x) { return x / cT<T>(a.rho_w)[q]; }, rho_avr);
+}
+
+// The predictor's near rows: a tile (32 x 8 columns) and row whose cells, or
+// the neighbours that its stencil reads, lie in a set segment of the
+// materials, or whose own cells lie in one of the face jumps' (now or old).
+// One thread per four segments; few are set, and those mark the tiles around
+// them (near starts at 0).
+__global__ void __launch_bounds__(NT) k_ab2_near(Params p, const uint8_t* __restrict__ mat,
+                                                 const uint8_t* __restrict__ jmp, const uint8_t* __restrict__ jmpold,
+                                                 uint8_t* __restrict__ near) {
+  const long long w = blockIdx.x * (long long)NT + threadIdx.x;
+  if (4 * w >= seg_count(p)) return;
+  // (the maps are padded with zeros to a multiple of four)
+  const unsigned m4 = reinterpret_cast<const unsigned*>(mat)[w];
+  const unsigned j4 = reinterpret_cast<const unsigned*>(jmp)[w] | reinterpret_cast<const unsigned*>(jmpold)[w];
+  if (!(m4 | j4)) return;
+  const int nsx = seg_row(p);
+  for (int b = 0; b < 4; ++b) {
+    const bool m = (m4 >> 8 * b) & 0xFFu, jj = (j4 >> 8 * b) & 0xFFu;
+    if (!m && !jj) continue;
+    const long long q = 4 * w + b, r = q / nsx;
+    const int sx = (int)(q - r * nsx), k = (int)(r / p.jmax), j = (int)(r - (long long)k * p.jmax) + 1;
+    auto set = [&](int s, int y, int kk) { near[((long long)s + (long long)nsx * ((y - 1) / kAb2Y)) * p.nCz + kk] = 1; };
+    if (!m) {
+      set(sx, j, k);
+      continue;
+    }
+    const int xm = sx ? sx - 1 : nsx - 1, xp = sx + 1 < nsx ? sx + 1 : 0;
+    const int ym = wrapy(p, j - 1), yp = wrapy(p, j + 1);
+    for (int kk = max(k - 1, 1); kk <= min(k + 1, p.kmax); ++kk)
+      for (int s : {xm, sx, xp}) {
+        set(s, ym, kk);
+        set(s, j, kk);
+        set(s, yp, kk);
+      }
+  }
 }
 
 // fillps (fillps.f90:36-53), optionally followed by p = p + p_jump
@@ -473,7 +509,7 @@ __device__ __forceinline__ void pupdate_pair(double p0, double p1, T o0, T o1, T
 template <typename T>
 __global__ void __launch_bounds__(NT) k_pupdate(Params p, const double* __restrict__ pp,
                                                 T* __restrict__ pnew, T* __restrict__ pold, int first,
-                                                int normalise, const DevScalars* __restrict__ dsc) {
+                                                int normalise, DevScalars* __restrict__ dsc) {
   typedef typename Vec2<T>::type T2;
   const long long n = 2 * (blockIdx.x * (long long)NT + threadIdx.x);
   if (n >= p.nC) return;
@@ -485,11 +521,13 @@ __global__ void __launch_bounds__(NT) k_pupdate(Params p, const double* __restri
     pupdate_pair<T>(pv.x, pv.y, ov.x, ov.y, nv.x, nv.y, dv.x, dv.y, first, normalise, norm, norm_old);
     *reinterpret_cast<T2*>(pold + n) = dv;
     *reinterpret_cast<T2*>(pnew + n) = nv;
+    if (!(isfinite(dv.x) && isfinite(dv.y) && isfinite(nv.x) && isfinite(nv.y))) dsc->p_bad = 1;
   } else {  // an odd last cell
     T n0, n1, d0, d1;
     pupdate_pair<T>(pp[n], 0., pnew[n], TC(0.), n0, n1, d0, d1, first, normalise, norm, norm_old);
     pold[n] = d0;
     pnew[n] = n0;
+    if (!(isfinite(d0) && isfinite(n0))) dsc->p_bad = 1;
   }
 }
 
@@ -619,6 +657,7 @@ MomArgs mom_args(Ctx& c) {
   a.pnew = c.pnew; a.pold = c.pold;
   a.px = c.px; a.py = c.py; a.pz = c.pz; a.pxold = c.pxold; a.pyold = c.pyold; a.pzold = c.pzold;
   a.rho_avr = &c.dsc->rho_avr;
+  a.near = nullptr; a.p_bad = &c.dsc->p_bad;
   return a;
 }
 CorrArgs corr_args(Ctx& c) {
@@ -637,11 +676,23 @@ template <typename T>
 T* fp(double* q) { return reinterpret_cast<T*>(q); }
 
 void launch_ab2(Ctx& c) {
-  Scope sc_(c.prof, c.s, "ab2", 1);
+  // the segment maps hold unless a caller wrote the fields they describe
+  const bool far = (c.P.f32 || c.ab2_ring) && !c.mat_dirty && !c.jmp_dirty[0] && !c.jmp_dirty[1];
+  Scope sc_(c.prof, c.s, "ab2", far ? 2 : 1);
   MomArgs a = mom_args(c);
+  if (far) {
+    cudaMemsetAsync(c.ab2_near, 0, (size_t)seg_row(c.P) * ((c.P.jmax + kAb2Y - 1) / kAb2Y) * c.P.nCz, c.s);
+    k_ab2_near<<<nblocks((seg_count(c.P) + 3) / 4), NT, 0, c.s>>>(c.P, c.seg_mat[c.mat_cur], c.seg_jmp[0],
+                                                                  c.seg_jmp[1], c.ab2_near);
+    a.near = c.ab2_near;
+    if (c.p_dirty) cudaMemsetAsync(&c.dsc->p_bad, 1, sizeof(int), c.s);  // unknown: nonzero
+  }
   const int o = c.hist ^ 1;
-  if (c.P.f32) ab2_launch_f32(c, a, o);     // k_ab2_f32.cu
-  else if (!ab2_tma_launch(c, a, o)) ab2_launch<double>(c, a, o);  // k_ab2_tma.cu when chosen, else the ring
+  if (c.P.f32) {
+    ab2_launch_f32(c, a, o);  // k_ab2_f32.cu
+  } else if (!ab2_tma_launch(c, a, o)) {  // k_ab2_tma.cu when chosen, else the ring
+    ab2_launch<double>(c, a, o);
+  }
   launch_ywalls_uvw(c, c.dudt, c.dvdt, c.dwdt);  // the y walls of bounduvw(dudt,dvdt,dwdt)
   c.hist = o;
 }
@@ -741,6 +792,8 @@ void launch_pressure_update(Ctx& c, int first) {
   // the plane-1 normalisation runs for BC_in_y Periodic and Walls only
   // (main.f90:169-185); otherwise pold = pnew, pnew = p
   const int norm = c.P.bcy == ICLS_BCY_PERIODIC || c.P.bcy == ICLS_BCY_WALLS;
+  cudaMemsetAsync(&c.dsc->p_bad, 0, sizeof(int), c.s);
+  c.p_dirty = false;
   if (norm) k_plane_norm<<<1, kNormThreads, 0, c.s>>>(c.P, c.p, c.dsc);
   if (c.P.f32)
     k_pupdate<float><<<nblocks((c.P.nC + 1) / 2), NT, 0, c.s>>>(c.P, c.p, fp<float>(c.pnew), fp<float>(c.pold), first, norm,
