@@ -626,15 +626,15 @@ void tube_batch(Ctx& c, LsBatch& b, bool list) {
   }
 }
 
-// the band cells a batch's list can hold at most: its tasks' computed
-// interior cells
+// the cells that a region, or a batch's regions, can put into a list at most:
+// the computed interior cells
+long long band_bound(const Ctx& c, const Region& r) {
+  const long long z = std::max(0, std::min(r.cz1, c.P.kmax) - std::max(r.cz0, 1) + 1);
+  return (long long)(r.cx1 - r.cx0 + 1) * (r.cy1 - r.cy0 + 1) * z;
+}
 long long band_bound(const Ctx& c, const LsBatch& b) {
   long long n = 0;
-  for (int q = 0; q < b.n; ++q) {
-    const Region& r = b.t[q].r;
-    const long long z = std::max(0, std::min(r.cz1, c.P.kmax) - std::max(r.cz0, 1) + 1);
-    n += (long long)(r.cx1 - r.cx0 + 1) * (r.cy1 - r.cy0 + 1) * z;
-  }
+  for (int q = 0; q < b.n; ++q) n += band_bound(c, b.t[q].r);
   return n;
 }
 
@@ -746,24 +746,55 @@ int inflation(Ctx& c, const std::vector<int>& drops) {
   c.nrm_stale = true;
   std::vector<double> bg0(c.P.L), bgg0(c.P.L);
   bool far_moved = false;
-  for (LsBatch& b : make_batches(drops, kStageRows, box)) {
-    // RK3: lv -> s1 -> s2 -> lv, or -> s3 where lv is still to be blended
-    auto stage = [&](int st, double a, double bb, double fdt) {
+  // batches whose moving cells the list holds (one drop's always fit)
+  std::vector<std::vector<int>> parts;
+  long long held = 0;
+  for (int l : drops) {
+    const long long n = band_bound(c, c.win[l].box);
+    if (parts.empty() || held + n > c.band_cap || parts.back().size() == (size_t)kTasks) {
+      parts.emplace_back();
+      held = 0;
+    }
+    parts.back().push_back(l);
+    held += n;
+  }
+  for (const std::vector<int>& part : parts) {
+    LsBatch b = make_batches(part, kStageRows, box)[0];
+    const long long need = band_bound(c, b);
+    // RK3 of lv, s1 and s2 in between: into s3 where lv is still to be
+    // blended; else from a copy, s1, over s2 and s3 into lv
+    auto set = [&](int st) {
       for (int q = 0; q < b.n; ++q) {
         LsTask& t = b.t[q];
         const Ctx::Member& m = member(c, t.l);
-        const DropWin& w = c.win[t.l];
-        const double g2 = 3. / 4. * w.bg + 1. / 4. * w.bg, h2 = 3. / 4. * w.bg_ghost + 1. / 4. * w.bg_ghost;
+        double* lv = c.lv[t.l];
+        double* base = gain_one ? lv : m.s1;
+        double* A = gain_one ? m.s1 : m.s2;
+        double* S = gain_one ? m.s2 : m.s3;
+        double* fin = gain_one ? m.s3 : lv;
         t.mask = m.mask;
         t.orig = m.cv;
         t.aux = m.fit;
-        t.phi0 = c.lv[t.l];
-        t.phis = st == 1 ? c.lv[t.l] : (st == 2 ? m.s1 : m.s2);
-        t.out = st == 1 ? m.s1 : (st == 2 ? m.s2 : (gain_one ? m.s3 : c.lv[t.l]));
-        t.bg = st == 1 ? w.bg : (st == 2 ? g2 : 1. / 3. * w.bg + 2. / 3. * g2);
-        t.bgg = st == 1 ? w.bg_ghost : (st == 2 ? h2 : 1. / 3. * w.bg_ghost + 2. / 3. * h2);
+        t.bg = rk3_still(c.win[t.l].bg);
+        t.bgg = rk3_still(c.win[t.l].bg_ghost);
+        if (st == 0) {
+          t.phi0 = lv;
+          t.out = m.s1;
+          t.out2 = m.s2;
+          t.out3 = gain_one ? nullptr : m.s3;
+          t.phis = fin;
+          continue;
+        }
+        t.phi0 = base;
+        t.phis = st == 1 ? base : (st == 2 ? A : S);
+        t.out = st == 1 ? A : (st == 2 ? S : fin);
       }
-      launch_inflate_stage(c, b, c.cfg.i_space, st == 1 ? 1 : 0, a, bb, fdt);
+    };
+    set(0);
+    launch_inflate_base(c, b);
+    auto stage = [&](int st, double a, double bb, double fdt) {
+      set(st);
+      launch_inflate_stage(c, b, c.cfg.i_space, st == 1 ? 1 : 0, a, bb, fdt, need);
     };
     stage(1, 1., 0., 1. * c.dt);
     stage(2, 3. / 4., 1. / 4., 1. / 4. * c.dt);
@@ -882,6 +913,11 @@ void reinit_batches(Ctx& c, std::vector<LsBatch>& bs) {
   const double dtau = 0.5 * dz;
   const double thr = dz * dz * dz * dz * dz;
   for (LsBatch& b : bs) {
+    // 8 rows per block, 5 (the fewest that hold a wall row and the two next
+    // to it) where 8 leave the SMs with two blocks or fewer (one drop at 64^3:
+    // 48 -> 34 us per stage)
+    set_tiles(b, kStageRows);
+    if (b.start[b.n] < 2 * 148) set_tiles(b, 5);
     double xg[kTasks], xh[kTasks], og[kTasks];
     bool partial[kTasks];
     for (int q = 0; q < b.n; ++q) {

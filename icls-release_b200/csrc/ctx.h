@@ -39,7 +39,7 @@ struct LsTask {
   const double* orig;    // reinitialisation: sgn source; mass correction: the drop's curvature (shape C)
   double* aux;           // mass correction: |grad phi| (shape I) of the curvature sweep, then H (shape C); else null
   double* out;
-  double *out2, *out3;   // tube with a band list: the clipped values go here as well
+  double *out2, *out3;   // tube with a band list: the clipped values go here as well; mass correction: k_inflate_base
   uint8_t* mask;         // the drop's band mask (tube writes, advection reads)
   Region vin;            // tube: phi0 holds valid data on vin's written cells,
   double bgin, bggin;    //       these far-field values elsewhere
@@ -264,7 +264,9 @@ void launch_materials(Ctx& c, const uint8_t* cur, const uint8_t* prev);
 void launch_seg_clear_jumps(Ctx& c, const uint8_t* faces, const uint8_t* lap);
 // mass correction of the tasks' drops; LsTask::far holds the interior cells outside a drop's region
 void launch_inflate_sums(Ctx& c, const LsBatch& b);
-void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt);
+void launch_inflate_base(Ctx& c, const LsBatch& b);
+void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
+                          long long need);
 void launch_gain(Ctx& c, const LsBatch& b);
 void launch_region_blend(Ctx& c, const LsBatch& b);
 // one RK3 stage over the band cells that the batch's tube listed; rest: and

@@ -110,6 +110,40 @@ struct BandCell {
   int k;
 };
 
+// Appends the cells that the block's threads marked (bit r of rows: row ka + r
+// of the thread's column) to the list (null: counts only): one addition to the
+// counter per block; within a warp the rows in order, lanes (x fastest) within
+// a row.  Returns the block's number of cells (in thread 0).
+__device__ __forceinline__ int append_cells(unsigned rows, int ka, unsigned ijt, BandCell* __restrict__ list,
+                                            int* __restrict__ count) {
+  __shared__ int wsum[NT / 32], base_sh;
+  const int lane = flat_tid() & 31, warp = flat_tid() >> 5;
+  const unsigned any = __reduce_or_sync(0xffffffffu, rows);
+  int n = 0, tot = 0;
+  for (unsigned r = any; r; r &= r - 1) n += __popc(__ballot_sync(0xffffffffu, rows >> (__ffs(r) - 1) & 1u));
+  if (lane == 0) wsum[warp] = n;
+  __syncthreads();
+  if (flat_tid() == 0) {
+    for (int w = 0; w < NT / 32; ++w) {
+      const int v = wsum[w];
+      wsum[w] = tot;
+      tot += v;
+    }
+    base_sh = (tot && list) ? atomicAdd(count, tot) : 0;
+  }
+  __syncthreads();
+  if (list && n) {
+    int at = base_sh + wsum[warp];
+    for (unsigned r = any; r; r &= r - 1) {
+      const int row = __ffs(r) - 1;
+      const unsigned m = __ballot_sync(0xffffffffu, rows >> row & 1u);
+      if (rows >> row & 1u) list[at + __popc(m & ((1u << lane) - 1u))] = BandCell{ijt, ka + row};
+      at += __popc(m);
+    }
+  }
+  return tot;
+}
+
 // Clip to +-NB (levelset.f90:120-128) and the band mask (130-160) over the
 // tasks' regions.  phi0 holds valid data on vin's written cells, bgin
 // (rows 0..k1) or bggin (ghost rows) elsewhere.  Counts the band per drop
@@ -130,9 +164,11 @@ struct BandCell {
 // instruction issue: the version before staged 2-D tiles of flags in shared
 // memory with a barrier per row and 64-bit index products per store, 580
 // instructions a warp row.  With the list and the two more copies a sweep
-// takes 0.25 ms instead of 0.20 (256^3 x 48, FP64; FP32 0.16 instead of 0.14),
-// and the three stages 0.34 instead of 0.67 ms (FP32 0.19 instead of 0.31).
-constexpr int kTubeRows = 16;
+// takes 0.244 ms instead of 0.203 (256^3 x 48, FP64; FP32 0.136 instead of
+// 0.140), and the three stages 0.34 instead of 0.67 ms (FP32 0.19 instead of
+// 0.31).  Chunks of 8 rows (16: 0.254 and 0.161 ms, one drop at 64^3 28 instead
+// of 22 us).
+constexpr int kTubeRows = 8;
 template <typename T>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_tube(Params p, const __grid_constant__ LsBatch B,
                                              long long* __restrict__ cnt, int* __restrict__ bbox_lo,
@@ -197,7 +233,10 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_tube(Params p,
         else val = clipNB(a2, NB);
         if (k >= 1 && k <= p.kmax) {
           bool m = in_band(a0) | in_band(a1) | in_band(a2) | in_band(a3) | in_band(a4);
-          if (!m) {
+          if (!m && held == 0x3FFu && k >= t.vin.z0 && k <= t.vin.z1) {  // every neighbour is stored
+            m = in_band(in[o - 2]) | in_band(in[o - 1]) | in_band(in[o + 1]) | in_band(in[o + 2]) |
+                in_band(in[o - 2 * sy]) | in_band(in[o - sy]) | in_band(in[o + sy]) | in_band(in[o + 2 * sy]);
+          } else if (!m) {
             const T fk = far(k);
             const bool kin = k >= t.vin.z0 && k <= t.vin.z1;
 #pragma unroll
@@ -224,37 +263,10 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_tube(Params p,
       a0 = a1; a1 = a2; a2 = a3; a3 = a4; a4 = nxt;
     }
   }
-  const int lane = flat_tid() & 31, warp = flat_tid() >> 5;
-  // the warp's band cells, then the block's: one addition to the drop's count
-  // and one to the list per block; within a warp the rows in order, lanes (x
-  // fastest) within a row
-  __shared__ int wsum[NT / 32], base_sh;
-  int n = 0;
-  for (unsigned any = __reduce_or_sync(0xffffffffu, rows), r = any; r; r &= r - 1)
-    n += __popc(__ballot_sync(0xffffffffu, rows >> (__ffs(r) - 1) & 1u));
-  if (lane == 0) wsum[warp] = n;
-  __syncthreads();
-  if (flat_tid() == 0) {
-    int tot = 0;
-    for (int w = 0; w < NT / 32; ++w) {
-      const int v = wsum[w];
-      wsum[w] = tot;
-      tot += v;
-    }
-    if (tot) atomicAdd((unsigned long long*)(cnt + t.l), (unsigned long long)tot);
-    base_sh = (tot && list) ? atomicAdd(count, tot) : 0;
-  }
-  __syncthreads();
-  if (list && n) {
-    int at = base_sh + wsum[warp];
-    const unsigned ijt = (unsigned)(i - 1) | ((unsigned)(j - 1) << 12) | ((unsigned)ti << 24);
-    for (unsigned r = __reduce_or_sync(0xffffffffu, rows); r; r &= r - 1) {
-      const int row = __ffs(r) - 1;
-      const unsigned m = __ballot_sync(0xffffffffu, rows >> row & 1u);
-      if (rows >> row & 1u) list[at + __popc(m & ((1u << lane) - 1u))] = BandCell{ijt, c.ka + row};
-      at += __popc(m);
-    }
-  }
+  const int lane = flat_tid() & 31;
+  const unsigned ijt = (unsigned)(i - 1) | ((unsigned)(j - 1) << 12) | ((unsigned)ti << 24);
+  const int tot = append_cells(rows, c.ka, ijt, list, count);
+  if (flat_tid() == 0 && tot) atomicAdd((unsigned long long*)(cnt + t.l), (unsigned long long)tot);
   int lo[5] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX, INT_MAX};
   int hi[5] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN};
   if (kmin != INT_MAX) {
@@ -392,18 +404,23 @@ __device__ __forceinline__ T infl_v_back(const Params& p, const T* __restrict__ 
   const T h = dheav[idxC(p, i, p.jmax, k)];
   return -divy(p, temp * (-h - h));
 }
-// (a, b, c) = u_lc, v_lc, w_lc at an interior cell; false where H is uniform
-// around it (the velocity is then +-0 and moves nothing)
+// H is not uniform around an interior cell (where it is, the velocity of a
+// finite temp is +-0 and moves nothing)
 template <typename T>
-__device__ __forceinline__ bool infl_velocity(const Params& p, const T* __restrict__ dheav,
+__device__ __forceinline__ bool infl_moves(const Params& p, const T* __restrict__ dheav, T temp, int i, int j, int k) {
+  const long long n = idxC(p, i, j, k), sy = p.nCx, sz = (long long)p.nCx * p.nCy;
+  const T h0 = dheav[n];
+  return !((p.bcy == ICLS_BCY_PERIODIC || (j != 1 && j != p.jmax)) && isfinite(temp) && dheav[n + 1] == h0 &&
+           dheav[n - 1] == h0 && dheav[n + sy] == h0 && dheav[n - sy] == h0 && dheav[n + sz] == h0 &&
+           dheav[n - sz] == h0);
+}
+// (a, b, c) = u_lc, v_lc, w_lc at an interior cell
+template <typename T>
+__device__ __forceinline__ void infl_velocity(const Params& p, const T* __restrict__ dheav,
                                               const T* __restrict__ kappa, T temp, int i, int j, int k,
                                               const double* __restrict__ vin, T& a, T& b, T& cc) {
-  const long long n = idxC(p, i, j, k), sy = p.nCx, sz = (long long)p.nCx * p.nCy;
+  const long long n = idxC(p, i, j, k);
   const bool inner_y = p.bcy == ICLS_BCY_PERIODIC || (j != 1 && j != p.jmax);
-  const T h0 = dheav[n];
-  if (inner_y && isfinite(temp) && dheav[n + 1] == h0 && dheav[n - 1] == h0 && dheav[n + sy] == h0 &&
-      dheav[n - sy] == h0 && dheav[n + sz] == h0 && dheav[n - sz] == h0)
-    return false;
   const T ul_m = infl_face(p, dheav, temp, 0, wrapx(p, i - 1), j, k);
   const T ul_0 = infl_face(p, dheav, temp, 0, i, j, k);
   T vl_m, vl_0;
@@ -425,20 +442,12 @@ __device__ __forceinline__ bool infl_velocity(const Params& p, const T* __restri
     b = b * kp;
     cc = cc * kp;
   }
-  return true;
 }
 
-// INFL: a stage of the mass correction.  The velocity is u_lc, v_lc, w_lc of
-// the inflation, formed at the cell (infl_velocity); where H is uniform
-// around the cell it is an exact zero and the value keeps its base without
-// the stencil (the correction moves only cells within 1.5dz of the
-// interface and their neighbours, a fifth of the band).
-template <int SCHEME, typename T, int PW, bool INFL>
+template <int SCHEME, typename T, int PW>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Params p, const __grid_constant__ LsBatch B, int stage1,
                                                      double a_, double bb_, double fdt_, const T* __restrict__ vu,
-                                                     const T* __restrict__ vv, const T* __restrict__ vw,
-                                                     const InflateState* __restrict__ inf,
-                                                     const double* __restrict__ vin) {
+                                                     const T* __restrict__ vv, const T* __restrict__ vw) {
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -458,8 +467,6 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Para
   T* const o2 = jj != INT_MIN ? out + idxL(p, i, jj, 0) : nullptr;
   T* const o3 = (ii != INT_MIN && jj != INT_MIN) ? out + idxL(p, ii, jj, 0) : nullptr;
   const long long qc = idxI(p, i, j, 1);  // row k at qc + (k - 1) * szI
-  T temp = TC(0.);
-  if constexpr (INFL) temp = TC(inf[t.l].temp);
   auto put = [&](int k, T v) {
     const int o = k * sz;
     o0[o] = v;
@@ -491,27 +498,9 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Para
         val = stage1 ? f0 : a * f0 + bb * fsc[o];
       } else {
         const long long q = qc + (long long)(k - 1) * szI;
-        uint8_t m = t.mask[q];
+        const uint8_t m = t.mask[q];
+        const T u = vu[q], v = vv[q], w = vw[q];
         const T* f = fsc + o;
-        T u, v, w;
-        if constexpr (INFL) {
-          u = v = w = TC(0.);
-          if (m) m = infl_velocity(p, cT<T>(t.aux), cT<T>(t.orig), temp, i, j, k, vin, u, v, w) ? 1 : 0;
-          if (!m) {
-            val = stage1 ? f0 : a * f0 + bb * f[0];
-            if (k == 1) v1 = val;
-            if (k == 2) v2 = val;
-            if (k == p.kmax - 1) vkm = val;
-            if (k == p.kmax) vk = val;
-            put(k, val);
-            if (k == 2 && wall0) put(0, TC(2.) * v1 - v2);
-            continue;
-          }
-        } else {
-          u = vu[q];
-          v = vv[q];
-          w = vw[q];
-        }
         Axial19<T> S;
         S.c = f[0];
 #pragma unroll
@@ -546,23 +535,48 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Para
 // Bound by the latency of the 19 stencil loads (a quarter of the box's cells
 // are band cells; the column stage loads all of them and walks every row):
 // 256^3 x 48, FP64 0.223 -> 0.112 ms, FP32 0.104 -> 0.063 ms per stage.
-template <int SCHEME, typename T, int PW>
+// INFL: a stage of the mass correction over its list of moving cells
+// (k_inflate_base), the velocity u_lc, v_lc, w_lc formed at the cell.
+template <int SCHEME, typename T, int PW, bool INFL>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4))
     k_adv_band(Params p, const __grid_constant__ LsBatch B, const BandCell* __restrict__ list,
                const int* __restrict__ count, int stage1, double a_, double bb_, double fdt_,
-               const T* __restrict__ vu, const T* __restrict__ vv, const T* __restrict__ vw) {
-  const int total = *count;
+               const T* __restrict__ vu, const T* __restrict__ vv, const T* __restrict__ vw,
+               const InflateState* __restrict__ inf, const double* __restrict__ vin) {
+  const int total = *count, stride = (int)gridDim.x * NT;
   const T a = TC(a_), bb = TC(bb_), fdt = TC(fdt_);
   const int sy = p.nLx, sz = p.nLx * p.nLy;
-  for (int n = (int)(blockIdx.x * NT + threadIdx.x); n < total; n += (int)gridDim.x * NT) {
-    const BandCell bc = list[n];
+  // the tasks' arrays, where a lane finds its cell's without a walk through
+  // the launch parameters
+  __shared__ const T *sf0[kTasks], *sfs[kTasks];
+  __shared__ T* so[kTasks];
+  for (int q = flat_tid(); q < B.n; q += NT) {
+    sf0[q] = cT<T>(B.t[q].phi0);
+    sfs[q] = cT<T>(B.t[q].phis);
+    so[q] = mT<T>(B.t[q].out);
+  }
+  __syncthreads();
+  int n = (int)(blockIdx.x * NT) + flat_tid();
+  BandCell next = n < total ? list[n] : BandCell{0u, 1};
+  for (; n < total; n += stride) {
+    const BandCell bc = next;
+    if (n + stride < total) next = list[n + stride];
     const int i = (int)(bc.ijt & 0xFFFu) + 1, j = (int)((bc.ijt >> 12) & 0xFFFu) + 1, k = bc.k;
-    const LsTask& t = B.t[bc.ijt >> 24];
-    const int o = (int)idxL(p, i, j, k);
-    const int q = (i - 1) + p.imax * ((j - 1) + p.jmax * (k - 1));
-    const T* f = cT<T>(t.phis) + o;
-    const T f0 = cT<T>(t.phi0)[o];
-    const T u = vu[q], v = vv[q], w = vw[q];
+    const int ti = (int)(bc.ijt >> 24);
+    const int o = (i + 2) + sy * (j + 2) + sz * (k + 2);
+    const T* f = sfs[ti] + o;
+    const T f0 = sf0[ti][o];
+    T u, v, w;
+    if constexpr (INFL) {
+      const LsTask& t = B.t[ti];
+      u = v = w = TC(0.);
+      infl_velocity(p, cT<T>(t.aux), cT<T>(t.orig), TC(inf[t.l].temp), i, j, k, vin, u, v, w);
+    } else {
+      const int q = (i - 1) + p.imax * ((j - 1) + p.jmax * (k - 1));
+      u = vu[q];
+      v = vv[q];
+      w = vw[q];
+    }
     Axial19<T> S;
     S.c = f[0];
 #pragma unroll
@@ -574,7 +588,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4))
     }
     S.x[3] = S.y[3] = S.z[3] = S.c;
     const T val = (stage1 ? f0 : a * f0 + bb * S.c) + fdt * adv_rhs<SCHEME, PW>(p, S, u, v, w, k);
-    T* const out = mT<T>(t.out);
+    T* const out = so[ti];
     out[o] = val;
     if (i <= 3 || i > p.imax - 3 || j <= 3 || j > p.jmax - 3) putL(p, out, i, j, k, val);
   }
@@ -1271,6 +1285,42 @@ __global__ void __launch_bounds__(kFinalThreads)
 // volumes before (V) and after (V1) the inflation: the blend removes the
 // measured error to first order in the (small) displacement.
 
+// The start of the mass correction's RK3 over the tasks' written cells: phi0
+// into the buffers that the stages read around the cells they move (out, out2
+// and, where set, out3), its RK3 combinations into phis, the last stage's
+// output (which may be phi0 itself), and the list of the band's moving cells
+// (infl_moves): about a twelfth of a box, which the column stages walked
+// three times to find (256^3 x 48 after a reinitialisation, three stages FP64
+// 1.20 -> 0.54 ms with this sweep, FP32 0.78 -> 0.39 ms).
+template <typename T>
+__global__ void __launch_bounds__(NT) k_inflate_base(Params p, const __grid_constant__ LsBatch B,
+                                                     const InflateState* __restrict__ inf,
+                                                     BandCell* __restrict__ list, int* __restrict__ count) {
+  const int ti = task_of(B);
+  const LsTask& t = B.t[ti];
+  const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
+  unsigned rows = 0;
+  if (c.ok) {
+    const T* src = cT<T>(t.phi0);
+    T* fin = const_cast<T*>(cT<T>(t.phis));
+    const T temp = TC(inf[t.l].temp);
+    for (int k = c.ka; k <= c.kb; ++k) {
+      const T x = src[idxL(p, c.i, c.j, k)];
+      const bool in = computed(c, t.r, k);
+      const T y = TC(3. / 4.) * x + TC(1. / 4.) * x;
+      putL(p, mT<T>(t.out), c.i, c.j, k, x);
+      putL(p, mT<T>(t.out2), c.i, c.j, k, x);
+      if (t.out3) putL(p, mT<T>(t.out3), c.i, c.j, k, x);
+      putL(p, fin, c.i, c.j, k,
+           in ? TC(1. / 3.) * x + TC(2. / 3.) * y : ((k < 0 || k > p.k1) ? TC(t.bgg) : TC(t.bg)));
+      if (in && k >= 1 && k <= p.kmax && t.mask[idxI(p, c.i, c.j, k)] &&
+          infl_moves(p, cT<T>(t.aux), temp, c.i, c.j, k))
+        rows |= 1u << (k - c.ka);
+    }
+  }
+  append_cells(rows, c.ka, (unsigned)(c.i - 1) | ((unsigned)(c.j - 1) << 12) | ((unsigned)ti << 24), list, count);
+}
+
 // per-(tile, chunk) exact sums of H(phi0) over the tasks' computed interior cells
 template <typename T>
 __global__ void __launch_bounds__(NT) k_region_heav(Params p, const __grid_constant__ LsBatch B,
@@ -1503,7 +1553,7 @@ void launch_band_extents(Ctx& c, int l) {
           (k_band_extents<double><<<g, NT, 0, c.s>>>(c.P, c.lv[l], l, lo, hi)));
 }
 
-template <typename T, bool INFL>
+template <typename T>
 void adv_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt, const double* vu,
                 const double* vv, const double* vw) {
   const T* u = reinterpret_cast<const T*>(vu);
@@ -1513,18 +1563,18 @@ void adv_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, doub
   // the FP32 form always takes the product by the reciprocal)
   const unsigned g = b.start[b.n];
   const bool pw = c.P.pow2 || sizeof(T) == 4;
-  auto go = [&](auto kernel) { kernel<<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w, c.dinf, c.vin); };
+  auto go = [&](auto kernel) { kernel<<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w); };
   if (scheme == ICLS_HOUC5) {
-    if (pw) go(k_adv_stage<ICLS_HOUC5, T, 1, INFL>);
-    else go(k_adv_stage<ICLS_HOUC5, T, 0, INFL>);
+    if (pw) go(k_adv_stage<ICLS_HOUC5, T, 1>);
+    else go(k_adv_stage<ICLS_HOUC5, T, 0>);
   } else {
-    if (pw) go(k_adv_stage<ICLS_WENO5, T, 1, INFL>);
-    else go(k_adv_stage<ICLS_WENO5, T, 0, INFL>);
+    if (pw) go(k_adv_stage<ICLS_WENO5, T, 1>);
+    else go(k_adv_stage<ICLS_WENO5, T, 0>);
   }
 }
 // one RK stage over the batch from the list of its tube sweep; need = the
 // upper bound of its length that the caller checked against c.band_cap
-template <typename T>
+template <typename T, bool INFL>
 void adv_band_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                      const double* vu, const double* vv, const double* vw, long long need, bool rest, bool walls) {
   const T* u = reinterpret_cast<const T*>(vu);
@@ -1533,14 +1583,14 @@ void adv_band_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a,
   const BandCell* list = reinterpret_cast<const BandCell*>(c.band_list);
   const unsigned nb = (unsigned)std::min<long long>((need + NT - 1) / NT, 8 * 148);
   const bool pw = c.P.pow2 || sizeof(T) == 4;
-  auto go = [&](auto kernel) { kernel<<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, stage1, a, bb, fdt, u, v, w); };
+  auto go = [&](auto kernel) { kernel<<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, stage1, a, bb, fdt, u, v, w, c.dinf, c.vin); };
   if (nb > 0) {
     if (scheme == ICLS_HOUC5) {
-      if (pw) go(k_adv_band<ICLS_HOUC5, T, 1>);
-      else go(k_adv_band<ICLS_HOUC5, T, 0>);
+      if (pw) go(k_adv_band<ICLS_HOUC5, T, 1, INFL>);
+      else go(k_adv_band<ICLS_HOUC5, T, 0, INFL>);
     } else {
-      if (pw) go(k_adv_band<ICLS_WENO5, T, 1>);
-      else go(k_adv_band<ICLS_WENO5, T, 0>);
+      if (pw) go(k_adv_band<ICLS_WENO5, T, 1, INFL>);
+      else go(k_adv_band<ICLS_WENO5, T, 0, INFL>);
     }
   }
   if (rest) k_adv_rest<T><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b);
@@ -1550,27 +1600,43 @@ void adv_band_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a,
     k_adv_ghosts<T><<<w1.start[w1.n], kTile, 0, c.s>>>(c.P, w1, stage1, a, bb);
   }
 }
+bool holds_walls(const LsBatch& b) {
+  for (int q = 0; q < b.n; ++q)
+    if (b.t[q].r.cz0 <= -2) return true;
+  return false;
+}
 void launch_adv_band(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                      const double* vu, const double* vv, const double* vw, long long need, bool rest) {
   if (b.n == 0) return;
-  bool walls = false;
-  for (int q = 0; q < b.n; ++q) walls = walls || b.t[q].r.cz0 <= -2;
+  const bool walls = holds_walls(b);
   Scope sc_(c.prof, c.s, "adv_stage", 1 + (walls ? 1 : 0) + (rest ? 1 : 0));
-  BY_FORM(c, adv_band_launch<float>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need, rest, walls),
-          adv_band_launch<double>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need, rest, walls));
+  BY_FORM(c, (adv_band_launch<float, false>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need, rest, walls)),
+          (adv_band_launch<double, false>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw, need, rest, walls)));
 }
+// the mass correction's stages: its buffers and list, then one stage over the list
+void launch_inflate_base(Ctx& c, const LsBatch& b) {
+  if (b.n == 0) return;
+  Scope sc_(c.prof, c.s, "inflate_stage", 1);
+  cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
+  BandCell* l = reinterpret_cast<BandCell*>(c.band_list);
+  BY_FORM(c, (k_inflate_base<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf, l, c.band_count)),
+          (k_inflate_base<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf, l, c.band_count)));
+}
+void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
+                          long long need) {
+  if (b.n == 0) return;
+  const bool walls = holds_walls(b);
+  Scope sc_(c.prof, c.s, "inflate_stage", 1 + (walls ? 1 : 0));
+  BY_FORM(c, (adv_band_launch<float, true>(c, b, scheme, stage1, a, bb, fdt, nullptr, nullptr, nullptr, need, false, walls)),
+          (adv_band_launch<double, true>(c, b, scheme, stage1, a, bb, fdt, nullptr, nullptr, nullptr, need, false, walls)));
+}
+
 void launch_adv_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                       const double* vu, const double* vv, const double* vw) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "adv_stage", 1);
-  BY_FORM(c, (adv_launch<float, false>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw)),
-          (adv_launch<double, false>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw)));
-}
-void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt) {
-  if (b.n == 0) return;
-  Scope sc_(c.prof, c.s, "inflate_stage", 1);
-  BY_FORM(c, (adv_launch<float, true>(c, b, scheme, stage1, a, bb, fdt, nullptr, nullptr, nullptr)),
-          (adv_launch<double, true>(c, b, scheme, stage1, a, bb, fdt, nullptr, nullptr, nullptr)));
+  BY_FORM(c, adv_launch<float>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw),
+          adv_launch<double>(c, b, scheme, stage1, a, bb, fdt, vu, vv, vw));
 }
 
 void launch_reinit_stage(Ctx& c, const LsBatch& b, int stage, double dtau) {
