@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <new>
 #include <vector>
 
@@ -112,81 +113,124 @@ constexpr int SB_H2T = SB_H1T + 32768;        // H2^T [128 x 128]
 constexpr int SB_DZT = SB_H2T + 32768;        // delta^T [128 x 128]
 constexpr int SB_TRAIN = SB_DZT + 32768;      // 196608
 
-// a weight matrix [n][k] (row-major BF16, global) into the B operand layout
-__device__ __forceinline__ void stage_b(unsigned char* sb, const __nv_bfloat16* __restrict__ w, int n, int k) {
-  for (int e = threadIdx.x; e < n * k; e += blockDim.x) {
-    const int r = e / k, c = e - r * k;
-    *reinterpret_cast<__nv_bfloat16*>(sb + kmajor_off(r, c, n)) = w[e];
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);  // a at the lower address
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// a weight matrix [n][k] (row-major BF16, 16-byte aligned rows) into the
+// B-operand layout, one 16-byte chunk per store
+__device__ __forceinline__ void stage_rows(unsigned char* dst, const __nv_bfloat16* __restrict__ w, int n, int k) {
+  for (int e = threadIdx.x; e < n * (k / 8); e += blockDim.x) {
+    const int c = e / n, r = e - c * n;
+    *reinterpret_cast<uint4*>(dst + kmajor_off(r, 8 * c, n)) =
+        *reinterpret_cast<const uint4*>(w + (size_t)r * k + 8 * c);
   }
 }
 
-// The forward pass of one 128-sample tile; x (FP32, [rows][32]) holds the
-// tile's inputs, sample t of the tile is row t.  Returns y (kappa*dx) of this
-// thread's sample.  Training keeps the pre-activations z1..z3 (zg, per sample
-// 320 floats) and the transposed activations in shared memory.
-template <bool TRAIN>
+// row t of the tile: the sample's 32 FP32 inputs (from registers; zeros
+// past the end) as BF16 hi (k 0..31) and lo (k 32..63)
+__device__ __forceinline__ void stage_inputs_regs(unsigned char* act, const float4 (&xv)[kIn / 4], int t) {
+#pragma unroll
+  for (int c = 0; c < kIn / 8; ++c) {
+    const float4 a = xv[2 * c], b = xv[2 * c + 1];
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    float hi[8], lo[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      hi[q] = __bfloat162float(__float2bfloat16(v[q]));
+      lo[q] = v[q] - hi[q];
+    }
+    *reinterpret_cast<uint4*>(act + kmajor_off(t, 8 * c, kRows)) =
+        make_uint4(pack_bf16(hi[0], hi[1]), pack_bf16(hi[2], hi[3]), pack_bf16(hi[4], hi[5]), pack_bf16(hi[6], hi[7]));
+    *reinterpret_cast<uint4*>(act + kmajor_off(t, kIn + 8 * c, kRows)) =
+        make_uint4(pack_bf16(lo[0], lo[1]), pack_bf16(lo[2], lo[3]), pack_bf16(lo[4], lo[5]), pack_bf16(lo[6], lo[7]));
+  }
+}
+
+// A training tile's epilogues work on 32 columns of a thread's row at a time.
+// Row t of a tile of 32 activations or deltas, columns c0.., as the next A
+// operand (16-byte stores) and transposed, for the weight gradients
+__device__ __forceinline__ void put_row32(unsigned char* act, int t, int c0, const float (&h)[32]) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+    *reinterpret_cast<uint4*>(act + kmajor_off(t, c0 + 8 * m, kRows)) =
+        make_uint4(pack_bf16(h[8 * m], h[8 * m + 1]), pack_bf16(h[8 * m + 2], h[8 * m + 3]),
+                   pack_bf16(h[8 * m + 4], h[8 * m + 5]), pack_bf16(h[8 * m + 6], h[8 * m + 7]));
+}
+// (two lanes' values of a column sit next to each other there: the even lane
+// stores the pair of an even column, the odd lane that of the next)
+__device__ __forceinline__ void put_col32(unsigned char* act, int t, int c0, int rows, const float (&h)[32]) {
+  const bool odd = t & 1;
+#pragma unroll
+  for (int q = 0; q < 32; q += 2) {
+    const float give = odd ? h[q] : h[q + 1];
+    const float got = __shfl_xor_sync(0xffffffffu, give, 1);
+    const uint32_t v = odd ? pack_bf16(got, h[q + 1]) : pack_bf16(h[q], got);
+    *reinterpret_cast<uint32_t*>(act + kmajor_off(c0 + q + (odd ? 1 : 0), t & ~1, rows)) = v;
+  }
+}
+
+// The forward pass of one 128-sample tile; xrow (FP32, 32 values) holds the
+// inputs of sample t of the tile.  Returns y (kappa*dx) of
+// this thread's sample.  Keeps the pre-activations z1..z3 (column c of sample
+// t at zt[128 c], so a warp's accesses are contiguous) and the transposed
+// activations in shared memory.
 __device__ float forward_tile(const Net& net, const float* __restrict__ xrow, unsigned char* sm, uint32_t tmem,
-                              uint64_t* bar, uint32_t& phase, float* __restrict__ zrow, bool& ok) {
+                              uint64_t* bar, uint32_t& phase, float* __restrict__ zt, bool& ok) {
   const int t = threadIdx.x, warp = t >> 5;
   const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-  // inputs
-  for (int j = 0; j < kIn; ++j) {
-    const float v = xrow ? xrow[j] : 0.f;
-    const float hi = __bfloat162float(__float2bfloat16(v));
-    const float lo = v - hi;
-    put_bf16(sm + SB_XA, kmajor_off(t, j, kRows), hi);
-    put_bf16(sm + SB_XA, kmajor_off(t, j + kIn, kRows), lo);
-    if (TRAIN) {
-      put_bf16(sm + SB_XT, kmajor_off(j, t, kIn2), hi);
-      put_bf16(sm + SB_XT, kmajor_off(j + kIn, t, kIn2), lo);
+  {
+    float4 xv[kIn / 4];
+    const bool vec = (reinterpret_cast<uintptr_t>(xrow) & 15) == 0;  // a caller's array need not be aligned
+#pragma unroll
+    for (int q = 0; q < kIn / 4; ++q)
+      xv[q] = vec ? reinterpret_cast<const float4*>(xrow)[q]
+                  : make_float4(xrow[4 * q], xrow[4 * q + 1], xrow[4 * q + 2], xrow[4 * q + 3]);
+    stage_inputs_regs(sm + SB_XA, xv, t);
+    float hi[32], lo[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      const float v = (&xv[q / 4].x)[q % 4];
+      hi[q] = __bfloat162float(__float2bfloat16(v));
+      lo[q] = v - hi[q];
     }
+    put_col32(sm + SB_XT, t, 0, kIn2, hi);
+    put_col32(sm + SB_XT, t, kIn, kIn2, lo);
   }
-  // layer 1
-  stage_b(sm + SB_B, net.w1, kH1, kIn2);
+  // the two hidden layers
+  auto hidden = [&](int n, int ob, int z0, unsigned char* ht) {
+    for (int c = 0; c < n; c += 32) {
+      float v[32];
+      umma::tmem_ld32(lane_addr + c, v);
+#pragma unroll
+      for (int q = 0; q < 32; ++q) {
+        const float z = v[q] + net.theta[ob + c + q];
+        zt[kRows * (z0 + c + q)] = z;
+        v[q] = silu(z);
+      }
+      put_row32(sm + SB_ACT, t, c, v);
+      put_col32(ht, t, c, n, v);
+    }
+  };
+  stage_rows(sm + SB_B, net.w1, kH1, kIn2);
   ok &= umma::tile_gemm(sm + SB_XA, sm + SB_B, kH1, kIn2, tmem, bar, phase);
-  for (int c = 0; c < kH1; c += 8) {
-    float v[8];
-    umma::tmem_ld8(lane_addr + c, v);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float z = v[q] + net.theta[oB1 + c + q];
-      const float h = silu(z);
-      put_bf16(sm + SB_ACT, kmajor_off(t, c + q, kRows), h);
-      if (TRAIN) {
-        put_bf16(sm + SB_H1T, kmajor_off(c + q, t, kH1), h);
-        zrow[c + q] = z;
-      }
-    }
-  }
-  // layer 2
-  stage_b(sm + SB_B, net.w2, kH2, kH1);
+  hidden(kH1, oB1, 0, sm + SB_H1T);
+  stage_rows(sm + SB_B, net.w2, kH2, kH1);
   ok &= umma::tile_gemm(sm + SB_ACT, sm + SB_B, kH2, kH1, tmem, bar, phase);
-  for (int c = 0; c < kH2; c += 8) {
-    float v[8];
-    umma::tmem_ld8(lane_addr + c, v);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float z = v[q] + net.theta[oB2 + c + q];
-      const float h = silu(z);
-      put_bf16(sm + SB_ACT, kmajor_off(t, c + q, kRows), h);
-      if (TRAIN) {
-        put_bf16(sm + SB_H2T, kmajor_off(c + q, t, kH2), h);
-        zrow[kH1 + c + q] = z;
-      }
-    }
-  }
+  hidden(kH2, oB2, kH1, sm + SB_H2T);
   // layer 3 and the linear head
-  stage_b(sm + SB_B, net.w3, kH3, kH2);
+  stage_rows(sm + SB_B, net.w3, kH3, kH2);
   ok &= umma::tile_gemm(sm + SB_ACT, sm + SB_B, kH3, kH2, tmem, bar, phase);
   float y = net.theta[oB4];
-  for (int c = 0; c < kH3; c += 8) {
-    float v[8];
-    umma::tmem_ld8(lane_addr + c, v);
+  for (int c = 0; c < kH3; c += 32) {
+    float v[32];
+    umma::tmem_ld32(lane_addr + c, v);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < 32; ++q) {
       const float z = v[q] + net.theta[oB3 + c + q];
       y += net.theta[oW4 + c + q] * silu(z);
-      if (TRAIN) zrow[kH1 + kH2 + c + q] = z;
+      zt[kRows * (kH1 + kH2 + c + q)] = z;
     }
   }
   return y;
@@ -197,6 +241,32 @@ __device__ __forceinline__ void warp_add(float* dst, float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(dst, v);
+}
+// the warp's sums of 32 columns added to dst[0..31]: at each halving a lane
+// keeps the half of the columns that its lane bit names and gives away the
+// other, 31 shuffles instead of 160, and lane l ends with column l
+__device__ __forceinline__ void warp_add32(float* dst, float (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      if (q < o) {
+        const float give = up ? v[q] : v[q + o], keep = up ? v[q + o] : v[q];
+        v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+  }
+  atomicAdd(dst + lane, v[0]);
+}
+// 32 consecutive gradients of this thread's row added to dst (16-byte aligned),
+// four per instruction
+__device__ __forceinline__ void row_add32(float* dst, const float (&v)[32]) {
+#pragma unroll
+  for (int q = 0; q < 32; q += 4)
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + q), "f"(v[q]), "f"(v[q + 1]),
+                 "f"(v[q + 2]), "f"(v[q + 3])
+                 : "memory");
 }
 
 // One training tile: forward, weighted squared-error gradient (dy = scale x
@@ -224,80 +294,72 @@ __global__ void __launch_bounds__(128) k_mlp_train_tile(Net net, const float* __
   bool ok = true;
   const long long gi = base + (long long)blockIdx.x * kRows + t;
   const long long s = (long long)(((unsigned long long)gi * pa + pb) & (unsigned long long)(n - 1));
-  float* zrow = zbuf + ((long long)blockIdx.x * kRows + t) * (kH1 + kH2 + kH3);
-  const float y = forward_tile<true>(net, X + s * kIn, sm, tmem, &bar, phase, zrow, ok);
+  float* zt = zbuf + (long long)blockIdx.x * kRows * (kH1 + kH2 + kH3) + t;
+  const float y = forward_tile(net, X + s * kIn, sm, tmem, &bar, phase, zt, ok);
   const float e = y - label[s];
   const float wt = weight ? weight[s] : 1.f;
   warp_add(loss, wt * e * e);
   const float dy = scale * wt * e;
   // head: dW4 = sum dy h3, db4 = sum dy; delta3 = dy W4 silu'(z3)
   warp_add(grad + oB4, dy);
-  for (int j = 0; j < kH3; ++j) {
-    const float z = zrow[kH1 + kH2 + j];
-    warp_add(grad + oW4 + j, dy * silu(z));
-    const float d3 = dy * net.theta[oW4 + j] * dsilu(z);
-    warp_add(grad + oB3 + j, d3);
-    put_bf16(sm + SB_ACT, kmajor_off(t, j, kRows), d3);
-    put_bf16(sm + SB_DZT, kmajor_off(j, t, kRows), d3);
-    put_bf16(sm + SB_DZT, kmajor_off(j + kH3, t, kRows), 0.f);  // rows 64..127 of delta3^T are padding
+  for (int c = 0; c < kH3; c += 32) {
+    float h[32], d[32], none[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      const float z = zt[kRows * (kH1 + kH2 + c + q)];
+      h[q] = dy * silu(z);
+      d[q] = dy * net.theta[oW4 + c + q] * dsilu(z);
+      none[q] = 0.f;
+    }
+    put_row32(sm + SB_ACT, t, c, d);
+    put_col32(sm + SB_DZT, t, c, kRows, d);
+    put_col32(sm + SB_DZT, t, c + kH3, kRows, none);  // rows 64..127 of delta3^T are padding
+    warp_add32(grad + oW4 + c, h);
+    warp_add32(grad + oB3 + c, d);
   }
   // dW3 = delta3^T H2 (rows 0..63 of a 128 x 128 tile)
   ok &= umma::tile_gemm(sm + SB_DZT, sm + SB_H2T, kH2, kRows, tmem, &bar, phase);
-  if (t < kH3)
-    for (int c = 0; c < kH2; c += 8) {
-      float v[8];
-      umma::tmem_ld8(lane_addr + c, v);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) atomicAdd(grad + oW3 + t * kH2 + c + q, v[q]);
-    }
-  else
-    for (int c = 0; c < kH2; c += 8) {  // every lane of the warp takes part in tcgen05.ld
-      float v[8];
-      umma::tmem_ld8(lane_addr + c, v);
-    }
-  // dH2 = delta3 W3 -> delta2 = dH2 silu'(z2)
-  stage_b(sm + SB_B, net.w3t, kH2, kH3);
-  ok &= umma::tile_gemm(sm + SB_ACT, sm + SB_B, kH2, kH3, tmem, &bar, phase);
-  for (int c = 0; c < kH2; c += 8) {
-    float v[8];
-    umma::tmem_ld8(lane_addr + c, v);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float d2 = v[q] * dsilu(zrow[kH1 + c + q]);
-      warp_add(grad + oB2 + c + q, d2);
-      put_bf16(sm + SB_ACT, kmajor_off(t, c + q, kRows), d2);
-      put_bf16(sm + SB_DZT, kmajor_off(c + q, t, kRows), d2);
-    }
+  for (int c = 0; c < kH2; c += 32) {  // every lane of a warp takes part in tcgen05.ld
+    float v[32];
+    umma::tmem_ld32(lane_addr + c, v);
+    if (t < kH3) row_add32(grad + oW3 + t * kH2 + c, v);
   }
+  // a hidden layer's deltas, dH silu'(z), and its bias gradients
+  auto deltas = [&](int n, int ob, int z0, bool keep) {
+    for (int c = 0; c < n; c += 32) {
+      float v[32];
+      umma::tmem_ld32(lane_addr + c, v);
+#pragma unroll
+      for (int q = 0; q < 32; ++q) v[q] *= dsilu(zt[kRows * (z0 + c + q)]);
+      if (keep) put_row32(sm + SB_ACT, t, c, v);
+      put_col32(sm + SB_DZT, t, c, kRows, v);
+      warp_add32(grad + ob + c, v);
+    }
+  };
+  // dH2 = delta3 W3 -> delta2 = dH2 silu'(z2)
+  stage_rows(sm + SB_B, net.w3t, kH2, kH3);
+  ok &= umma::tile_gemm(sm + SB_ACT, sm + SB_B, kH2, kH3, tmem, &bar, phase);
+  deltas(kH2, oB2, kH1, true);
   // dW2 = delta2^T H1
   ok &= umma::tile_gemm(sm + SB_DZT, sm + SB_H1T, kH1, kRows, tmem, &bar, phase);
-  for (int c = 0; c < kH1; c += 8) {
-    float v[8];
-    umma::tmem_ld8(lane_addr + c, v);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) atomicAdd(grad + oW2 + t * kH1 + c + q, v[q]);
+  for (int c = 0; c < kH1; c += 32) {
+    float v[32];
+    umma::tmem_ld32(lane_addr + c, v);
+    row_add32(grad + oW2 + t * kH1 + c, v);
   }
   // dH1 = delta2 W2 -> delta1
-  stage_b(sm + SB_B, net.w2t, kH1, kH2);
+  stage_rows(sm + SB_B, net.w2t, kH1, kH2);
   ok &= umma::tile_gemm(sm + SB_ACT, sm + SB_B, kH1, kH2, tmem, &bar, phase);
-  for (int c = 0; c < kH1; c += 8) {
-    float v[8];
-    umma::tmem_ld8(lane_addr + c, v);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float d1 = v[q] * dsilu(zrow[c + q]);
-      warp_add(grad + oB1 + c + q, d1);
-      put_bf16(sm + SB_DZT, kmajor_off(c + q, t, kRows), d1);
-    }
-  }
+  deltas(kH1, oB1, 0, false);
   // dW1 = delta1^T X (the hi and lo halves both act through W1)
   ok &= umma::tile_gemm(sm + SB_DZT, sm + SB_XT, kIn2, kRows, tmem, &bar, phase);
-  for (int c = 0; c < kIn; c += 8) {
-    float v[8], w[8];
-    umma::tmem_ld8(lane_addr + c, v);
-    umma::tmem_ld8(lane_addr + kIn + c, w);
+  {
+    float v[32], w[32];
+    umma::tmem_ld32(lane_addr, v);
+    umma::tmem_ld32(lane_addr + kIn, w);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) atomicAdd(grad + oW1 + t * kIn + c + q, v[q] + w[q]);
+    for (int q = 0; q < 32; ++q) v[q] += w[q];
+    row_add32(grad + oW1 + t * kIn, v);
   }
   if (!ok && t == 0) atomicExch(err, 1);
   umma::fence_before();
@@ -335,41 +397,6 @@ __device__ __forceinline__ float tanh_hw(float x) {
 __device__ __forceinline__ float silu_bf16(float z) {
   const float h = 0.5f * z;
   return fmaf(h, tanh_hw(h), h);
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);  // a at the lower address
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// a weight matrix [n][k] (row-major BF16, 16-byte aligned rows) into the
-// B-operand layout, one 16-byte chunk per store
-__device__ __forceinline__ void stage_rows(unsigned char* dst, const __nv_bfloat16* __restrict__ w, int n, int k) {
-  for (int e = threadIdx.x; e < n * (k / 8); e += blockDim.x) {
-    const int c = e / n, r = e - c * n;
-    *reinterpret_cast<uint4*>(dst + kmajor_off(r, 8 * c, n)) =
-        *reinterpret_cast<const uint4*>(w + (size_t)r * k + 8 * c);
-  }
-}
-
-// row t of the tile: the sample's 32 FP32 inputs (from registers; zeros
-// past the end) as BF16 hi (k 0..31) and lo (k 32..63)
-__device__ __forceinline__ void stage_inputs_regs(unsigned char* act, const float4 (&xv)[kIn / 4], int t) {
-#pragma unroll
-  for (int c = 0; c < kIn / 8; ++c) {
-    const float4 a = xv[2 * c], b = xv[2 * c + 1];
-    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    float hi[8], lo[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      hi[q] = __bfloat162float(__float2bfloat16(v[q]));
-      lo[q] = v[q] - hi[q];
-    }
-    *reinterpret_cast<uint4*>(act + kmajor_off(t, 8 * c, kRows)) =
-        make_uint4(pack_bf16(hi[0], hi[1]), pack_bf16(hi[2], hi[3]), pack_bf16(hi[4], hi[5]), pack_bf16(hi[6], hi[7]));
-    *reinterpret_cast<uint4*>(act + kmajor_off(t, kIn + 8 * c, kRows)) =
-        make_uint4(pack_bf16(lo[0], lo[1]), pack_bf16(lo[2], lo[3]), pack_bf16(lo[4], lo[5]), pack_bf16(lo[6], lo[7]));
-  }
 }
 
 // a hidden layer's epilogue: row t of SiLU(D + bias) as the next A operand
@@ -876,6 +903,7 @@ struct icls_mlp {
   float *theta = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr;
   __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr, *w2t = nullptr, *w3t = nullptr;
   float* zbuf = nullptr;     // pre-activations of one batch
+  float* h_out = nullptr;    // pinned: icls_mlp_grad's gradient, loss and error flag
   long long zcap = 0;        // samples zbuf holds
   float* loss = nullptr;     // per-epoch loss sums
   int nloss = 0;
@@ -1036,6 +1064,7 @@ extern "C" int icls_mlp_destroy(icls_mlp* m) {
                   (void*)m->X, (void*)m->label, (void*)m->weight, (void*)m->extra, (void*)m->Xh, (void*)m->labelh,
                   (void*)m->weighth, (void*)m->extrah, (void*)m->yh})
     if (p) cudaFree(p);
+  if (m->h_out) cudaFreeHost(m->h_out);
   if (m->s) cudaStreamDestroy(m->s);
   delete m;
   return ICLS_OK;
@@ -1179,18 +1208,23 @@ extern "C" int icls_mlp_grad(icls_mlp* m, const void* X, const float* label, lon
     if (cudaMalloc(&m->loss, sizeof(float)) != cudaSuccess) return ICLS_E_NOMEM;
     m->nloss = 1;
   }
+  // the results come through one pinned buffer: one wait for all of them
+  if (!m->h_out && cudaMallocHost((void**)&m->h_out, sizeof(float) * (kParams + 2)) != cudaSuccess) return ICLS_E_NOMEM;
   cudaMemsetAsync(m->loss, 0, sizeof(float), m->s);
   cudaMemsetAsync(m->grad, 0, sizeof(float) * kParams, m->s);
   icls::k_mlp_train_tile<<<(unsigned)(n / 128), 128, icls::SB_TRAIN, m->s>>>(
       net_of(m), static_cast<const float*>(X), label, nullptr, n, 0, 1ull, 0ull, scale, m->zbuf, m->grad, m->loss,
       m->err);
-  rc = sync_err(m);
-  if (rc) return rc;
-  cudaMemcpy(grad, m->grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost);
-  float l = 0.f;
-  cudaMemcpy(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost);
-  if (loss) *loss = l;
-  cudaMemset(m->grad, 0, sizeof(float) * kParams);
+  cudaMemcpyAsync(m->h_out, m->grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost, m->s);
+  cudaMemcpyAsync(m->h_out + kParams, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->s);
+  cudaMemcpyAsync(m->h_out + kParams + 1, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->s);
+  cudaMemsetAsync(m->grad, 0, sizeof(float) * kParams, m->s);
+  if (cudaStreamSynchronize(m->s) != cudaSuccess || cudaGetLastError() != cudaSuccess) return ICLS_E_CUDA;
+  int err = 0;
+  std::memcpy(&err, m->h_out + kParams + 1, sizeof(err));
+  if (err) return ICLS_E_CUDA;
+  std::memcpy(grad, m->h_out, sizeof(float) * kParams);
+  if (loss) *loss = m->h_out[kParams];
   return ICLS_OK;
 }
 
