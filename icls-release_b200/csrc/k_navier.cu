@@ -238,77 +238,94 @@ __device__ __forceinline__ T corr_val(const Params& p, T d, double pp, double p0
 // tests are made once per thread: with the map, FP64 0.373 -> 0.293 ms and
 // FP32 0.257 -> 0.232 ms; 128 x 128 x 256 FP64 with a rho0 that divides 0.126 ->
 // 0.093 ms.
+// A thread takes `rows` rows upwards, whose lower neighbours' corrections and
+// own pressures it then has in registers: one row per thread read the p planes
+// three times through L2 (256^3: FP64 0.293 -> 0.266 ms, FP32 0.232 -> 0.167).
+// Rows and blocks per SM: FP64 4 and 4 (8 and 5: 0.273 ms), FP32 8 and 8 (4
+// and 6: 0.179 ms).
+template <typename T>
+constexpr int kCorRows = sizeof(T) == 4 ? 8 : 4;
 template <typename T, int RP>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 8 : 5)) k_correc_own(Params p, CorrArgs a) {
+__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 8 : 4)) k_correc_own(Params p, CorrArgs a, int rows) {
   const int i = 1 + BX * (int)blockIdx.x + (int)threadIdx.x, j = 1 + BY * (int)blockIdx.y + (int)threadIdx.y;
-  const int k = 1 + (int)blockIdx.z;
+  const int ka = 1 + rows * (int)blockIdx.z, kb = min(ka + rows - 1, p.kmax);
   if (i > p.imax || j > p.jmax) return;
   const int sy = p.nCx, sz = p.nCx * p.nCy;
-  const int c = i + sy * j + sz * k;
-  const int cx = i > 1 ? c - 1 : c + p.imax - 1, cy = j > 1 ? c - sy : c + sy * (p.jmax - 1), cz = c - sz;
+  int c = i + sy * j + sz * ka;
+  const int ox = i > 1 ? -1 : p.imax - 1, oy = j > 1 ? -sy : sy * (p.jmax - 1);
   const T* __restrict__ du = cT<T>(a.dudt);
   const T* __restrict__ dv = cT<T>(a.dvdt);
   const T* __restrict__ dw = cT<T>(a.dwdt);
   const double* __restrict__ pp = a.p;
   const int nsx = seg_row(p), sp = nsx * p.jmax;
-  const uint8_t* __restrict__ seg = a.seg + ((int)blockIdx.x + nsx * (j - 1) + sp * k);
-  const uint8_t own = seg[0], west = seg[blockIdx.x ? -1 : nsx - 1];
-  const uint8_t south = seg[j > 1 ? -nsx : sp - nsx], below = seg[-sp];
-  const double p0 = pp[c];
-  const double pe = pp[c + 1], pn = pp[c + sy], pu = pp[c + sz], pw = pp[cx], ps = pp[cy], pd = pp[cz];
-  const T d0 = du[c], d1 = dv[c], d2 = dw[c], e0 = du[cx], e1 = dv[cy], e2 = dw[cz];
-  T qx = TC(0.), qy = TC(0.), qz = TC(0.), qxm = TC(0.), qym = TC(0.), qzm = TC(0.);
-  if (own) {
-    qx = cT<T>(a.px)[c];
-    qy = cT<T>(a.py)[c];
-    qz = cT<T>(a.pz)[c];
-  }
-  if (own | west) qxm = cT<T>(a.px)[cx];
-  if (south) qym = cT<T>(a.py)[cy];
-  if (below) qzm = cT<T>(a.pz)[cz];
-  const T uu = corr_val<T, RP>(p, d0, pe, p0, qx, p.cdx);
-  const T vv = corr_val<T, RP>(p, d1, pn, p0, qy, p.cdy);
-  const T ww = (k == p.kmax) ? TC(0.) : corr_val<T, RP>(p, d2, pu, p0, qz, p.cdz);
-  // the cell-centre average's (i-1), (j-1) and (k-1) corrections
-  const T um = corr_val<T, RP>(p, e0, p0, pw, qxm, p.cdx);
-  const T vm = corr_val<T, RP>(p, e1, p0, ps, qym, p.cdy);
-  const T wl = corr_val<T, RP>(p, e2, p0, pd, qzm, p.cdz);
+  const uint8_t* __restrict__ seg = a.seg + ((int)blockIdx.x + nsx * (j - 1) + sp * ka);
+  const int ow = blockIdx.x ? -1 : nsx - 1, os = j > 1 ? -nsx : sp - nsx;
   T* __restrict__ u = mT<T>(a.u);
   T* __restrict__ v = mT<T>(a.v);
   T* __restrict__ w = mT<T>(a.w);
-  const int q = (i - 1) + p.imax * ((j - 1) + p.jmax * (k - 1));
-  u[c] = uu;
-  v[c] = vv;
-  w[c] = ww;
-  mT<T>(a.ucc)[q] = (um + uu) / TC(2.);
-  mT<T>(a.vcc)[q] = (vm + vv) / TC(2.);
-  mT<T>(a.wcc)[q] = (((k == 1) ? TC(0.) : wl) + ww) / TC(2.);
+  T* __restrict__ uc = mT<T>(a.ucc);
+  T* __restrict__ vc = mT<T>(a.vcc);
+  T* __restrict__ wc = mT<T>(a.wcc);
+  int q = (i - 1) + p.imax * ((j - 1) + p.jmax * (ka - 1));
   const bool ex = i == 1 || i == p.imax, ey = j == 1 || j == p.jmax;
-  if (!(ex | ey | (k == 1) | (k == p.kmax))) return;
-  // images and wall rows
-  const int di = ex ? (i == 1 ? p.imax : -p.imax) : 0, dj = ey ? sy * (j == 1 ? p.jmax : -p.jmax) : 0;
-  auto put = [&](T* __restrict__ f, int n, T x) {
-    f[n] = x;
-    if (di) f[n + di] = x;
-    if (dj) {
-      f[n + dj] = x;
-      if (di) f[n + di + dj] = x;
+  double p0 = pp[c];
+  // the correction of the row below, or the wall's
+  T wl = corr_val<T, RP>(p, dw[c - sz], p0, pp[c - sz], seg[-sp] ? cT<T>(a.pz)[c - sz] : TC(0.), p.cdz);
+  for (int k = ka; k <= kb; ++k) {
+    const uint8_t own = seg[0], west = seg[ow], south = seg[os];
+    const double pe = pp[c + 1], pn = pp[c + sy], pu = pp[c + sz], pw = pp[c + ox], ps = pp[c + oy];
+    const T d0 = du[c], d1 = dv[c], d2 = dw[c], e0 = du[c + ox], e1 = dv[c + oy];
+    T qx = TC(0.), qy = TC(0.), qz = TC(0.), qxm = TC(0.), qym = TC(0.);
+    if (own) {
+      qx = cT<T>(a.px)[c];
+      qy = cT<T>(a.py)[c];
+      qz = cT<T>(a.pz)[c];
     }
-  };
-  put(u, c, uu);
-  put(v, c, vv);
-  put(w, c, ww);
-  if (k == 1) {
-    put(u, c - sz, -uu);
-    put(v, c - sz, TC(2. * p.v_lower) - vv);
-    put(w, c - sz, TC(0.));
+    if (own | west) qxm = cT<T>(a.px)[c + ox];
+    if (south) qym = cT<T>(a.py)[c + oy];
+    const T uu = corr_val<T, RP>(p, d0, pe, p0, qx, p.cdx);
+    const T vv = corr_val<T, RP>(p, d1, pn, p0, qy, p.cdy);
+    const T ww = (k == p.kmax) ? TC(0.) : corr_val<T, RP>(p, d2, pu, p0, qz, p.cdz);
+    // the cell-centre average's (i-1) and (j-1) corrections
+    const T um = corr_val<T, RP>(p, e0, p0, pw, qxm, p.cdx);
+    const T vm = corr_val<T, RP>(p, e1, p0, ps, qym, p.cdy);
+    u[c] = uu;
+    v[c] = vv;
+    w[c] = ww;
+    uc[q] = (um + uu) / TC(2.);
+    vc[q] = (vm + vv) / TC(2.);
+    wc[q] = (((k == 1) ? TC(0.) : wl) + ww) / TC(2.);
+    if (ex | ey | (k == 1) | (k == p.kmax)) {  // images and wall rows
+      const int di = ex ? (i == 1 ? p.imax : -p.imax) : 0, dj = ey ? sy * (j == 1 ? p.jmax : -p.jmax) : 0;
+      auto put = [&](T* __restrict__ f, int n, T x) {
+        f[n] = x;
+        if (di) f[n + di] = x;
+        if (dj) {
+          f[n + dj] = x;
+          if (di) f[n + di + dj] = x;
+        }
+      };
+      put(u, c, uu);
+      put(v, c, vv);
+      put(w, c, ww);
+      if (k == 1) {
+        put(u, c - sz, -uu);
+        put(v, c - sz, TC(2. * p.v_lower) - vv);
+        put(w, c - sz, TC(0.));
+      }
+      if (k == p.kmax) {
+        put(u, c + sz, -uu);
+        put(v, c + sz, TC(2. * p.v_upper) - vv);
+        put(w, c + sz, wl);
+      }
+      if (i == 1 && j == 1 && k == 1 && isnan(vv)) a.dsc->nan_flag = 1;
+    }
+    wl = ww;
+    p0 = pu;
+    c += sz;
+    q += p.imax * p.jmax;
+    seg += sp;
   }
-  if (k == p.kmax) {
-    put(u, c + sz, -uu);
-    put(v, c + sz, TC(2. * p.v_upper) - vv);
-    put(w, c + sz, wl);
-  }
-  if (i == 1 && j == 1 && k == 1 && isnan(vv)) a.dsc->nan_flag = 1;
 }
 
 // The halo cells of shape C by number: the planes k = 0 and k = k1, then the
@@ -721,12 +738,17 @@ void launch_correc(Ctx& c, int fused_bc) {
   // images (ICLS_CORREC=shapec: one thread per shape-C cell)
   if (fused_bc && !c.correc_shapec) {
     const bool rp = c.P.rho0_pow2 != 0;
+    // several rows per thread while the blocks still fill every SM
+    dim3 g = gridI(c.P);
+    int rows = c.P.f32 ? kCorRows<float> : kCorRows<double>;
+    while (rows > 1 && (long long)g.x * g.y * ((g.z + rows - 1) / rows) < 8 * 148) rows /= 2;
+    g.z = (g.z + rows - 1) / rows;
     if (c.P.f32) {
-      if (rp) k_correc_own<float, 1><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a);
-      else k_correc_own<float, 0><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a);
+      if (rp) k_correc_own<float, 1><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
+      else k_correc_own<float, 0><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
     } else {
-      if (rp) k_correc_own<double, 1><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a);
-      else k_correc_own<double, 0><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a);
+      if (rp) k_correc_own<double, 1><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
+      else k_correc_own<double, 0><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
     }
     return;
   }
