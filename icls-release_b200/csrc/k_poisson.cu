@@ -87,45 +87,55 @@ __device__ __forceinline__ void smem_fft(double2* buf, int nl, int N, int logN, 
   }
 }
 
-// split Z (FFT of a+ib) into the scaled half-complex spectra of a and b
-__device__ __forceinline__ void unpack_hc(const double2* Z, int N, int n, double s, double& ha, double& hb) {
-  // position n of the half-complex output
-  if (n == 0) { ha = s * Z[0].x; hb = s * Z[0].y; return; }
-  if (n == N - 1) { ha = s * Z[N / 2].x; hb = s * Z[N / 2].y; return; }
-  const int k = (n + 1) >> 1;
-  const double2 zk = Z[k], zn = Z[N - k];
+// A real line's spectrum is stored as N/2 aligned (re, im) pairs: r_0 and
+// r_{N/2} share pair 0, pair k holds Re_k and Im_k.  (VFFTPACK's order, r_0,
+// Re_1, Im_1, ..., r_{N/2}, puts the pairs at odd places; the values and their
+// scaling are its, and only the eigenvalues' order has to follow.)  A pair is
+// one 16-byte access, and Z_k and Z_{N-k} give it once: the four transforms of
+// a 256^3 solve with fillps took 0.354 ms with one position per access and
+// take 0.337 ms.
+// Position n (from 0) of a line belongs to wavenumber:
+__host__ __device__ __forceinline__ int wave_of(int n, int N) { return n == 1 ? N / 2 : n >> 1; }
+
+// pair k of the scaled spectra of a and b from Z (the FFT of a + i b)
+__device__ __forceinline__ void unpack_pair(const double2* Z, int N, int k, double s, double2& ha, double2& hb) {
+  if (k == 0) {
+    ha = make_double2(s * Z[0].x, s * Z[N / 2].x);
+    hb = make_double2(s * Z[0].y, s * Z[N / 2].y);
+    return;
+  }
   // A_k = (Z_k + conj Z_{N-k})/2 ; B_k = (Z_k - conj Z_{N-k})/(2i)
-  if (n & 1) {  // real parts
-    ha = s * (0.5 * (zk.x + zn.x));
-    hb = s * (0.5 * (zk.y + zn.y));
-  } else {      // imaginary parts
-    ha = s * (0.5 * (zk.y - zn.y));
-    hb = s * (-0.5 * (zk.x - zn.x));
-  }
+  const double2 zk = Z[k], zn = Z[N - k];
+  ha = make_double2(s * (0.5 * (zk.x + zn.x)), s * (0.5 * (zk.y - zn.y)));
+  hb = make_double2(s * (0.5 * (zk.y + zn.y)), s * (-0.5 * (zk.x - zn.x)));
+}
+// position n of them
+__device__ __forceinline__ void unpack_hc(const double2* Z, int N, int n, double s, double& ha, double& hb) {
+  double2 a, b;
+  unpack_pair(Z, N, n >> 1, s, a, b);
+  ha = n & 1 ? a.y : a.x;
+  hb = n & 1 ? b.y : b.x;
 }
 
-// Z_k of the Hermitian pair built from two half-complex lines a, b
+// Z_k of the Hermitian pair a, b from their pairs of wavenumber min(k, N - k)
+__device__ __forceinline__ double2 pack_pair(double2 a, double2 b, int N, int k) {
+  if (k == 0) return make_double2(a.x, b.x);
+  if (k == N / 2) return make_double2(a.y, b.y);
+  if (k < N / 2) return make_double2(a.x - b.y, a.y + b.x);
+  return make_double2(a.x + b.y, -a.y + b.x);
+}
+// the pair that Z_k reads
+__device__ __forceinline__ int pair_of(int N, int k) { return k < N / 2 ? k : (k == N / 2 ? 0 : N - k); }
+// from two lines with stride st between positions
 __device__ __forceinline__ double2 pack_hc(const double* a, const double* b, int N, int k, long long st) {
-  if (k == 0) return make_double2(a[0], b[0]);
-  if (k == N / 2) return make_double2(a[(N - 1) * st], b[(N - 1) * st]);
-  if (k < N / 2) {
-    const double ar = a[(2 * k - 1) * st], ai = a[(2 * k) * st];
-    const double br = b[(2 * k - 1) * st], bi = b[(2 * k) * st];
-    return make_double2(ar - bi, ai + br);
-  }
-  const int m = N - k;
-  const double ar = a[(2 * m - 1) * st], ai = a[(2 * m) * st];
-  const double br = b[(2 * m - 1) * st], bi = b[(2 * m) * st];
-  return make_double2(ar + bi, -ai + br);
+  const long long m = 2 * pair_of(N, k) * st;
+  return pack_pair(make_double2(a[m], a[m + st]), make_double2(b[m], b[m + st]), N, k);
 }
-
-// the same from a column pair held as 16-byte vectors, ab[n * st] = (a_n, b_n)
+// from a column pair held as 16-byte vectors, ab[n * st] = (a_n, b_n)
 __device__ __forceinline__ double2 pack_hc2(const double2* __restrict__ ab, int N, int k, int st) {
-  if (k == 0) return ab[0];
-  if (k == N / 2) return ab[(N - 1) * st];
-  const int m = k < N / 2 ? k : N - k;
-  const double2 r = ab[(2 * m - 1) * st], q = ab[2 * m * st];
-  return k < N / 2 ? make_double2(r.x - q.y, q.x + r.y) : make_double2(r.x + q.y, -q.x + r.y);
+  const int m = 2 * pair_of(N, k) * st;
+  const double2 r = ab[m], q = ab[m + st];
+  return pack_pair(make_double2(r.x, q.x), make_double2(r.y, q.y), N, k);
 }
 
 // ---- x pass: lines (j,k) of length imax; CL complex lines per CTA --------
@@ -355,20 +365,16 @@ struct RhsArgs {
   const double* pj;
   const uint8_t* row;  // rows (j, k) whose p_jump may be nonzero; null: p_jump is not added
 };
+// (the velocities read by the caller: two lines that share a face read it once)
 template <typename T>
-__device__ __forceinline__ double rhs_at(const Params& p, const RhsArgs& r, long long c, bool add) {
-  const T* __restrict__ du = static_cast<const T*>(r.du);
-  const T* __restrict__ dv = static_cast<const T*>(r.dv);
-  const T* __restrict__ dw = static_cast<const T*>(r.dw);
+__device__ __forceinline__ double rhs_of(const Params& p, T u, T um, T v, T vm, T w, T wm) {
   // explicitly rounded operations: this file allows multiply-add
   // contraction, k_fillps (k_navier.cu) does not
   const double coef = p.rho0 / p.dt;
-  const double vel_x = __dmul_rn(__dsub_rn((double)du[c], (double)du[c - 1]), p.dxi);
-  const double vel_y = __dmul_rn(__dsub_rn((double)dv[c], (double)dv[c - p.nCx]), p.dyi);
-  const double vel_z = __dmul_rn(__dsub_rn((double)dw[c], (double)dw[c - (long long)p.nCx * p.nCy]), p.dzi);
-  double v = __dmul_rn(coef, __dadd_rn(__dadd_rn(vel_x, vel_y), vel_z));
-  if (add) v = __dadd_rn(v, r.pj[c]);
-  return v;
+  const double vel_x = __dmul_rn(__dsub_rn((double)u, (double)um), p.dxi);
+  const double vel_y = __dmul_rn(__dsub_rn((double)v, (double)vm), p.dyi);
+  const double vel_z = __dmul_rn(__dsub_rn((double)w, (double)wm), p.dzi);
+  return __dmul_rn(coef, __dadd_rn(__dadd_rn(vel_x, vel_y), vel_z));
 }
 
 // One CTA transforms LPC complex lines (2 LPC real lines).  YPASS false:
@@ -442,17 +448,30 @@ __global__ void __launch_bounds__(256, (R1 > 16 || R2 > 16) ? 1 : 2)
 #pragma unroll
     for (int n1 = 0; n1 < R1; ++n1) {
       const int n = R2 * n1 + lane;
-      if constexpr (RHS != 0) {  // dir 0: lines a and b start at columns 1 of (ja,ka), (jb,kb)
+      if constexpr (RHS != 0) {
+        // dir 0: lines a and b start at columns 1 of (ja, ka) and (ja + 1, ka)
+        // (periodic y: jmax is even)
         using T = typename std::conditional<RHS == 4, float, double>::type;
-        x[n1] = make_double2(rhs_at<T>(p, ra, idxC(p, 1, ja, ka) + n, adda),
-                             rhs_at<T>(p, ra, idxC(p, 1, jb, kb) + n, addb));
+        const T* __restrict__ du = static_cast<const T*>(ra.du);
+        const T* __restrict__ dv = static_cast<const T*>(ra.dv);
+        const T* __restrict__ dw = static_cast<const T*>(ra.dw);
+        const int sy = p.nCx, sz = p.nCx * p.nCy, c = 1 + n + sy * (ja + p.nCy * ka), d = c + sy;
+        const T v = dv[c];
+        double va = rhs_of<T>(p, du[c], du[c - 1], v, dv[c - sy], dw[c], dw[c - sz]);
+        double vb = rhs_of<T>(p, du[d], du[d - 1], dv[d], v, dw[d], dw[d - sz]);
+        if (adda) va = __dadd_rn(va, ra.pj[c]);
+        if (addb) vb = __dadd_rn(vb, ra.pj[d]);
+        x[n1] = make_double2(va, vb);
+      } else if constexpr (YPASS) {
+        // columns 2c and 2c + 1: imax is even, so the pair is 16-byte aligned
+        const double2* ab = reinterpret_cast<const double2*>(colbase);
+        x[n1] = dir == 0 ? ab[n * (p.imax / 2)] : pack_hc2(ab, N, n, p.imax / 2);
       } else {
-        if constexpr (YPASS) {
-          // columns 2c and 2c + 1: imax is even, so the pair is 16-byte aligned
-          const double2* ab = reinterpret_cast<const double2*>(colbase);
-          x[n1] = dir == 0 ? ab[n * (p.imax / 2)] : pack_hc2(ab, N, n, p.imax / 2);
+        if (dir == 0) {
+          x[n1] = make_double2(A[n], B[n]);
         } else {
-          x[n1] = dir == 0 ? make_double2(A[n * st], B[n * st]) : pack_hc(A, B, N, n, st);
+          const int m = pair_of(N, n);
+          x[n1] = pack_pair(reinterpret_cast<const double2*>(A)[m], reinterpret_cast<const double2*>(B)[m], N, n);
         }
       }
     }
@@ -529,15 +548,17 @@ __global__ void __launch_bounds__(256, (R1 > 16 || R2 > 16) ? 1 : 2)
   }
   __syncthreads();
   if (!live) return;
-  for (int n = lane; n < N; n += TPL) {
-    double ha, hb;
-    unpack_hc(Z, N, n, s, ha, hb);
+  for (int k = lane; k < N / 2; k += TPL) {
+    double2 ha, hb;
+    unpack_pair(Z, N, k, s, ha, hb);
     if (YPASS) {
-      reinterpret_cast<double2*>(colbase)[n * (p.imax / 2)] = make_double2(ha, hb);
+      double2* ab = reinterpret_cast<double2*>(colbase) + (long long)k * p.imax;
+      ab[0] = make_double2(ha.x, hb.x);
+      ab[p.imax / 2] = make_double2(ha.y, hb.y);
     } else {
-      const long long la = 2 * ((long long)blockIdx.x * LPC + lt);
-      spec[la * N + n] = ha;
-      spec[(la + 1) * N + n] = hb;
+      double2* line = reinterpret_cast<double2*>(spec) + 2 * ((long long)blockIdx.x * LPC + lt) * (N / 2);
+      line[k] = ha;
+      line[N / 2 + k] = hb;
     }
   }
 }
@@ -552,7 +573,8 @@ constexpr size_t fft2_smem() {
 // and the raw last divisor at k=kmax.  The pivots depend on (i,j) only
 // through xy = xrt(i) + yrt(j), and xrt(2m) = xrt(2m+1), yrt likewise, so
 // one column per distinct pair d = (i/2) + (imax/2+1) (j/2) serves every
-// (i,j) that shares it: (imax/2+1)(jmax/2+1) columns, L2-resident at 256^2.
+// (i,j) that shares it (wave_of): (imax/2+1)(jmax/2+1) columns, L2-resident at
+// 256^2.
 __host__ __device__ __forceinline__ long long pivot_columns(const Params& p) {
   return (long long)(p.imax / 2 + 1) * (p.jmax / 2 + 1);
 }
@@ -710,7 +732,7 @@ __global__ void __launch_bounds__(NTH, MB) k_thomas_seg(Params p, TridiagLines L
   const int i = (live ? q % p.imax : 0) + 1, m = (live ? q / p.imax : 0) + 1;
   const int nxd = p.imax / 2 + 1;
   double* col = YL ? spec + (i - 1) + (long long)p.imax * p.jmax * (m - 1) : spec + (i - 1) + (long long)p.imax * (m - 1);
-  const double* zc = zpiv + (i >> 1) + (long long)nxd * (YL ? m - 1 : m >> 1);
+  const double* zc = zpiv + wave_of(i - 1, p.imax) + (long long)nxd * (YL ? m - 1 : wave_of(m - 1, p.jmax));
   thomas_seg(col, L, live, zc, sh);
 }
 
@@ -721,7 +743,7 @@ __global__ void __launch_bounds__(128) k_thomas(Params p, const double* __restri
   const long long nxy = (long long)p.imax * p.jmax, nd = pivot_columns(p);
   if (q >= nxy) return;
   const int i = (int)(q % p.imax) + 1, j = (int)(q / p.imax) + 1;
-  thomas_line(spec + q, nxy, p.kmax, zpiv + (i >> 1) + (long long)(p.imax / 2 + 1) * (j >> 1), nd, a, c);
+  thomas_line(spec + q, nxy, p.kmax, zpiv + wave_of(i - 1, p.imax) + (long long)(p.imax / 2 + 1) * wave_of(j - 1, p.jmax), nd, a, c);
 }
 // solver2d_cos (solver.f90:245-283): lines along y, one thread per (i,k),
 // diagonal b(j) + xzrt(i,k); the distinct columns are (i>>1, k)
@@ -732,7 +754,7 @@ __global__ void __launch_bounds__(128) k_thomas_y(Params p, const double* __rest
   if (q >= nxz) return;
   const int i = (int)(q % p.imax) + 1, k = (int)(q / p.imax) + 1;
   thomas_line(spec + (i - 1) + (long long)p.imax * p.jmax * (k - 1), p.imax, p.jmax,
-              zpiv + (i >> 1) + (long long)(p.imax / 2 + 1) * (k - 1), nd, a, c);
+              zpiv + wave_of(i - 1, p.imax) + (long long)(p.imax / 2 + 1) * (k - 1), nd, a, c);
 }
 
 // VCOSQB (dir 0) / VCOSQF (dir 1) along z of every (i,j) line of spec, as
