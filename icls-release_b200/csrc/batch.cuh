@@ -63,8 +63,8 @@ __device__ __forceinline__ Col col_of(const Params& p, const LsTask& t, int loca
   if (c.i > p.imax) c.i -= p.imax;
   c.j = t.r.ya + c.Y;
   if (c.j > p.jmax) c.j -= p.jmax;
-  c.ka = t.r.z0 + ch * t.kc;
-  c.kb = (ch == t.nch - 1) ? t.r.z1 : c.ka + t.kc - 1;
+  c.ka = t.r.z0 + ch * t.kc + (ch ? t.head : 0);
+  c.kb = (ch == t.nch - 1) ? t.r.z1 : t.r.z0 + (ch + 1) * t.kc + t.head - 1;
   c.cxy = c.X >= t.r.cx0 && c.X <= t.r.cx1 && c.Y >= t.r.cy0 && c.Y <= t.r.cy1;
   return c;
 }

@@ -235,7 +235,7 @@ int allocate(Ctx& c) {
   if (cudaMalloc((void**)&c.band_count, sizeof(int)) != cudaSuccess) return ICLS_E_NOMEM;
   AL(c.drs, (size_t)P.L);
   c.red_cap = ((P.imax + TBX - 1) / TBX) * ((P.jmax + TBY - 1) / TBY);
-  c.hcap = c.red_cap * ((P.kmax + 2 + kHeavRows - 1) / kHeavRows);
+  c.hcap = std::max(c.red_cap * ((P.kmax + 2 + kHeavRows - 1) / kHeavRows), 3 * kHeavBlocks);
   // per-(tile, chunk) exact sums of H (4 words each) for every drop, then
   // the mass correction's area sums
   AL(c.hpart, (size_t)5 * P.L * c.hcap);
@@ -581,6 +581,7 @@ void update_materials(Ctx& c) {
   for (int l = 0; l < L; ++l) all[l] = l;
   std::vector<int> ntiles(L, 0);  // partial sums per drop: column tiles x z chunks
   for (LsBatch& b : make_batches(all, kHeavRows, [&](int l) { return c_region(c.P, c.win[l].box, 0); })) {
+    size_tiles(c.P, b, kHeavRows, 4, kHeavBlocks);
     for (int q = 0; q < b.n; ++q) {
       b.t[q].phi0 = c.lv[b.t[q].l];
       ntiles[b.t[q].l] = b.t[q].tx * b.t[q].ty * b.t[q].nch;
@@ -913,11 +914,7 @@ void reinit_batches(Ctx& c, std::vector<LsBatch>& bs) {
   const double dtau = 0.5 * dz;
   const double thr = dz * dz * dz * dz * dz;
   for (LsBatch& b : bs) {
-    // 8 rows per block, 5 (the fewest that hold a wall row and the two next
-    // to it) where 8 leave the SMs with two blocks or fewer (one drop at 64^3:
-    // 48 -> 34 us per stage)
-    set_tiles(b, kStageRows);
-    if (b.start[b.n] < 2 * 148) set_tiles(b, 5);
+    size_tiles(P, b, kStageRows, 2, 7 * 148);
     double xg[kTasks], xh[kTasks], og[kTasks];
     bool partial[kTasks];
     for (int q = 0; q < b.n; ++q) {
@@ -1174,6 +1171,7 @@ int gfm4p(Ctx& c) {
         t.out = member(c, t.l).fit;
       }
       const bool mlp = c.cfg.curvature_model == ICLS_CURV_MLP;
+      size_tiles(c.P, b, kStageRows, 2, 7 * 148);
       launch_curvature(c, b, nullptr, mlp);
       if (mlp) launch_mlp_curvature(c, b);
     }
@@ -1183,6 +1181,7 @@ int gfm4p(Ctx& c) {
         t.phi0 = c.lv[t.l];
         t.phis = member(c, t.l).fit;
       }
+      size_tiles(c.P, b, kStageRows, 2, 7 * 148);
       launch_jumps(c, b);
     }
   }

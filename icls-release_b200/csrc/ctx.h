@@ -27,11 +27,12 @@ constexpr int TBX = 32, TBY = 8;    // column tile of a batched launch
 // One drop's share of a batched launch.  A block of TBX x TBY threads
 // sweeps one column tile of the region over one chunk of z rows, each
 // thread walking its column upwards: chunk m covers rows z0 + m*kc ..
-// z0 + (m+1)*kc - 1, the last chunk runs to z1.  Every chunk holds at least
-// kc rows, so the rows a wall row extrapolates from lie in its chunk.
+// z0 + (m+1)*kc - 1, the last chunk runs to z1 (chunk 0 has `head` rows more).
+// The rows a wall row extrapolates from lie in its chunk: set_tiles gives every
+// chunk at least kc >= 5 rows, size_tiles lengthens those at a wall.
 struct LsTask {
   Region r;
-  int tx, ty, nch, kc;
+  int tx, ty, nch, kc, head;
   int l, flat;           // flat: a block takes 256 consecutive columns (else TBX x TBY tiles)
   double bg, bgg;        // far-field values of the apron: rows 0..k1 / ghost rows
   const double* phi0;    // RK base (read at the thread's own cell only)
@@ -119,6 +120,9 @@ inline dim3 ab2_grid(const Params& p, bool fp64, int& kc) {
 // z rows per chunk of update_materials' Heaviside sweep (one exact partial
 // sum per column tile and chunk)
 constexpr int kHeavRows = 8;
+// and half as many while a batch has fewer blocks than this (size_tiles): at
+// most 3 kHeavBlocks partials then
+constexpr int kHeavBlocks = 4 * 148;
 
 struct Ctx {
   // tensor maps of the TMA predictor for up to four sets of its 18 input
@@ -249,6 +253,7 @@ Region full_region(const Params& P);
 bool region_full(const Params& P, const Region& r);
 Region c_region(const Params& P, const Region& r, int apron);
 void set_tiles(LsBatch& b, int kc, bool flat = true);
+void size_tiles(const Params& p, LsBatch& b, int kc, int kmin, int blocks);
 // tube_construction; list: the band cells also into c.band_list (sets the batch's own tiles)
 void launch_tube(Ctx& c, LsBatch& b, bool list);
 void launch_adv_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,

@@ -1084,16 +1084,16 @@ __global__ void __launch_bounds__(NT) k_materials_final(Params p, const T* __res
 // warp takes the set ones in turn, a lane per cell.  f(sx, j, k, q) for
 // segment q, bytes(q, sx, j, k) true where it is to be visited.
 template <class Bytes, class F>
-__device__ __forceinline__ void for_segments(const Params& p, const Bytes& bytes, const F& f) {
+__device__ __forceinline__ void for_segments(const Params& p, int per, const Bytes& bytes, const F& f) {
   const int nsx = seg_row(p);
   const long long ns = seg_count(p), lane = threadIdx.x & 31;
   const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long W = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long g = w0; g * 32 < ns; g += W) {
-    const long long q = g * 32 + lane;
+  for (long long g = w0; g * per < ns; g += W) {
+    const long long q = g * per + lane;
     int sx = 0, j = 0, k = 0;
     bool on = false;
-    if (q < ns) {
+    if (lane < per && q < ns) {
       const long long r = q / nsx;
       sx = (int)(q - r * nsx);
       k = (int)(r / p.jmax);
@@ -1111,9 +1111,9 @@ __device__ __forceinline__ void for_segments(const Params& p, const Bytes& bytes
 
 // jiemian = 1 in the segments of a map (with the periodic images)
 template <typename T>
-__global__ void __launch_bounds__(NT) k_seg_reset(Params p, const uint8_t* __restrict__ seg, T* __restrict__ jiemian) {
+__global__ void __launch_bounds__(NT) k_seg_reset(Params p, int per, const uint8_t* __restrict__ seg, T* __restrict__ jiemian) {
   for_segments(
-      p, [&](long long q, int, int, int) { return seg[q] != 0; },
+      p, per, [&](long long q, int, int, int) { return seg[q] != 0; },
       [&](int sx, int j, int k) {
         const int i = 1 + kSeg * sx + (int)(threadIdx.x & 31);
         if (i <= p.imax) putC(p, jiemian, i, j, k, TC(1.));
@@ -1122,12 +1122,12 @@ __global__ void __launch_bounds__(NT) k_seg_reset(Params p, const uint8_t* __res
 // p_x, p_y, p_z = 0 in the segments of `faces`, p_jump = 0 in those of `lap`
 // (interior cells: gfm4p writes no others)
 template <typename T>
-__global__ void __launch_bounds__(NT) k_seg_clear_jumps(Params p, const uint8_t* __restrict__ faces,
+__global__ void __launch_bounds__(NT) k_seg_clear_jumps(Params p, int per, const uint8_t* __restrict__ faces,
                                                         const uint8_t* __restrict__ lap, T* __restrict__ px,
                                                         T* __restrict__ py, T* __restrict__ pz,
                                                         double* __restrict__ pjump) {
   for_segments(
-      p, [&](long long q, int, int, int) { return (faces[q] | lap[q]) != 0; },
+      p, per, [&](long long q, int, int, int) { return (faces[q] | lap[q]) != 0; },
       [&](int sx, int j, int k) {
         const int i = 1 + kSeg * sx + (int)(threadIdx.x & 31);
         const long long q = sx + (long long)seg_row(p) * ((j - 1) + (long long)p.jmax * k);
@@ -1145,7 +1145,7 @@ __global__ void __launch_bounds__(NT) k_seg_clear_jumps(Params p, const uint8_t*
 // domain at 256^3 x 48, where the whole sweep wrote all of them (FP64
 // 0.19 -> 0.05 ms, FP32 0.13 -> 0.05 ms with the reset of jiemian).
 template <typename T>
-__global__ void __launch_bounds__(NT) k_materials_seg(Params p, const uint8_t* __restrict__ cur,
+__global__ void __launch_bounds__(NT) k_materials_seg(Params p, int per, const uint8_t* __restrict__ cur,
                                                       const uint8_t* __restrict__ prev, const T* __restrict__ jiemian,
                                                       T* __restrict__ miu, T* __restrict__ rho, T* __restrict__ rho_u,
                                                       T* __restrict__ rho_v, T* __restrict__ rho_w) {
@@ -1153,7 +1153,7 @@ __global__ void __launch_bounds__(NT) k_materials_seg(Params p, const uint8_t* _
   const T rho1 = TC(p.rho1), rho2 = TC(p.rho2);
   const long long sz = (long long)p.nCx * p.nCy;
   for_segments(
-      p,
+      p, per,
       [&](long long q, int sx, int j, int k) {
         const long long qx = sx + 1 < nsx ? q + 1 : q - sx;
         const long long qy = j < p.jmax ? q + nsx : q - (long long)nsx * (p.jmax - 1);
@@ -1507,6 +1507,7 @@ void set_tiles(LsBatch& b, int kc, bool flat) {
       t.ty = (t.r.yn + TBY - 1) / TBY;
     }
     const int nz = t.r.z1 - t.r.z0 + 1;
+    t.head = 0;
     if (kc <= 0 || kc >= nz) {
       t.nch = 1;
       t.kc = nz;
@@ -1518,6 +1519,43 @@ void set_tiles(LsBatch& b, int kc, bool flat) {
     s += t.tx * t.ty * t.nch;
   }
   b.start[b.n] = s;
+}
+
+// Flat tiles with chunks of kc rows, halved down to kmin while the batch has
+// fewer than `blocks` blocks: few drops leave SMs idle, and the cells of a
+// chunk are worked off one after the other.  The chunks at a wall are
+// lengthened to the five rows -2..2 or k1-2..k1+2.  Lines and minima are set
+// where each sweep is launched, from microseconds per call at 8 / 4 / 2 rows (drops,
+// grid, blocks at 8 rows):
+//                         reinit stage   Heaviside     curvature     jumps
+//   one, 64^3 (128)       48 / 31 / 25   17 / 13 / 11  27 / 21 / 18  24 / 17 / 15
+//   one, 128^2 x 256 (385) 45 / 34 / 31   18 / 14 / 18  27 / 21 / 21  22 / 18 / 18
+//   10, 96 x 192 x 100 (3000) 210 / 212 / 245  40 / 52 / 85
+//   24, 256^3 (600)                                    65 / 53 / 51  34 / 27 / 30
+//   48, 256^3 (3000-7000) 775 / 868 / 1066  79 / 107 / 178  172 / 185 / 218  110 / 122 / 156
+void size_tiles(const Params& p, LsBatch& b, int kc, int kmin, int blocks) {
+  for (;; kc /= 2) {
+    int s = 0;
+    for (int q = 0; q < b.n; ++q) {
+      LsTask& t = b.t[q];
+      t.flat = 1;
+      t.tx = (t.r.xn * t.r.yn + TBX * TBY - 1) / (TBX * TBY);
+      t.ty = 1;
+      const int nz = t.r.z1 - t.r.z0 + 1, more = std::max(0, 5 - kc);
+      t.kc = kc;
+      t.head = t.r.z0 <= 0 ? more : 0;
+      t.nch = (nz - t.head - (t.r.z1 >= p.k1 ? more : 0)) / kc;
+      if (t.nch < 1) {
+        t.nch = 1;
+        t.kc = nz;
+        t.head = 0;
+      }
+      b.start[q] = s;
+      s += t.tx * t.nch;
+    }
+    b.start[b.n] = s;
+    if (s >= blocks || kc / 2 < kmin) return;
+  }
 }
 
 // ================================================================ launchers
@@ -1534,8 +1572,9 @@ void set_tiles(LsBatch& b, int kc, bool flat) {
 void launch_tube(Ctx& c, LsBatch& b, bool list) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "tube", 1);
-  // chunks of 16 rows: the register window along z is filled once per chunk
-  set_tiles(b, kTubeRows);
+  // the register window along z is filled once per chunk (one drop at 64^3:
+  // 8 rows 21.0 us, 4 rows 19.1, 2 rows 23.2)
+  size_tiles(c.P, b, kTubeRows, 4, 4 * 148);
   int* lo = c.d_bbox;
   int* hi = c.d_bbox + 5 * c.P.L;
   if (list) cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
@@ -1707,21 +1746,32 @@ void launch_volumes(Ctx& c, const double* outside, const int* ntiles) {
 }
 // the warps of a sweep over the segments: enough for one group of 32 each, at
 // most eight blocks per SM
+// map bytes per warp (for_segments), 32 halved down to 2 while the warps are
+// fewer than 2^14: a warp takes its set segments one after the other
+// (k_materials_seg with 32 / 8 / 4 / 2: 64^3 22.8 / 10.6 / 9.6 / 8.4 us,
+// 128^2 x 256 21.0 / 12.6 / 14.6 / 20.5 us; 256^3 x 48, 16 instead of 32: 35.0
+// for 37.3 us, but the jumps' clearing 20.2 for 18.0)
+int seg_per_warp(const Params& p) {
+  int per = 32;
+  while (per > 2 && seg_count(p) < ((long long)per << 14)) per /= 2;
+  return per;
+}
 unsigned seg_blocks(const Params& p) {
-  return (unsigned)std::min<long long>((seg_count(p) + 32 * (NT / 32) - 1) / (32 * (NT / 32)), kRedBlocks);
+  const int n = seg_per_warp(p) * (NT / 32);
+  return (unsigned)std::min<long long>((seg_count(p) + n - 1) / n, kRedBlocks);
 }
 void launch_seg_reset(Ctx& c, const uint8_t* seg) {
   Scope sc_(c.prof, c.s, "fill", 1);
-  BY_FORM(c, (k_seg_reset<float><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg, reinterpret_cast<float*>(c.jiemian))),
-          (k_seg_reset<double><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg, c.jiemian)));
+  BY_FORM(c, (k_seg_reset<float><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), seg, reinterpret_cast<float*>(c.jiemian))),
+          (k_seg_reset<double><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), seg, c.jiemian)));
 }
 void launch_seg_clear_jumps(Ctx& c, const uint8_t* faces, const uint8_t* lap) {
   Scope sc_(c.prof, c.s, "clear_jumps", 1);
   auto f = [](double* q) { return reinterpret_cast<float*>(q); };
   BY_FORM(c,
-          (k_seg_clear_jumps<float><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, faces, lap, f(c.px), f(c.py), f(c.pz),
+          (k_seg_clear_jumps<float><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), faces, lap, f(c.px), f(c.py), f(c.pz),
                                                                      c.pjump)),
-          (k_seg_clear_jumps<double><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, faces, lap, c.px, c.py, c.pz, c.pjump)));
+          (k_seg_clear_jumps<double><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), faces, lap, c.px, c.py, c.pz, c.pjump)));
 }
 // miu, rho and the face densities; cur and prev: the maps of jiemian (null:
 // one thread per cell of the whole arrays, ICLS_MATERIALS=rows1)
@@ -1730,7 +1780,7 @@ void launch_materials(Ctx& c, const uint8_t* cur, const uint8_t* prev) {
   auto go = [&](auto zero, auto view) {
     using T = decltype(zero);
     if (cur) {
-      k_materials_seg<T><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, cur, prev, view(c.jiemian), view(c.miu), view(c.rho),
+      k_materials_seg<T><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), cur, prev, view(c.jiemian), view(c.miu), view(c.rho),
                                                           view(c.rho_u), view(c.rho_v), view(c.rho_w));
       return;
     }

@@ -109,3 +109,23 @@ def test_band_list_equals_columns(grid, scheme, drops, precision):
     for name in ("u", "v", "w", "pnew", "jiemian", "curv"):
         assert np.array_equal(lists.download(name), cols.download(name)), name
     assert np.array_equal(lists.volumes()[0], cols.volumes()[0])
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32])
+def test_short_chunks_equal_long_ones(precision):
+    """A batch of twelve drops has chunks of eight rows, a drop alone
+    (ICLS_GROUP=1) chunks of two, longer at the walls that the upper and lower
+    drops' regions reach; every step reinitialises."""
+    h = 1.0 / 64
+    cfg = make_config(itot=96, jtot=96, ktot=45, lmax=12, lx=96 * h, ly=96 * h, lz=45 * h, timestep=1e-3, rho2=10.0,
+                      miu2=10.0, Re=100.0, We=0.5, v_wall_lower=-0.5, v_wall_upper=0.5, reinit_step=1,
+                      reinit_iter_max=2, precision=precision)
+    pos = [(12 + 24 * (l % 4), 16 + 32 * (l // 4), (10, 22, 34)[l % 3]) for l in range(12)]
+    ls = init_drops(cfg, [tuple(h * x for x in q) for q in pos], [8 * h] * 12, all_images=True)
+    one = run_steps(cfg, ls, 3, ICLS_GROUP="1")
+    all_ = run_steps(cfg, ls, 3)
+    for l in range(1, 13):
+        assert np.array_equal(one.download("lvset", l), all_.download("lvset", l)), l
+    for name in ("u", "v", "w", "pnew", "jiemian", "miu", "rho_u", "p_x", "p_y", "p_z", "p_jump"):
+        assert np.array_equal(one.download(name), all_.download(name)), name
+    assert np.array_equal(one.volumes()[0], all_.volumes()[0])
