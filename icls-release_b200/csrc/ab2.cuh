@@ -232,6 +232,7 @@ template <typename T, int PW, int MB, bool FAR>
 __global__ void __launch_bounds__(MX * MY, MB)
     k_ab2(Params p, MomArgs a, T* __restrict__ dudt, T* __restrict__ dvdt, T* __restrict__ dwdt,
           T* __restrict__ duold_out, T* __restrict__ dvold_out, T* __restrict__ dwold_out, int kc) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char ab2_dyn[];
   typedef T PT;  // the pressure term's arithmetic
   typedef T Plane[MSY][MSX];
@@ -429,7 +430,7 @@ void ab2_launch_far(Ctx& c, const MomArgs& a, int o) {
     cudaFuncSetAttribute(k_ab2<T, PW, MB, FAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, ab2_smem<T>());
     attr |= 1u << (dev & 31);
   }
-  k_ab2<T, PW, MB, FAR><<<grid, dim3(MX, MY, 1), ab2_smem<T>(), c.s>>>(
+  pdl(k_ab2<T, PW, MB, FAR>, grid, dim3(MX, MY, 1), ab2_smem<T>(), c.s)(
       c.P, a, ab2_ptr<T>(c.dudt), ab2_ptr<T>(c.dvdt), ab2_ptr<T>(c.dwdt), ab2_ptr<T>(c.duold[o]),
       ab2_ptr<T>(c.dvold[o]), ab2_ptr<T>(c.dwold[o]), kc);
 }

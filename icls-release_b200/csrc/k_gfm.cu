@@ -106,6 +106,7 @@ __device__ __forceinline__ T curvature_at(const Params& p, const T* __restrict__
 template <typename T>
 __global__ void __launch_bounds__(NT, 4) k_curvature(Params p, const __grid_constant__ LsBatch B, T* __restrict__ nrm_m,
                                                   MlpCell* __restrict__ rec, int* __restrict__ count, int cap) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -177,6 +178,7 @@ __device__ __forceinline__ T recurvature_at(const Params& p, const T* __restrict
 // re_curvature + boundc over the tasks' regions: phis (get_curvature) -> out
 template <typename T>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 6 : 5)) k_recurvature(Params p, const __grid_constant__ LsBatch B) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const T* __restrict__ cin = cT<T>(t.phis);
@@ -255,6 +257,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_jumps(Params p
                                               double* __restrict__ pjump, T* __restrict__ px,
                                               T* __restrict__ py, T* __restrict__ pz, uint8_t* __restrict__ seg,
                                               uint8_t* __restrict__ row) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const T* __restrict__ cv = cT<T>(t.phis);
@@ -329,6 +332,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_ipot_pair(Params p, const __grid_constant__ LsBatch B, const T* __restrict__ pn,
                                                   Region rn, double bgn, double bggn,
                                                   unsigned long long* __restrict__ out) {
+  pdl_wait();
   const LsTask& t = B.t[0];
   const T* pm = cT<T>(t.phi0);
   const Col c = col_of(p, t, (int)blockIdx.x);
@@ -376,24 +380,24 @@ void launch_curvature(Ctx& c, const LsBatch& b, double* nrm_m_out, bool collect)
   MlpCell* rec = collect ? reinterpret_cast<MlpCell*>(c.mlp_rec) : nullptr;
   if (collect) cudaMemsetAsync(c.mlp_count, 0, sizeof(int), c.s);
   if (c.P.f32)
-    k_curvature<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, reinterpret_cast<float*>(nrm_m_out), rec, c.mlp_count,
+    pdl(k_curvature<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, reinterpret_cast<float*>(nrm_m_out), rec, c.mlp_count,
                                                         c.mlp_cap);
   else
-    k_curvature<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, nrm_m_out, rec, c.mlp_count, c.mlp_cap);
+    pdl(k_curvature<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, nrm_m_out, rec, c.mlp_count, c.mlp_cap);
 }
 void launch_recurvature(Ctx& c, const LsBatch& b) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "recurvature", 1);
   if (c.P.f32)
-    k_recurvature<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b);
+    pdl(k_recurvature<float>, b.start[b.n], kTile, 0, c.s)(c.P, b);
   else
-    k_recurvature<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b);
+    pdl(k_recurvature<double>, b.start[b.n], kTile, 0, c.s)(c.P, b);
 }
 void launch_jumps(Ctx& c, const LsBatch& b) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "jumps", 1);
   auto go = [&](auto kernel, auto* px, auto* py, auto* pz) {
-    kernel<<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.pjump, px, py, pz, c.seg_jmp[0], c.row_jmp);
+    pdl(kernel, b.start[b.n], kTile, 0, c.s)(c.P, b, c.pjump, px, py, pz, c.seg_jmp[0], c.row_jmp);
   };
   if (c.P.f32) {
     auto f = [](double* q) { return reinterpret_cast<float*>(q); };
@@ -441,11 +445,11 @@ void launch_ipot(Ctx& c, double* dmin_dev) {
       set_tiles(b, 8);
       Scope sc_(c.prof, c.s, "ipot", 1);
       if (c.P.f32)
-        k_ipot_pair<float><<<b.start[1], kTile, 0, c.s>>>(c.P, b, reinterpret_cast<const float*>(c.lv[n]),
+        pdl(k_ipot_pair<float>, b.start[1], kTile, 0, c.s)(c.P, b, reinterpret_cast<const float*>(c.lv[n]),
                                                           c.win[n].valid, c.win[n].bg, c.win[n].bg_ghost,
                                                           o + m + (long long)c.P.L * n);
       else
-        k_ipot_pair<double><<<b.start[1], kTile, 0, c.s>>>(c.P, b, c.lv[n], c.win[n].valid, c.win[n].bg,
+        pdl(k_ipot_pair<double>, b.start[1], kTile, 0, c.s)(c.P, b, c.lv[n], c.win[n].valid, c.win[n].bg,
                                                            c.win[n].bg_ghost, o + m + (long long)c.P.L * n);
     }
 }

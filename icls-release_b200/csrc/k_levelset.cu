@@ -63,6 +63,7 @@ __device__ __forceinline__ bool interior(const Params& p, int i, int j, int k) {
 template <typename T>
 __global__ void __launch_bounds__(NT) k_band_extents(Params p, const T* __restrict__ phi, int l,
                                                      int* __restrict__ bbox_lo, int* __restrict__ bbox_hi) {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)NT + threadIdx.x;
   int lo[5] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX, INT_MAX};
   int hi[5] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN};
@@ -174,6 +175,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_tube(Params p,
                                              long long* __restrict__ cnt, int* __restrict__ bbox_lo,
                                              int* __restrict__ bbox_hi, BandCell* __restrict__ list,
                                              int* __restrict__ count) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -448,6 +450,7 @@ template <int SCHEME, typename T, int PW>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4)) k_adv_stage(Params p, const __grid_constant__ LsBatch B, int stage1,
                                                      double a_, double bb_, double fdt_, const T* __restrict__ vu,
                                                      const T* __restrict__ vv, const T* __restrict__ vw) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -543,6 +546,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4))
                const int* __restrict__ count, int stage1, double a_, double bb_, double fdt_,
                const T* __restrict__ vu, const T* __restrict__ vv, const T* __restrict__ vw,
                const InflateState* __restrict__ inf, const double* __restrict__ vin) {
+  pdl_wait();
   const int total = *count, stride = (int)gridDim.x * NT;
   const T a = TC(a_), bb = TC(bb_), fdt = TC(fdt_);
   const int sy = p.nLx, sz = p.nLx * p.nLy;
@@ -600,6 +604,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 5 : 4))
 template <typename T>
 __global__ void __launch_bounds__(NT) k_adv_ghosts(Params p, const __grid_constant__ LsBatch B, int stage1, double a_,
                                                    double bb_) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -622,6 +627,7 @@ __global__ void __launch_bounds__(NT) k_adv_ghosts(Params p, const __grid_consta
 // no stage moves), and the far-field value on the aprons
 template <typename T>
 __global__ void __launch_bounds__(NT) k_adv_rest(Params p, const __grid_constant__ LsBatch B) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -732,6 +738,7 @@ __device__ __forceinline__ T reinit_val(int stage, T f0, T fs, T dtau, T rhs) {
 template <typename T, int PW>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 4 : 3)) k_reinit_stage(Params p, const __grid_constant__ LsBatch B, int stage,
                                                         double dtau_, ReinitState* __restrict__ rs) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -816,6 +823,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 4 : 3)) k_reinit_stage(P
 }
 
 __global__ void k_reinit_reset(const __grid_constant__ LsBatch B, int maxiter, ReinitState* __restrict__ rs) {
+  pdl_wait();
   for (int q = threadIdx.x; q < B.n; q += blockDim.x) {
     ReinitState& s = rs[B.t[q].l];
     s.residual = 0.;
@@ -829,6 +837,7 @@ __global__ void k_reinit_reset(const __grid_constant__ LsBatch B, int maxiter, R
 // as the scalars of the last ls_reinit call
 __global__ void k_reinit_check(const __grid_constant__ LsBatch B, int it, int maxiter, double thr,
                                ReinitState* __restrict__ rs, DevScalars* __restrict__ dsc, int last_drop) {
+  pdl_wait();
   for (int q = threadIdx.x; q < B.n; q += blockDim.x) {
     const int l = B.t[q].l;
     ReinitState& s = rs[l];
@@ -875,6 +884,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedThreads) k_disp(Params p, const T* __restrict__ phi,
                                                       const T* __restrict__ ucc, const T* __restrict__ vcc,
                                                       const T* __restrict__ wcc, double* __restrict__ part) {
+  pdl_wait();
   double s[7] = {0., 0., 0., 0., 0., 0., 0.};
   const int rows = p.jmax * p.kmax;
   const int W = (int)((gridDim.x * kRedThreads) >> 5);
@@ -906,6 +916,7 @@ __global__ void __launch_bounds__(kRedThreads) k_disp(Params p, const T* __restr
 }
 __global__ void __launch_bounds__(kRedThreads) k_disp_final(const double* __restrict__ part, int nblk,
                                                             double* __restrict__ out) {
+  pdl_wait();
 #pragma unroll 1
   for (int q = 0; q < 7; ++q) {
     double s = 0.;
@@ -965,6 +976,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT, 4) k_heaviside(Params p, const __grid_constant__ LsBatch B,
                                                   T* __restrict__ jiemian, uint8_t* __restrict__ seg,
                                                   XSum* __restrict__ part, int cap) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -1020,6 +1032,7 @@ struct PerDrop {
 // (below 2^53), and lane 0 rounds the exact total once.
 __global__ void k_volumes(Params p, const XSum* __restrict__ part, int cap, PerDrop pd, int uniform, int nb_all,
                           double* __restrict__ vol, DevScalars* __restrict__ dsc) {
+  pdl_wait();
   const double N = (1. * p.imax * p.jmax) * p.kmax;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int l = warp; l < p.L; l += nw) {
@@ -1046,6 +1059,7 @@ __global__ void k_volumes(Params p, const XSum* __restrict__ part, int cap, PerD
 
 template <typename T>
 __global__ void __launch_bounds__(NT) k_fill(T* __restrict__ a, long long n, double v) {
+  pdl_wait();
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
     a[q] = TC(v);
 }
@@ -1055,6 +1069,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_materials_final(Params p, const T* __restrict__ jiemian, T* __restrict__ miu,
                                                         T* __restrict__ rho, T* __restrict__ rho_u,
                                                         T* __restrict__ rho_v, T* __restrict__ rho_w) {
+  pdl_wait();
   const int r0[3] = {0, 0, 0}, r1[3] = {p.i1, p.j1, p.k1};
   int i, j, k;
   if (!cell3(r0, r1, i, j, k)) return;
@@ -1112,6 +1127,7 @@ __device__ __forceinline__ void for_segments(const Params& p, int per, const Byt
 // jiemian = 1 in the segments of a map (with the periodic images)
 template <typename T>
 __global__ void __launch_bounds__(NT) k_seg_reset(Params p, int per, const uint8_t* __restrict__ seg, T* __restrict__ jiemian) {
+  pdl_wait();
   for_segments(
       p, per, [&](long long q, int, int, int) { return seg[q] != 0; },
       [&](int sx, int j, int k) {
@@ -1126,6 +1142,7 @@ __global__ void __launch_bounds__(NT) k_seg_clear_jumps(Params p, int per, const
                                                         const uint8_t* __restrict__ lap, T* __restrict__ px,
                                                         T* __restrict__ py, T* __restrict__ pz,
                                                         double* __restrict__ pjump) {
+  pdl_wait();
   for_segments(
       p, per, [&](long long q, int, int, int) { return (faces[q] | lap[q]) != 0; },
       [&](int sx, int j, int k) {
@@ -1149,6 +1166,7 @@ __global__ void __launch_bounds__(NT) k_materials_seg(Params p, int per, const u
                                                       const uint8_t* __restrict__ prev, const T* __restrict__ jiemian,
                                                       T* __restrict__ miu, T* __restrict__ rho, T* __restrict__ rho_u,
                                                       T* __restrict__ rho_v, T* __restrict__ rho_w) {
+  pdl_wait();
   const int nsx = seg_row(p);
   const T rho1 = TC(p.rho1), rho2 = TC(p.rho2);
   const long long sz = (long long)p.nCx * p.nCy;
@@ -1199,6 +1217,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_inflate_sums(Params p, const __grid_constant__ LsBatch B,
                                                      double* __restrict__ part_area,
                                                      XSum* __restrict__ part_heav, int cap) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -1258,6 +1277,7 @@ __global__ void __launch_bounds__(kFinalThreads)
     k_inflate_final(Params p, const __grid_constant__ LsBatch B, const double* __restrict__ part_area,
                     const XSum* __restrict__ part_heav, int cap, double istep_dt, double* __restrict__ vol,
                     const double* __restrict__ vol0, double* __restrict__ maxchk, InflateState* __restrict__ inf) {
+  pdl_wait();
   const LsTask& t = B.t[blockIdx.x];
   const int l = t.l, n = t.tx * t.ty * t.nch;
   double sa = 0.;
@@ -1296,6 +1316,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_inflate_base(Params p, const __grid_constant__ LsBatch B,
                                                      const InflateState* __restrict__ inf,
                                                      BandCell* __restrict__ list, int* __restrict__ count) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -1325,6 +1346,7 @@ __global__ void __launch_bounds__(NT) k_inflate_base(Params p, const __grid_cons
 template <typename T>
 __global__ void __launch_bounds__(NT) k_region_heav(Params p, const __grid_constant__ LsBatch B,
                                                     XSum* __restrict__ part, int cap) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -1345,6 +1367,7 @@ __global__ void __launch_bounds__(NT) k_region_heav(Params p, const __grid_const
 __global__ void __launch_bounds__(kFinalThreads)
     k_gain_final(Params p, const __grid_constant__ LsBatch B, const XSum* __restrict__ part, int cap,
                  const double* __restrict__ vol, const double* __restrict__ vol0, InflateState* __restrict__ inf) {
+  pdl_wait();
   const LsTask& t = B.t[blockIdx.x];
   const XSum hs = task_heav(t, part, cap);
   if (threadIdx.x != 0) return;
@@ -1358,6 +1381,7 @@ __global__ void __launch_bounds__(kFinalThreads)
 __global__ void __launch_bounds__(kFinalThreads)
     k_volume_now(Params p, const __grid_constant__ LsBatch B, const XSum* __restrict__ part, int cap,
                  double* __restrict__ vnow) {
+  pdl_wait();
   const LsTask& t = B.t[blockIdx.x];
   const XSum hs = task_heav(t, part, cap);
   if (threadIdx.x == 0) vnow[t.l] = 1. - xs_value(hs) / ((1. * p.imax * p.jmax) * p.kmax);
@@ -1368,6 +1392,7 @@ __global__ void __launch_bounds__(kFinalThreads)
 template <typename T>
 __global__ void __launch_bounds__(NT) k_region_blend(Params p, const __grid_constant__ LsBatch B,
                                                      const InflateState* __restrict__ inf) {
+  pdl_wait();
   const int ti = task_of(B);
   const LsTask& t = B.t[ti];
   const Col c = col_of(p, t, (int)blockIdx.x - B.start[ti]);
@@ -1387,6 +1412,7 @@ __global__ void __launch_bounds__(NT) k_region_blend(Params p, const __grid_cons
 // copies.  Reads only interior cells, writes only the others.
 template <typename T>
 __global__ void __launch_bounds__(NT) k_boundmls(Params p, T* __restrict__ y) {
+  pdl_wait();
   const int r0[3] = {-2, -2, -2}, r1[3] = {p.i1 + 2, p.j1 + 2, p.k1 + 2};
   int i, j, k;
   if (!cell3(r0, r1, i, j, k)) return;
@@ -1415,6 +1441,7 @@ __global__ void __launch_bounds__(NT) k_boundmls(Params p, T* __restrict__ y) {
 // drop's stored array valid everywhere, e.g. before a download)
 template <typename T>
 __global__ void __launch_bounds__(NT) k_materialize(Params p, Region r, double bg, double bgg, T* __restrict__ y) {
+  pdl_wait();
   const int r0[3] = {-2, -2, -2}, r1[3] = {p.i1 + 2, p.j1 + 2, p.k1 + 2};
   int i, j, k;
   if (!cell3(r0, r1, i, j, k)) return;
@@ -1423,10 +1450,12 @@ __global__ void __launch_bounds__(NT) k_materialize(Params p, Region r, double b
 
 // field conversions of the precision form (upload / download)
 __global__ void k_to_float(float* __restrict__ dst, const double* __restrict__ src, long long n) {
+  pdl_wait();
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
     dst[q] = (float)src[q];
 }
 __global__ void k_to_double(double* __restrict__ dst, const float* __restrict__ src, long long n) {
+  pdl_wait();
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
     dst[q] = (double)src[q];
 }
@@ -1579,8 +1608,8 @@ void launch_tube(Ctx& c, LsBatch& b, bool list) {
   int* hi = c.d_bbox + 5 * c.P.L;
   if (list) cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
   BandCell* l = list ? reinterpret_cast<BandCell*>(c.band_list) : nullptr;
-  BY_FORM(c, (k_tube<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)),
-          (k_tube<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)));
+  BY_FORM(c, (pdl(k_tube<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)),
+          (pdl(k_tube<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)));
 }
 
 void launch_band_extents(Ctx& c, int l) {
@@ -1588,8 +1617,8 @@ void launch_band_extents(Ctx& c, int l) {
   int* lo = c.d_bbox;
   int* hi = c.d_bbox + 5 * c.P.L;
   const unsigned g = (unsigned)(((long long)c.P.imax * c.P.jmax + NT - 1) / NT);
-  BY_FORM(c, (k_band_extents<float><<<g, NT, 0, c.s>>>(c.P, reinterpret_cast<const float*>(c.lv[l]), l, lo, hi)),
-          (k_band_extents<double><<<g, NT, 0, c.s>>>(c.P, c.lv[l], l, lo, hi)));
+  BY_FORM(c, (pdl(k_band_extents<float>, g, NT, 0, c.s)(c.P, reinterpret_cast<const float*>(c.lv[l]), l, lo, hi)),
+          (pdl(k_band_extents<double>, g, NT, 0, c.s)(c.P, c.lv[l], l, lo, hi)));
 }
 
 template <typename T>
@@ -1602,7 +1631,7 @@ void adv_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, doub
   // the FP32 form always takes the product by the reciprocal)
   const unsigned g = b.start[b.n];
   const bool pw = c.P.pow2 || sizeof(T) == 4;
-  auto go = [&](auto kernel) { kernel<<<g, kTile, 0, c.s>>>(c.P, b, stage1, a, bb, fdt, u, v, w); };
+  auto go = [&](auto kernel) { pdl(kernel, g, kTile, 0, c.s)(c.P, b, stage1, a, bb, fdt, u, v, w); };
   if (scheme == ICLS_HOUC5) {
     if (pw) go(k_adv_stage<ICLS_HOUC5, T, 1>);
     else go(k_adv_stage<ICLS_HOUC5, T, 0>);
@@ -1622,7 +1651,7 @@ void adv_band_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a,
   const BandCell* list = reinterpret_cast<const BandCell*>(c.band_list);
   const unsigned nb = (unsigned)std::min<long long>((need + NT - 1) / NT, 8 * 148);
   const bool pw = c.P.pow2 || sizeof(T) == 4;
-  auto go = [&](auto kernel) { kernel<<<nb, NT, 0, c.s>>>(c.P, b, list, c.band_count, stage1, a, bb, fdt, u, v, w, c.dinf, c.vin); };
+  auto go = [&](auto kernel) { pdl(kernel, nb, NT, 0, c.s)(c.P, b, list, c.band_count, stage1, a, bb, fdt, u, v, w, c.dinf, c.vin); };
   if (nb > 0) {
     if (scheme == ICLS_HOUC5) {
       if (pw) go(k_adv_band<ICLS_HOUC5, T, 1, INFL>);
@@ -1632,11 +1661,11 @@ void adv_band_launch(Ctx& c, const LsBatch& b, int scheme, int stage1, double a,
       else go(k_adv_band<ICLS_WENO5, T, 0, INFL>);
     }
   }
-  if (rest) k_adv_rest<T><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b);
+  if (rest) pdl(k_adv_rest<T>, b.start[b.n], kTile, 0, c.s)(c.P, b);
   if (walls) {
     LsBatch w1 = b;
     set_tiles(w1, 0);
-    k_adv_ghosts<T><<<w1.start[w1.n], kTile, 0, c.s>>>(c.P, w1, stage1, a, bb);
+    pdl(k_adv_ghosts<T>, w1.start[w1.n], kTile, 0, c.s)(c.P, w1, stage1, a, bb);
   }
 }
 bool holds_walls(const LsBatch& b) {
@@ -1658,8 +1687,8 @@ void launch_inflate_base(Ctx& c, const LsBatch& b) {
   Scope sc_(c.prof, c.s, "inflate_stage", 1);
   cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
   BandCell* l = reinterpret_cast<BandCell*>(c.band_list);
-  BY_FORM(c, (k_inflate_base<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf, l, c.band_count)),
-          (k_inflate_base<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf, l, c.band_count)));
+  BY_FORM(c, (pdl(k_inflate_base<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.dinf, l, c.band_count)),
+          (pdl(k_inflate_base<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.dinf, l, c.band_count)));
 }
 void launch_inflate_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                           long long need) {
@@ -1683,19 +1712,19 @@ void launch_reinit_stage(Ctx& c, const LsBatch& b, int stage, double dtau) {
   Scope sc_(c.prof, c.s, "reinit_stage", 1);
   const unsigned g = b.start[b.n];
   // the FP32 form takes the product by the reciprocal at any spacing
-  if (c.P.f32) k_reinit_stage<float, 1><<<g, kTile, 0, c.s>>>(c.P, b, stage, dtau, c.drs);
-  else if (c.P.pow2) k_reinit_stage<double, 1><<<g, kTile, 0, c.s>>>(c.P, b, stage, dtau, c.drs);
-  else k_reinit_stage<double, 0><<<g, kTile, 0, c.s>>>(c.P, b, stage, dtau, c.drs);
+  if (c.P.f32) pdl(k_reinit_stage<float, 1>, g, kTile, 0, c.s)(c.P, b, stage, dtau, c.drs);
+  else if (c.P.pow2) pdl(k_reinit_stage<double, 1>, g, kTile, 0, c.s)(c.P, b, stage, dtau, c.drs);
+  else pdl(k_reinit_stage<double, 0>, g, kTile, 0, c.s)(c.P, b, stage, dtau, c.drs);
 }
 void launch_reinit_reset(Ctx& c, const LsBatch& b, int maxiter) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "reinit_reset", 1);
-  k_reinit_reset<<<1, 64, 0, c.s>>>(b, maxiter, c.drs);
+  pdl(k_reinit_reset, 1, 64, 0, c.s)(b, maxiter, c.drs);
 }
 void launch_reinit_check(Ctx& c, const LsBatch& b, int it, int maxiter, double thr) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "reinit_check", 1);
-  k_reinit_check<<<1, 64, 0, c.s>>>(b, it, maxiter, thr, c.drs, c.dsc, c.P.L - 1);
+  pdl(k_reinit_check, 1, 64, 0, c.s)(b, it, maxiter, thr, c.drs, c.dsc, c.P.L - 1);
 }
 
 // the per-(tile, chunk) exact sums of H: hcap per drop (4 words each)
@@ -1705,9 +1734,9 @@ void launch_heaviside(Ctx& c, const LsBatch& b) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "heaviside", 1);
   BY_FORM(c,
-          (k_heaviside<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, reinterpret_cast<float*>(c.jiemian),
+          (pdl(k_heaviside<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, reinterpret_cast<float*>(c.jiemian),
                                                                 c.seg_mat[c.mat_cur], hparts(c), c.hcap)),
-          (k_heaviside<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.jiemian, c.seg_mat[c.mat_cur], hparts(c),
+          (pdl(k_heaviside<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.jiemian, c.seg_mat[c.mat_cur], hparts(c),
                                                                  c.hcap)));
 }
 
@@ -1715,20 +1744,20 @@ void launch_heaviside(Ctx& c, const LsBatch& b) {
 void launch_fill(Ctx& c, double* a, long long n, double v, bool tfield) {
   Scope sc_(c.prof, c.s, "fill", 1);
   if (tfield && c.P.f32)
-    k_fill<float><<<1184, NT, 0, c.s>>>(reinterpret_cast<float*>(a), n, v);
+    pdl(k_fill<float>, 1184, NT, 0, c.s)(reinterpret_cast<float*>(a), n, v);
   else
-    k_fill<double><<<1184, NT, 0, c.s>>>(a, n, v);
+    pdl(k_fill<double>, 1184, NT, 0, c.s)(a, n, v);
 }
 
 // outside/ntiles: per drop (null: every drop swept its whole grid)
 void launch_disp(Ctx& c, int l) {
   Scope sc_(c.prof, c.s, "disp", 2);
-  BY_FORM(c, (k_disp<float><<<kRedBlocks, kRedThreads, 0, c.s>>>(c.P, reinterpret_cast<const float*>(c.lv[l]),
+  BY_FORM(c, (pdl(k_disp<float>, kRedBlocks, kRedThreads, 0, c.s)(c.P, reinterpret_cast<const float*>(c.lv[l]),
                                                                   reinterpret_cast<const float*>(c.ucc),
                                                                   reinterpret_cast<const float*>(c.vcc),
                                                                   reinterpret_cast<const float*>(c.wcc), c.diag)),
-          (k_disp<double><<<kRedBlocks, kRedThreads, 0, c.s>>>(c.P, c.lv[l], c.ucc, c.vcc, c.wcc, c.diag)));
-  k_disp_final<<<1, kRedThreads, 0, c.s>>>(c.diag, kRedBlocks, c.diag + 7 * kRedBlocks);
+          (pdl(k_disp<double>, kRedBlocks, kRedThreads, 0, c.s)(c.P, c.lv[l], c.ucc, c.vcc, c.wcc, c.diag)));
+  pdl(k_disp_final, 1, kRedThreads, 0, c.s)(c.diag, kRedBlocks, c.diag + 7 * kRedBlocks);
 }
 
 void launch_volumes(Ctx& c, const double* outside, const int* ntiles) {
@@ -1741,7 +1770,7 @@ void launch_volumes(Ctx& c, const double* outside, const int* ntiles) {
   }
   // uniform: every drop swept whole, (kmax + 2) / kStageRows z chunks of
   // red_cap column tiles
-  k_volumes<<<1, 1024, 0, c.s>>>(c.P, hparts(c), c.hcap, o, uniform, c.red_cap * ((c.P.kmax + 2) / kHeavRows), c.dvol,
+  pdl(k_volumes, 1, 1024, 0, c.s)(c.P, hparts(c), c.hcap, o, uniform, c.red_cap * ((c.P.kmax + 2) / kHeavRows), c.dvol,
                                 c.dsc);
 }
 // the warps of a sweep over the segments: enough for one group of 32 each, at
@@ -1762,16 +1791,16 @@ unsigned seg_blocks(const Params& p) {
 }
 void launch_seg_reset(Ctx& c, const uint8_t* seg) {
   Scope sc_(c.prof, c.s, "fill", 1);
-  BY_FORM(c, (k_seg_reset<float><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), seg, reinterpret_cast<float*>(c.jiemian))),
-          (k_seg_reset<double><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), seg, c.jiemian)));
+  BY_FORM(c, (pdl(k_seg_reset<float>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), seg, reinterpret_cast<float*>(c.jiemian))),
+          (pdl(k_seg_reset<double>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), seg, c.jiemian)));
 }
 void launch_seg_clear_jumps(Ctx& c, const uint8_t* faces, const uint8_t* lap) {
   Scope sc_(c.prof, c.s, "clear_jumps", 1);
   auto f = [](double* q) { return reinterpret_cast<float*>(q); };
   BY_FORM(c,
-          (k_seg_clear_jumps<float><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), faces, lap, f(c.px), f(c.py), f(c.pz),
+          (pdl(k_seg_clear_jumps<float>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), faces, lap, f(c.px), f(c.py), f(c.pz),
                                                                      c.pjump)),
-          (k_seg_clear_jumps<double><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), faces, lap, c.px, c.py, c.pz, c.pjump)));
+          (pdl(k_seg_clear_jumps<double>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), faces, lap, c.px, c.py, c.pz, c.pjump)));
 }
 // miu, rho and the face densities; cur and prev: the maps of jiemian (null:
 // one thread per cell of the whole arrays, ICLS_MATERIALS=rows1)
@@ -1780,12 +1809,12 @@ void launch_materials(Ctx& c, const uint8_t* cur, const uint8_t* prev) {
   auto go = [&](auto zero, auto view) {
     using T = decltype(zero);
     if (cur) {
-      k_materials_seg<T><<<seg_blocks(c.P), NT, 0, c.s>>>(c.P, seg_per_warp(c.P), cur, prev, view(c.jiemian), view(c.miu), view(c.rho),
+      pdl(k_materials_seg<T>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), cur, prev, view(c.jiemian), view(c.miu), view(c.rho),
                                                           view(c.rho_u), view(c.rho_v), view(c.rho_w));
       return;
     }
     const int r0[3] = {0, 0, 0}, r1[3] = {c.P.i1, c.P.j1, c.P.k1};
-    k_materials_final<T><<<grid_of(r0, r1), kBlock, 0, c.s>>>(c.P, view(c.jiemian), view(c.miu), view(c.rho),
+    pdl(k_materials_final<T>, grid_of(r0, r1), kBlock, 0, c.s)(c.P, view(c.jiemian), view(c.miu), view(c.rho),
                                                               view(c.rho_u), view(c.rho_v), view(c.rho_w));
   };
   BY_FORM(c, go(0.f, [](double* q) { return reinterpret_cast<float*>(q); }), go(0., [](double* q) { return q; }));
@@ -1799,56 +1828,56 @@ double* aparts(Ctx& c) { return c.hpart + (size_t)4 * c.P.L * c.hcap; }
 void launch_inflate_sums(Ctx& c, const LsBatch& b) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "inflate_sums", 2);
-  BY_FORM(c, (k_inflate_sums<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, aparts(c), hparts(c), c.hcap)),
-          (k_inflate_sums<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, aparts(c), hparts(c), c.hcap)));
-  k_inflate_final<<<b.n, kFinalThreads, 0, c.s>>>(c.P, b, aparts(c), hparts(c), c.hcap,
+  BY_FORM(c, (pdl(k_inflate_sums<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, aparts(c), hparts(c), c.hcap)),
+          (pdl(k_inflate_sums<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, aparts(c), hparts(c), c.hcap)));
+  pdl(k_inflate_final, b.n, kFinalThreads, 0, c.s)(c.P, b, aparts(c), hparts(c), c.hcap,
                                                   (double)c.cfg.inflate_step * c.dt, c.dvol, c.dvol0, c.dmaxchk,
                                                   c.dinf);
 }
 // gain-one inflation: the volume after it, and the blend
 void launch_region_heav(Ctx& c, const LsBatch& b) {
-  BY_FORM(c, (k_region_heav<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, hparts(c), c.hcap)),
-          (k_region_heav<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, hparts(c), c.hcap)));
+  BY_FORM(c, (pdl(k_region_heav<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, hparts(c), c.hcap)),
+          (pdl(k_region_heav<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, hparts(c), c.hcap)));
 }
 void launch_gain(Ctx& c, const LsBatch& b) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "gain_one", 2);
   launch_region_heav(c, b);
-  k_gain_final<<<b.n, kFinalThreads, 0, c.s>>>(c.P, b, hparts(c), c.hcap, c.dvol, c.dvol0, c.dinf);
+  pdl(k_gain_final, b.n, kFinalThreads, 0, c.s)(c.P, b, hparts(c), c.hcap, c.dvol, c.dvol0, c.dinf);
 }
 void launch_volume_now(Ctx& c, const LsBatch& b) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "gain_one", 2);
   launch_region_heav(c, b);
-  k_volume_now<<<b.n, kFinalThreads, 0, c.s>>>(c.P, b, hparts(c), c.hcap, c.dvolnow);
+  pdl(k_volume_now, b.n, kFinalThreads, 0, c.s)(c.P, b, hparts(c), c.hcap, c.dvolnow);
 }
 void launch_region_blend(Ctx& c, const LsBatch& b) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "gain_one", 1);
-  BY_FORM(c, (k_region_blend<float><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf)),
-          (k_region_blend<double><<<b.start[b.n], kTile, 0, c.s>>>(c.P, b, c.dinf)));
+  BY_FORM(c, (pdl(k_region_blend<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.dinf)),
+          (pdl(k_region_blend<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.dinf)));
 }
 
 void launch_boundmls(Ctx& c, double* phi) {
   Scope sc_(c.prof, c.s, "boundmls", 1);
   const int r0[3] = {-2, -2, -2}, r1[3] = {c.P.i1 + 2, c.P.j1 + 2, c.P.k1 + 2};
-  BY_FORM(c, (k_boundmls<float><<<grid_of(r0, r1), kBlock, 0, c.s>>>(c.P, reinterpret_cast<float*>(phi))),
-          (k_boundmls<double><<<grid_of(r0, r1), kBlock, 0, c.s>>>(c.P, phi)));
+  BY_FORM(c, (pdl(k_boundmls<float>, grid_of(r0, r1), kBlock, 0, c.s)(c.P, reinterpret_cast<float*>(phi))),
+          (pdl(k_boundmls<double>, grid_of(r0, r1), kBlock, 0, c.s)(c.P, phi)));
 }
 
 void launch_materialize(Ctx& c, const Region& r, double bg, double bgg, double* phi) {
   Scope sc_(c.prof, c.s, "materialize", 1);
   const int r0[3] = {-2, -2, -2}, r1[3] = {c.P.i1 + 2, c.P.j1 + 2, c.P.k1 + 2};
   BY_FORM(c,
-          (k_materialize<float><<<grid_of(r0, r1), kBlock, 0, c.s>>>(c.P, r, bg, bgg, reinterpret_cast<float*>(phi))),
-          (k_materialize<double><<<grid_of(r0, r1), kBlock, 0, c.s>>>(c.P, r, bg, bgg, phi)));
+          (pdl(k_materialize<float>, grid_of(r0, r1), kBlock, 0, c.s)(c.P, r, bg, bgg, reinterpret_cast<float*>(phi))),
+          (pdl(k_materialize<double>, grid_of(r0, r1), kBlock, 0, c.s)(c.P, r, bg, bgg, phi)));
 }
 
 void launch_to_float(Ctx& c, double* dst_f32, const double* src, long long n) {
-  k_to_float<<<1184, 256, 0, c.s>>>(reinterpret_cast<float*>(dst_f32), src, n);
+  pdl(k_to_float, 1184, 256, 0, c.s)(reinterpret_cast<float*>(dst_f32), src, n);
 }
 void launch_to_double(Ctx& c, double* dst, const double* src_f32, long long n) {
-  k_to_double<<<1184, 256, 0, c.s>>>(dst, reinterpret_cast<const float*>(src_f32), n);
+  pdl(k_to_double, 1184, 256, 0, c.s)(dst, reinterpret_cast<const float*>(src_f32), n);
 }
 
 }  // namespace icls

@@ -55,6 +55,7 @@ inline dim3 gridI(const Params& p) {
 template <typename T>
 __global__ void __launch_bounds__(NT) k_mom_main(Params p, MomArgs a, T* __restrict__ ru, T* __restrict__ rv,
                                                  T* __restrict__ rw) {
+  pdl_wait();
   int i, j, k;
   if (!cell3(kI0, cI1(p).v, i, j, k)) return;
   const long long q = idxI(p, i, j, k);
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(NT) k_mom_main(Params p, MomArgs a, T* __restr
 __global__ void __launch_bounds__(NT) k_ab2_near(Params p, const uint8_t* __restrict__ mat,
                                                  const uint8_t* __restrict__ jmp, const uint8_t* __restrict__ jmpold,
                                                  uint8_t* __restrict__ near) {
+  pdl_wait();
   const long long w = blockIdx.x * (long long)NT + threadIdx.x;
   if (4 * w >= seg_count(p)) return;
   // (the maps are padded with zeros to a multiple of four)
@@ -112,6 +114,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_fillps(Params p, const T* __restrict__ dudt, const T* __restrict__ dvdt,
                                                const T* __restrict__ dwdt, const double* __restrict__ pjump, int add,
                                                double* __restrict__ out) {
+  pdl_wait();
   int i, j, k;
   if (!cell3(kI0, cI1(p).v, i, j, k)) return;
   const long long q = idxI(p, i, j, k);
@@ -126,6 +129,7 @@ __global__ void __launch_bounds__(NT) k_fillps(Params p, const T* __restrict__ d
 }
 
 __global__ void __launch_bounds__(NT) k_add(Params p, double* __restrict__ a, const double* __restrict__ b) {
+  pdl_wait();
   const long long n = blockIdx.x * (long long)NT + threadIdx.x;
   if (n < p.nC) a[n] = a[n] + b[n];
 }
@@ -165,6 +169,7 @@ struct CorrArgs {
 // correc over the interior only (the separate reference call)
 template <typename T>
 __global__ void __launch_bounds__(NT) k_correc_interior(Params p, CorrArgs a) {
+  pdl_wait();
   int i, j, k;
   if (!cell3(kI0, cI1(p).v, i, j, k)) return;
   const long long c = idxC(p, i, j, k);
@@ -177,6 +182,7 @@ __global__ void __launch_bounds__(NT) k_correc_interior(Params p, CorrArgs a) {
 // (main.f90:159-160,190,207) over shape C
 template <typename T>
 __global__ void __launch_bounds__(NT) k_correc_fused(Params p, CorrArgs a) {
+  pdl_wait();
   int i, j, k;
   if (!cell3(kC0, cC1(p).v, i, j, k)) return;
   const long long n = idxC(p, i, j, k);
@@ -247,6 +253,7 @@ template <typename T>
 constexpr int kCorRows = sizeof(T) == 4 ? 8 : 4;
 template <typename T, int RP>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 8 : 4)) k_correc_own(Params p, CorrArgs a, int rows) {
+  pdl_wait();
   const int i = 1 + BX * (int)blockIdx.x + (int)threadIdx.x, j = 1 + BY * (int)blockIdx.y + (int)threadIdx.y;
   const int ka = 1 + rows * (int)blockIdx.z, kb = min(ka + rows - 1, p.kmax);
   if (i > p.imax || j > p.jmax) return;
@@ -371,6 +378,7 @@ __device__ __forceinline__ bool halo_cell(const Params& p, int q, int& i, int& j
 template <typename T>
 __global__ void __launch_bounds__(NT) k_bounduvw(Params p, T* __restrict__ u, T* __restrict__ v, T* __restrict__ w,
                                                  int halo) {
+  pdl_wait();
   const int q = (int)(blockIdx.x * NT + threadIdx.x);
   if (q >= halo) {
     const int e = q - halo;
@@ -399,6 +407,7 @@ __global__ void __launch_bounds__(NT) k_bounduvw(Params p, T* __restrict__ u, T*
 // boundp (bound.f90:182-287, BC_in_y='Periodic')
 template <typename T>
 __global__ void __launch_bounds__(NT) k_boundp(Params p, T* __restrict__ a, int halo) {
+  pdl_wait();
   const int q = (int)(blockIdx.x * NT + threadIdx.x);
   int i, j, k;
   if (q >= halo || !halo_cell(p, q, i, j, k)) return;
@@ -413,6 +422,7 @@ __global__ void __launch_bounds__(NT) k_boundp(Params p, T* __restrict__ a, int 
 template <typename T>
 __global__ void __launch_bounds__(NT) k_ywalls_uvw(Params p, T* __restrict__ u, T* __restrict__ v,
                                                    T* __restrict__ w, const double* __restrict__ vin) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1;
   if (i > p.imax) return;
   const long long f0 = idxC(p, i, 0, k), f1 = idxC(p, i, 1, k);
@@ -441,6 +451,7 @@ __global__ void __launch_bounds__(NT) k_ywalls_uvw(Params p, T* __restrict__ u, 
 // Dirichlet at an outflow end
 template <typename T>
 __global__ void __launch_bounds__(NT) k_ywalls_p(Params p, T* __restrict__ a) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1;
   if (i > p.imax) return;
   const T f = a[idxC(p, i, 1, k)], b = a[idxC(p, i, p.jmax, k)];
@@ -450,6 +461,7 @@ __global__ void __launch_bounds__(NT) k_ywalls_p(Params p, T* __restrict__ a) {
 // isnan(vnew(1,1,1)) (main.f90:207)
 template <typename T>
 __global__ void k_nan_probe(Params p, const T* __restrict__ v, DevScalars* __restrict__ dsc) {
+  pdl_wait();
   if (isnan(v[idxC(p, 1, 1, 1)])) dsc->nan_flag = 1;
 }
 
@@ -458,6 +470,7 @@ __global__ void k_nan_probe(Params p, const T* __restrict__ v, DevScalars* __res
 template <typename T>
 __global__ void __launch_bounds__(NT) k_gather_plane_x(const T* __restrict__ src, long long nx, long long nxy, long long ioff,
                                                        int n1, int n2, double* __restrict__ dst) {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)NT + threadIdx.x;
   if (q >= (long long)n1 * n2) return;
   const long long j = q % n1, k = q / n1;
@@ -469,6 +482,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_average_vel(Params p, const T* __restrict__ u, const T* __restrict__ v,
                                                     const T* __restrict__ w, T* __restrict__ ucc, T* __restrict__ vcc,
                                                     T* __restrict__ wcc) {
+  pdl_wait();
   int i, j, k;
   if (!cell3(kI0, cI1(p).v, i, j, k)) return;
   const long long q = idxI(p, i, j, k);
@@ -487,6 +501,7 @@ __global__ void __launch_bounds__(NT) k_average_vel(Params p, const T* __restric
 constexpr int kNormThreads = 1024;
 __global__ void __launch_bounds__(kNormThreads) k_plane_norm(Params p, const double* __restrict__ pp,
                                                              DevScalars* __restrict__ dsc) {
+  pdl_wait();
   const long long n = (long long)p.nCx * p.nCy, base = idxC(p, 0, 0, 1);
   double s = 0.;
   for (long long e = threadIdx.x; e < n; e += kNormThreads) s += pp[base + e];
@@ -527,6 +542,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_pupdate(Params p, const double* __restrict__ pp,
                                                 T* __restrict__ pnew, T* __restrict__ pold, int first,
                                                 int normalise, DevScalars* __restrict__ dsc) {
+  pdl_wait();
   typedef typename Vec2<T>::type T2;
   const long long n = 2 * (blockIdx.x * (long long)NT + threadIdx.x);
   if (n >= p.nC) return;
@@ -555,6 +571,7 @@ __global__ void __launch_bounds__(NT) k_pupdate(Params p, const double* __restri
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) k_sum_interior(Params p, const T* __restrict__ a,
                                                               double* __restrict__ partial) {
+  pdl_wait();
   const int rows = p.jmax * p.kmax;
   const int W = (int)((gridDim.x * kRedThreads) >> 5);
   const int lane = threadIdx.x & 31;
@@ -575,6 +592,7 @@ __global__ void __launch_bounds__(kRedThreads) k_sum_interior(Params p, const T*
 }
 __global__ void __launch_bounds__(kRedThreads) k_stream_final(Params p, const double* __restrict__ partial, int nblk,
                                                               DevScalars* __restrict__ dsc) {
+  pdl_wait();
   double s = 0.;
   for (int b = threadIdx.x; b < nblk; b += kRedThreads) s += partial[b];
   s = block_sum<double, kRedThreads>(s);
@@ -587,6 +605,7 @@ __global__ void __launch_bounds__(kRedThreads) k_chkdiv(Params p, const T* __res
                                                         const T* __restrict__ w,
                                                         double* __restrict__ part_sum, double* __restrict__ part_max,
                                                         long long* __restrict__ part_loc) {
+  pdl_wait();
   double s = 0., m = 0.;
   long long loc = -1;
   for (int q = blockIdx.x * kRedThreads + threadIdx.x; q < (int)p.nI; q += gridDim.x * kRedThreads) {
@@ -619,6 +638,7 @@ __global__ void __launch_bounds__(kRedThreads) k_chkdiv(Params p, const T* __res
 }
 __global__ void k_chkdiv_final(const double* __restrict__ part_sum, const double* __restrict__ part_max,
                                const long long* __restrict__ part_loc, int nblk, DevScalars* __restrict__ dsc) {
+  pdl_wait();
   if (threadIdx.x) return;
   double s = 0., m = 0.;
   long long l = -1;
@@ -635,6 +655,7 @@ __global__ void k_chkdiv_final(const double* __restrict__ part_sum, const double
 template <typename T>
 __global__ void __launch_bounds__(NT) k_chkdt(Params p, const T* __restrict__ u, const T* __restrict__ v,
                                               const T* __restrict__ w, DevScalars* __restrict__ dsc) {
+  pdl_wait();
   double a = 0., b = 0., c = 0.;
   int i, j, k;
   const I3 hi = cC1(p);
@@ -656,6 +677,7 @@ __global__ void __launch_bounds__(NT) k_chkdt(Params p, const T* __restrict__ u,
 template <typename T>
 __global__ void __launch_bounds__(NT) k_maxvel(Params p, const T* __restrict__ ucc, const T* __restrict__ vcc,
                                                const T* __restrict__ wcc, DevScalars* __restrict__ dsc) {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)NT + threadIdx.x;
   double m = 0.;
   if (q < p.nI) {
@@ -699,7 +721,7 @@ void launch_ab2(Ctx& c) {
   MomArgs a = mom_args(c);
   if (far) {
     cudaMemsetAsync(c.ab2_near, 0, (size_t)seg_row(c.P) * ((c.P.jmax + kAb2Y - 1) / kAb2Y) * c.P.nCz, c.s);
-    k_ab2_near<<<nblocks((seg_count(c.P) + 3) / 4), NT, 0, c.s>>>(c.P, c.seg_mat[c.mat_cur], c.seg_jmp[0],
+    pdl(k_ab2_near, nblocks((seg_count(c.P) + 3) / 4), NT, 0, c.s)(c.P, c.seg_mat[c.mat_cur], c.seg_jmp[0],
                                                                   c.seg_jmp[1], c.ab2_near);
     a.near = c.ab2_near;
     if (c.p_dirty) cudaMemsetAsync(&c.dsc->p_bad, 1, sizeof(int), c.s);  // unknown: nonzero
@@ -717,20 +739,20 @@ void launch_mom_main(Ctx& c, double* du, double* dv, double* dw) {
   Scope sc_(c.prof, c.s, "mom_main", 1);
   MomArgs a = mom_args(c);
   if (c.P.f32)
-    k_mom_main<float><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a, fp<float>(du), fp<float>(dv), fp<float>(dw));
+    pdl(k_mom_main<float>, gridI(c.P), kBlock, 0, c.s)(c.P, a, fp<float>(du), fp<float>(dv), fp<float>(dw));
   else
-    k_mom_main<double><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a, du, dv, dw);
+    pdl(k_mom_main<double>, gridI(c.P), kBlock, 0, c.s)(c.P, a, du, dv, dw);
 }
 void launch_fillps(Ctx& c, int add_pjump) {
   Scope sc_(c.prof, c.s, "fillps", 1);
   if (c.P.f32)
-    k_fillps<float><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, fp<float>(c.dudt), fp<float>(c.dvdt), fp<float>(c.dwdt),
+    pdl(k_fillps<float>, gridI(c.P), kBlock, 0, c.s)(c.P, fp<float>(c.dudt), fp<float>(c.dvdt), fp<float>(c.dwdt),
                                                      c.pjump, add_pjump, c.p);
   else
-    k_fillps<double><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, c.dudt, c.dvdt, c.dwdt, c.pjump, add_pjump, c.p);
+    pdl(k_fillps<double>, gridI(c.P), kBlock, 0, c.s)(c.P, c.dudt, c.dvdt, c.dwdt, c.pjump, add_pjump, c.p);
 }
 void launch_add_pjump(Ctx& c) {
-  Scope sc_(c.prof, c.s, "add_pjump", 1); k_add<<<nblocks(c.P.nC), NT, 0, c.s>>>(c.P, c.p, c.pjump); }
+  Scope sc_(c.prof, c.s, "add_pjump", 1); pdl(k_add, nblocks(c.P.nC), NT, 0, c.s)(c.P, c.p, c.pjump); }
 void launch_correc(Ctx& c, int fused_bc) {
   Scope sc_(c.prof, c.s, "correc", 1);
   CorrArgs a = corr_args(c);
@@ -744,28 +766,28 @@ void launch_correc(Ctx& c, int fused_bc) {
     while (rows > 1 && (long long)g.x * g.y * ((g.z + rows - 1) / rows) < 8 * 148) rows /= 2;
     g.z = (g.z + rows - 1) / rows;
     if (c.P.f32) {
-      if (rp) k_correc_own<float, 1><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
-      else k_correc_own<float, 0><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
+      if (rp) pdl(k_correc_own<float, 1>, g, kBlock, 0, c.s)(c.P, a, rows);
+      else pdl(k_correc_own<float, 0>, g, kBlock, 0, c.s)(c.P, a, rows);
     } else {
-      if (rp) k_correc_own<double, 1><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
-      else k_correc_own<double, 0><<<g, kBlock, 0, c.s>>>(c.P, a, rows);
+      if (rp) pdl(k_correc_own<double, 1>, g, kBlock, 0, c.s)(c.P, a, rows);
+      else pdl(k_correc_own<double, 0>, g, kBlock, 0, c.s)(c.P, a, rows);
     }
     return;
   }
   if (c.P.f32) {
-    if (fused_bc) k_correc_fused<float><<<gridC(c.P), kBlock, 0, c.s>>>(c.P, a);
-    else k_correc_interior<float><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a);
+    if (fused_bc) pdl(k_correc_fused<float>, gridC(c.P), kBlock, 0, c.s)(c.P, a);
+    else pdl(k_correc_interior<float>, gridI(c.P), kBlock, 0, c.s)(c.P, a);
   } else {
-    if (fused_bc) k_correc_fused<double><<<gridC(c.P), kBlock, 0, c.s>>>(c.P, a);
-    else k_correc_interior<double><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, a);
+    if (fused_bc) pdl(k_correc_fused<double>, gridC(c.P), kBlock, 0, c.s)(c.P, a);
+    else pdl(k_correc_interior<double>, gridI(c.P), kBlock, 0, c.s)(c.P, a);
   }
 }
 void launch_bounduvw(Ctx& c, double* u, double* v, double* w) {
   Scope sc_(c.prof, c.s, "bounduvw", 1);
   const int halo = halo_cells(c.P);
   const unsigned g = nblocks(halo + halo_plane_cells(c.P));
-  if (c.P.f32) k_bounduvw<float><<<g, NT, 0, c.s>>>(c.P, fp<float>(u), fp<float>(v), fp<float>(w), halo);
-  else k_bounduvw<double><<<g, NT, 0, c.s>>>(c.P, u, v, w, halo);
+  if (c.P.f32) pdl(k_bounduvw<float>, g, NT, 0, c.s)(c.P, fp<float>(u), fp<float>(v), fp<float>(w), halo);
+  else pdl(k_bounduvw<double>, g, NT, 0, c.s)(c.P, u, v, w, halo);
   launch_ywalls_uvw(c, u, v, w);
 }
 inline dim3 grid_ik(const Params& p) { return dim3((unsigned)((p.imax + NT - 1) / NT), (unsigned)p.kmax, 1); }
@@ -773,41 +795,41 @@ void launch_boundp(Ctx& c, double* pp, bool tfield) {
   Scope sc_(c.prof, c.s, "boundp", 1);
   const int halo = halo_cells(c.P);
   if (tfield && c.P.f32) {
-    k_boundp<float><<<nblocks(halo), NT, 0, c.s>>>(c.P, fp<float>(pp), halo);
-    if (c.P.bcy != ICLS_BCY_PERIODIC) k_ywalls_p<float><<<grid_ik(c.P), NT, 0, c.s>>>(c.P, fp<float>(pp));
+    pdl(k_boundp<float>, nblocks(halo), NT, 0, c.s)(c.P, fp<float>(pp), halo);
+    if (c.P.bcy != ICLS_BCY_PERIODIC) pdl(k_ywalls_p<float>, grid_ik(c.P), NT, 0, c.s)(c.P, fp<float>(pp));
     return;
   }
-  k_boundp<double><<<nblocks(halo), NT, 0, c.s>>>(c.P, pp, halo);
+  pdl(k_boundp<double>, nblocks(halo), NT, 0, c.s)(c.P, pp, halo);
   launch_ywalls_p(c, pp);
 }
 void launch_ywalls_uvw(Ctx& c, double* u, double* v, double* w) {
   if (c.P.bcy == ICLS_BCY_PERIODIC) return;
   if (c.P.f32)
-    k_ywalls_uvw<float><<<grid_ik(c.P), NT, 0, c.s>>>(c.P, fp<float>(u), fp<float>(v), fp<float>(w), c.vin);
+    pdl(k_ywalls_uvw<float>, grid_ik(c.P), NT, 0, c.s)(c.P, fp<float>(u), fp<float>(v), fp<float>(w), c.vin);
   else
-    k_ywalls_uvw<double><<<grid_ik(c.P), NT, 0, c.s>>>(c.P, u, v, w, c.vin);
+    pdl(k_ywalls_uvw<double>, grid_ik(c.P), NT, 0, c.s)(c.P, u, v, w, c.vin);
 }
 void launch_ywalls_p(Ctx& c, double* pp) {
   if (c.P.bcy == ICLS_BCY_PERIODIC) return;
-  k_ywalls_p<double><<<grid_ik(c.P), NT, 0, c.s>>>(c.P, pp);
+  pdl(k_ywalls_p<double>, grid_ik(c.P), NT, 0, c.s)(c.P, pp);
 }
 void launch_gather_plane_x(Ctx& c, const double* d, bool f32, long long nx, long long ny, long long ioff, int n1,
                            int n2, double* dst) {
   const unsigned g = nblocks((long long)n1 * n2);
-  if (f32) k_gather_plane_x<float><<<g, NT, 0, c.s>>>(reinterpret_cast<const float*>(d), nx, nx * ny, ioff, n1, n2, dst);
-  else k_gather_plane_x<double><<<g, NT, 0, c.s>>>(d, nx, nx * ny, ioff, n1, n2, dst);
+  if (f32) pdl(k_gather_plane_x<float>, g, NT, 0, c.s)(reinterpret_cast<const float*>(d), nx, nx * ny, ioff, n1, n2, dst);
+  else pdl(k_gather_plane_x<double>, g, NT, 0, c.s)(d, nx, nx * ny, ioff, n1, n2, dst);
 }
 void launch_nan_probe(Ctx& c) {
-  if (c.P.f32) k_nan_probe<float><<<1, 1, 0, c.s>>>(c.P, fp<float>(c.v), c.dsc);
-  else k_nan_probe<double><<<1, 1, 0, c.s>>>(c.P, c.v, c.dsc);
+  if (c.P.f32) pdl(k_nan_probe<float>, 1, 1, 0, c.s)(c.P, fp<float>(c.v), c.dsc);
+  else pdl(k_nan_probe<double>, 1, 1, 0, c.s)(c.P, c.v, c.dsc);
 }
 void launch_average_vel(Ctx& c) {
   Scope sc_(c.prof, c.s, "average_vel", 1);
   if (c.P.f32)
-    k_average_vel<float><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, fp<float>(c.u), fp<float>(c.v), fp<float>(c.w),
+    pdl(k_average_vel<float>, gridI(c.P), kBlock, 0, c.s)(c.P, fp<float>(c.u), fp<float>(c.v), fp<float>(c.w),
                                                           fp<float>(c.ucc), fp<float>(c.vcc), fp<float>(c.wcc));
   else
-    k_average_vel<double><<<gridI(c.P), kBlock, 0, c.s>>>(c.P, c.u, c.v, c.w, c.ucc, c.vcc, c.wcc);
+    pdl(k_average_vel<double>, gridI(c.P), kBlock, 0, c.s)(c.P, c.u, c.v, c.w, c.ucc, c.vcc, c.wcc);
 }
 void launch_pressure_update(Ctx& c, int first) {
   Scope sc_(c.prof, c.s, "pressure_update", 2);
@@ -816,43 +838,43 @@ void launch_pressure_update(Ctx& c, int first) {
   const int norm = c.P.bcy == ICLS_BCY_PERIODIC || c.P.bcy == ICLS_BCY_WALLS;
   cudaMemsetAsync(&c.dsc->p_bad, 0, sizeof(int), c.s);
   c.p_dirty = false;
-  if (norm) k_plane_norm<<<1, kNormThreads, 0, c.s>>>(c.P, c.p, c.dsc);
+  if (norm) pdl(k_plane_norm, 1, kNormThreads, 0, c.s)(c.P, c.p, c.dsc);
   if (c.P.f32)
-    k_pupdate<float><<<nblocks((c.P.nC + 1) / 2), NT, 0, c.s>>>(c.P, c.p, fp<float>(c.pnew), fp<float>(c.pold), first, norm,
+    pdl(k_pupdate<float>, nblocks((c.P.nC + 1) / 2), NT, 0, c.s)(c.P, c.p, fp<float>(c.pnew), fp<float>(c.pold), first, norm,
                                                        c.dsc);
   else
-    k_pupdate<double><<<nblocks((c.P.nC + 1) / 2), NT, 0, c.s>>>(c.P, c.p, c.pnew, c.pold, first, norm, c.dsc);
+    pdl(k_pupdate<double>, nblocks((c.P.nC + 1) / 2), NT, 0, c.s)(c.P, c.p, c.pnew, c.pold, first, norm, c.dsc);
 }
 void launch_stream_vel(Ctx& c) {
   Scope sc_(c.prof, c.s, "stream_vel", 2);
-  if (c.P.f32) k_sum_interior<float><<<kRedBlocks, kRedThreads, 0, c.s>>>(c.P, fp<float>(c.v), c.partials);
-  else k_sum_interior<double><<<kRedBlocks, kRedThreads, 0, c.s>>>(c.P, c.v, c.partials);
-  k_stream_final<<<1, kRedThreads, 0, c.s>>>(c.P, c.partials, kRedBlocks, c.dsc);
+  if (c.P.f32) pdl(k_sum_interior<float>, kRedBlocks, kRedThreads, 0, c.s)(c.P, fp<float>(c.v), c.partials);
+  else pdl(k_sum_interior<double>, kRedBlocks, kRedThreads, 0, c.s)(c.P, c.v, c.partials);
+  pdl(k_stream_final, 1, kRedThreads, 0, c.s)(c.P, c.partials, kRedBlocks, c.dsc);
 }
 void launch_chkdiv(Ctx& c) {
   Scope sc_(c.prof, c.s, "chkdiv", 2);
   double* ps = c.partials;
   double* pm = c.partials + kRedBlocks;
   if (c.P.f32)
-    k_chkdiv<float><<<kRedBlocks, kRedThreads, 0, c.s>>>(c.P, fp<float>(c.u), fp<float>(c.v), fp<float>(c.w), ps, pm,
+    pdl(k_chkdiv<float>, kRedBlocks, kRedThreads, 0, c.s)(c.P, fp<float>(c.u), fp<float>(c.v), fp<float>(c.w), ps, pm,
                                                           c.lpartials);
   else
-    k_chkdiv<double><<<kRedBlocks, kRedThreads, 0, c.s>>>(c.P, c.u, c.v, c.w, ps, pm, c.lpartials);
-  k_chkdiv_final<<<1, 32, 0, c.s>>>(ps, pm, c.lpartials, kRedBlocks, c.dsc);
+    pdl(k_chkdiv<double>, kRedBlocks, kRedThreads, 0, c.s)(c.P, c.u, c.v, c.w, ps, pm, c.lpartials);
+  pdl(k_chkdiv_final, 1, 32, 0, c.s)(ps, pm, c.lpartials, kRedBlocks, c.dsc);
 }
 void launch_chkdt(Ctx& c) {
   Scope sc_(c.prof, c.s, "chkdt", 1);
   cudaMemsetAsync(&c.dsc->umax, 0, 3 * sizeof(double), c.s);
-  if (c.P.f32) k_chkdt<float><<<gridC(c.P), kBlock, 0, c.s>>>(c.P, fp<float>(c.u), fp<float>(c.v), fp<float>(c.w), c.dsc);
-  else k_chkdt<double><<<gridC(c.P), kBlock, 0, c.s>>>(c.P, c.u, c.v, c.w, c.dsc);
+  if (c.P.f32) pdl(k_chkdt<float>, gridC(c.P), kBlock, 0, c.s)(c.P, fp<float>(c.u), fp<float>(c.v), fp<float>(c.w), c.dsc);
+  else pdl(k_chkdt<double>, gridC(c.P), kBlock, 0, c.s)(c.P, c.u, c.v, c.w, c.dsc);
 }
 void launch_maxvel(Ctx& c) {
   Scope sc_(c.prof, c.s, "maxvel", 1);
   cudaMemsetAsync(&c.dsc->velmax, 0, sizeof(double), c.s);
   if (c.P.f32)
-    k_maxvel<float><<<nblocks(c.P.nI), NT, 0, c.s>>>(c.P, fp<float>(c.ucc), fp<float>(c.vcc), fp<float>(c.wcc), c.dsc);
+    pdl(k_maxvel<float>, nblocks(c.P.nI), NT, 0, c.s)(c.P, fp<float>(c.ucc), fp<float>(c.vcc), fp<float>(c.wcc), c.dsc);
   else
-    k_maxvel<double><<<nblocks(c.P.nI), NT, 0, c.s>>>(c.P, c.ucc, c.vcc, c.wcc, c.dsc);
+    pdl(k_maxvel<double>, nblocks(c.P.nI), NT, 0, c.s)(c.P, c.ucc, c.vcc, c.wcc, c.dsc);
 }
 
 }  // namespace icls

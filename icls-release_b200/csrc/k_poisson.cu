@@ -142,6 +142,7 @@ __device__ __forceinline__ double2 pack_hc2(const double2* __restrict__ ab, int 
 // dir 0: p (shape C interior) -> spec ; dir 1: spec -> p (+ boundp halos)
 __global__ void __launch_bounds__(FT) k_fft_x(Params p, int dir, int CL, int logN, const double2* __restrict__ tw,
                                               double* __restrict__ pp, double* __restrict__ spec, int halos) {
+  pdl_wait();
   extern __shared__ double2 sm[];
   const int N = p.imax;
   const int ld = N + 1;
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(FT) k_fft_x(Params p, int dir, int CL, int log
 // ---- y pass: columns (i,k) of length jmax, TI real columns per CTA -------
 __global__ void __launch_bounds__(FT) k_fft_y(Params p, int dir, int TI, int logN, const double2* __restrict__ tw,
                                               double* __restrict__ spec) {
+  pdl_wait();
   extern __shared__ double2 sm[];
   const int N = p.jmax;
   const int CL = TI / 2;
@@ -391,6 +393,7 @@ template <int R1, int R2, bool YPASS, int LPC, int RHS = 0>
 __global__ void __launch_bounds__(256, (R1 > 16 || R2 > 16) ? 1 : 2)
     k_fft2(Params p, int dir, const double2* __restrict__ tw, double* __restrict__ pp, double* __restrict__ spec,
            int halos, RhsArgs ra) {
+  pdl_wait();
   static_assert(RHS == 0 || !YPASS, "the right-hand side is formed in the forward x pass");
   constexpr int N = R1 * R2;
   constexpr int TPL = R1 > R2 ? R1 : R2;
@@ -584,6 +587,7 @@ __host__ __device__ __forceinline__ long long pivot_columns(const Params& p) {
 __global__ void k_thomas_setup(const double* __restrict__ eig, long long nd, int K, const double* __restrict__ a,
                                const double* __restrict__ b, const double* __restrict__ c,
                                double* __restrict__ zpiv) {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= nd) return;
   const double xy = eig[q];
@@ -726,6 +730,7 @@ __device__ __forceinline__ void thomas_seg(double* __restrict__ col, const Tridi
 template <bool YL, int NTH, int MB>
 __global__ void __launch_bounds__(NTH, MB) k_thomas_seg(Params p, TridiagLines L, const double* __restrict__ zpiv,
                                                         double* __restrict__ spec) {
+  pdl_wait();
   __shared__ double sh[2 * (NTH / SEGC) * (SEGC + 1)];
   const int q = (int)blockIdx.x * SEGC + (int)threadIdx.x;
   const bool live = q < L.nlines;
@@ -739,6 +744,7 @@ __global__ void __launch_bounds__(NTH, MB) k_thomas_seg(Params p, TridiagLines L
 // solver2d: lines along z, one thread per (i,j)
 __global__ void __launch_bounds__(128) k_thomas(Params p, const double* __restrict__ a, const double* __restrict__ c,
                                                 const double* __restrict__ zpiv, double* __restrict__ spec) {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long nxy = (long long)p.imax * p.jmax, nd = pivot_columns(p);
   if (q >= nxy) return;
@@ -749,6 +755,7 @@ __global__ void __launch_bounds__(128) k_thomas(Params p, const double* __restri
 // diagonal b(j) + xzrt(i,k); the distinct columns are (i>>1, k)
 __global__ void __launch_bounds__(128) k_thomas_y(Params p, const double* __restrict__ a, const double* __restrict__ c,
                                                   const double* __restrict__ zpiv, double* __restrict__ spec) {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long nxz = (long long)p.imax * p.kmax, nd = (long long)(p.imax / 2 + 1) * p.kmax;
   if (q >= nxz) return;
@@ -766,6 +773,7 @@ __global__ void __launch_bounds__(128) k_thomas_y(Params p, const double* __rest
 constexpr int CZ_TI = 32, CZ_ROWS = 4;
 constexpr int kCosqFftMaxN = 512;  // CZ_LINES x (N+1) complex values in shared memory
 __global__ void __launch_bounds__(256) k_cosq_z(Params p, const double* __restrict__ T, double* __restrict__ spec) {
+  pdl_wait();
   extern __shared__ double czx[];  // [kmax][CZ_TI]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i0 = 1 + CZ_TI * (int)blockIdx.x, j = 1 + (int)blockIdx.y;
@@ -813,6 +821,7 @@ constexpr int CZF_TI = 32, CZ_LINES = CZF_TI / 2;  // columns and complex lines 
 __device__ __forceinline__ int makhoul_pos(int k, int N) { return (k & 1) ? N - 1 - (k >> 1) : (k >> 1); }
 __global__ void __launch_bounds__(256) k_cosq_fft_z(Params p, int dir, int logN, const double2* __restrict__ tw,
                                                     const double2* __restrict__ cw, double* __restrict__ spec) {
+  pdl_wait();
   extern __shared__ double2 czb[];  // [CZ_LINES][N+1]
   const int N = p.kmax, ld = N + 1;
   const int i0 = 1 + CZF_TI * (int)blockIdx.x, j = 1 + (int)blockIdx.y;
@@ -924,7 +933,7 @@ void poisson_setup(Ctx& c) {
   cudaMemcpyAsync(c.twx, tx.data(), tx.size() * sizeof(double2), cudaMemcpyHostToDevice, c.s);
   cudaMemcpyAsync(c.twy, ty.data(), ty.size() * sizeof(double2), cudaMemcpyHostToDevice, c.s);
   const long long nd = pivot_columns(P);
-  k_thomas_setup<<<(unsigned)((nd + 127) / 128), 128, 0, c.s>>>(c.xyrt, nd, P.kmax, c.tri_a, c.tri_b, c.tri_c,
+  pdl(k_thomas_setup, (unsigned)((nd + 127) / 128), 128, 0, c.s)(c.xyrt, nd, P.kmax, c.tri_a, c.tri_b, c.tri_c,
                                                                  c.zpiv);
   cudaStreamSynchronize(c.s);  // host vectors above go out of scope
 }
@@ -1000,7 +1009,7 @@ void poisson_setup_cos(Ctx& c) {
   cudaMemcpyAsync(c.twy, tz.data(), tz.size() * sizeof(double2), cudaMemcpyHostToDevice, c.s);
   cudaMemcpyAsync(c.czw, wz.data(), wz.size() * sizeof(double2), cudaMemcpyHostToDevice, c.s);
   const long long nd = (long long)nxd * kmax;
-  k_thomas_setup<<<(unsigned)((nd + 127) / 128), 128, 0, c.s>>>(c.xyrt, nd, jtot, c.tri_a, c.tri_b, c.tri_c, c.zpiv);
+  pdl(k_thomas_setup, (unsigned)((nd + 127) / 128), 128, 0, c.s)(c.xyrt, nd, jtot, c.tri_a, c.tri_b, c.tri_c, c.zpiv);
   cudaStreamSynchronize(c.s);  // host vectors above go out of scope
 }
 
@@ -1018,13 +1027,13 @@ void launch_thomas(Ctx& c) {
   const unsigned g = (unsigned)((L.nlines + SEGC - 1) / SEGC);
   const int nseg = (L.K + SEGR - 1) / SEGR;
   if (nseg * SEGC <= 256) {
-    k_thomas_seg<YL, 256, 3><<<g, dim3(SEGC, nseg), 0, c.s>>>(P, L, c.zpiv, c.spec);
+    pdl(k_thomas_seg<YL, 256, 3>, g, dim3(SEGC, nseg), 0, c.s)(P, L, c.zpiv, c.spec);
   } else if (nseg * SEGC <= 512) {
-    k_thomas_seg<YL, 512, 1><<<g, dim3(SEGC, nseg), 0, c.s>>>(P, L, c.zpiv, c.spec);
+    pdl(k_thomas_seg<YL, 512, 1>, g, dim3(SEGC, nseg), 0, c.s)(P, L, c.zpiv, c.spec);
   } else {
     const unsigned g1 = (unsigned)((L.nlines + 127) / 128);
-    if (YL) k_thomas_y<<<g1, 128, 0, c.s>>>(P, c.tri_a, c.tri_c, c.zpiv, c.spec);
-    else k_thomas<<<g1, 128, 0, c.s>>>(P, c.tri_a, c.tri_c, c.zpiv, c.spec);
+    if (YL) pdl(k_thomas_y, g1, 128, 0, c.s)(P, c.tri_a, c.tri_c, c.zpiv, c.spec);
+    else pdl(k_thomas, g1, 128, 0, c.s)(P, c.tri_a, c.tri_c, c.zpiv, c.spec);
   }
 }
 
@@ -1053,8 +1062,7 @@ void fft2_launch(Ctx& c, int dir, const double2* tw, int halos, const RhsArgs& r
   }
   const long long units = Y ? (long long)(P.imax / (2 * LPC)) * P.kmax
                             : ((long long)P.jmax * P.kmax + 2 * LPC - 1) / (2 * LPC);
-  k_fft2<R1, R2, Y, LPC, RHS>
-      <<<(unsigned)units, 256, fft2_smem<R1, R2, LPC>(), c.s>>>(P, dir, tw, c.p, c.spec, halos, ra);
+  pdl(k_fft2<R1, R2, Y, LPC, RHS>, (unsigned)units, 256, fft2_smem<R1, R2, LPC>(), c.s)(P, dir, tw, c.p, c.spec, halos, ra);
 }
 // the lengths with a radix-3 factor: 16 lines per CTA where the columns tile
 // by 32 (y pass) and the lines need at most 16 threads, else 8
@@ -1148,12 +1156,12 @@ void solver2d_periodic(Ctx& c, int write_halos, const RhsArgs* ra) {
     if (P.f32) fft2_pass<false, 4>(c, 0, 0, *ra);
     else fft2_pass<false, 8>(c, 0, 0, *ra);
   } else if (!fft2_pass<false>(c, 0, 0)) {
-    k_fft_x<<<gx, FT, smx, c.s>>>(P, 0, CL, lx, c.twx, c.p, c.spec, 0);
+    pdl(k_fft_x, gx, FT, smx, c.s)(P, 0, CL, lx, c.twx, c.p, c.spec, 0);
   }
-  if (!fft2_pass<true>(c, 0, 0)) k_fft_y<<<gy, FT, smy, c.s>>>(P, 0, TI, ly, c.twy, c.spec);
+  if (!fft2_pass<true>(c, 0, 0)) pdl(k_fft_y, gy, FT, smy, c.s)(P, 0, TI, ly, c.twy, c.spec);
   launch_thomas<false>(c);
-  if (!fft2_pass<true>(c, 1, 0)) k_fft_y<<<gy, FT, smy, c.s>>>(P, 1, TI, ly, c.twy, c.spec);
-  if (!fft2_pass<false>(c, 1, write_halos)) k_fft_x<<<gx, FT, smx, c.s>>>(P, 1, CL, lx, c.twx, c.p, c.spec, write_halos);
+  if (!fft2_pass<true>(c, 1, 0)) pdl(k_fft_y, gy, FT, smy, c.s)(P, 1, TI, ly, c.twy, c.spec);
+  if (!fft2_pass<false>(c, 1, write_halos)) pdl(k_fft_x, gx, FT, smx, c.s)(P, 1, CL, lx, c.twx, c.p, c.spec, write_halos);
 }
 
 // solver2d_cos (solver.f90:202-317): x FFT, VCOSQB in z, Thomas in y,
@@ -1183,14 +1191,14 @@ void launch_solver2d_cos(Ctx& c, int write_halos) {
   const size_t smf = (size_t)CZ_LINES * (P.kmax + 1) * sizeof(double2);
   const dim3 gzf((unsigned)((P.imax + CZF_TI - 1) / CZF_TI), (unsigned)P.jmax, 1);
   auto cosq = [&](int dir) {
-    if (fz) k_cosq_fft_z<<<gzf, 256, smf, c.s>>>(P, dir, lz, c.twy, c.czw, c.spec);
-    else k_cosq_z<<<gz, 256, smz, c.s>>>(P, dir ? c.cosf : c.cosb, c.spec);
+    if (fz) pdl(k_cosq_fft_z, gzf, 256, smf, c.s)(P, dir, lz, c.twy, c.czw, c.spec);
+    else pdl(k_cosq_z, gz, 256, smz, c.s)(P, dir ? c.cosf : c.cosb, c.spec);
   };
-  if (!fft2_pass<false>(c, 0, 0)) k_fft_x<<<gx, FT, smx, c.s>>>(P, 0, CL, lx, c.twx, c.p, c.spec, 0);
+  if (!fft2_pass<false>(c, 0, 0)) pdl(k_fft_x, gx, FT, smx, c.s)(P, 0, CL, lx, c.twx, c.p, c.spec, 0);
   cosq(0);
   launch_thomas<true>(c);
   cosq(1);
-  if (!fft2_pass<false>(c, 1, write_halos)) k_fft_x<<<gx, FT, smx, c.s>>>(P, 1, CL, lx, c.twx, c.p, c.spec, write_halos);
+  if (!fft2_pass<false>(c, 1, write_halos)) pdl(k_fft_x, gx, FT, smx, c.s)(P, 1, CL, lx, c.twx, c.p, c.spec, write_halos);
   if (write_halos) launch_ywalls_p(c, c.p);
 }
 
