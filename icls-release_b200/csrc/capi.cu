@@ -216,7 +216,7 @@ int allocate(Ctx& c) {
     AL(c.xyrt, (size_t)(P.imax / 2 + 1) * P.kmax);                      // distinct xzrt
     AL(c.zpiv, (size_t)(P.imax / 2 + 1) * P.kmax * P.jmax);             // pivots per distinct (xrt, zrt)
     AL(c.tri_a, (size_t)P.jmax + 1); AL(c.tri_b, (size_t)P.jmax + 1); AL(c.tri_c, (size_t)P.jmax + 1);
-    AL(c.cosb, (size_t)P.kmax * P.kmax); AL(c.cosf, (size_t)P.kmax * P.kmax);
+    AL(c.cosb, cosq_coefs(P.kmax)); AL(c.cosf, cosq_coefs(P.kmax));
     AL(c.czw, (size_t)P.kmax);
   }
   AL(c.vin, (size_t)(P.i1 + 1) * (P.k1 + 1));

@@ -17,6 +17,7 @@
 namespace icls {
 
 constexpr int kRedBlocks = 1184;   // 8 x 148 SMs: fixed grid of the reduction kernels
+size_t cosq_coefs(int K);  // doubles in a cosine table (k_poisson.cu)
 constexpr int kCosqMaxN = 768;     // longest z line of solver2d_cos (one shared-memory tile)
 constexpr int kRedThreads = 256;
 constexpr int kMaxDropsParam = 256;  // drops whose far-field counts travel as a kernel parameter

@@ -22,6 +22,7 @@
 // flight), the N-point twiddles, one padded shared-memory exchange, and a
 // radix-R2 DFT in registers; other powers of two take radix-2 passes in
 // shared memory (k_fft_x, k_fft_y).
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -29,6 +30,13 @@
 #include "ctx.h"
 
 namespace icls {
+
+constexpr int CZ_ROWS = 8;  // rows of both products per warp of k_cosq_z
+// doubles in its table for lines of K
+size_t cosq_coefs(int K) {
+  const size_t H = (K + 1) / 2;
+  return (H + CZ_ROWS - 1) / CZ_ROWS * H * 2 * CZ_ROWS;
+}
 
 namespace {
 
@@ -765,45 +773,110 @@ __global__ void __launch_bounds__(128) k_thomas_y(Params p, const double* __rest
 }
 
 // VCOSQB (dir 0) / VCOSQF (dir 1) along z of every (i,j) line of spec, as
-// the matrix product out[m] = sum_k T[m][k] x[k] with the kmax x kmax table
-// T of the transform's definition (fft.f:120-124, 270-274).  A CTA holds 32
-// consecutive i of one j (all k) in shared memory; warp w forms rows
-// m = 4w.., 4 at a time, each lane one i, summing in k order with fused
-// multiply-adds.
-constexpr int CZ_TI = 32, CZ_ROWS = 4;
+// products with the transform's definition (fft.f:120-124, 270-274), any
+// length K.  The table's columns are even or odd about the middle of the line
+// (cos(pi m (2k+1)/2K) at k and K-1-k differ by (-1)^m), so with H = ceil(K/2):
+//   VCOSQB: out[2m] = sum_q T[2m][q] (x_q + x_{K-1-q}),
+//           out[2m+1] = sum_q T[2m+1][q] (x_q - x_{K-1-q}),   q < H;
+//   VCOSQF: out[k], out[K-1-k] = E_k + O_k, E_k - O_k,  k < H, with
+//           E_k = sum_q T[k][2q] x_{2q}, O_k = sum_q T[k][2q+1] x_{2q+1}:
+// two products of half the rows and half the columns either way.  A CTA
+// holds the two inputs of 32 consecutive i of one j in shared memory; a warp
+// forms CZ_ROWS rows of both products, each lane one i, in order of q with fused
+// multiply-adds.  W: the coefficients of group g of CZ_ROWS rows at q, the even
+// product's then the odd one's, adjacent, so a lane's 2 CZ_ROWS multiply-adds
+// take CZ_ROWS uniform 16-byte loads; a warp copies them into shared memory
+// CZ_Q steps at a time, the next ones under way meanwhile (one K x K product,
+// four rows and scalar loads per warp, bound by its loads: 128 x 90 x 75 35.5 ->
+// 15 us; uniform loads from global memory 23).
+constexpr int CZ_TI = 32, CZ_Q = 16;
 constexpr int kCosqFftMaxN = 512;  // CZ_LINES x (N+1) complex values in shared memory
-__global__ void __launch_bounds__(256) k_cosq_z(Params p, const double* __restrict__ T, double* __restrict__ spec) {
+__global__ void __launch_bounds__(256) k_cosq_z(Params p, int dir, const double2* __restrict__ W,
+                                                double* __restrict__ spec) {
   pdl_wait();
-  extern __shared__ double czx[];  // [kmax][CZ_TI]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  extern __shared__ double2 czx[];  // [H][CZ_TI]: the even and the odd product's inputs
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int i0 = 1 + CZ_TI * (int)blockIdx.x, j = 1 + (int)blockIdx.y;
-  const int K = p.kmax;
+  const int K = p.kmax, H = (K + 1) / 2;
   const long long plane = (long long)p.imax * p.jmax;
-  double* __restrict__ base = spec + (i0 - 1) + (long long)p.imax * (j - 1);
-  const int ni = min(CZ_TI, p.imax - i0 + 1);
-  for (int t = threadIdx.x; t < K * CZ_TI; t += blockDim.x) {
-    const int k = t / CZ_TI, l = t - k * CZ_TI;
-    czx[t] = l < ni ? base[l + plane * k] : 0.;
+  double* __restrict__ base = spec + (i0 - 1) + (long long)p.imax * (j - 1) + lane;
+  const bool ok = lane < p.imax - i0 + 1;
+  __shared__ double2 coef[8][CZ_Q * CZ_ROWS];
+#pragma unroll 4
+  for (int q = warp; q < H; q += nw) {
+    const int a = dir == 0 ? q : 2 * q, b = dir == 0 ? K - 1 - q : 2 * q + 1;
+    const double xa = ok ? base[plane * a] : 0., xb = ok && b < K ? base[plane * b] : 0.;
+    // (the middle of an odd line: once, and 0 for the odd product)
+    czx[q * CZ_TI + lane] = dir ? make_double2(xa, xb) : make_double2(a == b ? xa : xa + xb, xa - xb);
   }
   __syncthreads();
-  if (lane >= ni) return;
-  for (int m0 = CZ_ROWS * warp; m0 < K; m0 += CZ_ROWS * 8) {
-    double acc[CZ_ROWS];
-    const double* __restrict__ tr[CZ_ROWS];
+  double2* __restrict__ c = coef[warp];
+  constexpr int NC = CZ_Q * CZ_ROWS / 32;
+  for (int g = warp; g * CZ_ROWS < H; g += nw) {
+    const double2* __restrict__ w = W + (long long)g * H * CZ_ROWS;
+    const int n = H * CZ_ROWS;
+    double e[CZ_ROWS], o[CZ_ROWS];
+    double2 next[NC];
+    auto fetch = [&](int q0) {
+#pragma unroll
+      for (int t = 0; t < NC; ++t) {
+        const int m = q0 * CZ_ROWS + 32 * t + lane;
+        next[t] = m < n ? __ldg(w + m) : make_double2(0., 0.);
+      }
+    };
+#pragma unroll
+    for (int r = 0; r < CZ_ROWS; ++r) e[r] = o[r] = 0.;
+    fetch(0);
+    for (int q0 = 0; q0 < H; q0 += CZ_Q) {
+      __syncwarp();
+#pragma unroll
+      for (int t = 0; t < NC; ++t) c[32 * t + lane] = next[t];
+      __syncwarp();
+      fetch(q0 + CZ_Q);
+      const int q1 = min(CZ_Q, H - q0);
+      for (int q = 0; q < q1; ++q) {
+        const double2 x = czx[(q0 + q) * CZ_TI + lane];
+#pragma unroll
+        for (int r = 0; r < CZ_ROWS / 2; ++r) {
+          const double2 a = c[q * CZ_ROWS + r], b = c[q * CZ_ROWS + CZ_ROWS / 2 + r];
+          e[2 * r] = __fma_rn(a.x, x.x, e[2 * r]);
+          e[2 * r + 1] = __fma_rn(a.y, x.x, e[2 * r + 1]);
+          o[2 * r] = __fma_rn(b.x, x.y, o[2 * r]);
+          o[2 * r + 1] = __fma_rn(b.y, x.y, o[2 * r + 1]);
+        }
+      }
+    }
+    if (!ok) continue;
 #pragma unroll
     for (int r = 0; r < CZ_ROWS; ++r) {
-      acc[r] = 0.;
-      tr[r] = T + (long long)min(m0 + r, K - 1) * K;
+      const int m = g * CZ_ROWS + r;
+      if (m >= H) break;
+      if (dir == 0) {
+        base[plane * (2 * m)] = e[r];
+        if (2 * m + 1 < K) base[plane * (2 * m + 1)] = o[r];
+      } else {
+        base[plane * m] = e[r] + o[r];
+        if (K - 1 - m > m) base[plane * (K - 1 - m)] = e[r] - o[r];
+      }
     }
-    for (int k = 0; k < K; ++k) {
-      const double xv = czx[k * CZ_TI + lane];
-#pragma unroll
-      for (int r = 0; r < CZ_ROWS; ++r) acc[r] = __fma_rn(__ldg(tr[r] + k), xv, acc[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < CZ_ROWS; ++r)
-      if (m0 + r < K) base[lane + plane * (m0 + r)] = acc[r];
   }
+}
+// its coefficients from the table T[m][k] of the definition
+std::vector<double> cosq_pack(const std::vector<double>& T, int K, int dir) {
+  const int H = (K + 1) / 2;
+  std::vector<double> W(cosq_coefs(K), 0.);
+  for (int m = 0; m < H; ++m)
+    for (int q = 0; q < H; ++q) {
+      double* w = &W[((size_t)(m / CZ_ROWS) * H + q) * 2 * CZ_ROWS + m % CZ_ROWS];
+      if (dir == 0) {
+        w[0] = T[(size_t)(2 * m) * K + q];
+        if (2 * m + 1 < K) w[CZ_ROWS] = T[(size_t)(2 * m + 1) * K + q];
+      } else {
+        w[0] = T[(size_t)m * K + 2 * q];
+        if (2 * q + 1 < K) w[CZ_ROWS] = T[(size_t)m * K + 2 * q + 1];
+      }
+    }
+  return W;
 }
 
 // The same transforms for a power-of-two kmax up to kCosqFftMaxN through one
@@ -992,8 +1065,9 @@ void poisson_setup_cos(Ctx& c) {
   cudaMemcpyAsync(c.tri_a, a.data(), a.size() * sizeof(double), cudaMemcpyHostToDevice, c.s);
   cudaMemcpyAsync(c.tri_b, b.data(), b.size() * sizeof(double), cudaMemcpyHostToDevice, c.s);
   cudaMemcpyAsync(c.tri_c, cc.data(), cc.size() * sizeof(double), cudaMemcpyHostToDevice, c.s);
-  cudaMemcpyAsync(c.cosb, tb.data(), tb.size() * sizeof(double), cudaMemcpyHostToDevice, c.s);
-  cudaMemcpyAsync(c.cosf, tf.data(), tf.size() * sizeof(double), cudaMemcpyHostToDevice, c.s);
+  const std::vector<double> wb = cosq_pack(tb, kmax, 0), wf = cosq_pack(tf, kmax, 1);
+  cudaMemcpyAsync(c.cosb, wb.data(), wb.size() * sizeof(double), cudaMemcpyHostToDevice, c.s);
+  cudaMemcpyAsync(c.cosf, wf.data(), wf.size() * sizeof(double), cudaMemcpyHostToDevice, c.s);
   std::vector<double2> tx;
   make_twiddles(itot, tx);
   cudaMemcpyAsync(c.twx, tx.data(), tx.size() * sizeof(double2), cudaMemcpyHostToDevice, c.s);
@@ -1174,13 +1248,14 @@ void launch_solver2d_cos(Ctx& c, int write_halos) {
   const long long nlines = (long long)P.jmax * P.kmax;
   const unsigned gx = (unsigned)((nlines + 2 * CL - 1) / (2 * CL));
   const size_t smx = (size_t)CL * (P.imax + 1) * sizeof(double2);
-  const size_t smz = (size_t)P.kmax * CZ_TI * sizeof(double);
+  const int H = (P.kmax + 1) / 2;
+  const size_t smz = (size_t)H * CZ_TI * sizeof(double2);
   static unsigned attr = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr & (1u << (dev & 31)))) {
     cudaFuncSetAttribute(k_fft_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_cosq_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kCosqMaxN * CZ_TI * sizeof(double)));
+    cudaFuncSetAttribute(k_cosq_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((kCosqMaxN + 1) / 2 * CZ_TI * sizeof(double2)));
     cudaFuncSetAttribute(k_cosq_fft_z, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(CZ_LINES * (kCosqFftMaxN + 1) * sizeof(double2)));
     attr |= 1u << (dev & 31);
@@ -1192,7 +1267,7 @@ void launch_solver2d_cos(Ctx& c, int write_halos) {
   const dim3 gzf((unsigned)((P.imax + CZF_TI - 1) / CZF_TI), (unsigned)P.jmax, 1);
   auto cosq = [&](int dir) {
     if (fz) pdl(k_cosq_fft_z, gzf, 256, smf, c.s)(P, dir, lz, c.twy, c.czw, c.spec);
-    else pdl(k_cosq_z, gz, 256, smz, c.s)(P, dir ? c.cosf : c.cosb, c.spec);
+    else pdl(k_cosq_z, gz, 32 * std::min(8, (H + CZ_ROWS - 1) / CZ_ROWS), smz, c.s)(P, dir, reinterpret_cast<const double2*>(dir ? c.cosf : c.cosb), c.spec);
   };
   if (!fft2_pass<false>(c, 0, 0)) pdl(k_fft_x, gx, FT, smx, c.s)(P, 0, CL, lx, c.twx, c.p, c.spec, 0);
   cosq(0);

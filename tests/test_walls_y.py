@@ -231,3 +231,30 @@ def test_gpu_walls_fp32_form_tracks_fp64():
         assert np.max(np.abs(a - b)) <= 1e-4 * max(1e-3, np.max(np.abs(b))), k
     v = p32.download("v")
     assert np.all(v[1:-1, 0, 1:-1] == 0) and np.all(v[1:-1, -2, 1:-1] == 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,bc", [
+    # cosine lines: the shortest, odd, one past a group of rows, the longest odd one
+    ((16, 12, 6), BCS[0]), ((16, 10, 7), BCS[1]), ((48, 10, 17), BCS[2]), ((64, 12, 75), BCS[0]), ((8, 8, 767), BCS[1]),
+    # elimination split over threads: both block sizes and the lines beyond them, along y and along z
+    ((8, 254, 12), BCS[0]), ((8, 274, 6), BCS[1]), ((8, 520, 10), BCS[2]),
+    ((8, 8, 31), 0), ((16, 8, 256), 0), ((8, 16, 272), 0), ((8, 8, 515), 0)])
+def test_gpu_solver2d_line_lengths(n, bc):
+    nx, ny, nz = n
+    cfg = make_config(itot=nx, jtot=ny, ktot=nz, ly=ny / nx, lz=nz / nx, bc_y=bc)
+    o, g = Oracle(cfg), _gpu_solver(cfg)
+    ls = init_drops(cfg, [(0.5, 0.5 * cfg.ly, 0.5 * cfg.lz)], [0.25])
+    o.setup(ls)
+    g.setup(ls)
+    f = np.random.default_rng(nx + ny + nz).standard_normal(n)
+    singular = bc in (0, BCY_WALLS)
+    if singular:
+        f -= f.mean()
+    a, b = _solve(g, cfg, f), _solve(o, cfg, f)
+    if singular:
+        a, b = a - a.mean(), b - b.mean()
+    # 64-bit transforms and eliminations in another order: eps / 2 times the
+    # square of the longest line, which its smallest eigenvalue's condition
+    # stays below (4 K^2 / pi^2), and 1e-11 as for the lengths above
+    assert np.max(np.abs(a - b)) <= max(1e-11, 1e-16 * max(n) ** 2) * np.max(np.abs(b))
