@@ -129,3 +129,24 @@ def test_short_chunks_equal_long_ones(precision):
     for name in ("u", "v", "w", "pnew", "jiemian", "miu", "rho_u", "p_x", "p_y", "p_z", "p_jump"):
         assert np.array_equal(one.download(name), all_.download(name)), name
     assert np.array_equal(one.volumes()[0], all_.volumes()[0])
+
+
+@pytest.mark.parametrize("n,precision", [((64, 48, 50), FP64), ((48, 32, 41), FP32), ((64, 32, 6), FP64)])
+def test_separate_projection_calls_equal_whole_sweeps(n, precision):
+    """correc reads the jumps near the drops only, against a context told (by
+    an upload of the same values) that it knows nothing of them; row counts
+    that the rows per thread do and do not divide."""
+    nx, ny, nz = n
+    h = 1.0 / 64
+    cfg = make_config(itot=nx, jtot=ny, ktot=nz, lx=nx * h, ly=ny * h, lz=nz * h, timestep=1e-3, rho2=10.0, miu2=10.0,
+                      Re=100.0, We=0.5, v_wall_lower=-0.5, v_wall_upper=0.5, precision=precision)
+    ls = init_drops(cfg, [(0.02, 0.3, 0.5 * nz * h)], [0.1], all_images=True)
+    near, told = run_steps(cfg, ls, 2), run_steps(cfg, ls, 2)
+    told.upload("p_x", told.download("p_x"))
+    for s in (near, told):
+        s.fillps()
+        s.add_pjump()
+        s.correc()
+    for name in ("p", "u", "v", "w"):
+        assert np.array_equal(near.download(name), told.download(name)), name
+    assert np.any(near.download("p_x"))
