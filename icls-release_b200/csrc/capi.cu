@@ -565,18 +565,19 @@ void field_written(Ctx& c, int id) {
   }
 }
 
-void update_materials(Ctx& c) {
+// extents: the step's band extents are read back with the volumes
+void update_materials(Ctx& c, bool extents = false) {
   const int L = c.P.L;
   const size_t ns = (size_t)seg_count(c.P);
   const int prev = c.mat_cur;
   if (c.mat_dirty || c.materials_rows1) {
     cudaMemsetAsync(c.seg_mat[prev], 1, ns, c.s);
+    cudaMemsetAsync(c.seg_mat[prev ^ 1], 0, ns, c.s);
     launch_fill(c, c.jiemian, c.P.nC, 1.0, true);
   } else {
-    launch_seg_reset(c, c.seg_mat[prev]);
+    launch_seg_reset(c, c.seg_mat[prev], c.seg_mat[prev ^ 1]);
   }
   c.mat_cur ^= 1;
-  cudaMemsetAsync(c.seg_mat[c.mat_cur], 0, ns, c.s);
   std::vector<int> all(L);
   for (int l = 0; l < L; ++l) all[l] = l;
   std::vector<int> ntiles(L, 0);  // partial sums per drop: column tiles x z chunks
@@ -589,12 +590,12 @@ void update_materials(Ctx& c) {
     launch_heaviside(c, b);
   }
   for (int l = 0; l < L; ++l) c.outside[l] = outside_count(c, c.win[l].box);
-  launch_volumes(c, c.outside.data(), ntiles.data());
+  launch_volumes(c, c.outside.data(), ntiles.data(), extents);
+  cudaEventRecord(c.ev_vol, c.s);
+  if (extents) cudaEventRecord(c.ev_bbox, c.s);
   if (c.materials_rows1) launch_materials(c, nullptr, nullptr);
   else launch_materials(c, c.seg_mat[c.mat_cur], c.seg_mat[prev]);
   c.mat_dirty = false;
-  cudaMemcpyAsync(c.h_vol, c.dvol, sizeof(double) * L, cudaMemcpyDeviceToHost, c.s);
-  cudaEventRecord(c.ev_vol, c.s);
   c.vol_pending = true;
   std::fill(c.vol_dirty.begin(), c.vol_dirty.end(), 0);
 }
@@ -603,7 +604,7 @@ void update_materials(Ctx& c) {
 // their members' s1 and band masks; every cell outside the measured band
 // box is +6dz afterwards.  list: the band cells into c.band_list, and the
 // clipped values into s2 and s3 too.
-void tube_batch(Ctx& c, LsBatch& b, bool list) {
+void tube_batch(Ctx& c, LsBatch& b, bool list, bool fresh = false) {
   for (int q = 0; q < b.n; ++q) {
     LsTask& t = b.t[q];
     const DropWin& w = c.win[t.l];
@@ -617,7 +618,7 @@ void tube_batch(Ctx& c, LsBatch& b, bool list) {
     t.out3 = m.s3;
     t.mask = m.mask;
   }
-  launch_tube(c, b, list);
+  launch_tube(c, b, list, fresh);
   for (int q = 0; q < b.n; ++q) {
     DropWin& w = c.win[b.t[q].l];
     w.valid = w.box;
@@ -1063,9 +1064,8 @@ int ls_main(Ctx& c, int istep) {
     c.win[l].box = sweep_region(c, l, g_now);
     c.win[l].pending_grow = g_now;
   }
-  cudaMemsetAsync(c.d_nbcnt, 0, sizeof(long long) * L, c.s);
-  cudaMemsetAsync(c.d_bbox, 0x7F, sizeof(int) * 5 * L, c.s);
-  cudaMemsetAsync(c.d_bbox + 5 * L, 0x80, sizeof(int) * 5 * L, c.s);
+  launch_band_begin(c);
+  bool fresh = true;  // the list is empty
   // per group: tube_construction, ls_advection, ls_mass_correction (which
   // still reads the drop's band mask) and ls_reinit, as the reference runs
   // them for each drop
@@ -1078,7 +1078,8 @@ int ls_main(Ctx& c, int istep) {
       const bool list = !c.adv_column && c.P.imax <= 4096 && c.P.jmax <= 4096 && bound <= c.band_cap;
       bool unmeasured = false;
       for (int q = 0; q < b.n; ++q) unmeasured = unmeasured || (c.use_boxes && !c.win[b.t[q].l].have_D);
-      tube_batch(c, b, list);
+      tube_batch(c, b, list, fresh);
+      fresh = false;
       if (unmeasured) {
         std::vector<int> in_b;
         for (int q = 0; q < b.n; ++q) in_b.push_back(b.t[q].l);
@@ -1103,10 +1104,8 @@ int ls_main(Ctx& c, int istep) {
     }
     if (reinit_now && !correct_last) reinit_batches(c, bs);
   }
-  cudaMemcpyAsync(c.h_bbox, c.d_bbox, sizeof(int) * 10 * L, cudaMemcpyDeviceToHost, c.s);
-  cudaEventRecord(c.ev_bbox, c.s);
+  update_materials(c, true);
   c.bbox_pending = true;
-  update_materials(c);
   return check_launch();
 }
 
@@ -1152,13 +1151,10 @@ int gfm4p(Ctx& c) {
   // the jump fields start at zero: p_x, p_y, p_z where the step before last
   // left jumps, p_jump where the last one did
   const size_t bytes = sizeof(double) * (size_t)c.P.nC, tbytes = sizeof(double) * tn(c.P, c.P.nC);
-  const size_t ns = (size_t)seg_count(c.P);
   if (c.jmp_dirty[0])
     for (double* f : {c.px, c.py, c.pz}) cudaMemsetAsync(f, 0, tbytes, c.s);
   if (c.pjump_dirty) cudaMemsetAsync(c.pjump, 0, bytes, c.s);
   launch_seg_clear_jumps(c, c.seg_jmp[0], c.seg_jmp[1]);
-  cudaMemsetAsync(c.seg_jmp[0], 0, ns, c.s);
-  cudaMemsetAsync(c.row_jmp, 0, (size_t)c.P.jmax * c.P.nCz, c.s);
   c.jmp_dirty[0] = c.pjump_dirty = false;
   for (int g = 0; g < n_groups(c); ++g) {
     const std::vector<int> drops = group_drops(c, g);

@@ -256,7 +256,8 @@ Region c_region(const Params& P, const Region& r, int apron);
 void set_tiles(LsBatch& b, int kc, bool flat = true);
 void size_tiles(const Params& p, LsBatch& b, int kc, int kmin, int blocks);
 // tube_construction; list: the band cells also into c.band_list (sets the batch's own tiles)
-void launch_tube(Ctx& c, LsBatch& b, bool list);
+void launch_band_begin(Ctx& c);
+void launch_tube(Ctx& c, LsBatch& b, bool list, bool fresh);
 void launch_adv_stage(Ctx& c, const LsBatch& b, int scheme, int stage1, double a, double bb, double fdt,
                       const double* vu, const double* vv, const double* vw);
 void launch_reinit_stage(Ctx& c, const LsBatch& b, int stage, double dtau);
@@ -264,10 +265,10 @@ void launch_reinit_reset(Ctx& c, const LsBatch& b, int maxiter);
 void launch_reinit_check(Ctx& c, const LsBatch& b, int it, int maxiter, double thr);
 void launch_heaviside(Ctx& c, const LsBatch& b);
 void launch_fill(Ctx& c, double* a, long long n, double v, bool tfield);
-void launch_seg_reset(Ctx& c, const uint8_t* seg);
-void launch_volumes(Ctx& c, const double* outside, const int* ntiles);
+void launch_seg_reset(Ctx& c, const uint8_t* seg, uint8_t* next);
+void launch_volumes(Ctx& c, const double* outside, const int* ntiles, bool extents = false);
 void launch_materials(Ctx& c, const uint8_t* cur, const uint8_t* prev);
-void launch_seg_clear_jumps(Ctx& c, const uint8_t* faces, const uint8_t* lap);
+void launch_seg_clear_jumps(Ctx& c, uint8_t* faces, const uint8_t* lap);
 // mass correction of the tasks' drops; LsTask::far holds the interior cells outside a drop's region
 void launch_inflate_sums(Ctx& c, const LsBatch& b);
 void launch_inflate_base(Ctx& c, const LsBatch& b);

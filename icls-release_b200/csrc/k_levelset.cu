@@ -1030,9 +1030,16 @@ struct PerDrop {
 // One warp per drop: its lanes merge every 32nd partial, the lanes' sums
 // (limbs below 2^48 after each merge) add limb by limb across the warp
 // (below 2^53), and lane 0 rounds the exact total once.
+// (and into pinned memory for the host, with the band extents where asked:
+// copies and small memsets between the step's kernels left the GPU idle for
+// their length and broke the overlapped launches; without two copies and eight
+// memsets one drop at 64^3 takes 334 instead of 370 us)
 __global__ void k_volumes(Params p, const XSum* __restrict__ part, int cap, PerDrop pd, int uniform, int nb_all,
-                          double* __restrict__ vol, DevScalars* __restrict__ dsc) {
+                          double* __restrict__ vol, DevScalars* __restrict__ dsc, double* __restrict__ h_vol,
+                          const int* __restrict__ bbox, int* __restrict__ h_bbox) {
   pdl_wait();
+  if (bbox)
+    for (int t = threadIdx.x; t < 10 * p.L; t += blockDim.x) h_bbox[t] = bbox[t];
   const double N = (1. * p.imax * p.jmax) * p.kmax;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int l = warp; l < p.L; l += nw) {
@@ -1047,6 +1054,7 @@ __global__ void k_volumes(Params p, const XSum* __restrict__ part, int cap, PerD
       xs_norm(s);
       if (!uniform) xs_add_count(s, (long long)pd.v[l]);
       vol[l] = 1. - xs_value(s) / N;
+      h_vol[l] = vol[l];
     }
   }
   __syncthreads();
@@ -1096,8 +1104,8 @@ __global__ void __launch_bounds__(NT) k_materials_final(Params p, const T* __res
 }
 
 // One warp per 32 segments: the lanes read the segments' bytes, then the
-// warp takes the set ones in turn, a lane per cell.  f(sx, j, k, q) for
-// segment q, bytes(q, sx, j, k) true where it is to be visited.
+// warp takes the set ones in turn, a lane per cell.  bytes(q, sx, j, k): what
+// segment q is to be visited for (0: not), and f(sx, j, k, that) visits it.
 template <class Bytes, class F>
 __device__ __forceinline__ void for_segments(const Params& p, int per, const Bytes& bytes, const F& f) {
   const int nsx = seg_row(p);
@@ -1107,7 +1115,7 @@ __device__ __forceinline__ void for_segments(const Params& p, int per, const Byt
   for (long long g = w0; g * per < ns; g += W) {
     const long long q = g * per + lane;
     int sx = 0, j = 0, k = 0;
-    bool on = false;
+    int on = 0;
     if (lane < per && q < ns) {
       const long long r = q / nsx;
       sx = (int)(q - r * nsx);
@@ -1115,46 +1123,59 @@ __device__ __forceinline__ void for_segments(const Params& p, int per, const Byt
       j = (int)(r - (long long)k * p.jmax) + 1;
       on = bytes(q, sx, j, k);
     }
-    unsigned m = __ballot_sync(0xffffffffu, on);
+    unsigned m = __ballot_sync(0xffffffffu, on != 0);
     while (m) {
       const int b = __ffs(m) - 1;
       m &= m - 1;
-      f(__shfl_sync(0xffffffffu, sx, b), __shfl_sync(0xffffffffu, j, b), __shfl_sync(0xffffffffu, k, b));
+      f(__shfl_sync(0xffffffffu, sx, b), __shfl_sync(0xffffffffu, j, b), __shfl_sync(0xffffffffu, k, b),
+        __shfl_sync(0xffffffffu, on, b));
     }
   }
 }
 
-// jiemian = 1 in the segments of a map (with the periodic images)
+// jiemian = 1 in the segments of a map (with the periodic images), and the
+// next map zero
 template <typename T>
-__global__ void __launch_bounds__(NT) k_seg_reset(Params p, int per, const uint8_t* __restrict__ seg, T* __restrict__ jiemian) {
+__global__ void __launch_bounds__(NT) k_seg_reset(Params p, int per, const uint8_t* __restrict__ seg,
+                                                  uint8_t* __restrict__ next, T* __restrict__ jiemian) {
   pdl_wait();
   for_segments(
-      p, per, [&](long long q, int, int, int) { return seg[q] != 0; },
-      [&](int sx, int j, int k) {
+      p, per,
+      [&](long long q, int, int, int) {
+        next[q] = 0;
+        return (int)seg[q];
+      },
+      [&](int sx, int j, int k, int) {
         const int i = 1 + kSeg * sx + (int)(threadIdx.x & 31);
         if (i <= p.imax) putC(p, jiemian, i, j, k, TC(1.));
       });
 }
 // p_x, p_y, p_z = 0 in the segments of `faces`, p_jump = 0 in those of `lap`
-// (interior cells: gfm4p writes no others)
+// (interior cells: gfm4p writes no others); then faces and the row map are
+// zero, for the jumps that follow
 template <typename T>
-__global__ void __launch_bounds__(NT) k_seg_clear_jumps(Params p, int per, const uint8_t* __restrict__ faces,
-                                                        const uint8_t* __restrict__ lap, T* __restrict__ px,
-                                                        T* __restrict__ py, T* __restrict__ pz,
+__global__ void __launch_bounds__(NT) k_seg_clear_jumps(Params p, int per, uint8_t* faces,
+                                                        const uint8_t* __restrict__ lap, uint8_t* __restrict__ row,
+                                                        T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz,
                                                         double* __restrict__ pjump) {
   pdl_wait();
+  for (long long q = blockIdx.x * (long long)NT + threadIdx.x; q < (long long)p.jmax * p.nCz; q += (long long)gridDim.x * NT)
+    row[q] = 0;
   for_segments(
-      p, per, [&](long long q, int, int, int) { return (faces[q] | lap[q]) != 0; },
-      [&](int sx, int j, int k) {
+      p, per,
+      [&](long long q, int, int, int) {
+        const int on = (faces[q] ? 1 : 0) | (lap[q] ? 2 : 0);
+        if (on & 1) faces[q] = 0;
+        return on;
+      },
+      [&](int sx, int j, int k, int on) {
         const int i = 1 + kSeg * sx + (int)(threadIdx.x & 31);
-        const long long q = sx + (long long)seg_row(p) * ((j - 1) + (long long)p.jmax * k);
         if (i > p.imax || k < 1 || k > p.kmax) return;
         const long long n = idxC(p, i, j, k);
-        if (faces[q]) px[n] = py[n] = pz[n] = TC(0.);
-        if (lap[q]) pjump[n] = 0.;
+        if (on & 1) px[n] = py[n] = pz[n] = TC(0.);
+        if (on & 2) pjump[n] = 0.;
       });
 }
-
 // k_materials_final's fields where they can have changed: a segment whose
 // own cells, or the + neighbours that its face densities read, are or were
 // (prev) set; everywhere else they hold the carrier's values already.
@@ -1176,9 +1197,9 @@ __global__ void __launch_bounds__(NT) k_materials_seg(Params p, int per, const u
         const long long qx = sx + 1 < nsx ? q + 1 : q - sx;
         const long long qy = j < p.jmax ? q + nsx : q - (long long)nsx * (p.jmax - 1);
         const long long qz = k < p.k1 ? q + (long long)nsx * p.jmax : q;
-        return (cur[q] | cur[qx] | cur[qy] | cur[qz] | prev[q] | prev[qx] | prev[qy] | prev[qz]) != 0;
+        return cur[q] | cur[qx] | cur[qy] | cur[qz] | prev[q] | prev[qx] | prev[qy] | prev[qz];
       },
-      [&](int sx, int j, int k) {
+      [&](int sx, int j, int k, int) {
         const int i = 1 + kSeg * sx + (int)(threadIdx.x & 31);
         if (i > p.imax) return;
         const long long n = idxC(p, i, j, k);
@@ -1598,7 +1619,19 @@ void size_tiles(const Params& p, LsBatch& b, int kc, int kmin, int blocks) {
     }                                   \
   } while (0)
 
-void launch_tube(Ctx& c, LsBatch& b, bool list) {
+// the band counts, extents and list length before the tubes of a step
+__global__ void k_band_begin(int L, long long* __restrict__ nbcnt, int* __restrict__ bbox, int* __restrict__ count) {
+  pdl_wait();
+  for (int t = threadIdx.x; t < 10 * L; t += blockDim.x) {
+    bbox[t] = t < 5 * L ? 0x7F7F7F7F : (int)0x80808080;
+    if (t < L) nbcnt[t] = 0;
+  }
+  if (threadIdx.x == 0) *count = 0;
+}
+void launch_band_begin(Ctx& c) {
+  pdl(k_band_begin, 1, 256, 0, c.s)(c.P.L, c.d_nbcnt, c.d_bbox, c.band_count);
+}
+void launch_tube(Ctx& c, LsBatch& b, bool list, bool fresh) {
   if (b.n == 0) return;
   Scope sc_(c.prof, c.s, "tube", 1);
   // the register window along z is filled once per chunk (one drop at 64^3:
@@ -1606,7 +1639,7 @@ void launch_tube(Ctx& c, LsBatch& b, bool list) {
   size_tiles(c.P, b, kTubeRows, 4, 4 * 148);
   int* lo = c.d_bbox;
   int* hi = c.d_bbox + 5 * c.P.L;
-  if (list) cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
+  if (list && !fresh) cudaMemsetAsync(c.band_count, 0, sizeof(int), c.s);
   BandCell* l = list ? reinterpret_cast<BandCell*>(c.band_list) : nullptr;
   BY_FORM(c, (pdl(k_tube<float>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)),
           (pdl(k_tube<double>, b.start[b.n], kTile, 0, c.s)(c.P, b, c.d_nbcnt, lo, hi, l, c.band_count)));
@@ -1760,7 +1793,7 @@ void launch_disp(Ctx& c, int l) {
   pdl(k_disp_final, 1, kRedThreads, 0, c.s)(c.diag, kRedBlocks, c.diag + 7 * kRedBlocks);
 }
 
-void launch_volumes(Ctx& c, const double* outside, const int* ntiles) {
+void launch_volumes(Ctx& c, const double* outside, const int* ntiles, bool extents) {
   Scope sc_(c.prof, c.s, "volumes", 1);
   PerDrop o;
   const int uniform = (outside == nullptr || c.P.L > kMaxDropsParam) ? 1 : 0;
@@ -1771,7 +1804,7 @@ void launch_volumes(Ctx& c, const double* outside, const int* ntiles) {
   // uniform: every drop swept whole, (kmax + 2) / kStageRows z chunks of
   // red_cap column tiles
   pdl(k_volumes, 1, 1024, 0, c.s)(c.P, hparts(c), c.hcap, o, uniform, c.red_cap * ((c.P.kmax + 2) / kHeavRows), c.dvol,
-                                c.dsc);
+                                c.dsc, c.h_vol, extents ? c.d_bbox : nullptr, c.h_bbox);
 }
 // the warps of a sweep over the segments: enough for one group of 32 each, at
 // most eight blocks per SM
@@ -1789,18 +1822,22 @@ unsigned seg_blocks(const Params& p) {
   const int n = seg_per_warp(p) * (NT / 32);
   return (unsigned)std::min<long long>((seg_count(p) + n - 1) / n, kRedBlocks);
 }
-void launch_seg_reset(Ctx& c, const uint8_t* seg) {
+void launch_seg_reset(Ctx& c, const uint8_t* seg, uint8_t* next) {
   Scope sc_(c.prof, c.s, "fill", 1);
-  BY_FORM(c, (pdl(k_seg_reset<float>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), seg, reinterpret_cast<float*>(c.jiemian))),
-          (pdl(k_seg_reset<double>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), seg, c.jiemian)));
+  const int per = seg_per_warp(c.P);
+  BY_FORM(c,
+          (pdl(k_seg_reset<float>, seg_blocks(c.P), NT, 0, c.s)(c.P, per, seg, next, reinterpret_cast<float*>(c.jiemian))),
+          (pdl(k_seg_reset<double>, seg_blocks(c.P), NT, 0, c.s)(c.P, per, seg, next, c.jiemian)));
 }
-void launch_seg_clear_jumps(Ctx& c, const uint8_t* faces, const uint8_t* lap) {
+void launch_seg_clear_jumps(Ctx& c, uint8_t* faces, const uint8_t* lap) {
   Scope sc_(c.prof, c.s, "clear_jumps", 1);
+  const int per = seg_per_warp(c.P);
   auto f = [](double* q) { return reinterpret_cast<float*>(q); };
   BY_FORM(c,
-          (pdl(k_seg_clear_jumps<float>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), faces, lap, f(c.px), f(c.py), f(c.pz),
-                                                                     c.pjump)),
-          (pdl(k_seg_clear_jumps<double>, seg_blocks(c.P), NT, 0, c.s)(c.P, seg_per_warp(c.P), faces, lap, c.px, c.py, c.pz, c.pjump)));
+          (pdl(k_seg_clear_jumps<float>, seg_blocks(c.P), NT, 0, c.s)(c.P, per, faces, lap, c.row_jmp, f(c.px), f(c.py),
+                                                                      f(c.pz), c.pjump)),
+          (pdl(k_seg_clear_jumps<double>, seg_blocks(c.P), NT, 0, c.s)(c.P, per, faces, lap, c.row_jmp, c.px, c.py, c.pz,
+                                                                       c.pjump)));
 }
 // miu, rho and the face densities; cur and prev: the maps of jiemian (null:
 // one thread per cell of the whole arrays, ICLS_MATERIALS=rows1)
