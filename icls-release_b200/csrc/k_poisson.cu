@@ -40,6 +40,7 @@ size_t cosq_coefs(int K) {
 
 namespace {
 
+constexpr int kRhsU = 4;  // iterations of the right-hand side's loop under way
 constexpr int FT = 256;  // threads per FFT CTA
 
 __device__ __forceinline__ int bitrev(int x, int logn) { return (int)(__brev((unsigned)x) >> (32 - logn)); }
@@ -393,7 +394,7 @@ __device__ __forceinline__ double rhs_of(const Params& p, T u, T um, T v, T vm, 
 // are adjacent threads.  dir 0: p (x) or spec (y) -> half-complex spec;
 // dir 1: the inverse, into spec (y) or p (x, with the boundp images when
 // halos is set).  RHS (forward x pass only): 0 reads p; 4 or 8 forms
-// fillps' right-hand side from float or double velocities instead (rhs_at),
+// fillps' right-hand side from float or double velocities instead (rhs_of),
 // so p is neither written by fillps nor read here.
 // LPC complex lines per CTA of 256 threads, TPL = max(R1, R2) threads per
 // line; LPC * TPL <= 256 (the other threads idle)
@@ -446,33 +447,45 @@ __global__ void __launch_bounds__(256, (R1 > 16 || R2 > 16) ? 1 : 2)
     B = colbase + 1;
   }
   double2* S = sm + lt * LS;
-  // step 1: lane n2 < R2 transforms z[R2 n1 + n2] over n1
-  if (lane < R2 && live) {
-    double2 x[R1];
-    bool adda = false, addb = false;
-    if constexpr (RHS != 0) {
-      if (ra.row) {
-        adda = ra.row[(ja - 1) + (long long)p.jmax * ka] != 0;
-        addb = ra.row[(jb - 1) + (long long)p.jmax * kb] != 0;
-      }
-    }
-#pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) {
-      const int n = R2 * n1 + lane;
-      if constexpr (RHS != 0) {
-        // dir 0: lines a and b start at columns 1 of (ja, ka) and (ja + 1, ka)
-        // (periodic y: jmax is even)
-        using T = typename std::conditional<RHS == 4, float, double>::type;
-        const T* __restrict__ du = static_cast<const T*>(ra.du);
-        const T* __restrict__ dv = static_cast<const T*>(ra.dv);
-        const T* __restrict__ dw = static_cast<const T*>(ra.dw);
-        const int sy = p.nCx, sz = p.nCx * p.nCy, c = 1 + n + sy * (ja + p.nCy * ka), d = c + sy;
+  if constexpr (RHS != 0) {
+    // the right-hand side of lines a and b, (ja, ka) and (ja + 1, ka)
+    // (periodic y: jmax is even), into shared memory, whole rows per warp
+    // (formed at the transform's loads, 11 of them at each of a thread's 16
+    // points and half a row per warp: the solve at 256^3 FP64 0.412 -> 0.402 ms,
+    // at 128 x 128 x 256 142 -> 129 us; 8 iterations under way are no faster)
+    using T = typename std::conditional<RHS == 4, float, double>::type;
+    const T* __restrict__ du = static_cast<const T*>(ra.du);
+    const T* __restrict__ dv = static_cast<const T*>(ra.dv);
+    const T* __restrict__ dw = static_cast<const T*>(ra.dw);
+    const int sy = p.nCx, sz = p.nCx * p.nCy;
+    for (int l = (int)threadIdx.x >> 5; l < LPC; l += 8) {
+      const long long la = 2 * ((long long)blockIdx.x * LPC + l);
+      if (la >= (long long)p.jmax * p.kmax) break;
+      const int j = (int)(la % p.jmax) + 1, k = (int)(la / p.jmax) + 1;
+      const bool adda = ra.row && ra.row[(j - 1) + (long long)p.jmax * k] != 0;
+      const bool addb = ra.row && ra.row[j + (long long)p.jmax * k] != 0;
+      double2* __restrict__ z = sm + l * ZLD;
+#pragma unroll kRhsU
+      for (int n = (int)threadIdx.x & 31; n < N; n += 32) {
+        const int c = 1 + n + sy * (j + p.nCy * k), d = c + sy;
         const T v = dv[c];
         double va = rhs_of<T>(p, du[c], du[c - 1], v, dv[c - sy], dw[c], dw[c - sz]);
         double vb = rhs_of<T>(p, du[d], du[d - 1], dv[d], v, dw[d], dw[d - sz]);
         if (adda) va = __dadd_rn(va, ra.pj[c]);
         if (addb) vb = __dadd_rn(vb, ra.pj[d]);
-        x[n1] = make_double2(va, vb);
+        z[n] = make_double2(va, vb);
+      }
+    }
+    __syncthreads();
+  }
+  // step 1: lane n2 < R2 transforms z[R2 n1 + n2] over n1
+  double2 x[R1];
+  if (lane < R2 && live) {
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) {
+      const int n = R2 * n1 + lane;
+      if constexpr (RHS != 0) {
+        x[n1] = sm[lt * ZLD + n];
       } else if constexpr (YPASS) {
         // columns 2c and 2c + 1: imax is even, so the pair is 16-byte aligned
         const double2* ab = reinterpret_cast<const double2*>(colbase);
@@ -486,6 +499,9 @@ __global__ void __launch_bounds__(256, (R1 > 16 || R2 > 16) ? 1 : 2)
         }
       }
     }
+  }
+  if (RHS != 0) __syncthreads();  // every right-hand side is read
+  if (lane < R2 && live) {
     reg_dft<R1>(x, tw, N, dir);
 #pragma unroll
     for (int k1 = 1; k1 < R1; ++k1) {
