@@ -93,18 +93,16 @@ def initial_state(wl):
 # cells, B band cells of all drops (one batched scope covers every drop),
 # S |phi| <= 2dz shell cells of all drops.
 ALG_VALUES = {
-    "ab2": (24, 0, "N"),             # u,v,w,miu,rho_uvw,duold x3,pnew,pold,p_xyz,p_xyz_old -> dudt x3,duold x3
-    "correc": (12, 1, "N"),          # dudt x3,p_xyz | p -> u,v,w, ucc,vcc,wcc
+    "ab2": (14, 0, "N"),             # u,v,w,duold x3,pnew,pold -> dudt x3,duold x3 (miu,rho_uvw,p_xyz,p_xyz_old near drops only)
+    "correc": (9, 1, "N"),           # dudt x3 | p -> u,v,w, ucc,vcc,wcc (p_xyz near drops only)
     "fillps": (3, 2, "N"),           # dudt x3 | pjump -> p
     "solver2d": (3, 2, "N"),         # dudt x3 | p_jump -> p: fillps folded into the first pass (the transposes and sweeps between are not compulsory)
     "pressure_update": (3, 1, "N"),  # pnew | p -> pnew, pold
     "stream_vel": (1, 0, "N"),
-    "materials_final": (6, 0, "N"),  # jiemian -> miu, rho, rho_uvw
     "tube": (2, 0, "B"),             # phi -> clipped phi on the band
     "adv_stage": (17.0 / 3.0, 0, "B"),  # one RK3 stage on the band
     "heaviside": (1, 0, "B"),
     "curvature": (2, 0, "S"),
-    "recurvature": (2, 0, "S"),
     "jumps": (8, 2, "S"),            # phi, kappa_re, p_xyz (read+write) | p_jump (read+write)
 }
 
@@ -117,7 +115,7 @@ MLP_FLOPS_PER_CELL = 2 * (128 * 64 + 128 * 128 + 64 * 128)
 # (kernel, FP32 form) -> bytes: ncu's dram__bytes_read.sum + write.sum of the
 # launch in a capture of the static_drop_256 workload (the predictor's grid
 # and fields do not depend on the drops)
-TRAFFIC = {("ab2", False): 2.504199e9 + 0.801062e9, ("ab2", True): 1.245101e9 + 0.389982e9}
+TRAFFIC = {("ab2", False): 1.095140e9 + 0.771508e9, ("ab2", True): 0.555361e9 + 0.362161e9}
 
 
 def alg_bytes_per_launch(name, cfg, stats, f32=False):
