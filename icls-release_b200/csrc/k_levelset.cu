@@ -1021,8 +1021,12 @@ __global__ void __launch_bounds__(NT, 4) k_heaviside(Params p, const __grid_cons
   if (flat_tid() == 0) part[(long long)t.l * cap + c.tile + (long long)t.tx * t.ty * c.ch] = bs;
 }
 
-// volume(l) and rho_avr from the per-tile sums (misc.f90:139-173);
-// outside[l] interior cells of drop l lie in its far field, where H = 1
+// volume(l) and rho_avr from the per-(tile, chunk) sums (misc.f90:139-173) of
+// drops l0 .. l0 + nl - 1: n[l - l0] partials each, and v[l - l0] interior
+// cells in the drop's far field, where H = 1.  The counts travel as a kernel
+// parameter, so a launch takes up to kMaxDropsParam drops; launches of more
+// drops follow one another, and the last one, which sees every volume, sums
+// them in order.
 struct PerDrop {
   double v[kMaxDropsParam];
   int n[kMaxDropsParam];
@@ -1034,31 +1038,32 @@ struct PerDrop {
 // copies and small memsets between the step's kernels left the GPU idle for
 // their length and broke the overlapped launches; without two copies and eight
 // memsets one drop at 64^3 takes 334 instead of 370 us)
-__global__ void k_volumes(Params p, const XSum* __restrict__ part, int cap, PerDrop pd, int uniform, int nb_all,
+__global__ void k_volumes(Params p, const XSum* __restrict__ part, int cap, PerDrop pd, int l0, int nl,
                           double* __restrict__ vol, DevScalars* __restrict__ dsc, double* __restrict__ h_vol,
                           const int* __restrict__ bbox, int* __restrict__ h_bbox) {
   pdl_wait();
-  if (bbox)
+  const bool last = l0 + nl == p.L;
+  if (bbox && last)
     for (int t = threadIdx.x; t < 10 * p.L; t += blockDim.x) h_bbox[t] = bbox[t];
   const double N = (1. * p.imax * p.jmax) * p.kmax;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int l = warp; l < p.L; l += nw) {
-    const int nb = uniform ? nb_all : pd.n[l];
+  for (int q = warp; q < nl; q += nw) {
+    const int l = l0 + q, nb = pd.n[q];
     XSum s;
     xs_zero(s);
     for (int b = lane; b < nb; b += 32) xs_merge(s, part[(long long)l * cap + b]);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      for (int d = 16; d > 0; d >>= 1) s.L[q] += __shfl_down_sync(0xffffffffu, s.L[q], d);
+    for (int m = 0; m < 4; ++m)
+      for (int d = 16; d > 0; d >>= 1) s.L[m] += __shfl_down_sync(0xffffffffu, s.L[m], d);
     if (lane == 0) {
       xs_norm(s);
-      if (!uniform) xs_add_count(s, (long long)pd.v[l]);
+      xs_add_count(s, (long long)pd.v[q]);
       vol[l] = 1. - xs_value(s) / N;
       h_vol[l] = vol[l];
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (last && threadIdx.x == 0) {
     double sv = 0.;
     for (int l = 0; l < p.L; ++l) sv += vol[l];
     dsc->rho_avr = p.rho1 * (1. - sv) + p.rho2 * sv;
@@ -1782,7 +1787,6 @@ void launch_fill(Ctx& c, double* a, long long n, double v, bool tfield) {
     pdl(k_fill<double>, 1184, NT, 0, c.s)(a, n, v);
 }
 
-// outside/ntiles: per drop (null: every drop swept its whole grid)
 void launch_disp(Ctx& c, int l) {
   Scope sc_(c.prof, c.s, "disp", 2);
   BY_FORM(c, (pdl(k_disp<float>, kRedBlocks, kRedThreads, 0, c.s)(c.P, reinterpret_cast<const float*>(c.lv[l]),
@@ -1793,18 +1797,18 @@ void launch_disp(Ctx& c, int l) {
   pdl(k_disp_final, 1, kRedThreads, 0, c.s)(c.diag, kRedBlocks, c.diag + 7 * kRedBlocks);
 }
 
+// outside, ntiles: each drop's far-field cells and its partials
 void launch_volumes(Ctx& c, const double* outside, const int* ntiles, bool extents) {
-  Scope sc_(c.prof, c.s, "volumes", 1);
-  PerDrop o;
-  const int uniform = (outside == nullptr || c.P.L > kMaxDropsParam) ? 1 : 0;
-  for (int l = 0; l < kMaxDropsParam; ++l) {
-    o.v[l] = (!uniform && l < c.P.L) ? outside[l] : 0.;
-    o.n[l] = (!uniform && l < c.P.L) ? ntiles[l] : 0;
+  const int L = c.P.L;
+  Scope sc_(c.prof, c.s, "volumes", (L + kMaxDropsParam - 1) / kMaxDropsParam);
+  for (int l0 = 0; l0 < L; l0 += kMaxDropsParam) {
+    const int nl = std::min(kMaxDropsParam, L - l0);
+    PerDrop o = {};
+    std::copy(outside + l0, outside + l0 + nl, o.v);
+    std::copy(ntiles + l0, ntiles + l0 + nl, o.n);
+    pdl(k_volumes, 1, 1024, 0, c.s)(c.P, hparts(c), c.hcap, o, l0, nl, c.dvol, c.dsc, c.h_vol,
+                                  extents ? c.d_bbox : nullptr, c.h_bbox);
   }
-  // uniform: every drop swept whole, (kmax + 2) / kStageRows z chunks of
-  // red_cap column tiles
-  pdl(k_volumes, 1, 1024, 0, c.s)(c.P, hparts(c), c.hcap, o, uniform, c.red_cap * ((c.P.kmax + 2) / kHeavRows), c.dvol,
-                                c.dsc, c.h_vol, extents ? c.d_bbox : nullptr, c.h_bbox);
 }
 // the warps of a sweep over the segments: enough for one group of 32 each, at
 // most eight blocks per SM
