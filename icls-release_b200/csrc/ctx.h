@@ -319,7 +319,7 @@ void launch_boundp(Ctx& c, double* p, bool tfield = false);
 // the y-wall rows of bounduvw / boundp (bound.f90:81-282) for bc_y != periodic,
 // applied after the periodic halos (i = 1..imax, k = 1..kmax)
 void launch_ywalls_uvw(Ctx& c, double* u, double* v, double* w);
-void launch_ywalls_p(Ctx& c, double* p);
+void launch_ywalls_p(Ctx& c, double* p, bool tfield);
 void launch_nan_probe(Ctx& c);
 // drop l's band box as a whole-array tube sweep would measure it, into d_bbox
 void launch_band_extents(Ctx& c, int l);

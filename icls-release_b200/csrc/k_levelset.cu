@@ -1634,6 +1634,7 @@ __global__ void k_band_begin(int L, long long* __restrict__ nbcnt, int* __restri
   if (threadIdx.x == 0) *count = 0;
 }
 void launch_band_begin(Ctx& c) {
+  Scope sc_(c.prof, c.s, "band_begin", 1);
   pdl(k_band_begin, 1, 256, 0, c.s)(c.P.L, c.d_nbcnt, c.d_bbox, c.band_count);
 }
 void launch_tube(Ctx& c, LsBatch& b, bool list, bool fresh) {

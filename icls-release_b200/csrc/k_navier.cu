@@ -748,9 +748,9 @@ T* fp(double* q) { return reinterpret_cast<T*>(q); }
 void launch_ab2(Ctx& c) {
   // the segment maps hold unless a caller wrote the fields they describe
   const bool far = (c.P.f32 || c.ab2_ring) && !c.mat_dirty && !c.jmp_dirty[0] && !c.jmp_dirty[1];
-  Scope sc_(c.prof, c.s, "ab2", far ? 2 : 1);
   MomArgs a = mom_args(c);
   if (far) {
+    Scope sc_(c.prof, c.s, "ab2_near", 1);
     cudaMemsetAsync(c.ab2_near, 0, (size_t)seg_row(c.P) * ((c.P.jmax + kAb2Y - 1) / kAb2Y) * c.P.nCz, c.s);
     pdl(k_ab2_near, nblocks((seg_count(c.P) + 3) / 4), NT, 0, c.s)(c.P, c.seg_mat[c.mat_cur], c.seg_jmp[0],
                                                                   c.seg_jmp[1], c.ab2_near);
@@ -758,10 +758,13 @@ void launch_ab2(Ctx& c) {
     if (c.p_dirty) cudaMemsetAsync(&c.dsc->p_bad, 1, sizeof(int), c.s);  // unknown: nonzero
   }
   const int o = c.hist ^ 1;
-  if (c.P.f32) {
-    ab2_launch_f32(c, a, o);  // k_ab2_f32.cu
-  } else if (!ab2_tma_launch(c, a, o)) {  // k_ab2_tma.cu when chosen, else the ring
-    ab2_launch<double>(c, a, o);
+  {
+    Scope sc_(c.prof, c.s, "ab2", 1);
+    if (c.P.f32) {
+      ab2_launch_f32(c, a, o);  // k_ab2_f32.cu
+    } else if (!ab2_tma_launch(c, a, o)) {  // k_ab2_tma.cu when chosen, else the ring
+      ab2_launch<double>(c, a, o);
+    }
   }
   launch_ywalls_uvw(c, c.dudt, c.dvdt, c.dwdt);  // the y walls of bounduvw(dudt,dvdt,dwdt)
   c.hist = o;
@@ -811,35 +814,38 @@ void launch_correc(Ctx& c, int fused_bc) {
   }
 }
 void launch_bounduvw(Ctx& c, double* u, double* v, double* w) {
-  Scope sc_(c.prof, c.s, "bounduvw", 1);
   const int halo = halo_cells(c.P);
   const unsigned g = nblocks(halo + halo_plane_cells(c.P));
-  if (c.P.f32) pdl(k_bounduvw<float>, g, NT, 0, c.s)(c.P, fp<float>(u), fp<float>(v), fp<float>(w), halo);
-  else pdl(k_bounduvw<double>, g, NT, 0, c.s)(c.P, u, v, w, halo);
+  {
+    Scope sc_(c.prof, c.s, "bounduvw", 1);
+    if (c.P.f32) pdl(k_bounduvw<float>, g, NT, 0, c.s)(c.P, fp<float>(u), fp<float>(v), fp<float>(w), halo);
+    else pdl(k_bounduvw<double>, g, NT, 0, c.s)(c.P, u, v, w, halo);
+  }
   launch_ywalls_uvw(c, u, v, w);
 }
 inline dim3 grid_ik(const Params& p) { return dim3((unsigned)((p.imax + NT - 1) / NT), (unsigned)p.kmax, 1); }
 void launch_boundp(Ctx& c, double* pp, bool tfield) {
-  Scope sc_(c.prof, c.s, "boundp", 1);
   const int halo = halo_cells(c.P);
-  if (tfield && c.P.f32) {
-    pdl(k_boundp<float>, nblocks(halo), NT, 0, c.s)(c.P, fp<float>(pp), halo);
-    if (c.P.bcy != ICLS_BCY_PERIODIC) pdl(k_ywalls_p<float>, grid_ik(c.P), NT, 0, c.s)(c.P, fp<float>(pp));
-    return;
+  {
+    Scope sc_(c.prof, c.s, "boundp", 1);
+    if (tfield && c.P.f32) pdl(k_boundp<float>, nblocks(halo), NT, 0, c.s)(c.P, fp<float>(pp), halo);
+    else pdl(k_boundp<double>, nblocks(halo), NT, 0, c.s)(c.P, pp, halo);
   }
-  pdl(k_boundp<double>, nblocks(halo), NT, 0, c.s)(c.P, pp, halo);
-  launch_ywalls_p(c, pp);
+  launch_ywalls_p(c, pp, tfield);
 }
 void launch_ywalls_uvw(Ctx& c, double* u, double* v, double* w) {
   if (c.P.bcy == ICLS_BCY_PERIODIC) return;
+  Scope sc_(c.prof, c.s, "ywalls", 1);
   if (c.P.f32)
     pdl(k_ywalls_uvw<float>, grid_ik(c.P), NT, 0, c.s)(c.P, fp<float>(u), fp<float>(v), fp<float>(w), c.vin);
   else
     pdl(k_ywalls_uvw<double>, grid_ik(c.P), NT, 0, c.s)(c.P, u, v, w, c.vin);
 }
-void launch_ywalls_p(Ctx& c, double* pp) {
+void launch_ywalls_p(Ctx& c, double* pp, bool tfield) {
   if (c.P.bcy == ICLS_BCY_PERIODIC) return;
-  pdl(k_ywalls_p<double>, grid_ik(c.P), NT, 0, c.s)(c.P, pp);
+  Scope sc_(c.prof, c.s, "ywalls", 1);
+  if (tfield && c.P.f32) pdl(k_ywalls_p<float>, grid_ik(c.P), NT, 0, c.s)(c.P, fp<float>(pp));
+  else pdl(k_ywalls_p<double>, grid_ik(c.P), NT, 0, c.s)(c.P, pp);
 }
 void launch_gather_plane_x(Ctx& c, const double* d, bool f32, long long nx, long long ny, long long ioff, int n1,
                            int n2, double* dst) {
@@ -848,6 +854,7 @@ void launch_gather_plane_x(Ctx& c, const double* d, bool f32, long long nx, long
   else pdl(k_gather_plane_x<double>, g, NT, 0, c.s)(d, nx, nx * ny, ioff, n1, n2, dst);
 }
 void launch_nan_probe(Ctx& c) {
+  Scope sc_(c.prof, c.s, "nan_probe", 1);
   if (c.P.f32) pdl(k_nan_probe<float>, 1, 1, 0, c.s)(c.P, fp<float>(c.v), c.dsc);
   else pdl(k_nan_probe<double>, 1, 1, 0, c.s)(c.P, c.v, c.dsc);
 }

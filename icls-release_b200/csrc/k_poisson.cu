@@ -1207,6 +1207,7 @@ void solver2d_periodic(Ctx& c, int write_halos, const RhsArgs* ra);
 void launch_solver2d(Ctx& c, int write_halos) {
   if (c.P.bcy != ICLS_BCY_PERIODIC) {
     launch_solver2d_cos(c, write_halos);
+    if (write_halos) launch_ywalls_p(c, c.p, false);
     return;
   }
   solver2d_periodic(c, write_halos, nullptr);
@@ -1255,7 +1256,7 @@ void solver2d_periodic(Ctx& c, int write_halos, const RhsArgs* ra) {
 }
 
 // solver2d_cos (solver.f90:202-317): x FFT, VCOSQB in z, Thomas in y,
-// VCOSQF in z, inverse x FFT (+ boundp halos and the y-wall rows)
+// VCOSQF in z, inverse x FFT (+ boundp halos)
 void launch_solver2d_cos(Ctx& c, int write_halos) {
   Scope sc_(c.prof, c.s, "solver2d", 5);
   const Params& P = c.P;
@@ -1290,7 +1291,6 @@ void launch_solver2d_cos(Ctx& c, int write_halos) {
   launch_thomas<true>(c);
   cosq(1);
   if (!fft2_pass<false>(c, 1, write_halos)) pdl(k_fft_x, gx, FT, smx, c.s)(P, 1, CL, lx, c.twx, c.p, c.spec, write_halos);
-  if (write_halos) launch_ywalls_p(c, c.p);
 }
 
 }  // namespace icls
