@@ -93,7 +93,7 @@ def initial_state(wl):
 # cells, B band cells of all drops (one batched scope covers every drop),
 # S |phi| <= 2dz shell cells of all drops.
 ALG_VALUES = {
-    "ab2": (14, 0, "N"),             # u,v,w,duold x3,pnew,pold -> dudt x3,duold x3 (miu,rho_uvw,p_xyz,p_xyz_old near drops only)
+    "ab2": (12, 0, "N"),             # u,v,w,duold x3 -> dudt x3,duold x3 (miu,rho_uvw,p_xyz,p_xyz_old near drops only; pnew,pold: alg_bytes_per_launch)
     "correc": (9, 1, "N"),           # dudt x3 | p -> u,v,w, ucc,vcc,wcc (p_xyz near drops only)
     "fillps": (3, 2, "N"),           # dudt x3 | pjump -> p
     "solver2d": (3, 2, "N"),         # dudt x3 | p_jump -> p: fillps folded into the first pass (the transposes and sweeps between are not compulsory)
@@ -111,11 +111,12 @@ ALG_VALUES = {
 # (layer 1 takes its 32 inputs as hi + lo pairs, K = 64)
 MLP_FLOPS_PER_CELL = 2 * (128 * 64 + 128 * 128 + 64 * 128)
 
-# DRAM bytes (read + write) of one launch of the dominant kernel at 256^3,
-# (kernel, FP32 form) -> bytes: ncu's dram__bytes_read.sum + write.sum of the
-# launch in a capture of the static_drop_256 workload (the predictor's grid
-# and fields do not depend on the drops)
-TRAFFIC = {("ab2", False): 1.095140e9 + 0.771508e9, ("ab2", True): 0.555361e9 + 0.362161e9}
+# DRAM bytes (read + write) of one launch of the dominant kernel, (workload,
+# kernel, FP32 form) -> bytes: ncu's dram__bytes_read.sum + write.sum of the
+# launch in a capture of that workload (how many rows of the predictor read
+# the materials and jumps depends on the drops)
+TRAFFIC = {("multi_drop_256_48", "ab2", False): 1.264e9 + 0.771e9,
+           ("multi_drop_256_48", "ab2", True): 0.650e9 + 0.365e9}
 
 
 def alg_bytes_per_launch(name, cfg, stats, f32=False):
@@ -124,6 +125,10 @@ def alg_bytes_per_launch(name, cfg, stats, f32=False):
     if e is None:
         return None
     bulk, f64, unit = e
+    if name == "ab2" and cfg.rho1 > cfg.rho2:
+        # the carrier is the heavier phase: the pressure-split factor
+        # 1/rho - 1/min(rho1, rho2) is nonzero far from the drops too
+        bulk += 2
     n = {"N": cfg.itot * cfg.jtot * cfg.ktot, "B": stats.get("band_total", 0.0),
          "S": stats.get("shell_total", 0.0)}[unit]
     return (bulk * (4.0 if f32 else 8.0) + f64 * 8.0) * n
@@ -355,11 +360,11 @@ def kernel_table(s, args, cfg, stats, istep, f32, mlp_cells=None):
     if name == "mlp_curvature" and mlp_cells:
         tf = MLP_FLOPS_PER_CELL * mlp_cells / (per_launch_ms / 1000.0) / 1e12
         roofline = {"bound": "tensor", "kernel": name, "achieved": tf, "peak": tpeak, "unit": "TFLOP/s",
-                    "frac": tf / tpeak, "traffic": TRAFFIC.get((name, f32)), "flops": MLP_FLOPS_PER_CELL * mlp_cells,
+                    "frac": tf / tpeak, "traffic": TRAFFIC.get((args.workload, name, f32)), "flops": MLP_FLOPS_PER_CELL * mlp_cells,
                     "share": ent["ms"] / tot, "launch_ms": per_launch_ms, "peak_source": tsrc}
     else:
         roofline = {"bound": "hbm", "kernel": name, "achieved": achieved, "peak": peak, "unit": "GB/s",
-                    "frac": (achieved / peak) if achieved else None, "traffic": TRAFFIC.get((name, f32)),
+                    "frac": (achieved / peak) if achieved else None, "traffic": TRAFFIC.get((args.workload, name, f32)),
                     "alg_bytes": alg, "share": ent["ms"] / tot, "launch_ms": per_launch_ms,
                     "peak_source": "measured (burst copy)" if "hbm_gbs" in peaks else "fallback"}
     kernels = {}

@@ -53,3 +53,20 @@ def test_y_walls_are_scopes_of_their_own():
     for name in ("ab2", "bounduvw", "nan_probe"):
         assert table[name]["launches"] == table[name]["timed"] == 1, name
     s.close()
+
+
+def test_predictor_bytes_follow_the_pressures_it_reads():
+    """Far from the drops the predictor reads the two pressures only where the
+    carrier is the heavier phase (1/rho1 - 1/min(rho1, rho2) is zero
+    otherwise): 12 values per cell, or 14."""
+    from icls_gpu import make_config
+    n = 8 * 8 * 8
+    for rho2, values in ((10.0, 12), (1.0, 12), (0.1, 14)):
+        cfg = make_config(itot=8, jtot=8, ktot=8, rho1=1.0, rho2=rho2)
+        assert bench.alg_bytes_per_launch("ab2", cfg, {}) == 8 * values * n
+        assert bench.alg_bytes_per_launch("ab2", cfg, {}, True) == 4 * values * n
+
+
+def test_captured_traffic_stands_for_its_own_workload():
+    for workload, kernel, _ in bench.TRAFFIC:
+        assert bench.make_workload(workload).name == workload and kernel in bench.ALG_VALUES
