@@ -3,9 +3,9 @@
 // A batched launch carries up to kTasks drops (LsTask, ctx.h) in one
 // __grid_constant__ kernel parameter.  Its 1-D grid is the concatenation of
 // the drops' blocks: block b belongs to the task whose [start, next start)
-// holds b, and within the task it is one TBX x TBY column tile times one
-// chunk of z rows.  Each thread owns one column of the tile and walks the
-// rows of its chunk upwards.
+// holds b, and within the task it is one tile of 256 columns times one chunk
+// of z rows.  Each thread owns one column of the tile and walks the rows of
+// its chunk upwards.
 //
 // Periodic images: a thread that writes interior column (i,j) also writes
 // every halo cell that is a periodic copy of it (three layers in shape L,
@@ -39,26 +39,19 @@ struct Col {
   bool ok;     // inside the written spans
   bool cxy;    // a computed column
 };
-// Flat tasks: block bx of a chunk takes the region's written columns
-// 256 bx .. 256 bx + 255 in row-major order (x fastest), so a region of any
-// width fills whole warps; otherwise a block is a TBX x TBY column tile.
+// Block bx of a chunk takes the region's written columns 256 bx .. 256 bx +
+// 255 in row-major order (x fastest), so a region of any width fills whole
+// warps (tiles of 32 x 8 columns left a quarter of the lanes idle in a box 47
+// columns wide).
 __device__ __forceinline__ Col col_of(const Params& p, const LsTask& t, int local) {
   Col c;
-  const int bx = local % t.tx;
-  const int r = local / t.tx;
-  const int by = r % t.ty;
-  const int ch = r / t.ty;
-  c.tile = bx + t.tx * by;
+  const int ch = local / t.tx;
+  c.tile = local - ch * t.tx;
   c.ch = ch;
-  if (t.flat) {
-    const int col = bx * (TBX * TBY) + (int)threadIdx.x + TBX * (int)threadIdx.y;
-    c.Y = col / t.r.xn;
-    c.X = col - c.Y * t.r.xn;
-  } else {
-    c.X = bx * TBX + (int)threadIdx.x;
-    c.Y = by * TBY + (int)threadIdx.y;
-  }
-  c.ok = c.X < t.r.xn && c.Y < t.r.yn;
+  const int col = c.tile * (TBX * TBY) + (int)threadIdx.x + TBX * (int)threadIdx.y;
+  c.Y = col / t.r.xn;
+  c.X = col - c.Y * t.r.xn;
+  c.ok = c.Y < t.r.yn;
   c.i = t.r.xa + c.X;
   if (c.i > p.imax) c.i -= p.imax;
   c.j = t.r.ya + c.Y;

@@ -234,8 +234,8 @@ int allocate(Ctx& c) {
   if (cudaMalloc(&c.band_list, (size_t)c.band_cap * 8) != cudaSuccess) return ICLS_E_NOMEM;
   if (cudaMalloc((void**)&c.band_count, sizeof(int)) != cudaSuccess) return ICLS_E_NOMEM;
   AL(c.drs, (size_t)P.L);
-  c.red_cap = ((P.imax + TBX - 1) / TBX) * ((P.jmax + TBY - 1) / TBY);
-  c.hcap = std::max(c.red_cap * ((P.kmax + 2 + kHeavRows - 1) / kHeavRows), 3 * kHeavBlocks);
+  const int tiles = (P.imax * P.jmax + TBX * TBY - 1) / (TBX * TBY);  // column tiles of a whole plane
+  c.hcap = std::max(tiles * ((P.kmax + 2 + kHeavRows - 1) / kHeavRows), 3 * kHeavBlocks);
   // per-(tile, chunk) exact sums of H (4 words each) for every drop, then
   // the mass correction's area sums
   AL(c.hpart, (size_t)5 * P.L * c.hcap);
@@ -585,7 +585,7 @@ void update_materials(Ctx& c, bool extents = false) {
     size_tiles(c.P, b, kHeavRows, 4, kHeavBlocks);
     for (int q = 0; q < b.n; ++q) {
       b.t[q].phi0 = c.lv[b.t[q].l];
-      ntiles[b.t[q].l] = b.t[q].tx * b.t[q].ty * b.t[q].nch;
+      ntiles[b.t[q].l] = b.t[q].tx * b.t[q].nch;
     }
     launch_heaviside(c, b);
   }

@@ -23,18 +23,18 @@ constexpr int kRedThreads = 256;
 constexpr int kMaxDropsParam = 256;  // drops whose far-field counts travel as a kernel parameter
 
 constexpr int kTasks = 64;          // drops per batched launch (tasks travel as a kernel parameter)
-constexpr int TBX = 32, TBY = 8;    // column tile of a batched launch
+constexpr int TBX = 32, TBY = 8;    // threads of a batched launch's block
 
 // One drop's share of a batched launch.  A block of TBX x TBY threads
-// sweeps one column tile of the region over one chunk of z rows, each
+// sweeps one tile of the region's columns over one chunk of z rows, each
 // thread walking its column upwards: chunk m covers rows z0 + m*kc ..
 // z0 + (m+1)*kc - 1, the last chunk runs to z1 (chunk 0 has `head` rows more).
 // The rows a wall row extrapolates from lie in its chunk: set_tiles gives every
 // chunk at least kc >= 5 rows, size_tiles lengthens those at a wall.
 struct LsTask {
   Region r;
-  int tx, ty, nch, kc, head;
-  int l, flat;           // flat: a block takes 256 consecutive columns (else TBX x TBY tiles)
+  int tx, nch, kc, head;  // column tiles, chunks
+  int l;                  // the drop
   double bg, bgg;        // far-field values of the apron: rows 0..k1 / ghost rows
   const double* phi0;    // RK base (read at the thread's own cell only)
   const double* phis;    // stage input (stencil reads)
@@ -205,8 +205,7 @@ struct Ctx {
   double* stage = nullptr;              // precision form: FP64 staging of one field (upload/download)
   double* hpart = nullptr;              // per (tile, chunk): exact sums of H (XSum), hcap per drop, then area sums
   InflateState* dinf = nullptr;         // per drop
-  int red_cap = 0;                      // column tiles of a whole x-y plane
-  int hcap = 0;                         // Heaviside partials per drop: red_cap x the z chunks of shape C
+  int hcap = 0;                         // exact sums of H per drop: column tiles x z chunks of shape C
   // pinned host mirrors
   double* h_vol = nullptr;
   DevScalars* h_sc = nullptr;
@@ -253,7 +252,7 @@ void set_pseudo_inverse(const double* P270, cudaStream_t s);
 Region full_region(const Params& P);
 bool region_full(const Params& P, const Region& r);
 Region c_region(const Params& P, const Region& r, int apron);
-void set_tiles(LsBatch& b, int kc, bool flat = true);
+void set_tiles(LsBatch& b, int kc);
 void size_tiles(const Params& p, LsBatch& b, int kc, int kmin, int blocks);
 // tube_construction; list: the band cells also into c.band_list (sets the batch's own tiles)
 void launch_band_begin(Ctx& c);

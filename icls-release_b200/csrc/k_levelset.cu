@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(NT, 4) k_heaviside(Params p, const __grid_cons
   xs_add_count(s, ones);
   const XSum bs = block_xsum<NT>(s);
   // one partial per (column tile, z chunk) of the task
-  if (flat_tid() == 0) part[(long long)t.l * cap + c.tile + (long long)t.tx * t.ty * c.ch] = bs;
+  if (flat_tid() == 0) part[(long long)t.l * cap + c.tile + (long long)t.tx * c.ch] = bs;
 }
 
 // volume(l) and rho_avr from the per-(tile, chunk) sums (misc.f90:139-173) of
@@ -1281,7 +1281,7 @@ __global__ void __launch_bounds__(NT) k_inflate_sums(Params p, const __grid_cons
   const double ba = block_sum<double, NT>(sa);
   const XSum bh = block_xsum<NT>(sh);
   if (flat_tid() == 0) {
-    const long long at = (long long)t.l * cap + c.tile + (long long)t.tx * t.ty * c.ch;
+    const long long at = (long long)t.l * cap + c.tile + (long long)t.tx * c.ch;
     part_area[at] = ba;
     part_heav[at] = bh;
   }
@@ -1293,7 +1293,7 @@ constexpr int kFinalThreads = 256;
 __device__ __forceinline__ XSum task_heav(const LsTask& t, const XSum* __restrict__ part, int cap) {
   XSum hs;
   xs_zero(hs);
-  const int n = t.tx * t.ty * t.nch;
+  const int n = t.tx * t.nch;
   for (int b = threadIdx.x; b < n; b += kFinalThreads) xs_merge(hs, part[(long long)t.l * cap + b]);
   hs = block_xsum<kFinalThreads>(hs);
   xs_add_count(hs, (long long)t.far);
@@ -1305,7 +1305,7 @@ __global__ void __launch_bounds__(kFinalThreads)
                     const double* __restrict__ vol0, double* __restrict__ maxchk, InflateState* __restrict__ inf) {
   pdl_wait();
   const LsTask& t = B.t[blockIdx.x];
-  const int l = t.l, n = t.tx * t.ty * t.nch;
+  const int l = t.l, n = t.tx * t.nch;
   double sa = 0.;
   for (int b = threadIdx.x; b < n; b += kFinalThreads) sa += part_area[(long long)l * cap + b];
   sa = block_sum<double, kFinalThreads>(sa);
@@ -1386,7 +1386,7 @@ __global__ void __launch_bounds__(NT) k_region_heav(Params p, const __grid_const
       if (computed(c, t.r, k)) heav_add(sh, ones, heav_trig(p, phi[idxL(p, c.i, c.j, k)], s1));
   xs_add_count(sh, ones);
   const XSum bh = block_xsum<NT>(sh);
-  if (flat_tid() == 0) part[(long long)t.l * cap + c.tile + (long long)t.tx * t.ty * c.ch] = bh;
+  if (flat_tid() == 0) part[(long long)t.l * cap + c.tile + (long long)t.tx * c.ch] = bh;
 }
 
 // g = (V0 - V)/(V1 - V) of each task's drop, V1 from the partials and the far-field count
@@ -1546,21 +1546,13 @@ Region c_region(const Params& P, const Region& r, int ap) {
   return q;
 }
 
-// tiles, z chunks (kc rows each, the last one longer; kc <= 0: one chunk)
-// and block offsets of a batch; flat tiles of 256 consecutive columns
-// (col_of), or TBX x TBY tiles for the kernels that stage a 2-D tile
-void set_tiles(LsBatch& b, int kc, bool flat) {
+// tiles of 256 consecutive columns (col_of), z chunks (kc rows each, the last
+// one longer; kc <= 0: one chunk) and block offsets of a batch
+void set_tiles(LsBatch& b, int kc) {
   int s = 0;
   for (int q = 0; q < b.n; ++q) {
     LsTask& t = b.t[q];
-    t.flat = flat ? 1 : 0;
-    if (flat) {
-      t.tx = (t.r.xn * t.r.yn + TBX * TBY - 1) / (TBX * TBY);
-      t.ty = 1;
-    } else {
-      t.tx = (t.r.xn + TBX - 1) / TBX;
-      t.ty = (t.r.yn + TBY - 1) / TBY;
-    }
+    t.tx = (t.r.xn * t.r.yn + TBX * TBY - 1) / (TBX * TBY);
     const int nz = t.r.z1 - t.r.z0 + 1;
     t.head = 0;
     if (kc <= 0 || kc >= nz) {
@@ -1571,12 +1563,12 @@ void set_tiles(LsBatch& b, int kc, bool flat) {
       t.kc = kc;
     }
     b.start[q] = s;
-    s += t.tx * t.ty * t.nch;
+    s += t.tx * t.nch;
   }
   b.start[b.n] = s;
 }
 
-// Flat tiles with chunks of kc rows, halved down to kmin while the batch has
+// Tiles with chunks of kc rows, halved down to kmin while the batch has
 // fewer than `blocks` blocks: few drops leave SMs idle, and the cells of a
 // chunk are worked off one after the other.  The chunks at a wall are
 // lengthened to the five rows -2..2 or k1-2..k1+2.  Lines and minima are set
@@ -1593,9 +1585,7 @@ void size_tiles(const Params& p, LsBatch& b, int kc, int kmin, int blocks) {
     int s = 0;
     for (int q = 0; q < b.n; ++q) {
       LsTask& t = b.t[q];
-      t.flat = 1;
       t.tx = (t.r.xn * t.r.yn + TBX * TBY - 1) / (TBX * TBY);
-      t.ty = 1;
       const int nz = t.r.z1 - t.r.z0 + 1, more = std::max(0, 5 - kc);
       t.kc = kc;
       t.head = t.r.z0 <= 0 ? more : 0;

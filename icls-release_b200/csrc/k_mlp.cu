@@ -99,9 +99,6 @@ __device__ __forceinline__ float dsilu(float z) {
   const float s = 1.f / (1.f + __expf(-z));
   return s * (1.f + z * (1.f - s));
 }
-__device__ __forceinline__ void put_bf16(unsigned char* base, uint32_t off, float v) {
-  *reinterpret_cast<__nv_bfloat16*>(base + off) = __float2bfloat16(v);
-}
 
 // shared-memory plan of one tile (bytes)
 constexpr int SB_B = 0;                       // weight operand, up to 128 x 128
