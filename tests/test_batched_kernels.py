@@ -150,3 +150,52 @@ def test_separate_projection_calls_equal_whole_sweeps(n, precision):
     for name in ("p", "u", "v", "w"):
         assert np.array_equal(near.download(name), told.download(name)), name
     assert np.any(near.download("p_x"))
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32])
+@pytest.mark.parametrize("rho1,rho2,miu1,iFr", [(1.5, 0.3, 0.7, 0.0), (0.75, 2.5, 1.3, 0.98), (2.0, 1.0, 1.0, 0.98)])
+def test_far_rows_of_the_predictor_equal_general_ones(rho1, rho2, miu1, iFr, precision):
+    """The predictor's far rows against a context told (by an upload of the
+    same values) that it knows nothing of the fields: a carrier that is the
+    heavier phase, so that far rows read the pressures, densities that are and
+    are not powers of two, buoyancy along all three axes.  FP64: the same
+    bits.  FP32, whose rows may contract and divide differently: du/dt is u
+    plus a step dt R of some hundredths of it, so a few ulps of R are below an
+    ulp of u, and the last sums round to within four."""
+    cfg = make_config(itot=64, jtot=48, ktot=50, ly=0.75, lz=50 / 64, timestep=1e-3, rho1=rho1, rho2=rho2, miu1=miu1,
+                      miu2=0.4, Re=100.0, We=0.5, iFr=iFr, g_unit=(0.3, -0.2, -1.0), v_wall_lower=-0.5,
+                      v_wall_upper=0.5, precision=precision)
+    ls = init_drops(cfg, [(0.15, 0.15, 0.4)], [0.1], all_images=True)
+    far, told = run_steps(cfg, ls, 2), run_steps(cfg, ls, 2)
+    told.upload("p_x", told.download("p_x"))
+    for s in (far, told):
+        s.ab2()
+    for name in ("dudt", "dvdt", "dwdt", "duold", "dvold", "dwold"):
+        a, b = far.download(name), told.download(name)
+        if precision == FP64:
+            assert np.array_equal(a, b), name
+        elif name.endswith("dt"):
+            assert np.max(np.abs(a - b)) <= 4 * 2.0 ** -23 * np.max(np.abs(b)), name
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32])
+def test_far_rows_read_a_pressure_that_is_not_finite(precision):
+    """Far rows skip the pressures where their factor is zero; an infinite one
+    far from the drop still reaches the cells whose gradient reads it."""
+    cfg = make_config(itot=64, jtot=48, ktot=50, ly=0.75, lz=50 / 64, timestep=1e-3, rho2=10.0, miu2=10.0, Re=100.0,
+                      We=0.5, v_wall_lower=-0.5, v_wall_upper=0.5, precision=precision)
+    ls = init_drops(cfg, [(0.15, 0.15, 0.4)], [0.1], all_images=True)
+    far, told = run_steps(cfg, ls, 2), run_steps(cfg, ls, 2)
+    for s in (far, told):
+        p = s.download("p")
+        p[56, 40, 9] = np.inf
+        s.upload("p", p)
+        s.pressure_update(3, 0)
+    told.upload("p_x", told.download("p_x"))
+    for s in (far, told):
+        s.ab2()
+    for name in ("dudt", "dvdt", "dwdt"):
+        a, b = far.download(name), told.download(name)
+        assert np.array_equal(np.isnan(a), np.isnan(b)) and np.isnan(b).any(), name
+        if precision == FP64:
+            assert np.array_equal(a, b, equal_nan=True), name
