@@ -208,16 +208,19 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // runs the same expressions with one viscosity and one density: the same
 // bits.  Where the carrier is the lighter phase the pressure-split factor
 // 1/rho1 - 1/rho0 is exactly zero too, and while every pressure is finite
-// (p_bad) its product is: the two pressures are not read either.  Nine tenths
-// of the rows are far at 256^3 with 48 drops.  FAR false: the fields were
-// written by a caller, every row is general.
+// (p_bad) its product is: the two pressures are not read either.  Three
+// quarters of the rows are far at 256^3 with 48 drops.  FAR false: the fields
+// were written by a caller, every row is general.
 // The planes arrive one row ahead of their use, and so do the AB2 history
 // values; a near row's other operands are read at the row.  (Waiting for a
 // row's planes right after issuing them, the long-scoreboard and barrier
 // stalls were a third of the FP64 form's issue slots.)
 //
-// 256^3 with 48 drops: FP64 0.843 -> 0.626 ms, FP32 0.489 -> 0.357 ms; every row
-// general: FP64 0.842 -> 0.762 ms, 384 x 192 x 150 FP32 0.360 -> 0.283 ms.  FP64
+// 256^3 with 48 drops, k_ab2_near (0.013 ms) included: FP64 0.843 -> 0.626 ms,
+// FP32 0.489 -> 0.357 ms; every row general: 256^3 FP64 0.865 -> 0.788 ms, 384 x
+// 192 x 150 FP32 0.305 -> 0.283 ms.  The general FP32 row issues in 76 % of the
+// cycles and waits two more per issue on global loads, the nine operands that
+// are read at the row.  FP64
 // takes two blocks per SM at 128 registers (three at 80: 0.660 and 0.808 ms),
 // FP32 four.  Two cells per thread (adjacent in y, sharing their stencil) were
 // slower in both forms (FP64 0.743, FP32 0.396): the registers they take cost

@@ -258,9 +258,9 @@ int allocate(Ctx& c) {
   c.use_boxes = (P.L <= kMaxDropsParam) && !(fs && fs[0] == '1');
   // Alternative kernels of the same arithmetic (bit-identical fields), kept
   // for comparison:
-  // ICLS_AB2=tma: the FP64 predictor on the TMA-fed kernel in place of the
-  // cp.async-ring one (the ring kernel measured faster at 256^3, 1.37 vs
-  // 1.68 ms);
+  // ICLS_AB2=tma: the FP64 predictor on the TMA-fed kernel, which has no far
+  // rows, in place of the cp.async-ring one (256^3 with 48 drops 1.505 against
+  // 0.613 ms);
   // ICLS_ADV=column: the advection stages after tube_construction as
   // sweeps of each drop's columns in place of the list of its band cells;
   // ICLS_CORREC=shapec: the fused correction one thread per shape-C cell

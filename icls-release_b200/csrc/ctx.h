@@ -20,7 +20,7 @@ constexpr int kRedBlocks = 1184;   // 8 x 148 SMs: fixed grid of the reduction k
 size_t cosq_coefs(int K);  // doubles in a cosine table (k_poisson.cu)
 constexpr int kCosqMaxN = 768;     // longest z line of solver2d_cos (one shared-memory tile)
 constexpr int kRedThreads = 256;
-constexpr int kMaxDropsParam = 256;  // drops whose far-field counts travel as a kernel parameter
+constexpr int kMaxDropsParam = 256;  // drops whose counts travel as a kernel parameter of k_volumes
 
 constexpr int kTasks = 64;          // drops per batched launch (tasks travel as a kernel parameter)
 constexpr int TBX = 32, TBY = 8;    // threads of a batched launch's block

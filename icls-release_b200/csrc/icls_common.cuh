@@ -358,6 +358,10 @@ struct DevScalars {
 // projection 148 -> 133, bubble step 790 -> 736, 48 drops at 256^3 2703 ->
 // 2664 us).  The network's kernels keep plain launches: with theirs
 // overlapped the step with the learned curvature took 2125 us instead of 1987.
+// The price: blocks that only wait hold slots of their SMs, which kernels of
+// other streams then lack.  Where passes of two solvers share the GPU, the
+// 96 x 192 x 100 level-set sweep with reinitialisation takes 811 us instead of
+// 780.
 __device__ __forceinline__ void pdl_wait() {
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();

@@ -927,11 +927,10 @@ __global__ void __launch_bounds__(kRedThreads) k_disp_final(const double* __rest
 }
 
 // jiemian = min(jiemian, H_l) over the tasks' computed cells (shape-C
-// regions) and per-tile sums of H_l over their interior cells
-// (misc.f90:110-141), the sums in FP64.  jiemian starts at 1, the
-// far-field value of H, so only cells with H < 1 are touched; min is
-// order-free, so drops may share cells.  One chunk per tile:
-// part[l*cap + tile] is deterministic.
+// regions) and exact sums of H_l over their interior cells (misc.f90:110-141),
+// one per column tile and z chunk: part[l*cap + tile + tiles*chunk].  jiemian
+// starts at 1, the far-field value of H, so only cells with H < 1 are touched;
+// min is order-free, so drops may share cells.
 // For v >= +0 the signed-integer order of the bit patterns is the numeric
 // order against every non-negative value, and every negative value (sign
 // bit set) compares below it, as it does numerically: one atomicMin that

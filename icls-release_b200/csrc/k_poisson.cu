@@ -3,15 +3,16 @@
 // are held to a tolerance against the oracle, not to its rounding).
 //
 // Forward: real FFT along x of every (j,k) line, then along y of every
-// (i,k) column of those coefficients, with VFFTPACK's contract (fft.f:
-// 1123-1142): half-complex layout r0, Re1, Im1, ..., r_{N/2} and sqrt(1/N)
-// scaling.  Thomas elimination in z per (i,j) with diagonal b(k)+xyrt(i,j)
-// (solver.f90:119-160), the exactly-zero last pivot of mode (0,0) giving
-// p=0.  Inverse: y then x, the exact inverse of the forward transform
-// (fft.f:403-452).  The 2decomp transposes of the reference
+// (i,k) column of those coefficients, with VFFTPACK's values and sqrt(1/N)
+// scaling (fft.f:1123-1142), stored as (re, im) pairs in place of its r0, Re1,
+// Im1, ..., r_{N/2} (wave_of).  Thomas elimination in z per (i,j) with diagonal
+// b(k)+xyrt(i,j) (solver.f90:119-160), the exactly-zero last pivot of mode
+// (0,0) giving p=0.  Inverse: y then x, the exact inverse of the forward
+// transform (fft.f:403-452).  The 2decomp transposes of the reference
 // (transpose_*.f90) are replaced by the access pattern of each kernel: the
-// x pass streams contiguous lines, the y pass loads 16-wide column tiles,
-// the z pass walks k with one thread per (i,j).  In the fused time step the
+// x pass streams contiguous lines, the y pass moves column pairs of a plane,
+// the z pass holds 16 rows of a line per thread (lines of more than 512 rows
+// are walked by one thread each).  In the fused time step the
 // forward x pass forms fillps' right-hand side itself from the predicted
 // velocities (and p_jump), so p is not written and read back in between.
 //
