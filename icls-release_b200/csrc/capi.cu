@@ -882,11 +882,14 @@ int measure_volumes_now(Ctx& c, const std::vector<int>& drops) {
 // ls_mass_correction (levelset.f90:377-400) of the given drops.  The
 // reference tests the volume of the last update_materials; the gain-one
 // correction tests the drop's volume as it is now (after this step's
-// advection and reinitialisation, measured by measure_volumes_now into
-// h_volnow)
+// advection and reinitialisation), which it measures first
 int ls_mass_correction(Ctx& c, int istep, const std::vector<int>& drops) {
   for (int l : drops) c.inflated[l] = 0;
   if (istep % c.cfg.inflate_step != 0) return ICLS_OK;
+  if (c.cfg.mass_gain_one) {
+    const int rc = measure_volumes_now(c, drops);
+    if (rc) return rc;
+  }
   std::vector<int> sel;
   for (int l : drops) {
     double vol;
@@ -1094,10 +1097,6 @@ int ls_main(Ctx& c, int istep) {
     // removes the volume change of the reinitialisation in the same step
     const bool correct_last = c.cfg.mass_gain_one != 0;
     if (reinit_now && correct_last) reinit_batches(c, bs);
-    if (c.cfg.mass_correction && correct_last && istep % c.cfg.inflate_step == 0) {
-      rc = measure_volumes_now(c, drops);
-      if (rc) return rc;
-    }
     if (c.cfg.mass_correction) {
       rc = ls_mass_correction(c, istep, drops);
       if (rc) return rc;

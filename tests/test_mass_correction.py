@@ -171,3 +171,31 @@ def test_gpu_gain_one_with_reinitialisation_matches_oracle():
         assert rel_l2(g.download(name), o.download(name)) <= 1e-10, name
     vg, v0 = g.volumes()
     assert np.max(np.abs(vg / v0 - 1)) <= 1e-8
+
+
+@pytest.mark.gpu
+def test_gpu_gain_one_called_alone_measures_the_volume():
+    """ls_mass_correction called by itself tests the drop's volume as it is,
+    like the oracle's: not that of the last step that corrected (the level
+    set has been replaced since), and in a new context not an unset one."""
+    from icls_gpu import Solver
+    cfg = make_config(itot=32, jtot=32, ktot=32, lmax=1, timestep=1e-5, inflate_step=2, reinit_step=100000,
+                      mass_gain_one=1, mass_threshold=1e-6)
+    whole, small = (init_drops(cfg, [(0.5, 0.5, 0.5)], [R]) for R in (0.25, 0.249))
+    for steps in (0, 2):
+        made = [Solver(cfg), Oracle(cfg)]
+        for s in made:
+            s.setup(whole, *initial_velocity(cfg, 0.0))
+            for istep in range(1, steps + 1):
+                s.step(istep, 0)
+            s.tube_construction(1)
+            s.ls_mass_correction(2, 1)
+        assert [s.scalars()["last_inflated"] for s in made] == [0, 0], steps
+        for s in made:
+            s.upload("lvset", small[..., 0], 1)
+            s.tube_construction(1)
+            s.ls_mass_correction(2, 1)
+            s.update_materials()
+        assert [s.scalars()["last_inflated"] for s in made] == [1, 1], steps
+        (a, v0), (b, _) = (s.volumes() for s in made)
+        assert abs(a[0] - b[0]) <= 1e-12 and abs(a[0] - v0[0]) < 1e-3 * v0[0]  # downstream of cosines, as the others
