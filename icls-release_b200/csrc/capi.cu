@@ -168,17 +168,18 @@ void fill_params(Ctx& c) {
 
 void init_matrix(Ctx& c) { pseudo_inverse(c.P.dx, c.P.dy, c.P.dz, c.P10x27); }
 
+// zeroed on the context's stream: that stream does not wait for the legacy one
 template <typename T>
-int dalloc(T** p, size_t n) {
+int dalloc(T** p, size_t n, cudaStream_t s) {
   if (cudaMalloc((void**)p, n * sizeof(T) + 16) != cudaSuccess) return ICLS_E_NOMEM;
-  if (cudaMemset(*p, 0, n * sizeof(T) + 16) != cudaSuccess) return ICLS_E_CUDA;
+  if (cudaMemsetAsync(*p, 0, n * sizeof(T) + 16, s) != cudaSuccess) return ICLS_E_CUDA;
   return ICLS_OK;
 }
 
-#define AL(ptr, n)                  \
-  do {                              \
-    int rc_ = dalloc(&(ptr), (n));  \
-    if (rc_) return rc_;            \
+#define AL(ptr, n)                       \
+  do {                                   \
+    int rc_ = dalloc(&(ptr), (n), c.s);  \
+    if (rc_) return rc_;                 \
   } while (0)
 
 // doubles that hold n elements of the form's field type

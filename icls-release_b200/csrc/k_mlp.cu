@@ -988,6 +988,7 @@ int mlp_constants() {
   for (int q = 0; q < 270; ++q) puf[q] = (float)pu[q];
   if (cudaMemcpyToSymbol(cPu, pu, sizeof(pu)) != cudaSuccess) return 1;
   if (cudaMemcpyToSymbol(cPuf, puf, sizeof(puf)) != cudaSuccess) return 1;
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) return 1;  // the copies may still be under way
   set |= 1u << (dev & 31);
   return 0;
 }
@@ -999,7 +1000,7 @@ int mlp_buffers(Ctx& c, int cap) {
   if (cudaMalloc(&c.mlp_rec, (size_t)cap * sizeof(MlpCell)) != cudaSuccess) return ICLS_E_NOMEM;
   if (cudaMalloc(&c.mlp_count, sizeof(int)) != cudaSuccess) return ICLS_E_NOMEM;
   if (cudaMalloc(&c.mlp_stats, 2 * sizeof(unsigned long long)) != cudaSuccess) return ICLS_E_NOMEM;
-  cudaMemset(c.mlp_stats, 0, 2 * sizeof(unsigned long long));
+  cudaMemsetAsync(c.mlp_stats, 0, 2 * sizeof(unsigned long long), c.s);
   c.mlp_cap = cap;
   return cudaFuncSetAttribute(k_mlp_curv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SB_INFER) ==
                      cudaSuccess &&
@@ -1188,7 +1189,9 @@ extern "C" int icls_mlp_params(icls_mlp* m, float* host, int get) {
     if (cudaMemcpy(host, m->theta, sizeof(float) * kParams, cudaMemcpyDeviceToHost) != cudaSuccess) return ICLS_E_CUDA;
     return ICLS_OK;
   }
-  if (cudaMemcpy(m->theta, host, sizeof(float) * kParams, cudaMemcpyHostToDevice) != cudaSuccess) return ICLS_E_CUDA;
+  // on the network's stream, ahead of the kernel that reads them
+  if (cudaMemcpyAsync(m->theta, host, sizeof(float) * kParams, cudaMemcpyHostToDevice, m->s) != cudaSuccess)
+    return ICLS_E_CUDA;
   refresh_copies(m);
   return sync_err(m);
 }

@@ -42,3 +42,16 @@ def test_overlapped_kernels_wait_first(name):
         assert launched
     for k in launched:
         assert waits[k], k
+
+
+@pytest.mark.parametrize("name", list(TEXT))
+def test_device_memory_is_set_on_the_streams_that_use_it(name):
+    """The contexts' and networks' streams do not wait for the legacy stream,
+    and a memset or a copy from pageable memory there may still be under way
+    when it returns: no memset goes there, and no copy to the device but the
+    constants', which are waited for."""
+    s = TEXT[name]
+    assert not re.search(r"\bcudaMemset\(", s)
+    assert not re.search(r"\bcudaMemcpy\([^;]*cudaMemcpyHostToDevice", s)
+    for m in re.finditer(r"\bcudaMemcpyToSymbol\(", s):
+        assert "cudaStreamSynchronize(nullptr)" in s[m.end():m.end() + 400]
